@@ -1,4 +1,5 @@
-// Decode GEMV over the packed device layout, M = 1..16 activation rows.
+// Decode GEMV over the packed device layout, M = 1..16 activation rows, on the CUDA cores; b200_gemv dispatches between
+// this kernel and gemv_mma.cu.
 //
 // One warp streams R output rows: every lane issues one 16-byte load per row
 // and block (32 lanes x 16 B = 512 contiguous bytes of each row), dequantises
@@ -16,6 +17,9 @@
 #include "common.cuh"
 
 namespace b200 {
+
+bool gemv_mma_takes(const b200_weight *w, const b200_gemv_args *a);
+int gemv_mma_run(const b200_weight *w, const b200_gemv_args *a, cudaStream_t st);
 
 struct GemvP {
   const void *x;
@@ -582,6 +586,11 @@ int b200::gemv_run(const b200_weight *w, const b200_gemv_args *a, const TpPush *
     return fail(B200_EINVAL, "gemv: silu_pairs excludes accumulate/residual");
   if (int rc = ensure_device())
     return rc;
+  // int8 and int4 weights go to the integer tensor cores.  What stays here: one row over less than 6 MB of weights (the
+  // kernel below is done in 2.6 - 7 us, the other one's longer code and its quantisation of the row cost 1.3 us more; they
+  // meet at 8 MB), f32 weights, other group sizes and scale types, and the tensor-parallel push.
+  if (push == nullptr && gemv_mma_takes(w, a))
+    return gemv_mma_run(w, a, stream);
 
   GemvP p{};
   if (push != nullptr) {

@@ -1,0 +1,75 @@
+"""b200_gemv on the integer tensor cores at the sizes where its tiling can go wrong: ragged rows, short last
+blocks (int8: K % 512, int4: every K % 1024 that is a multiple of 128), every tile of activation rows, activation
+slabs that do not fit shared memory at once, 16-bit activations, non-finite activations."""
+import numpy as np
+import pytest
+
+import oracle_lib as orc
+from buddy_mlir_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return float(np.abs(a - b).max() / np.abs(b).max())
+
+
+@pytest.mark.parametrize("M,N,K", [(2, 8, 64), (2, 1, 16), (3, 77, 528), (5, 1001, 1040), (8, 33, 5008), (12, 333, 8976),
+                                   (16, 250, 12304), (1, 4099, 1552), (2, 50, 1001)])
+def test_int8_edges(M, N, K):
+    from gpu_util import dev, gemv, packed_weight
+    rng = np.random.default_rng(M * 7 + N + K)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    Q = rng.integers(-128, 128, (K, N)).astype(np.int8)
+    s = rng.uniform(0.001, 0.01, N).astype(np.float32)
+    y = gemv(_lib.W_I8, packed_weight(_lib.W_I8, Q, K, N), dev(s), K, N, dev(x)).cpu().numpy()
+    assert rel(y, orc.gemv_w8_f32(x, Q, s)) < 1e-5
+
+
+@pytest.mark.parametrize("M,N,K", [(2, 500, 128), (3, 66, 384), (2, 130, 640), (4, 34, 896), (5, 1000, 1152), (1, 9000, 1664),
+                                   (7, 18, 1280), (10, 250, 1792), (16, 100, 9088), (16, 64, 2944)])
+def test_int4_group128_edges(M, N, K):
+    from gpu_util import dev, gemv, packed_scales, packed_weight
+    rng = np.random.default_rng(M + N * 3 + K)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    P = rng.integers(0, 256, (K, N // 2)).astype(np.uint8)
+    s = rng.uniform(0.001, 0.01, (K // 128, N)).astype(np.float16)
+    y = gemv(_lib.W_U4, packed_weight(_lib.W_U4, P, K, N, 0), packed_scales(s, _lib.F16, K // 128, N), K, N, dev(x),
+             group=128, scale_dtype=_lib.F16).cpu().numpy()
+    assert rel(y, orc.gemv_w4g_f32(x, P, s, 128)) < 1e-5
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16"])
+@pytest.mark.parametrize("M", [2, 9])
+def test_norm_silu_and_16_bit_rows(dtype, M):
+    import torch
+    from gpu_util import dev, gemv, packed_weight
+    rng = np.random.default_rng(M)
+    K, N = 1552, 2 * 77
+    xt = torch.from_numpy((rng.standard_normal((M, K)) * 50).astype(np.float32)).to(
+        torch.float16 if dtype == "f16" else torch.bfloat16).cuda()
+    x = xt.float().cpu().numpy()
+    nw = (1 + 0.1 * rng.standard_normal(K)).astype(np.float32)
+    Q = rng.integers(-127, 128, (K, N)).astype(np.int8)
+    s = rng.uniform(0.0005, 0.001, N).astype(np.float32)
+    y = gemv(_lib.W_I8, packed_weight(_lib.W_I8, Q, K, N), dev(s), K, N, xt, norm_w=dev(nw), silu=True,
+             x_dtype=_lib.F16 if dtype == "f16" else _lib.BF16).cpu().numpy()
+    for m in range(M):
+        r = orc.gemv_w8_f32(orc.rmsnorm(x[m], nw, 1e-6)[None, :], Q, s)[0]
+        assert rel(y[m], orc.silu_mul(np.ascontiguousarray(r[0::2]), np.ascontiguousarray(r[1::2]))) < 1e-5
+
+
+def test_rows_of_very_different_size_and_a_row_with_a_nan():
+    """Every activation row has a fixed-point scale of its own; a non-finite row yields no finite result."""
+    from gpu_util import dev, gemv, packed_weight
+    rng = np.random.default_rng(3)
+    M, N, K = 4, 40, 1024
+    x = rng.standard_normal((M, K)).astype(np.float32) * np.float32([[1e-30], [1e20], [1.0], [1.0]])
+    x[2, 5] = np.nan
+    x[3, :] = 0
+    Q = rng.integers(-127, 128, (K, N)).astype(np.int8)
+    s = rng.uniform(0.001, 0.01, N).astype(np.float32)
+    y = gemv(_lib.W_I8, packed_weight(_lib.W_I8, Q, K, N), dev(s), K, N, dev(x)).cpu().numpy()
+    ref = orc.gemv_w8_f32(x[[0, 1, 3]], Q, s)
+    assert rel(y[0], ref[0]) < 1e-5 and rel(y[1], ref[1]) < 1e-5
+    assert not np.isfinite(y[2]).any() and (y[3] == 0).all()
