@@ -11,7 +11,7 @@
 // q/k/v/gate/up, row-parallel o/down, sum after each, vocab-sharded lm_head;
 // buddy-deepseek-r1-distributed.cpp:521-617) with NCCL in place of MPI.
 #include "common.cuh"
-#include "mega.cuh"
+#include "decode.cuh"
 
 #include <dlfcn.h>
 
@@ -301,15 +301,14 @@ struct b200_model {
   float *h_rows_pinned = nullptr;   // this step's K/V rows, fetched together with the logits
   bool rows_fresh = false;
   int32_t *h_state_pinned = nullptr;
-  // persistent decode-step kernel (batch 1, int8): see mega.cu
-  bool mega = false;
-  MegaParams mp{};
-  int mega_grid = 0;
-  size_t mega_smem = 0;
-  int64_t mega_stream_bytes = 0;
-  uint8_t *mega_stream = nullptr;
-  int64_t *mega_offsets = nullptr;   // [(4L+1)+1][grid]: per-phase and per-CTA stream offsets
-  const float **lvec_dev = nullptr;
+  // persistent decode-step kernel (batch 1): see decode.cu
+  bool persistent = false;
+  DecParams dp{};
+  int dec_grid = 0;
+  size_t dec_smem = 0;
+  uint8_t *dec_stream = nullptr;     // the weights once more, as the kernel's warps consume them
+  int64_t *dec_offsets = nullptr;    // [(4L+1)+1][grid * warps]: offsets of every projection, starts of the streams
+  DecLayer *dec_layers = nullptr;
   uint2 *ll_buf = nullptr;           // tagged activation buffers
   long long *d_trace = nullptr;
   // prefill (many rows at once): activations of all rows, grown on demand
@@ -549,164 +548,116 @@ int issue_step(b200_model *m, int *n_kernels) {
 
 
 // ---- persistent-kernel path ------------------------------------------------------
-void rows_of_host(int N, int cta, int grid, int &begin, int &count) {  // N in dealing units
-  const int base = N / grid, rem = N % grid;
-  begin = cta * base + (cta < rem ? cta : rem);
-  count = base + (cta < rem ? 1 : 0);
-}
-
-bool mega_eligible(const b200_model *m, const Layer &L0) {
+// Whether the persistent kernel can run this model's decode steps (batch 1, one GPU, head_dim 128): every projection int8
+// per channel, int4 (group 128 or per channel, f16 scales) or f32, with vectors a CTA can stage.  Fills the projections.
+bool persistent_eligible(const b200_model *m, int grid, DecPhase (&ph)[5]) {
   const char *env = std::getenv("BUDDY_B200_DECODE");
   if (env && !strcmp(env, "graph"))
     return false;
   const b200_model_config &c = m->cfg;
-  if (m->tp != 1 || c.head_dim != 128)
+  if (m->tp != 1 || c.head_dim != 128 || c.kv_heads > grid || !dec_group_built(c.q_heads / c.kv_heads) || c.hidden % 4)
     return false;
-  const int G = c.q_heads / c.kv_heads;
-  if (G != 1 && G != 2 && G != 4 && G != 6 && G != 8)
-    return false;
-  auto ok = [](const DevLinear &l) {
-    return l.set && l.w.kind == B200_W_I8 && l.w.scale_dtype == B200_F32 && l.w.K % 16 == 0 &&
-           l.w.K <= 12288;
+  auto fits = [&](const DevLinear &l, DecPhase &q) {
+    const b200_weight &w = l.w;
+    if (!l.set || w.K > kDecMaxK || w.K % 4 != 0)
+      return false;
+    if (w.kind == B200_W_I8) {
+      if (w.scale_dtype != B200_F32)
+        return false;
+    } else if (w.kind == B200_W_U4) {
+      if (w.scale_dtype != B200_F16 || w.K % 256 != 0 || (w.group > 0 && w.group < w.K && w.group != 128))
+        return false;
+    } else if (w.K % 32 != 0) {
+      return false;
+    }
+    const int tiles = (int)((w.N + 15) / 16), kb = dec_block_k(w.kind);
+    const DecPhase want{w.kind, (int)w.K, (int)w.N, tiles, (int)((w.K + kb - 1) / kb)};
+    if (q.tiles && (q.kind != want.kind || q.K != want.K || q.N != want.N))
+      return false;   // the layers share one plan
+    q = want;
+    return (tiles + grid - 1) / grid <= 128;
   };
   for (const auto &L : m->layers)
-    if (!ok(L.qkv) || !ok(L.o) || !ok(L.gate) || !ok(L.up) || !ok(L.down))
+    if (!fits(L.qkv, ph[0]) || !fits(L.o, ph[1]) || !fits(L.gateup, ph[2]) || !fits(L.down, ph[3]))
       return false;
-  (void)L0;
-  return ok(m->lm_head);
+  return fits(m->lm_head, ph[4]);
 }
 
-int build_mega(b200_model *m) {
+int build_persistent(b200_model *m) {
   const b200_model_config &c = m->cfg;
   int dev = 0, sms = 0, coop = 0;
   B200_CUDA(cudaGetDevice(&dev));
   B200_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   B200_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-  const int G = c.q_heads / c.kv_heads;
-  const int grid = sms, L = c.n_layers, D = c.head_dim;
-  // attention work items: every CTA takes one (kv head, split) pair
-  int splits = grid / c.kv_heads;
-  if (splits > 128) splits = 128;
-  while (splits > 1 && G * splits > 768) --splits;
-  // the split fold keeps (outputs per warp) x (splits per lane) partials in registers
-  const bool fold_fits =
-      splits >= 1 && (((G * D + splits - 1) / splits + 15) / 16) * ((splits + 31) / 32) <= 8;
-  if (!coop || !fold_fits)
+  const int grid = sms, L = c.n_layers, D = c.head_dim, warps = grid * kDecWarps;
+  DecParams &p = m->dp;
+  p = DecParams{};
+  if (!coop || !persistent_eligible(m, grid, p.phase))
     return B200_OK;  // stays on the graph path
-  const int H = c.hidden, QD = c.q_heads * D, KD = c.kv_heads * D, F = c.ffn, V = c.vocab;
-  MegaParams &p = m->mp;
-  const int Ks[5] = {H, QD, H, F, H}, Ns[5] = {QD + 2 * KD, H, 2 * F, H, V};
-  if (H > 1536 || QD > 1536 || H % 16 != 0 || QD % 16 != 0 || F % 16 != 0)
-    return B200_OK;
-  int slot_bytes = 0;
+  const int H = c.hidden, QD = c.q_heads * D, KD = c.kv_heads * D, F = c.ffn;
+  p.H = H; p.F = F; p.V = c.vocab; p.qh = c.q_heads; p.kvh = c.kv_heads; p.L = L;
+  p.max_len = c.max_len;
+  p.block_bytes = kDecBlockBytes;
+  p.part_rows = 0;
   for (int i = 0; i < 5; ++i) {
-    if (i == 3)
-      continue;
-    MegaPhase &ph = p.phase[i];
-    ph.K = Ks[i];
-    ph.N = Ns[i];
-    ph.row_bytes = Ks[i] + kMegaTrailer;
-    ph.mode = 0;
-    ph.unit = i == 2 ? 2 : 1;
-    ph.rps = 16;   // a stage is 16 rows: 16 warps x 1 row, 4 x 4 or 2 x 8
-    if (ph.rps * ph.row_bytes > slot_bytes)
-      slot_bytes = ph.rps * ph.row_bytes;
+    if (p.phase[i].kind == B200_W_U4)
+      p.block_bytes = kDecBlockBytes + kDecScaleBytes;
+    const int rows = (p.phase[i].tiles + grid - 1) / grid + kDecWarps;
+    if (rows > p.part_rows) p.part_rows = rows;
   }
-  {
-    // down projection: long rows, a few per stage, one warp per row
-    MegaPhase &ph = p.phase[3];
-    ph.K = F;
-    ph.N = H;
-    ph.row_bytes = F + kMegaTrailer;
-    ph.mode = 0;
-    ph.unit = 1;
-    ph.rps = slot_bytes / ph.row_bytes;
-    if (ph.rps > 8) ph.rps = 8;
-    if (ph.rps < 1 || (ph.rps & (ph.rps - 1)) != 0) {   // 1, 2, 4 or 8 rows: the warps split evenly over stages
-      if (ph.rps >= 4) ph.rps = 4;
-      else if (ph.rps >= 2) ph.rps = 2;
-      else if (ph.rps < 1) return B200_OK;
-    }
-  }
-  slot_bytes = (slot_bytes + 127) / 128 * 128;
-  int xs_floats = H > QD ? H : QD;                          // staged activations of a projection
-  if (xs_floats < F) xs_floats = F;
-  if (xs_floats < (G + 2 + 7 * G) * D) xs_floats = (G + 2 + 7 * G) * D;   // staged q | k | v + states of the 7 scanning warps
-  if (xs_floats < 3 * G * splits + 8) xs_floats = 3 * G * splits + 8;   // split fold: m, l, weights
-  xs_floats = (xs_floats + 31) / 32 * 32;
-  const size_t fixed = mega_fixed_shared_bytes() + (size_t)xs_floats * 4;
-  int slots = (int)((227 * 1024 - (long)fixed) / slot_bytes);
-  if (slots > kMegaMaxSlots) slots = kMegaMaxSlots;
-  if (slots < 4)
+  p.union_bytes = (int)dec_union_bytes(p.phase, c.q_heads / c.kv_heads, &p.planes_bytes);
+  if (dec_shared_bytes(p) > 227 * 1024)
     return B200_OK;
-  for (int cta = 0; cta < grid; ++cta) {   // the in-kernel stage table is fixed-size
-    int per_layer = 0;
-    for (int i = 0; i < 4; ++i) {
-      int b, n;
-      rows_of_host(p.phase[i].N / p.phase[i].unit, cta, grid, b, n);
-      per_layer += (n * p.phase[i].unit + p.phase[i].rps - 1) / p.phase[i].rps;
-    }
-    if (per_layer > kMegaMaxLayerStages)
-      return B200_OK;
-  }
-  // per-phase, per-CTA stream offsets
+  // Every warp's stream: its blocks of the four projections of layer 0, of layer 1, ..., then of the lm_head.
   const int nph = 4 * L + 1;
-  std::vector<int64_t> table((size_t)(nph + 1) * grid);
+  std::vector<int64_t> table((size_t)(nph + 1) * warps);   // bytes before projection i; last row: start of the stream
   int64_t total = 0;
-  for (int cta = 0; cta < grid; ++cta) {
-    table[(size_t)nph * grid + cta] = total;  // start of this CTA's stream
+  for (int w = 0; w < warps; ++w) {
+    table[(size_t)nph * warps + w] = total;
+    int64_t own = 0;
     for (int i = 0; i < nph; ++i) {
-      const MegaPhase &ph = p.phase[i < 4 * L ? i % 4 : 4];
-      int b, n;
-      rows_of_host(ph.N / ph.unit, cta, grid, b, n);
-      table[(size_t)i * grid + cta] = total;
-      total += (int64_t)n * ph.unit * ph.row_bytes;
+      const DecPhase &q = p.phase[i < 4 * L ? i % 4 : 4];
+      const int cta = w / kDecWarps, k = w % kDecWarps;
+      const int nb = (share_begin(q.tiles, cta + 1, grid) - share_begin(q.tiles, cta, grid)) * q.blocks;
+      table[(size_t)i * warps + w] = own;
+      own += (int64_t)(warp_begin(nb, k + 1) - warp_begin(nb, k)) * p.block_bytes;
     }
+    total += own;
   }
-  if (int rc = dev_alloc((void **)&m->mega_stream, total)) return rc;
-  if (int rc = dev_alloc((void **)&m->mega_offsets, table.size() * 8)) return rc;
-  B200_CUDA(cudaMemcpy(m->mega_offsets, table.data(), table.size() * 8, cudaMemcpyHostToDevice));
+  if (int rc = dev_alloc((void **)&m->dec_stream, total)) return rc;
+  if (int rc = dev_alloc((void **)&m->dec_offsets, table.size() * 8)) return rc;
+  // everything on the session's stream: it does not wait for the default stream, and a synchronous copy from pageable
+  // memory may return while its last bytes are still on their way
   cudaStream_t st = m->stream;
-  for (int l = 0; l < L; ++l) {
-    Layer &Ly = m->layers[l];
-    const int64_t *o0 = m->mega_offsets + (size_t)(4 * l) * grid;
-    if (int rc = mega_build_rows(Ly.qkv.w_buf, H, Ns[0], 1, 0, Ns[0], 1, (const float *)Ly.qkv.scale_buf,
-                                 Ly.qkv.bias_buf, grid, p.phase[0].row_bytes, o0, m->mega_stream, st))
-      return rc;
-    if (int rc = mega_build_rows(Ly.o.w_buf, QD, H, 1, 0, H, 1, (const float *)Ly.o.scale_buf, nullptr,
-                                 grid, p.phase[1].row_bytes, o0 + grid, m->mega_stream, st))
-      return rc;
-    // gate_j -> row 2j, up_j -> row 2j+1: one warp then holds the pair of a SiLU gate
-    if (int rc = mega_build_rows(Ly.gate.w_buf, H, F, 2, 0, 2 * F, 2, (const float *)Ly.gate.scale_buf,
-                                 nullptr, grid, p.phase[2].row_bytes, o0 + 2 * grid, m->mega_stream, st))
-      return rc;
-    if (int rc = mega_build_rows(Ly.up.w_buf, H, F, 2, 1, 2 * F, 2, (const float *)Ly.up.scale_buf, nullptr,
-                                 grid, p.phase[2].row_bytes, o0 + 2 * grid, m->mega_stream, st))
-      return rc;
-    if (int rc = mega_build_rows(Ly.down.w_buf, F, H, 1, 0, H, 1, (const float *)Ly.down.scale_buf, nullptr,
-                                 grid, p.phase[3].row_bytes, o0 + 3 * grid, m->mega_stream, st))
+  B200_CUDA(cudaMemcpyAsync(m->dec_offsets, table.data(), table.size() * 8, cudaMemcpyHostToDevice, st));
+  const int64_t *starts = m->dec_offsets + (size_t)nph * warps;
+  for (int i = 0; i < nph; ++i) {
+    const DevLinear *lin = &m->lm_head;
+    if (i < 4 * L) {
+      const Layer &Ly = m->layers[i / 4];
+      lin = i % 4 == 0 ? &Ly.qkv : i % 4 == 1 ? &Ly.o : i % 4 == 2 ? &Ly.gateup : &Ly.down;
+    }
+    if (int rc = dec_build_phase(&lin->w, p.phase[i < 4 * L ? i % 4 : 4], grid, p.block_bytes, starts,
+                                 m->dec_offsets + (size_t)i * warps, m->dec_stream, st))
       return rc;
   }
-  if (int rc = mega_build_rows(m->lm_head.w_buf, H, V, 1, 0, V, 1, (const float *)m->lm_head.scale_buf,
-                               nullptr, grid, p.phase[4].row_bytes,
-                               m->mega_offsets + (size_t)(4 * L) * grid, m->mega_stream, st))
-    return rc;
-  std::vector<const float *> lvec(4 * L);
+  std::vector<DecLayer> layers(L);
+  auto i8_scale = [](const DevLinear &l) { return l.w.kind == B200_W_I8 ? (const float *)l.scale_buf : nullptr; };
   for (int l = 0; l < L; ++l) {
-    lvec[4 * l] = m->layers[l].in_norm;
-    lvec[4 * l + 1] = m->layers[l].post_norm;
-    lvec[4 * l + 2] = m->layers[l].q_norm;
-    lvec[4 * l + 3] = m->layers[l].k_norm;
+    const Layer &Ly = m->layers[l];
+    layers[l] = DecLayer{Ly.in_norm, Ly.post_norm, Ly.q_norm, Ly.k_norm,
+                         {i8_scale(Ly.qkv), i8_scale(Ly.o), i8_scale(Ly.gateup), i8_scale(Ly.down)},
+                         Ly.qkv.bias_buf, m->kv[2 * l], m->kv[2 * l + 1]};
   }
-  if (int rc = dev_alloc((void **)&m->lvec_dev, lvec.size() * sizeof(float *))) return rc;
-  B200_CUDA(cudaMemcpy(m->lvec_dev, lvec.data(), lvec.size() * sizeof(float *), cudaMemcpyHostToDevice));
+  if (int rc = dev_alloc((void **)&m->dec_layers, layers.size() * sizeof(DecLayer))) return rc;
+  B200_CUDA(cudaMemcpyAsync(m->dec_layers, layers.data(), layers.size() * sizeof(DecLayer), cudaMemcpyHostToDevice, st));
   // tagged activation buffers, all in one allocation (zero tags never match)
   const size_t n_qkv = 2 * (size_t)(QD + 2 * KD), n_attn = 2 * (size_t)QD, n_x = 2 * (size_t)H,
-               n_mid = 2 * (size_t)F, n_part = 2 * (size_t)c.q_heads * splits * (D + 2),
+               n_mid = 2 * (size_t)F, n_part = 2 * (size_t)c.q_heads * kDecMaxSplits * (D + 2),
                n_cand = 2 * (size_t)grid;
   const size_t n_ll = n_qkv + n_attn + 2 * n_x + n_mid + n_part + n_cand + 16;
   if (int rc = dev_alloc((void **)&m->ll_buf, n_ll * sizeof(uint2))) return rc;
-  B200_CUDA(cudaMemset(m->ll_buf, 0, n_ll * sizeof(uint2)));
+  B200_CUDA(cudaMemsetAsync(m->ll_buf, 0, n_ll * sizeof(uint2), st));
   uint2 *q = m->ll_buf;
   auto take = [&](size_t n) { uint2 *r = q; q += (n + 1) / 2 * 2; return r; };   // keep 16-byte alignment
   p.ll_qkv = take(n_qkv);
@@ -716,38 +667,30 @@ int build_mega(b200_model *m) {
   p.ll_xa = take(n_x);
   p.ll_part = take(n_part);
   p.ll_cand = take(n_cand);
-  p.stream = m->mega_stream;
-  p.cta_off = m->mega_offsets + (size_t)nph * grid;
-  p.H = H; p.F = F; p.V = V; p.qh = c.q_heads; p.kvh = c.kv_heads; p.L = L;
-  p.max_len = c.max_len;
-  p.splits = splits;
-  p.slots = slots;
-  p.slot_bytes = slot_bytes;
-  p.xs_floats = xs_floats;
+  p.stream = m->dec_stream;
+  p.warp_off = starts;
+  p.layers = m->dec_layers;
+  p.lm_scale = i8_scale(m->lm_head);
   p.eps = c.eps;
   p.embed = m->embed; p.inv_freq = m->inv_freq; p.final_norm = m->final_norm;
-  p.lvec = m->lvec_dev;
-  p.kv = m->kv_dev;
   p.logits = m->logits;
   p.kv_stage = m->kv_stage;
   p.state = m->d_state;
   p.history = m->d_history;
   p.history_cap = m->history_cap;
   p.error = m->d_state + 6;
-  p.trace = nullptr;
   p.trace_stride = 1;
   if (const char *t = std::getenv("BUDDY_B200_TRACE")) {
     p.trace_stride = std::atoi(t) > 0 ? std::atoi(t) : 1;
-    const size_t n = (size_t)(grid / p.trace_stride + 1) * (L + 1) * kMegaTraceSlots;
+    const size_t n = (size_t)(grid / p.trace_stride + 1) * (L + 1) * kDecTraceSlots;
     if (int rc = dev_alloc((void **)&m->d_trace, n * 8)) return rc;
-    B200_CUDA(cudaMemset(m->d_trace, 0, n * 8));
+    B200_CUDA(cudaMemsetAsync(m->d_trace, 0, n * 8, st));
     p.trace = m->d_trace;
   }
-  m->mega_grid = grid;
-  m->mega_smem = fixed + (size_t)slots * slot_bytes;
-  m->mega_stream_bytes = total;
+  m->dec_grid = grid;
+  m->dec_smem = dec_shared_bytes(p);
   B200_CUDA(cudaStreamSynchronize(st));
-  m->mega = true;
+  m->persistent = true;
   return B200_OK;
 }
 
@@ -791,8 +734,8 @@ int run_step_int8(b200_model *m) {
 int run_step(b200_model *m) {
   if (m->act_int8)
     return run_step_int8(m);
-  if (m->mega)
-    return mega_launch(m->mp, m->mega_grid, m->mega_smem, m->stream);
+  if (m->persistent)
+    return dec_launch(m->dp, m->dec_grid, m->dec_smem, m->stream);
   B200_CUDA(cudaGraphLaunch(m->exec, m->stream));
   count_launch(m->kernels_per_step);
   return B200_OK;
@@ -963,7 +906,7 @@ void b200_model_destroy(b200_model *m) {
   cudaFree(m->part); cudaFree(m->logits); cudaFree(m->logits_shard);
   cudaFree(m->attn_scratch); cudaFree(m->argmax_scratch); cudaFree(m->kv_stage);
   cudaFree(m->d_state); cudaFree(m->d_history);
-  cudaFree(m->mega_stream); cudaFree(m->mega_offsets); cudaFree(m->lvec_dev);
+  cudaFree(m->dec_stream); cudaFree(m->dec_offsets); cudaFree(m->dec_layers);
   cudaFree(m->ll_buf); cudaFree(m->d_trace);
   cudaFree(m->pf_x); cudaFree(m->pf_qkv); cudaFree(m->pf_att); cudaFree(m->pf_mid); cudaFree(m->pf_logits);
   cudaFree(m->pf_ws); cudaFree(m->pf_tokens); cudaFree(m->pf_norm);
@@ -1588,6 +1531,8 @@ int b200_model_finalize(b200_model *m) {
   if (m->finalized)
     return B200_OK;
   const b200_model_config &c = m->cfg;
+  // uploads and clears so far went through the default stream, which the session's stream does not wait for
+  B200_CUDA(cudaStreamSynchronize(nullptr));
   if (!m->embed || !m->final_norm || !m->lm_head.set)
     return fail(B200_ESTATE, "finalize: embedding, final norm or lm_head missing");
   if (!m->inv_freq) {
@@ -1608,10 +1553,9 @@ int b200_model_finalize(b200_model *m) {
     if (int rc = fuse_linears({&L.gate, &L.up}, true, &L.gateup, m->stream)) return rc;
     L.q.release(); L.k.release(); L.v.release();
   }
-  if (mega_eligible(m, m->layers[0]))
-    if (int rc = build_mega(m)) return rc;
+  if (int rc = build_persistent(m)) return rc;
   for (auto &L : m->layers) { L.gate.release(); L.up.release(); }
-  if (m->mega) {
+  if (m->persistent) {
     // warm the kernel once (shared-memory attribute, module load), then clear the row it wrote
     if (int rc = set_state(m, 0, 0)) return rc;
     if (int rc = run_step(m)) return rc;
@@ -1820,7 +1764,7 @@ static int prefill_reserve(b200_model *m, int rows, int logit_rows) {
     if (int rc = dev_alloc((void **)&m->pf_att, (size_t)rows * m->qh * D * 4)) return rc;
     if (int rc = dev_alloc((void **)&m->pf_mid, (size_t)rows * m->ffn * 4)) return rc;
     if (int rc = dev_alloc(&m->pf_ws, (size_t)m->pf_ws_bytes)) return rc;
-    B200_CUDA(cudaMemset(m->pf_ws, 0, 256));   // the GEMM's error word (float projections never touch it)
+    B200_CUDA(cudaMemsetAsync(m->pf_ws, 0, 256, m->stream));   // the GEMM's error word (float projections never touch it)
     if (int rc = dev_alloc((void **)&m->pf_tokens, (size_t)rows * 4)) return rc;
     if (m->act_int8)
       if (int rc = dev_alloc((void **)&m->pf_norm, (size_t)rows * c.hidden * 4)) return rc;
@@ -2024,7 +1968,7 @@ int b200_batch_create(b200_model *m, int max_seqs, int page_size, int n_pages, i
   if (rc == B200_OK)
     rc = dev_alloc((void **)&b->d_part,
                    (size_t)gqa_paged_scratch_floats(b->part_rows, m->qh, m->cfg.head_dim, b->max_context) * 4);
-  if (rc == B200_OK && cudaMemset(b->d_part, 0, (size_t)b->part_rows * m->qh * 4) != cudaSuccess)   // the counters
+  if (rc == B200_OK && cudaMemsetAsync(b->d_part, 0, (size_t)b->part_rows * m->qh * 4, m->stream) != cudaSuccess)   // the counters
     rc = fail(B200_ECUDA, "batch_create: cudaMemset failed");
   if (rc != B200_OK) {
     b200_batch_destroy(b);
@@ -2133,7 +2077,7 @@ float *b200_model_kv_ptr(b200_model *m, int buffer) {
   return (m && buffer >= 0 && buffer < (int)m->kv.size()) ? m->kv[buffer] : nullptr;
 }
 
-int b200_model_uses_persistent_kernel(const b200_model *m) { return m && m->mega ? 1 : 0; }
+int b200_model_uses_persistent_kernel(const b200_model *m) { return m && m->persistent ? 1 : 0; }
 // Diagnostic: move the persistent kernel's launch counter, the base of the 32-bit tags its
 // CTAs exchange activations under (tag = (launches + 1) * 8 * (layers + 3) + phase), so that
 // the wrap of the tag space (after 2^32 / (8 * (layers + 3)) launches, 17 million tokens for
@@ -2141,7 +2085,7 @@ int b200_model_uses_persistent_kernel(const b200_model *m) { return m && m->mega
 int b200_model_set_launch_counter(b200_model *m, uint32_t launches) {
   if (!m || !m->finalized)
     return fail(B200_ESTATE, "set_launch_counter: a finalised model is required");
-  if (!m->mega)
+  if (!m->persistent)
     return fail(B200_ESTATE, "set_launch_counter: the model does not run the persistent kernel");
   B200_CUDA(cudaStreamSynchronize(m->stream));
   m->h_state_pinned[4] = (int32_t)launches;
@@ -2156,7 +2100,7 @@ int b200_model_tp_sum_kind(const b200_model *m) {
 int b200_model_read_trace(b200_model *m, long long *host, int64_t capacity) {
   if (!m || !host || !m->d_trace)
     return fail(B200_ESTATE, "read_trace: tracing is off (set BUDDY_B200_TRACE=<cta stride>)");
-  const int64_t n = (int64_t)(m->mega_grid / m->mp.trace_stride + 1) * (m->cfg.n_layers + 1) * kMegaTraceSlots;
+  const int64_t n = (int64_t)(m->dec_grid / m->dp.trace_stride + 1) * (m->cfg.n_layers + 1) * kDecTraceSlots;
   B200_CUDA(cudaMemcpy(host, m->d_trace, (size_t)(n < capacity ? n : capacity) * 8,
                        cudaMemcpyDeviceToHost));
   return (int)(n < capacity ? n : capacity);
