@@ -82,9 +82,15 @@ __device__ __forceinline__ uint4 ll_load2(const uint2 *p) {   // two pairs, 16-b
   return v;
 }
 
+// Bring [p, p + bytes) to L2 (whole 16-byte pieces; p 16-byte aligned).  One thread.
+__device__ __forceinline__ void prefetch_l2(const void *p, int64_t bytes) {
+  const uint32_t n = (uint32_t)bytes & ~15u;
+  if (n > 0)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(n) : "memory");
+}
+
 struct Shared {
   DecParams p;                  // a copy for the function that cannot reach the kernel's parameters cheaply
-  alignas(16) uint32_t red[kDecWarps];   // per-warp largest magnitude (bits)
   alignas(16) float redf[kDecWarps];     // per-warp sum of squares
   float bestv[kDecWarps];
   int besti[kDecWarps];
@@ -93,7 +99,7 @@ struct Shared {
   int first[5][kDecWarps + 1];  // first block of every warp, in this CTA's list of blocks (tile by tile)
   int ftile[5][kDecWarps];      // and its tile
   int abort_flag;
-  // attention: this CTA's (kv head, key range), or head -1; the number of key ranges; its outputs of the fold
+  // attention: this CTA's (kv head, key range), or head -1; the number of key ranges; its outputs of the fold (in fours)
   int a_head, a_split, a_first, a_end, splits, out0, out1;
   uint8_t wfirst[5][kMaxTiles], wlast[5][kMaxTiles];   // warps that hold shares of a tile
 };
@@ -104,7 +110,7 @@ struct Ctx {
   const DecParams &p;
   Shared &sh;
   const DecLayer *layers;   // shared-memory copy
-  uint8_t *planes, *xf;     // activation planes, activations as f32 (attention: scratch, from `planes` on)
+  uint8_t *planes;          // activation planes or values; attention scratch
   float *part;              // partial sums of the tiles, [part_rows][16]
   uint32_t ring;            // this warp's ring (shared-memory address)
   const uint8_t *ring_ptr;
@@ -151,6 +157,14 @@ __device__ __forceinline__ bool poll_expired(const DecParams &p, Shared &sh, Pol
   }
   return false;
 }
+// The same for a whole warp, lanes with `ok` still waiting for the others: one decision for all of them.  Poll loops leave
+// together: lanes that fall out of a loop one by one stay apart, and every shuffle after it pays for it.
+__device__ __forceinline__ bool poll_done(const DecParams &p, Shared &sh, Poll &w, int code, bool ok) {
+  if (__all_sync(0xffffffffu, ok))
+    return true;
+  __nanosleep(20);
+  return __any_sync(0xffffffffu, poll_expired(p, sh, w, code));
+}
 __device__ __forceinline__ float ll_wait1(Ctx &c, const uint2 *p, uint32_t tag) {
   uint2 v = ll_load1(p);
   Poll w;
@@ -163,9 +177,10 @@ __device__ __forceinline__ float ll_wait1(Ctx &c, const uint2 *p, uint32_t tag) 
   return __uint_as_float(v.x);
 }
 
-// n pairs at once: their round trips overlap.
+// N pairs per lane at once, whole warps: the round trips overlap.  Lanes that want nothing pass any valid pair and !live.
 template <int N>
-__device__ __forceinline__ void ll_wait(const DecParams &dp, Shared &sh, const uint2 *const (&p)[N], uint32_t tag, float (&out)[N]) {
+__device__ __forceinline__ void ll_wait(const DecParams &dp, Shared &sh, const uint2 *const (&p)[N], uint32_t tag, float (&out)[N],
+                                        bool live = true) {
   Poll w;
   bool ok;
   do {
@@ -179,9 +194,7 @@ __device__ __forceinline__ void ll_wait(const DecParams &dp, Shared &sh, const u
       ok = ok && v[i].y == tag;
       out[i] = __uint_as_float(v[i].x);
     }
-    if (!ok)
-      __nanosleep(20);
-  } while (!ok && !poll_expired(dp, sh, w, 400 + (int)(tag & 7)));
+  } while (!poll_done(dp, sh, w, 400 + (int)(tag & 7), ok || !live));
 }
 
 // ---- weight stream ---------------------------------------------------------------------------------------------------
@@ -223,18 +236,20 @@ struct XSrc {
   const float *norm_w;  // RMSNorm weight, or null
 };
 
-// The vector goes to shared memory as f32 (times the norm weight), kXBatch groups of four per thread in flight at a time,
-// while every thread follows the largest magnitude; then, for int8 and int4 rows, into planes.  Both passes are loops: the
-// code is run 4 L times a token by whoever needs it, and what does not fit the instruction cache costs more than a loop.
-// Returns what the row sums have to be multiplied by.
-__device__ __forceinline__ float stage_x(Ctx &c, const XSrc &xs, int K, int kind, int *z) {
+// A thread takes k = 4i .. 4i+3 for i = tid, tid + 512, ..; kXBatch of them are in flight at a time.  f32 rows: the values
+// (times the norm weight) go to shared memory.  int8 and int4: a warp's 32 threads hold 128 k, which get a fixed-point
+// scale of their own (one warp reduction, no barrier) and go to planes; `gscale` receives what a group's sums have to be
+// multiplied by.  Loops, not straight lines: this code runs 4 L times a token.  Returns the RMSNorm factor.
+template <int MODE>
+__device__ __forceinline__ float stage_x(Ctx &c, const XSrc &xs, int K, int kind, float *gscale, int *z) {
   const int n4 = K >> 2;
-  float4 *xf = reinterpret_cast<float4 *>(c.xf);
   float ss = 0.f;
-  uint32_t mx = 0;
 #pragma unroll 1
-  for (int i0 = c.tid; i0 < n4; i0 += kXBatch * kCT) {
+  for (int i0 = c.tid; i0 - c.lane < n4; i0 += kXBatch * kCT) {   // whole warps
     float4 v[kXBatch], nw[kXBatch];
+#pragma unroll
+    for (int r = 0; r < kXBatch; ++r)
+      v[r] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (xs.norm_w != nullptr) {   // depends on nothing: requested before the wait
 #pragma unroll
       for (int r = 0; r < kXBatch; ++r)
@@ -265,50 +280,44 @@ __device__ __forceinline__ float stage_x(Ctx &c, const XSrc &xs, int K, int kind
             v[r] = make_float4(__uint_as_float(a[r].x), __uint_as_float(a[r].z), __uint_as_float(b[r].x),
                                __uint_as_float(b[r].z));
           }
-        if (!ok)
-          __nanosleep(20);
-      } while (!ok && !poll_expired(c.p, c.sh, w, 400 + (int)(xs.tag & 7)));
+      } while (!poll_done(c.p, c.sh, w, 400 + (int)(xs.tag & 7), ok));
     }
 #pragma unroll
-    for (int r = 0; r < kXBatch; ++r)
-      if (i0 + r * kCT < n4) {
-        if (xs.norm_w != nullptr) {
-          ss = fmaf(v[r].x, v[r].x, ss);
-          ss = fmaf(v[r].y, v[r].y, ss);
-          ss = fmaf(v[r].z, v[r].z, ss);
-          ss = fmaf(v[r].w, v[r].w, ss);
-          v[r] = make_float4(v[r].x * nw[r].x, v[r].y * nw[r].y, v[r].z * nw[r].z, v[r].w * nw[r].w);
-        }
-        const uint32_t m = 0x7fffffffu;
-        mx = max(mx, max(max(__float_as_uint(v[r].x) & m, __float_as_uint(v[r].y) & m),
-                         max(__float_as_uint(v[r].z) & m, __float_as_uint(v[r].w) & m)));
-        xf[i0 + r * kCT] = v[r];
+    for (int r = 0; r < kXBatch; ++r) {
+      const int i = i0 + r * kCT;
+      if (i - c.lane >= n4)   // warp-uniform
+        break;
+      if (xs.norm_w != nullptr && i < n4) {
+        ss = fmaf(v[r].x, v[r].x, ss);
+        ss = fmaf(v[r].y, v[r].y, ss);
+        ss = fmaf(v[r].z, v[r].z, ss);
+        ss = fmaf(v[r].w, v[r].w, ss);
+        v[r] = make_float4(v[r].x * nw[r].x, v[r].y * nw[r].y, v[r].z * nw[r].z, v[r].w * nw[r].w);
       }
-  }
-  mx = __reduce_max_sync(0xffffffffu, mx);
-  if (xs.norm_w != nullptr)
-    ss = warp_sum(ss);
-  if (c.lane == 0) {
-    c.sh.red[c.warp] = mx;
-    c.sh.redf[c.warp] = ss;
-  }
-  __syncthreads();
-  float inv = 1.f;
-  if (kind != B200_W_F32) {
-    const float scale = fixed_scale(__reduce_max_sync(0xffffffffu, c.sh.red[c.lane & (kDecWarps - 1)]), &inv);
-#pragma unroll 1
-    for (int i = c.tid; i < n4; i += kCT) {   // every thread its own values again
-      const float4 v = xf[i];
+      if (MODE >= 1 && kind == B200_W_F32) {
+        if (i < n4)
+          reinterpret_cast<float4 *>(c.planes)[i] = v[r];
+        continue;
+      }
+      const uint32_t m = 0x7fffffffu;
+      const uint32_t mx = __reduce_max_sync(0xffffffffu, max(max(__float_as_uint(v[r].x) & m, __float_as_uint(v[r].y) & m),
+                                                             max(__float_as_uint(v[r].z) & m, __float_as_uint(v[r].w) & m)));
+      float inv;
+      const float scale = fixed_scale(mx, &inv);
+      if (c.lane == 0)
+        gscale[i >> 5] = inv;
       uint32_t w[4];
-      plane_words(fixed_digits(v.x, scale), fixed_digits(v.y, scale), fixed_digits(v.z, scale), fixed_digits(v.w, scale), w);
+      plane_words(fixed_digits(v[r].x, scale), fixed_digits(v[r].y, scale), fixed_digits(v[r].z, scale),
+                  fixed_digits(v[r].w, scale), w);
       const int set = i >> 4, e = i & 15;
       // word e of the set's 64 k: int8: k = 16t + 4j; int4: k = 32(j/2) + 8t + 4(j%2)
-      const int t = kind == B200_W_I8 ? e >> 2 : (e >> 1) & 3, j = kind == B200_W_I8 ? e & 3 : (e >> 3) * 2 + (e & 1);
+      const bool i8 = MODE < 2 || kind == B200_W_I8;
+      const int t = i8 ? e >> 2 : (e >> 1) & 3, j = i8 ? e & 3 : (e >> 3) * 2 + (e & 1);
       uint8_t *at = c.planes + set * kSet + t * 16 + j * 4;
 #pragma unroll
       for (int pl = 0; pl < 4; ++pl)
         *reinterpret_cast<uint32_t *>(at + pl * 64) = w[pl];
-      if (kind == B200_W_U4) {   // K is a multiple of 256: whole warps, and a warp's 128 k are one scale group
+      if (!i8) {   // start values of the group's sums
 #pragma unroll
         for (int pl = 0; pl < 4; ++pl) {
           const int s = __reduce_add_sync(0xffffffffu, __dp4a((int)w[pl], 0x01010101, 0));
@@ -317,48 +326,54 @@ __device__ __forceinline__ float stage_x(Ctx &c, const XSrc &xs, int K, int kind
         }
       }
     }
-    __syncthreads();
   }
   if (xs.norm_w != nullptr) {
-    float s = 0.f;
-#pragma unroll
-    for (int w = 0; w < kDecWarps; w += 4) {
-      const float4 q = *reinterpret_cast<const float4 *>(&c.sh.redf[w]);
-      s += (q.x + q.y) + (q.z + q.w);
-    }
-    inv *= rsqrtf(s * (1.0f / (float)K) + c.p.eps);
+    ss = warp_sum(ss);
+    if (c.lane == 0)
+      c.sh.redf[c.warp] = ss;
   }
-  return inv;
+  __syncthreads();
+  if (xs.norm_w == nullptr)
+    return 1.f;
+  float s = 0.f;
+#pragma unroll
+  for (int w = 0; w < kDecWarps; w += 4) {
+    const float4 q = *reinterpret_cast<const float4 *>(&c.sh.redf[w]);
+    s += (q.x + q.y) + (q.z + q.w);
+  }
+  return rsqrtf(s * (1.0f / (float)K) + c.p.eps);
 }
 
 // ---- one stream block times the staged activations ---------------------------------------------------------------------
+// int8, int4: the planes' sums (f32, each group of 128 k exact); f32: four partial sums.
 struct Acc {
-  int i[2][4];   // int8: plane sums, two independent MMA chains
-  float f[4];    // int4: plane sums; f32: four partial sums
-  __device__ __forceinline__ void clear() {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      i[0][e] = i[1][e] = 0;
-      f[e] = 0.f;
-    }
-  }
+  float f[4];
+  __device__ __forceinline__ void clear() { f[0] = f[1] = f[2] = f[3] = 0.f; }
 };
-__device__ __forceinline__ void block_i8(const uint8_t *blk, const uint8_t *planes, int lane, Acc &a) {
+__device__ __forceinline__ void block_i8(const uint8_t *blk, const uint8_t *planes, float gscale, int lane, Acc &a) {
   const uint8_t *b = planes + lane_at<4>();
+  int d[2][4] = {{kFloatBias, kFloatBias, kFloatBias, kFloatBias}, {0, 0, 0, 0}};   // |sums| <= 2^21: see start_u4
 #pragma unroll
   for (int s = 0; s < 2; ++s) {
     const uint4 w0 = *reinterpret_cast<const uint4 *>(blk + (s * 64 + lane) * 16);
     const uint4 w8 = *reinterpret_cast<const uint4 *>(blk + (s * 64 + 32 + lane) * 16);
     const uint4 x = *reinterpret_cast<const uint4 *>(b + s * kSet);
-    mma_s8(a.i[s], w0.x, w8.x, w0.y, w8.y, x.x, x.y);
-    mma_s8(a.i[s], w0.z, w8.z, w0.w, w8.w, x.z, x.w);
+    mma_s8(d[s], w0.x, w8.x, w0.y, w8.y, x.x, x.y);
+    mma_s8(d[s], w0.z, w8.z, w0.w, w8.w, x.z, x.w);
   }
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+    a.f[e] = fmaf(__int_as_float(d[0][e] + d[1][e]) - 12582912.0f, gscale, a.f[e]);
 }
-__device__ __forceinline__ void block_u4(const uint8_t *blk, const uint8_t *planes, const int *z, int lane, Acc &a) {
+__device__ __forceinline__ void block_u4(const uint8_t *blk, const uint8_t *planes, const float *gscale, const int *z, int lane,
+                                         Acc &a) {
   const uint8_t *b = planes + lane_at<4>();
   const int g = lane >> 2;
-  const float2 s0 = __half22float2(*reinterpret_cast<const __half2 *>(blk + kDecBlockBytes + g * 4));
-  const float2 s8 = __half22float2(*reinterpret_cast<const __half2 *>(blk + kDecBlockBytes + (g + 8) * 4));
+  const float2 gs = *reinterpret_cast<const float2 *>(gscale);
+  float2 s0 = __half22float2(*reinterpret_cast<const __half2 *>(blk + kDecBlockBytes + g * 4));
+  float2 s8 = __half22float2(*reinterpret_cast<const __half2 *>(blk + kDecBlockBytes + (g + 8) * 4));
+  s0 = make_float2(s0.x * gs.x, s0.y * gs.y);
+  s8 = make_float2(s8.x * gs.x, s8.y * gs.y);
   int d[2][4];
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
@@ -424,25 +439,28 @@ __device__ __forceinline__ void gemv_phase(Ctx &c, int ph, const XSrc &xs, const
   const int tiles = c.sh.tiles[ph], kind = MODE == 0 ? (int)B200_W_I8 : q.kind;
   if (tiles == 0)
     return;
-  // what the epilogue needs of row tid is requested now
-  const int row0 = c.sh.tile0[ph] * kTileRows, nrows = tiles * kTileRows;
+  // Epilogue: a warp takes tile `warp`, `warp` + 16, ..; two lanes a row (each half of the shares).  What the first tile
+  // needs is requested now.
+  const int tile0 = c.sh.tile0[ph];
   float e_scale = 1.f, e_bias = 0.f;
   uint2 e_res = make_uint2(0u, 0u);
-  if (c.tid < nrows && row0 + c.tid < q.N) {
-    if (ep.scale != nullptr) {
-      e_scale = ld_row(ep.scale + row0 + c.tid);
-      if (ep.next_scale != nullptr && (c.tid & 15) == 0)   // the next layer's rows: in L2 by then
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(ep.next_scale + row0 + c.tid));
-    }
+  auto row_data = [&](int row) {
+    if (ep.scale != nullptr)
+      e_scale = ld_row(ep.scale + row);
     if (ep.bias != nullptr)
-      e_bias = ld_row(ep.bias + row0 + c.tid);
+      e_bias = ld_row(ep.bias + row);
     if (ep.res_ll != nullptr)
-      e_res = ll_load1(ep.res_ll + row0 + c.tid);   // as a rule complete long ago; the tag is checked when it is used
+      e_res = ll_load1(ep.res_ll + row);   // as a rule complete long ago; the tag is checked when it is used
     else if (ep.res != nullptr)
-      e_res.x = __float_as_uint(ld_row(ep.res + row0 + c.tid));
-  }
-  int *z = reinterpret_cast<int *>(c.planes + (q.K + 127) / 128 * (2 * kSet));   // int4: start values of the group sums
-  const float inv = stage_x(c, xs, q.K, kind, z);
+      e_res.x = __float_as_uint(ld_row(ep.res + row));
+  };
+  if (c.warp < tiles)
+    row_data(min((tile0 + c.warp) * kTileRows + (c.lane & 15), q.N - 1));
+  if (c.tid == 0 && ep.next_scale != nullptr)   // the next layer's rows: in L2 by then
+    prefetch_l2(ep.next_scale + tile0 * kTileRows, 4 * min(tiles * kTileRows, q.N - tile0 * kTileRows));
+  float *gscale = reinterpret_cast<float *>(c.planes + (q.K + 127) / 128 * (2 * kSet));
+  int *z = reinterpret_cast<int *>(gscale + ((q.K + 255) / 256 * 2 + 3) / 4 * 4);   // int4: start values of the group sums
+  const float inv = stage_x<MODE>(c, xs, q.K, kind, gscale, z);
   trace(c, layer, 10 + 4 * ph);
   int b = c.sh.first[ph][c.warp], tile = c.sh.ftile[ph][c.warp], st = b - tile * q.blocks;
   const int b1 = c.sh.first[ph][c.warp + 1];
@@ -452,11 +470,11 @@ __device__ __forceinline__ void gemv_phase(Ctx &c, int ph, const XSrc &xs, const
   for (; b < b1; ++b) {
     const uint8_t *blk = wait_block<MODE>(c);
     if (kind == B200_W_I8)
-      block_i8(blk, c.planes + st * (2 * kSet), c.lane, a);
+      block_i8(blk, c.planes + st * (2 * kSet), gscale[st], c.lane, a);
     else if (MODE == 2 && kind == B200_W_U4)
-      block_u4(blk, c.planes + st * (4 * kSet), z + st * 8, c.lane, a);
+      block_u4(blk, c.planes + st * (4 * kSet), gscale + st * 2, z + st * 8, c.lane, a);
     else if (MODE >= 1)
-      block_f32(blk, reinterpret_cast<const float *>(c.xf) + st * 32, c.lane, a);
+      block_f32(blk, reinterpret_cast<const float *>(c.planes) + st * 32, c.lane, a);
     if (MODE == 2)
       __syncwarp();   // the scales are read across lanes
     request_block<MODE>(c);
@@ -469,11 +487,6 @@ __device__ __forceinline__ void gemv_phase(Ctx &c, int ph, const XSrc &xs, const
         if (c.lane < 16)
           dst[c.lane] = v;
       } else {
-        if (kind == B200_W_I8) {
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            a.f[e] = (float)(a.i[0][e] + a.i[1][e]);
-        }
         const bool lowp = c.lane & 1;   // odd: planes 2 and 3
         const float f0 = lowp ? 256.f : 16777216.f, f1 = lowp ? 1.f : 65536.f;
         float v0 = fmaf(a.f[0], f0, a.f[1] * f1), v1 = fmaf(a.f[2], f0, a.f[3] * f1);
@@ -491,32 +504,24 @@ __device__ __forceinline__ void gemv_phase(Ctx &c, int ph, const XSrc &xs, const
   }
   __syncthreads();
   trace(c, layer, 11 + 4 * ph);
-  // ---- rows: shares of the warps in warp order, epilogue ------------------------------------------------------------
+  // ---- rows: shares of the warps, epilogue -------------------------------------------------------------------------
 #pragma unroll 1
-  for (int i = c.tid; i < ((nrows + 31) & ~31); i += kCT) {   // whole warps
-    const int t = i >> 4, row = row0 + i;
-    const bool in = i < nrows && row < q.N;
+  for (int t = c.warp; t < tiles; t += kDecWarps) {
+    const int r = c.lane & 15, row = (tile0 + t) * kTileRows + r;
+    const bool in = c.lane < 16 && row < q.N;
+    if (t != c.warp)
+      row_data(min(row, q.N - 1));
     float v = 0.f;
-    if (in) {
-      const int w1 = c.sh.wlast[ph][t];
+    const int w1 = c.sh.wlast[ph][t];
 #pragma unroll 4
-      for (int w = c.sh.wfirst[ph][t]; w <= w1; ++w)
-        v += c.part[(t + w) * kTileRows + (i & 15)];
-      if (i >= kCT) {
-        if (ep.scale != nullptr)
-          e_scale = ld_row(ep.scale + row);
-        if (ep.bias != nullptr)
-          e_bias = ld_row(ep.bias + row);
-        e_res = make_uint2(0u, ep.res_tag + 1u);
-        if (ep.res != nullptr)
-          e_res.x = __float_as_uint(ld_row(ep.res + row));
-      }
-      v = v * (inv * e_scale) + e_bias;
-    }
+    for (int w = c.sh.wfirst[ph][t] + (c.lane >> 4); w <= w1; w += 2)
+      v += c.part[(t + w) * kTileRows + r];
+    v += __shfl_xor_sync(0xffffffffu, v, 16);
+    v = v * (inv * e_scale) + e_bias;
     if (ep.kind == EP_SILU) {
       const float up = __shfl_down_sync(0xffffffffu, v, 1);   // (gate, up) rows are neighbours
       // (g * sigmoid(g)) * u; e^-g is kept finite (g * 1e-30 is as good a zero as g / inf)
-      if (in && (i & 1) == 0)
+      if (in && (r & 1) == 0)
         ll_store(ep.out + (row >> 1), v * div_normal(1.f, 1.f + fminf(expf(-v), 1e30f)) * up, ep.tag);
     } else if (in) {
       if (ep.kind == EP_LOGITS) {
@@ -576,12 +581,10 @@ __device__ __noinline__ void attention_range(Shared &sh, const DecLayer *layers,
   };
   load(k, ly.k_cache, s0 + warp * 4);   // the cache does not depend on this layer's q, k, v
   load(v, ly.v_cache, s0 + warp * 4);
-  if (layer + 1 < p.L) {   // and the next layer's share of it can come from L2 by then
-    const DecLayer &nx = layers[layer + 1];
-#pragma unroll 1
-    for (int i = tid; i < (s1 - s0) * 8; i += kCT)   // 128-byte lines: four per row of K and of V
-      asm volatile("prefetch.global.L2 [%0];" ::"l"((i & 4 ? nx.v_cache : nx.k_cache) + head + (size_t)(s0 + (i >> 3)) * D +
-                                                    (i & 3) * 32));
+  if (layer + 1 < p.L && tid == 0) {   // and the next layer's share of it can come from L2 by then
+    const size_t at = head + (size_t)s0 * D;
+    prefetch_l2(layers[layer + 1].k_cache + at, (int64_t)(s1 - s0) * D * 4);
+    prefetch_l2(layers[layer + 1].v_cache + at, (int64_t)(s1 - s0) * D * 4);
   }
   // ---- q heads (one warp each), then k, then v: (head norm,) rotation ---------------------------------------------
   const uint2 *qkv = p.ll_qkv + (size_t)par * (QD + 2 * KD);
@@ -626,22 +629,27 @@ __device__ __noinline__ void attention_range(Shared &sh, const DecLayer *layers,
   for (int g = 0; g < G; ++g)
     acc[g] = make_float4(0.f, 0.f, 0.f, 0.f);
   float m = kSeed, l = 0.f;   // of head `warp`
-#pragma unroll 1
-  for (int j0 = s0; j0 < s1; j0 += kPass) {
+  auto store_k = [&]() {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
       *reinterpret_cast<float4 *>(&s.k[warp * 4 + i][lane * 4]) = k[i];
-    if (j0 + kPass < s1)
-      load(k, ly.k_cache, j0 + kPass + warp * 4);
-    __syncthreads();
-    {
+  };
+  // Two barriers per pass: scores of pass i + 1 share a section with P*V of pass i, the K rows of pass i + 1 are stored
+  // beside the softmax of pass i.
+  store_k();
+  if (s0 + kPass < s1)
+    load(k, ly.k_cache, s0 + kPass + warp * 4);
+  __syncthreads();
+#pragma unroll 1
+  for (int j0 = s0 - kPass; j0 < s1; j0 += kPass) {
+    if (j0 + kPass < s1) {   // scores of the pass at j0 + 64
       const int key = (warp >> 3) * 32 + lane, d0 = (warp & 7) * 16;
-      const float *kr = (j0 + key == pos ? s.knew : s.k[key]) + d0;
+      const float *kr = (j0 + kPass + key == pos ? s.knew : s.k[key]) + d0;
       float sc[G];
 #pragma unroll
       for (int g = 0; g < G; ++g)
         sc[g] = 0.f;
-#pragma unroll 1
+#pragma unroll 2
       for (int i = 0; i < 16; i += 4) {
         const float4 x = *reinterpret_cast<const float4 *>(kr + i);
 #pragma unroll
@@ -654,16 +662,41 @@ __device__ __noinline__ void attention_range(Shared &sh, const DecLayer *layers,
       for (int g = 0; g < G; ++g)
         s.part[warp & 7][g][key] = sc[g];
     }
+    if (j0 >= s0) {   // P*V of the pass at j0
+      if (pos >= j0 + warp * 4 && pos < j0 + warp * 4 + 4) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (j0 + warp * 4 + i == pos)
+            v[i] = *reinterpret_cast<const float4 *>(&s.vnew[lane * 4]);
+      }
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        const float4 pg = *reinterpret_cast<const float4 *>(&s.p[g][warp * 4]);
+        const float ag = s.alpha[g];
+        acc[g].x = fmaf(pg.x, v[0].x, fmaf(pg.y, v[1].x, fmaf(pg.z, v[2].x, fmaf(pg.w, v[3].x, acc[g].x * ag))));
+        acc[g].y = fmaf(pg.x, v[0].y, fmaf(pg.y, v[1].y, fmaf(pg.z, v[2].y, fmaf(pg.w, v[3].y, acc[g].y * ag))));
+        acc[g].z = fmaf(pg.x, v[0].z, fmaf(pg.y, v[1].z, fmaf(pg.z, v[2].z, fmaf(pg.w, v[3].z, acc[g].z * ag))));
+        acc[g].w = fmaf(pg.x, v[0].w, fmaf(pg.y, v[1].w, fmaf(pg.z, v[2].w, fmaf(pg.w, v[3].w, acc[g].w * ag))));
+      }
+      if (j0 + kPass >= s1)
+        break;
+      load(v, ly.v_cache, j0 + kPass + warp * 4);
+    }
     __syncthreads();
-    if (warp < G) {
+    if (j0 + 2 * kPass < s1) {
+      store_k();
+      if (j0 + 3 * kPass < s1)
+        load(k, ly.k_cache, j0 + 3 * kPass + warp * 4);
+    }
+    if (warp < G) {   // softmax of the pass at j0 + 64
       float a = 0.f, b = 0.f;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         a += s.part[i][warp][lane];
         b += s.part[i][warp][lane + 32];
       }
-      a = j0 + lane < s1 ? a : -INFINITY;
-      b = j0 + lane + 32 < s1 ? b : -INFINITY;
+      a = j0 + kPass + lane < s1 ? a : -INFINITY;
+      b = j0 + kPass + lane + 32 < s1 ? b : -INFINITY;
       const float nm = fmaxf(m, warp_max(fmaxf(a, b)));
       const float al = ex2(m - nm);
       a = ex2(a - nm);
@@ -678,24 +711,7 @@ __device__ __noinline__ void attention_range(Shared &sh, const DecLayer *layers,
         s.l[warp] = l;
       }
     }
-    if (pos >= j0 + warp * 4 && pos < j0 + warp * 4 + 4) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (j0 + warp * 4 + i == pos)
-          v[i] = *reinterpret_cast<const float4 *>(&s.vnew[lane * 4]);
-    }
     __syncthreads();
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-      const float4 pg = *reinterpret_cast<const float4 *>(&s.p[g][warp * 4]);
-      const float ag = s.alpha[g];
-      acc[g].x = fmaf(pg.x, v[0].x, fmaf(pg.y, v[1].x, fmaf(pg.z, v[2].x, fmaf(pg.w, v[3].x, acc[g].x * ag))));
-      acc[g].y = fmaf(pg.x, v[0].y, fmaf(pg.y, v[1].y, fmaf(pg.z, v[2].y, fmaf(pg.w, v[3].y, acc[g].y * ag))));
-      acc[g].z = fmaf(pg.x, v[0].z, fmaf(pg.y, v[1].z, fmaf(pg.z, v[2].z, fmaf(pg.w, v[3].z, acc[g].z * ag))));
-      acc[g].w = fmaf(pg.x, v[0].w, fmaf(pg.y, v[1].w, fmaf(pg.z, v[2].w, fmaf(pg.w, v[3].w, acc[g].w * ag))));
-    }
-    if (j0 + kPass < s1)
-      load(v, ly.v_cache, j0 + kPass + warp * 4);
   }
   if (tr != nullptr && tid == 0)
     tr[layer * kDecTraceSlots + 2] = clock64();
@@ -728,20 +744,37 @@ template <int G> __device__ __forceinline__ void attention_phase(Ctx &c, int lay
   const DecParams &p = c.p;
   if (c.sh.a_head >= 0)
     attention_range<G>(c.sh, c.layers, *reinterpret_cast<AttnScratch<G> *>(c.planes), layer, pos, tag_of(c, layer, 0), c.tr);
-  // ---- fold the ranges: one warp per output, one lane per range ---------------------------------------------------------
+  // ---- fold the ranges: one warp per four outputs, one lane per range ---------------------------------------------------
   if (c.sh.splits > 1) {
     const int par = layer & 1, o1 = c.sh.out1;
 #pragma unroll 1
-    for (int o = c.sh.out0 + c.warp; o < o1; o += kDecWarps) {
-      const uint2 *part = p.ll_part + (((size_t)par * p.qh + (o >> 7)) * kDecMaxSplits + c.lane) * (D + 2);
-      float in[3] = {0.f, kSeed, 0.f};
-      if (c.lane < c.sh.splits)
-        ll_wait<3>(p, c.sh, {part + (o & (D - 1)), part + D, part + D + 1}, tag_of(c, layer, T_PART), in);
-      __syncwarp();
-      const float b = ex2(in[1] - warp_max(in[1]));
-      const float A = warp_sum(in[0] * b), L = warp_sum(in[2] * b);
-      if (c.lane == 0)
-        ll_store(p.ll_attn + (size_t)par * p.qh * D + o, div_normal(A, L), tag_of(c, layer, T_ATTN));
+    for (int o = (c.sh.out0 + c.warp) * 4; o < o1 * 4; o += kDecWarps * 4) {
+      const bool live = c.lane < c.sh.splits;
+      const uint2 *part = p.ll_part + (((size_t)par * p.qh + (o >> 7)) * kDecMaxSplits + (live ? c.lane : 0)) * (D + 2);
+      float in[6];
+      Poll w;
+      const uint32_t tag = tag_of(c, layer, T_PART);
+      bool ok;
+      do {
+        const uint4 v[3] = {ll_load2(part + (o & (D - 1))), ll_load2(part + (o & (D - 1)) + 2), ll_load2(part + D)};
+        ok = true;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          ok = ok && v[i].y == tag && v[i].w == tag;
+          in[2 * i] = __uint_as_float(v[i].x);
+          in[2 * i + 1] = __uint_as_float(v[i].z);
+        }
+      } while (!poll_done(p, c.sh, w, 400 + (int)(tag & 7), ok));
+      if (!live)
+        in[4] = kSeed;
+      const float b = ex2(in[4] - warp_max(in[4]));
+      const float L = warp_sum(in[5] * b);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float A = warp_sum(in[i] * b);
+        if (c.lane == i)
+          ll_store(p.ll_attn + (size_t)par * p.qh * D + o + i, div_normal(A, L), tag_of(c, layer, T_ATTN));
+      }
     }
     __syncthreads();   // as at the end of a projection
   }
@@ -766,7 +799,7 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_step_kernel(const __gri
   constexpr int kBlock = kDecBlockBytes + (MODE == 2 ? kDecScaleBytes : 0);
   uint8_t *ring = at + (size_t)warp * dec_slots(MODE) * kBlock;
 
-  Ctx c{p, sh, layers, planes, planes + p.planes_bytes, part, smem_u32(ring), ring,
+  Ctx c{p, sh, layers, planes, part, smem_u32(ring), ring,
         p.stream + p.warp_off[blockIdx.x * kDecWarps + warp] + lane * 16, 0, 0, 0ull, (int)threadIdx.x, lane, warp,
         ((uint32_t)p.state[4] + 1u) * (8u * (uint32_t)(p.L + 3)),
         (p.trace != nullptr && blockIdx.x % p.trace_stride == 0)
@@ -815,8 +848,8 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_step_kernel(const __gri
     sh.a_split = sp;
     sh.a_first = sp * chunk;
     sh.a_end = min(len, (sp + 1) * chunk);
-    sh.out0 = share_begin(p.qh * D, blockIdx.x, gridDim.x);
-    sh.out1 = share_begin(p.qh * D, blockIdx.x + 1, gridDim.x);
+    sh.out0 = share_begin(p.qh * D / 4, blockIdx.x, gridDim.x);
+    sh.out1 = share_begin(p.qh * D / 4, blockIdx.x + 1, gridDim.x);
   }
 #pragma unroll 1
   for (int i = threadIdx.x; i < p.L * (int)(sizeof(DecLayer) / 8); i += kCT)
@@ -873,14 +906,12 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_step_kernel(const __gri
     gemv_phase<MODE>(c, step, xs, ep, l, bestv, besti);
     if (step == 0) {
       trace(c, l, 0);
-      // the next layer's norm weights and q|k|v bias: in L2 by then
-      const int at = threadIdx.x * 32;
-      if (blockIdx.x == gridDim.x - 1 && at < H) {
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(nx->in_norm + at));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(nx->post_norm + at));
+      if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {   // the next layer's norm weights and bias: in L2 by then
+        prefetch_l2(nx->in_norm, 4 * H);
+        prefetch_l2(nx->post_norm, 4 * H);
+        if (nx->qkv_bias != nullptr)
+          prefetch_l2(nx->qkv_bias, 4 * (QD + 2 * KD));
       }
-      if (blockIdx.x == gridDim.x - 1 && nx->qkv_bias != nullptr && at < QD + 2 * KD)
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(nx->qkv_bias + at));
       attention_phase<G>(c, l, pos);
     }
   }
@@ -915,10 +946,13 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_step_kernel(const __gri
     if (blockIdx.x == 0) {
       bestv = -INFINITY;
       besti = 0x7fffffff;
-      for (int i = lane; i < (int)gridDim.x; i += 32) {
+      for (int i = 0; i < (int)gridDim.x; i += 32) {
+        const bool live = i + lane < (int)gridDim.x;
+        const uint2 *cand = p.ll_cand + 2 * (live ? i + lane : 0);
         float in[2];
-        ll_wait<2>(p, sh, {p.ll_cand + 2 * i, p.ll_cand + 2 * i + 1}, ctag, in);
-        better(in[0], __float_as_int(in[1]));
+        ll_wait<2>(p, sh, {cand, cand + 1}, ctag, in, live);
+        if (live)
+          better(in[0], __float_as_int(in[1]));
       }
       __syncwarp();
       warp_best();
@@ -1005,22 +1039,19 @@ int dec_build_phase(const b200_weight *w, const DecPhase &ph, int grid, int bloc
   return B200_OK;
 }
 
-size_t dec_union_bytes(const DecPhase *ph, int G, int *planes_bytes) {
-  size_t attn = 0, planes = 0, xf = 0;
+size_t dec_union_bytes(const DecPhase *ph, int G) {
+  size_t n = 0;
   switch (G) {
-#define B200_G(G_) case G_: attn = sizeof(AttnScratch<G_>); break;
+#define B200_G(G_) case G_: n = sizeof(AttnScratch<G_>); break;
     B200_G(1) B200_G(2) B200_G(3) B200_G(4) B200_G(6) B200_G(8)
 #undef B200_G
   default: break;
   }
   for (int i = 0; i < 5; ++i) {
-    if (ph[i].kind != B200_W_F32)
-      planes = std::max(planes, (size_t)(ph[i].K + 127) / 128 * (2 * kSet + 16));
-    xf = std::max(xf, (size_t)ph[i].K * 4);
+    const size_t groups = (size_t)(ph[i].K + 255) / 256 * 2;   // planes, scale and start values of 128 k
+    n = std::max(n, ph[i].kind == B200_W_F32 ? (size_t)ph[i].K * 4 : groups * (2 * kSet + 4 + 16) + 16);
   }
-  planes = (planes + 127) / 128 * 128;
-  *planes_bytes = (int)planes;
-  return (std::max(planes + xf, attn) + 127) / 128 * 128;
+  return (n + 127) / 128 * 128;
 }
 // Which weight kinds the kernel has to be compiled for: 0: int8; 1: int8 and f32; 2: all three.
 static int dec_mode(const DecPhase *ph) {

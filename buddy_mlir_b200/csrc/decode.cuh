@@ -35,7 +35,7 @@ struct DecParams {
   const float *lm_scale, *final_norm, *embed, *inv_freq;
   int H, F, V, qh, kvh, L, max_len;
   int block_bytes;
-  int planes_bytes, union_bytes, part_rows;   // shared memory: planes; planes + f32 vector / attention scratch; partial sums
+  int union_bytes, part_rows;   // shared memory: activation planes / attention scratch; partial sums
   float eps;
   // tagged (value, tag) activation buffers, two copies each (layer parity)
   uint2 *ll_qkv;                // [2][QD + 2*KD]
@@ -56,7 +56,7 @@ struct DecParams {
 };
 
 int dec_block_k(int kind);                           // k per stream block
-size_t dec_union_bytes(const DecPhase *ph, int G, int *planes_bytes);
+size_t dec_union_bytes(const DecPhase *ph, int G);   // shared memory of the planes / attention scratch
 size_t dec_shared_bytes(const DecParams &p);
 bool dec_group_built(int G);                         // q heads per kv head the kernel is compiled for
 // The blocks of every CTA's every warp of one projection, from the packed rows (all layers' streams share one layout;

@@ -605,7 +605,7 @@ int build_persistent(b200_model *m) {
     const int rows = (p.phase[i].tiles + grid - 1) / grid + kDecWarps;
     if (rows > p.part_rows) p.part_rows = rows;
   }
-  p.union_bytes = (int)dec_union_bytes(p.phase, c.q_heads / c.kv_heads, &p.planes_bytes);
+  p.union_bytes = (int)dec_union_bytes(p.phase, c.q_heads / c.kv_heads);
   if (dec_shared_bytes(p) > 227 * 1024)
     return B200_OK;
   // Every warp's stream: its blocks of the four projections of layer 0, of layer 1, ..., then of the lm_head.
