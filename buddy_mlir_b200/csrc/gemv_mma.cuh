@@ -29,12 +29,12 @@ __device__ __forceinline__ void mma_s8(int (&c)[4], uint32_t a0, uint32_t a1, ui
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// Fixed-point scale of a row from the bit pattern of its largest magnitude; *inv undoes it.  A row with an infinity or a
-// NaN gets inv = NaN, so its results are NaN.
-__device__ __forceinline__ float fixed_scale(uint32_t absbits, float *inv) {
+// Fixed-point scale of a row from the bit pattern of its largest magnitude, so that |X| < 2^(TOP+1); *inv undoes it.  A row
+// with an infinity or a NaN gets inv = NaN, so its results are NaN.
+template <int TOP = 29> __device__ __forceinline__ float fixed_scale(uint32_t absbits, float *inv) {
   const int e = max((int)(absbits >> 23) - 127, -90);
-  *inv = absbits >= 0x7f800000u ? __uint_as_float(0x7fffffffu) : __uint_as_float((uint32_t)(e - 29 + 127) << 23);
-  return __uint_as_float((uint32_t)(29 - e + 127) << 23);
+  *inv = absbits >= 0x7f800000u ? __uint_as_float(0x7fffffffu) : __uint_as_float((uint32_t)(e - TOP + 127) << 23);
+  return __uint_as_float((uint32_t)(TOP - e + 127) << 23);
 }
 // The four signed digits of X, most significant in the top byte.
 __device__ __forceinline__ uint32_t fixed_digits(float v, float scale) {
