@@ -132,6 +132,10 @@ __host__ __device__ inline int64_t packed_offset(int kind, int64_t K, int64_t k,
   return unit_off + el * 4; // f32: one group of 4 floats, byte offset
 }
 
+// engine.cu: cache rows between a host buffer and a session's cache without waiting (b200_model_kv_upload / _download wait)
+int model_kv_upload_async(b200_model *m, int buffer, const float *host, int pos0, int n_pos);
+int model_kv_download_async(b200_model *m, int buffer, float *host, int pos0, int n_pos);
+int model_synchronize(b200_model *m);
 // prefill.cu: the row-batched small ops around the dense GEMMs
 int embed_rows_launch(const float *table, const int32_t *tokens_dev, float *x, int64_t H, int M, cudaStream_t st);
 int rope_kv_rows_launch(float *qkv, int64_t ld, float *k_cache, float *v_cache, const float *inv_freq,

@@ -1603,7 +1603,7 @@ int b200_model_finalize(b200_model *m) {
 }
 
 static int kv_copy(b200_model *m, int buffer, float *host, int pos0, int n_pos,
-                   bool upload) {
+                   bool upload, bool wait = true) {
   if (!m || !host || buffer < 0 || buffer >= (int)m->kv.size() || pos0 < 0 ||
       n_pos < 0 || pos0 + n_pos > m->cfg.max_len)
     return fail(B200_EINVAL, "kv copy: bad argument");
@@ -1620,9 +1620,24 @@ static int kv_copy(b200_model *m, int buffer, float *host, int pos0, int n_pos,
   else
     B200_CUDA(cudaMemcpy2DAsync(h0, pitch, d0, pitch, width, m->kvh,
                                 cudaMemcpyDeviceToHost, m->stream));
+  if (wait)
+    B200_CUDA(cudaStreamSynchronize(m->stream));
+  return B200_OK;
+}
+}  // extern "C"
+// Queue the upload on the session's stream: what runs on the session next sees the rows.  `host` (page-locked, or the call
+// waits) must stay as it is until then.
+int b200::model_kv_upload_async(b200_model *m, int buffer, const float *host, int pos0, int n_pos) {
+  return kv_copy(m, buffer, const_cast<float *>(host), pos0, n_pos, true, false);
+}
+int b200::model_kv_download_async(b200_model *m, int buffer, float *host, int pos0, int n_pos) {
+  return kv_copy(m, buffer, host, pos0, n_pos, false, false);
+}
+int b200::model_synchronize(b200_model *m) {
   B200_CUDA(cudaStreamSynchronize(m->stream));
   return B200_OK;
 }
+extern "C" {
 int b200_model_kv_upload(b200_model *m, int buffer, const float *host, int pos0,
                          int n_pos) {
   return kv_copy(m, buffer, const_cast<float *>(host), pos0, n_pos, true);

@@ -8,7 +8,9 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
+#include <thread>
 #include <tuple>
 #include <string>
 #include <vector>
@@ -93,16 +95,42 @@ std::mutex g_cache_mu;
 uint64_t g_cache_clock = 0;
 size_t g_cache_bytes = 0;
 
+// Hash of up to `samples` evenly spaced words.  The samples of a large tensor are cache (and TLB) misses: they are
+// requested well ahead, and four independent chains keep the multiplies out of the way.
 uint64_t fingerprint_bytes(const void *p, size_t bytes, uint64_t h, size_t samples = 4096) {
   const size_t words = bytes / 8;
   const uint64_t *q = (const uint64_t *)p;
   const size_t n = words < samples ? words : samples;
-  for (size_t i = 0; i < n; ++i) {
-    uint64_t v;
-    memcpy(&v, q + (n > 1 ? i * (words - 1) / (n - 1) : 0), 8);
-    h = (h ^ v) * 0x100000001B3ull;
-    h ^= h >> 29;
+  uint64_t c[4] = {h, h + 1, h + 2, h + 3};
+  if (n > 0) {
+    // word i is at i * (words - 1) / (n - 1), stepped without a division
+    const size_t d = n > 1 ? n - 1 : 1, step = (words - 1) / d, rem = (words - 1) % d;
+    constexpr size_t kAhead = 24;
+    size_t at = 0, acc = 0, pat = 0, pacc = 0, pi = 0;
+    for (size_t i = 0; i < n; ++i) {
+      for (; pi < n && pi < i + kAhead; ++pi) {
+        __builtin_prefetch(q + pat, 0, 0);
+        pat += step;
+        if ((pacc += rem) >= d) {
+          pacc -= d;
+          ++pat;
+        }
+      }
+      uint64_t v;
+      memcpy(&v, q + at, 8);
+      uint64_t &x = c[i & 3];
+      x = (x ^ v) * 0x100000001B3ull;
+      x ^= x >> 29;
+      at += step;
+      if ((acc += rem) >= d) {
+        acc -= d;
+        ++at;
+      }
+    }
   }
+  for (int i = 1; i < 4; ++i)
+    c[0] = (c[0] ^ c[i]) * 0x100000001B3ull;
+  h = c[0] ^ (c[0] >> 29);
   const unsigned char *tail = (const unsigned char *)p + words * 8;
   for (size_t i = 0; i < bytes - words * 8; ++i)
     h = (h ^ tail[i]) * 0x100000001B3ull;
@@ -168,21 +196,41 @@ int pack_weight_from_host(int kind, const void *src, const void *host_scale, int
   return B200_OK;
 }
 
-// src / host_scale: dense host copies (what is packed and fingerprinted);
-// key: what identifies the caller's tensor.  The returned descriptor stays
-// valid until the next cache call (the entry points hold g_entry_mu).
-int cached_weight(int kind, const void *src, const void *host_scale, int sdt,
-                  int signed_nibbles, int64_t K, int64_t N, int64_t groups,
-                  WeightKey key, const b200_weight **out) {
+// A weight operand of a call: dense host copies (what is packed and fingerprinted), and what identifies the caller's
+// tensor.
+struct WeightSource {
+  int kind;
+  const void *src, *scale;
+  int sdt, signed_nibbles;
+  int64_t K, N, groups;
+  WeightKey key;
+};
+uint64_t fingerprint_of(const WeightSource &w) {
+  const size_t src_bytes = w.kind == B200_W_F32 ? (size_t)w.K * w.N * 4
+                         : w.kind == B200_W_I8  ? (size_t)w.K * w.N
+                                                : (size_t)w.K * w.N / 2;
+  uint64_t fp = fingerprint_bytes(w.src, src_bytes, 0xCBF29CE484222325ull);
+  if (w.scale)
+    fp = fingerprint_bytes(w.scale, (size_t)w.groups * w.N * (w.sdt == B200_F32 ? 4 : 2), fp);
+  return fp;
+}
+WeightKey full_key(const WeightSource &w) {
+  WeightKey key = w.key;
+  key.K = w.K; key.N = w.N; key.groups = w.groups;
+  key.kind = w.kind; key.signed_nibbles = w.signed_nibbles; key.sdt = w.sdt;
+  return key;
+}
+// The cached device copy under the tensor's key, contents unchecked, or null.  Returned descriptors stay valid until the
+// next cache call (the entry points hold g_entry_mu).
+const CachedWeight *cached_candidate(const WeightSource &w) {
   std::lock_guard<std::mutex> lock(g_cache_mu);
-  key.K = K; key.N = N; key.groups = groups;
-  key.kind = kind; key.signed_nibbles = signed_nibbles; key.sdt = sdt;
-  const size_t src_bytes = kind == B200_W_F32 ? (size_t)K * N * 4
-                         : kind == B200_W_I8  ? (size_t)K * N
-                                              : (size_t)K * N / 2;
-  uint64_t fp = fingerprint_bytes(src, src_bytes, 0xCBF29CE484222325ull);
-  if (host_scale)
-    fp = fingerprint_bytes(host_scale, (size_t)groups * N * (sdt == B200_F32 ? 4 : 2), fp);
+  auto it = g_cache.find(full_key(w));
+  return it == g_cache.end() ? nullptr : it->second;
+}
+// The device copy of the tensor whose host bytes have fingerprint fp: the cached one, or packed afresh.
+int cached_weight(const WeightSource &w, uint64_t fp, const b200_weight **out) {
+  std::lock_guard<std::mutex> lock(g_cache_mu);
+  const WeightKey key = full_key(w);
   auto it = g_cache.find(key);
   if (it != g_cache.end()) {
     if (it->second->fingerprint == fp) {
@@ -195,7 +243,7 @@ int cached_weight(int kind, const void *src, const void *host_scale, int sdt,
     g_cache.erase(it);
   }
   auto *cw = new CachedWeight();
-  if (int rc = pack_weight_from_host(kind, src, host_scale, sdt, signed_nibbles, K, N, groups, cw)) {
+  if (int rc = pack_weight_from_host(w.kind, w.src, w.scale, w.sdt, w.signed_nibbles, w.K, w.N, w.groups, cw)) {
     delete cw;
     return rc;
   }
@@ -208,6 +256,7 @@ int cached_weight(int kind, const void *src, const void *host_scale, int sdt,
   *out = &cw->desc;
   return B200_OK;
 }
+int cached_weight(const WeightSource &w, const b200_weight **out) { return cached_weight(w, fingerprint_of(w), out); }
 template <typename MRW, typename MRS> WeightKey key_of(const MRW *W, const MRS *S) {
   WeightKey k{};
   k.w = W->aligned + W->offset;
@@ -221,26 +270,116 @@ template <typename MRW, typename MRS> WeightKey key_of(const MRW *W, const MRS *
 // the call that uses it.
 std::mutex g_entry_mu;
 
-// y[M,N] = x[M,K] * W through the GEMV kernel, 16 activation rows at a time.
-int run_gemv_host(const b200_weight *w, const void *x_host, int x_dtype, int M,
-                  void *y_host, int y_dtype) {
+// Staging for the vectors of the per-op calls: page-locked and device buffers and a stream, kept between calls (allocating
+// and freeing them cost more than the operation), one call at a time.  Bounded: larger operands use buffers of their own.
+// b200_release_cached_weights gives it back.
+struct Stage {
+  static constexpr size_t kMost = 8 << 20;
+  int device = -1;
+  cudaStream_t stream = nullptr;
+  char *host = nullptr, *dev = nullptr;
+  size_t bytes = 0;
+  void release() {
+    if (host) cudaFreeHost(host);
+    if (dev) cudaFree(dev);
+    if (stream) cudaStreamDestroy(stream);
+    host = dev = nullptr;
+    stream = nullptr;
+    bytes = 0;
+    device = -1;
+  }
+  int reserve(size_t need) {
+    int d = 0;
+    B200_CUDA(cudaGetDevice(&d));
+    if (d == device && need <= bytes)
+      return B200_OK;
+    release();
+    const size_t n = need < (1 << 20) ? (1 << 20) : kMost;
+    if (cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaMallocHost((void **)&host, n) != cudaSuccess || cudaMalloc((void **)&dev, n) != cudaSuccess) {
+      (void)cudaGetLastError();
+      release();
+      return fail(B200_ENOMEM, "staging buffers of %zu bytes", n);
+    }
+    bytes = n;
+    device = d;
+    return B200_OK;
+  }
+};
+Stage g_stage;
+std::mutex g_stage_mu;
+
+// y[M,N] = x[M,K] * W through the GEMV kernel, 16 activation rows at a time.  `meanwhile` (optional) runs on the host while
+// the GPU works; a failure of it is returned after the GPU is done.
+template <typename F>
+int run_gemv_host(const b200_weight *w, const void *x_host, int x_dtype, int M, void *y_host, int y_dtype, F meanwhile) {
+  if (int rc = ensure_device()) return rc;
   const int64_t K = w->K, N = w->N;
   const size_t xe = x_dtype == B200_F32 ? 4 : 2, ye = y_dtype == B200_F32 ? 4 : 2;
-  DevBuf dx, dy;
-  if (int rc = dx.alloc((size_t)M * K * xe)) return rc;
-  if (int rc = dy.alloc((size_t)M * N * ye)) return rc;
-  B200_CUDA(cudaMemcpy(dx.p, x_host, (size_t)M * K * xe, cudaMemcpyHostToDevice));
+  const size_t xb = (size_t)M * K * xe, yb = (size_t)M * N * ye, xa = (xb + 255) / 256 * 256;
+  std::lock_guard<std::mutex> lock(g_stage_mu);
+  Stage *st = &g_stage;
+  DevBuf big;
+  char *dx;
+  const bool staged = xa + yb <= Stage::kMost;
+  if (int rc = st->reserve(staged ? xa + yb : 0)) return rc;
+  if (staged) {
+    dx = st->dev;
+    memcpy(st->host, x_host, xb);
+    B200_CUDA(cudaMemcpyAsync(dx, st->host, xb, cudaMemcpyHostToDevice, st->stream));
+  } else {
+    if (int rc = big.alloc(xa + yb)) return rc;
+    dx = (char *)big.p;
+    B200_CUDA(cudaMemcpyAsync(dx, x_host, xb, cudaMemcpyHostToDevice, st->stream));
+  }
+  char *dy = dx + xa;
   for (int m0 = 0; m0 < M; m0 += 16) {
     b200_gemv_args a{};
-    a.x = (const char *)dx.p + (size_t)m0 * K * xe;
+    a.x = dx + (size_t)m0 * K * xe;
     a.x_dtype = x_dtype;
-    a.y = (char *)dy.p + (size_t)m0 * N * ye;
+    a.y = dy + (size_t)m0 * N * ye;
     a.y_dtype = y_dtype;
     a.M = M - m0 < 16 ? M - m0 : 16;
-    if (int rc = b200_gemv(w, &a, nullptr)) return rc;
+    if (int rc = b200_gemv(w, &a, st->stream)) {
+      cudaStreamSynchronize(st->stream);
+      return rc;
+    }
   }
-  B200_CUDA(cudaMemcpy(y_host, dy.p, (size_t)M * N * ye, cudaMemcpyDeviceToHost));
-  return B200_OK;
+  if (staged)
+    B200_CUDA(cudaMemcpyAsync(st->host + xa, dy, yb, cudaMemcpyDeviceToHost, st->stream));
+  const int rc = meanwhile();
+  if (!staged)
+    B200_CUDA(cudaMemcpyAsync(y_host, dy, yb, cudaMemcpyDeviceToHost, st->stream));
+  B200_CUDA(cudaStreamSynchronize(st->stream));
+  if (staged && rc == B200_OK)
+    memcpy(y_host, st->host + xa, yb);
+  return rc;
+}
+int run_gemv_host(const b200_weight *w, const void *x_host, int x_dtype, int M, void *y_host, int y_dtype) {
+  return run_gemv_host(w, x_host, x_dtype, M, y_host, y_dtype, [] { return (int)B200_OK; });
+}
+
+// The same with a cached weight.  The host bytes are fingerprinted while the GPU already works with the copy found under
+// the tensor's key; a result from a copy that turns out to be stale is thrown away.
+int run_cached_gemv(const WeightSource &src, const void *x_host, int x_dtype, int M, void *y_host, int y_dtype) {
+  const CachedWeight *cand = cached_candidate(src);
+  uint64_t fp = 0;
+  if (cand) {
+    int rc = run_gemv_host(&cand->desc, x_host, x_dtype, M, y_host, y_dtype, [&] {
+      fp = fingerprint_of(src);
+      return (int)B200_OK;
+    });
+    if (rc)
+      return rc;
+    const bool fresh = fp == cand->fingerprint;
+    const b200_weight *w = nullptr;
+    if ((rc = cached_weight(src, fp, &w)) != B200_OK || fresh)   // marks the use, or repacks
+      return rc;
+    return run_gemv_host(w, x_host, x_dtype, M, y_host, y_dtype);
+  }
+  const b200_weight *w = nullptr;
+  if (int rc = cached_weight(src, &w)) return rc;
+  return run_gemv_host(w, x_host, x_dtype, M, y_host, y_dtype);
 }
 
 template <typename T> T *host_alloc(size_t n) {
@@ -263,6 +402,8 @@ void b200_release_cached_weights(void) {
     delete kv.second;
   g_cache.clear();
   g_cache_bytes = 0;
+  std::lock_guard<std::mutex> stage(g_stage_mu);
+  g_stage.release();
 }
 
 void _mlir_ciface_buddy_matmul_f32(b200_memref_f32_2 *result, b200_memref_f32_2 *A,
@@ -302,13 +443,10 @@ void _mlir_ciface_buddy_gemv_w8_f32(b200_memref_f32_2 *result, b200_memref_f32_2
   std::vector<int8_t> tw;
   const float *a = dense2<float>(A, ta), *s = dense2<float>(scale, ts);
   const int8_t *q = dense2<int8_t>(W, tw);
-  const b200_weight *w = nullptr;
   std::lock_guard<std::mutex> entry(g_entry_mu);
-  if (cached_weight(B200_W_I8, q, s, B200_F32, 1, K, N, 1, key_of(W, scale), &w))
-    return;
   float *y = host_alloc<float>((size_t)M * N);
   if (!y) return;
-  if (run_gemv_host(w, a, B200_F32, (int)M, y, B200_F32)) {
+  if (run_cached_gemv({B200_W_I8, q, s, B200_F32, 1, K, N, 1, key_of(W, scale)}, a, B200_F32, (int)M, y, B200_F32)) {
     std::free(y);
     return;
   }
@@ -329,7 +467,7 @@ void _mlir_ciface_buddy_matmul_w8a8_f32(b200_memref_f32_2 *result, b200_memref_f
   const int8_t *q = dense2<int8_t>(W, tw);
   const b200_weight *w = nullptr;
   std::lock_guard<std::mutex> entry(g_entry_mu);
-  if (cached_weight(B200_W_I8, q, s, B200_F32, 1, K, N, 1, key_of(W, scale), &w))
+  if (cached_weight({B200_W_I8, q, s, B200_F32, 1, K, N, 1, key_of(W, scale)}, &w))
     return;
   DevBuf da, dc, ws;
   const int64_t wsb = b200_gemm_w8a8_workspace_bytes((int)M, K);
@@ -364,13 +502,10 @@ void _mlir_ciface_buddy_gemv_w4_f16(b200_memref_f16_2 *result, b200_memref_f16_2
   std::vector<int8_t> tw;
   const uint16_t *a = dense2<uint16_t>(A, ta), *s = dense2<uint16_t>(scale, ts);
   const int8_t *q = dense2<int8_t>(P, tw);
-  const b200_weight *w = nullptr;
   std::lock_guard<std::mutex> entry(g_entry_mu);
-  if (cached_weight(B200_W_U4, q, s, B200_F16, 1, K, N, 1, key_of(P, scale), &w))
-    return;
   uint16_t *y = host_alloc<uint16_t>((size_t)M * N);
   if (!y) return;
-  if (run_gemv_host(w, a, B200_F16, (int)M, y, B200_F16)) {
+  if (run_cached_gemv({B200_W_U4, q, s, B200_F16, 1, K, N, 1, key_of(P, scale)}, a, B200_F16, (int)M, y, B200_F16)) {
     std::free(y);
     return;
   }
@@ -392,13 +527,10 @@ void _mlir_ciface_buddy_gemv_w4g_f32(b200_memref_f32_2 *result, b200_memref_f32_
   const float *a = dense2<float>(A, ta);
   const uint16_t *s = dense2<uint16_t>(scale, ts);
   const int8_t *q = dense2<int8_t>(P, tw);
-  const b200_weight *w = nullptr;
   std::lock_guard<std::mutex> entry(g_entry_mu);
-  if (cached_weight(B200_W_U4, q, s, B200_F16, 0, K, N, groups, key_of(P, scale), &w))
-    return;
   float *y = host_alloc<float>((size_t)M * N);
   if (!y) return;
-  if (run_gemv_host(w, a, B200_F32, (int)M, y, B200_F32)) {
+  if (run_cached_gemv({B200_W_U4, q, s, B200_F16, 0, K, N, groups, key_of(P, scale)}, a, B200_F32, (int)M, y, B200_F32)) {
     std::free(y);
     return;
   }
@@ -575,7 +707,28 @@ struct ForwardSession {
   const void *alias_w0 = nullptr;
   uint64_t alias_quick = 0;
   int valid_rows = 0;                      // rows [0, valid_rows) of shadow == device cache
-  std::vector<std::vector<float>> shadow;  // [2*layers][kv_heads*max_len*D]
+  // [2*layers][kv_heads*max_len*D]: page-locked when it can be (cache rows then move to and from the device by DMA, queued
+  // behind each other), at most kMostPinned bytes of it
+  static constexpr size_t kMostPinned = (size_t)512 << 20;
+  std::shared_ptr<float> shadow_mem;
+  size_t shadow_each = 0;
+  float *shadow(size_t b) const { return shadow_mem.get() + b * shadow_each; }
+  int make_shadow(size_t buffers, size_t each) {
+    const size_t bytes = buffers * each * 4;
+    float *p = nullptr;
+    if (bytes <= kMostPinned && cudaMallocHost((void **)&p, bytes) == cudaSuccess) {
+      shadow_mem = std::shared_ptr<float>(p, [](float *q) { cudaFreeHost(q); });
+    } else {
+      (void)cudaGetLastError();
+      p = (float *)std::malloc(bytes);
+      if (!p)
+        return fail(B200_ENOMEM, "host copy of the cache: %zu bytes", bytes);
+      shadow_mem = std::shared_ptr<float>(p, [](float *q) { std::free(q); });
+    }
+    memset(p, 0, bytes);
+    shadow_each = each;
+    return B200_OK;
+  }
   std::vector<float> rows;
   std::vector<float> logits;
   bool failed = false;
@@ -665,8 +818,11 @@ int session_for(ForwardSession &s, const b200_model_config *cfg, const char *var
   s.variant = variant;
   g_fwd_builds.fetch_add(1);
   s.rows.resize((size_t)2 * c.n_layers * c.kv_heads * c.head_dim);
-  s.shadow.assign((size_t)2 * c.n_layers,
-                  std::vector<float>((size_t)c.kv_heads * c.max_len * c.head_dim, 0.f));
+  if ((rc = s.make_shadow((size_t)2 * c.n_layers, (size_t)c.kv_heads * c.max_len * c.head_dim)) != B200_OK) {
+    b200_model_destroy(s.model);
+    s = ForwardSession();
+    return rc;
+  }
   s.valid_rows = 0;
   return B200_OK;
 }
@@ -718,6 +874,30 @@ inline bool same_row(const uint16_t *host, const float *shadow, size_t n) {
   return true;
 }
 
+// fn(b) for every cache buffer: host copies of `bytes` in all, beside the transfers they feed; shared between a few threads
+// when they would take longer than starting those.
+template <typename F> int for_buffers(int nbuf, size_t bytes, F fn) {
+  const int n = bytes < ((size_t)4 << 20) ? 1 : 4;
+  std::atomic<int> next{0}, status{B200_OK};
+  int dev = 0;
+  B200_CUDA(cudaGetDevice(&dev));
+  auto work = [&] {
+    for (int b; (b = next.fetch_add(1)) < nbuf && status.load() == B200_OK;)
+      if (const int rc = fn(b))
+        status.store(rc);
+  };
+  std::vector<std::thread> helpers;
+  for (int i = 1; i < n; ++i)
+    helpers.emplace_back([&] {
+      if (cudaSetDevice(dev) == cudaSuccess)
+        work();
+    });
+  work();
+  for (auto &t : helpers)
+    t.join();
+  return status.load() == B200_OK ? B200_OK : fail(status.load(), "copying the cache between host and device failed");
+}
+
 // Does the host cache still hold, in rows [0, pos), what the device cache holds?
 // Row pos-1 of every buffer depends on every earlier token of the sequence, row
 // 0 and the middle row catch a rewritten or shifted cache
@@ -734,10 +914,10 @@ bool host_matches_device(const ForwardSession &s, const b200_model_config *cfg,
     return true;
   const size_t D = cfg->head_dim, KH = cfg->kv_heads, L = cfg->max_len;
   const long long probe[3] = {0, (pos - 1) / 2, pos - 1};
-  for (size_t b = 0; b < s.shadow.size(); ++b)
+  for (size_t b = 0; b < (size_t)2 * cfg->n_layers; ++b)
     for (size_t h = 0; h < KH; ++h)
       for (long long r : probe)
-        if (!same_row(host_kv[b] + (h * HL + (size_t)r) * D, s.shadow[b].data() + (h * L + (size_t)r) * D, D))
+        if (!same_row(host_kv[b] + (h * HL + (size_t)r) * D, s.shadow((size_t)b) + (h * L + (size_t)r) * D, D))
           return false;
   return true;
 }
@@ -761,10 +941,15 @@ int forward_decode(const b200_model_config *cfg, const char *variant, int all_li
   if (!host_matches_device(s, cfg, host_kv, pos, HL)) {
     // hand-off from the host (CPU prefill, another sequence, a shifted cache):
     // everything before `pos` comes from host_kv
-    for (int b = 0; b < nbuf; ++b) {
+    const int rc = for_buffers(nbuf, (size_t)pos * D * KH * nbuf * sizeof(T), [&](int b) {
       for (size_t h = 0; h < KH; ++h)
-        from_host(s.shadow[b].data() + h * L * D, host_kv[b] + h * HL * D, (size_t)pos * D);
-      if (int rc = b200_model_kv_upload(s.model, b, s.shadow[b].data(), 0, (int)pos)) return rc;
+        from_host(s.shadow((size_t)b) + h * L * D, host_kv[b] + h * HL * D, (size_t)pos * D);
+      return model_kv_upload_async(s.model, b, s.shadow((size_t)b), 0, (int)pos);
+    });
+    if (rc) {
+      s.valid_rows = 0;
+      model_synchronize(s.model);
+      return rc;
     }
     s.valid_rows = (int)pos;
   }
@@ -789,7 +974,7 @@ int forward_decode(const b200_model_config *cfg, const char *variant, int all_li
     for (size_t h = 0; h < KH; ++h) {
       const float *row = &s.rows[((size_t)b * KH + h) * D];
       to_host(host_kv[b] + (h * HL + (size_t)pos) * D, row, D);
-      memcpy(s.shadow[b].data() + (h * L + (size_t)pos) * D, row, D * 4);
+      memcpy(s.shadow((size_t)b) + (h * L + (size_t)pos) * D, row, D * 4);
     }
   if (s.valid_rows < pos + 1)
     s.valid_rows = (int)pos + 1;
@@ -843,14 +1028,18 @@ int forward_prefill(const b200_model_config *cfg, const char *variant, int all_l
       to_host(logits_out, lf.data(), lf.size());
     }
   }
-  for (int b = 0; b < nbuf; ++b) {
-    if (int rc = b200_model_kv_download(s.model, b, s.shadow[b].data(), 0, n_rows)) return rc;
-    for (size_t h = 0; h < KH; ++h) {
-      to_host(host_kv_out[b] + h * HL * D, s.shadow[b].data() + h * L * D, (size_t)n_rows * D);
-      if ((size_t)n_rows < HL)   // rows the prefill did not reach read as zero
-        memset(host_kv_out[b] + (h * HL + (size_t)n_rows) * D, 0, (HL - (size_t)n_rows) * D * sizeof(T));
-    }
-  }
+  for (int b = 0; b < nbuf; ++b)
+    if (int rc = model_kv_download_async(s.model, b, s.shadow((size_t)b), 0, n_rows)) return rc;
+  if (int rc = model_synchronize(s.model)) return rc;
+  if (int rc = for_buffers(nbuf, HL * D * KH * nbuf * sizeof(T), [&](int b) {
+        for (size_t h = 0; h < KH; ++h) {
+          to_host(host_kv_out[b] + h * HL * D, s.shadow((size_t)b) + h * L * D, (size_t)n_rows * D);
+          if ((size_t)n_rows < HL)   // rows the prefill did not reach read as zero
+            memset(host_kv_out[b] + (h * HL + (size_t)n_rows) * D, 0, (HL - (size_t)n_rows) * D * sizeof(T));
+        }
+        return (int)B200_OK;
+      }))
+    return rc;
   s.valid_rows = n_rows;
   return B200_OK;
 }

@@ -62,15 +62,36 @@ def from_result(m, dtype):
     return out
 
 
+_fns = {}
+
+
+def _descriptor(a):
+    """The bytes of a's descriptor (every field of a MemRef is 64 bits wide): what to_memref fills, without a
+    structure class per (type, rank)."""
+    if a.dtype not in _CT:
+        raise KeyError(a.dtype)
+    p, size = a.__array_interface__["data"][0], a.itemsize
+    return (C.c_int64 * (3 + 2 * a.ndim))(p, p, 0, *a.shape, *[s // size for s in a.strides])
+
+
 def _call(name, result_dtype, result_rank, *arrays):
-    lib = _lib.load()
-    fn = getattr(lib, name)
-    res = memref_type(result_dtype, result_rank)()
-    descs = [to_memref(a) for a in arrays]
-    fn.restype = None
-    fn.argtypes = [C.c_void_p] * (1 + len(descs))
+    fn = _fns.get(name)
+    if fn is None:
+        fn = getattr(_lib.load(), name)
+        fn.restype = None
+        fn.argtypes = [C.c_void_p] * (1 + len(arrays))
+        _fns[name] = fn
+    res = (C.c_int64 * (3 + 2 * result_rank))()
+    descs = [_descriptor(a) for a in arrays]
     fn(C.byref(res), *[C.byref(d) for d in descs])
-    return from_result(res, result_dtype)
+    allocated, aligned, offset = res[0], res[1], res[2]
+    if not aligned:
+        raise _lib.B200Error(_lib.load().b200_last_error().decode())
+    # copy the result out and free it, as the generated code does when it destroys the descriptor
+    out = np.empty(tuple(res[3:3 + result_rank]), dtype=result_dtype)
+    C.memmove(out.__array_interface__["data"][0], aligned + offset * out.itemsize, out.nbytes)
+    _libc.free(allocated)
+    return out
 
 
 def buddy_matmul_f32(A, B):
