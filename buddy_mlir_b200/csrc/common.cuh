@@ -152,10 +152,15 @@ int gqa_paged_launch(const float *qkv, int64_t ld, const float *k_pool, const fl
                      int q_heads, int kv_heads, int D, int page, const int32_t *row_seq, const int32_t *row_pos,
                      const int32_t *block_table, int table_stride, int M, float *scratch, int scratch_rows,
                      int max_context, cudaStream_t st);
-int gqa_paged_prefill_launch(const float *qkv, int64_t ld, const float *k_pool, const float *v_pool, float *out,
-                             int64_t ldo, int q_heads, int kv_heads, int D, int page, const int32_t *seq_table,
-                             int pos0, int M, int max_context, cudaStream_t st);
 int64_t gqa_paged_scratch_floats(int rows, int q_heads, int D, int max_context);
+// prefill_attn.cu: causal attention of M rows at positions pos0, pos0 + 1, .. of one sequence on the tensor cores.  kc / vc:
+// the contiguous cache [kv_heads][max_len][D] (table null), or page pools [pages][kv_heads][page][D] and the sequence's row
+// of the block table.  error: a device word that takes the code of a wait that gave up.
+bool prefill_attn_takes(const float *qkv, int64_t ld, const float *kc, const float *vc, const float *out, int64_t ldo, int D, int M);
+int64_t prefill_attn_workspace_bytes(int n_keys, int kv_heads, int D);
+int prefill_attn_launch(const float *qkv, int64_t ld, const float *kc, const float *vc, float *out, int64_t ldo, int q_heads,
+                        int kv_heads, int D, int max_len, int pos0, int M, const int32_t *table, int page, void *workspace,
+                        int64_t workspace_bytes, int *error, cudaStream_t st);
 // gemm_tc.cu: b200_gemm_w8a8 with the residual sum or the SiLU pair folded into the store
 int gemm_w8a8_fused(const b200_weight *w, const float *A, int M, int64_t lda, float *C, int64_t ldc,
                     const float *residual, int64_t ldr, int silu_pairs, void *workspace, int64_t workspace_bytes,

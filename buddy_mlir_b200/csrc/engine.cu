@@ -321,6 +321,8 @@ struct b200_model {
   cudaGraphExec_t exec_q = nullptr;
   int kernels_per_step_q = 0;
   void *pf_ws = nullptr;
+  void *pf_kv = nullptr;                // head (error word), then the attention's K and V images
+  int64_t pf_kv_bytes = 0;              // without the head
   int32_t *pf_tokens = nullptr;
   int pf_rows = 0, pf_logit_rows = 0;
   int64_t pf_ws_bytes = 0;
@@ -875,7 +877,7 @@ int b200_model_create(const b200_model_config *cfg, b200_model **out) {
   if (rc == B200_OK && (cudaMallocHost((void **)&m->h_logits_pinned, (size_t)c.vocab * 4) != cudaSuccess ||
                         cudaMallocHost((void **)&m->h_rows_pinned,
                                        (size_t)2 * c.n_layers * m->kvh * D * 4) != cudaSuccess ||
-                        cudaMallocHost((void **)&m->h_state_pinned, 32) != cudaSuccess))
+                        cudaMallocHost((void **)&m->h_state_pinned, 64) != cudaSuccess))
     rc = fail(B200_ENOMEM, "pinned host allocation failed");
   if (rc != B200_OK) {
     b200_model_destroy(m);
@@ -909,7 +911,7 @@ void b200_model_destroy(b200_model *m) {
   cudaFree(m->dec_stream); cudaFree(m->dec_offsets); cudaFree(m->dec_layers);
   cudaFree(m->ll_buf); cudaFree(m->d_trace);
   cudaFree(m->pf_x); cudaFree(m->pf_qkv); cudaFree(m->pf_att); cudaFree(m->pf_mid); cudaFree(m->pf_logits);
-  cudaFree(m->pf_ws); cudaFree(m->pf_tokens); cudaFree(m->pf_norm);
+  cudaFree(m->pf_ws); cudaFree(m->pf_tokens); cudaFree(m->pf_norm); cudaFree(m->pf_kv);
   cudaFree(m->q_row); cudaFree(m->q_scale);
   if (m->exec_q) cudaGraphExecDestroy(m->exec_q);
   if (m->graph_q) cudaGraphDestroy(m->graph_q);
@@ -1795,6 +1797,45 @@ static int prefill_reserve(b200_model *m, int rows, int logit_rows) {
   return B200_OK;
 }
 
+constexpr int64_t kPrefillKvHead = 1024;
+// Attention of M rows of one sequence at positions pos0 .. over the contiguous cache (table null) or over pages.
+static int prefill_attention(b200_model *m, const float *kc, const float *vc, int max_len, int pos0, int M, const int32_t *table,
+                             int page) {
+  const int D = m->cfg.head_dim;
+  const int64_t QD = (int64_t)m->qh * D, QKV = QD + 2 * (int64_t)m->kvh * D;
+  return prefill_attn_launch(m->pf_qkv, QKV, kc, vc, m->pf_att, QD, m->qh, m->kvh, D, max_len, pos0, M, table, page,
+                             (uint8_t *)m->pf_kv + kPrefillKvHead, m->pf_kv_bytes, (int *)m->pf_kv, m->stream);
+}
+// Images for n_keys of limit keys; room for twice as many, so that a growing sequence comes here rarely.
+static int prefill_attention_reserve(b200_model *m, int n_keys, int limit) {
+  if (m->pf_kv && prefill_attn_workspace_bytes(n_keys, m->kvh, m->cfg.head_dim) <= m->pf_kv_bytes)
+    return B200_OK;
+  cudaFree(m->pf_kv);
+  m->pf_kv = nullptr;
+  m->pf_kv_bytes = 0;
+  const int64_t bytes = prefill_attn_workspace_bytes((int)std::min<int64_t>(limit, 2 * (int64_t)n_keys), m->kvh, m->cfg.head_dim);
+  if (int rc = dev_alloc(&m->pf_kv, (size_t)(bytes + kPrefillKvHead))) return rc;
+  B200_CUDA(cudaMemsetAsync(m->pf_kv, 0, kPrefillKvHead, m->stream));
+  m->pf_kv_bytes = bytes;
+  return B200_OK;
+}
+// Queue the error words of a pass's GEMMs and attention behind it; after the stream is synchronised, rows_status reads them.
+static int rows_status_queue(b200_model *m) {
+  m->h_state_pinned[8] = m->h_state_pinned[9] = 0;
+  B200_CUDA(cudaMemcpyAsync(m->h_state_pinned + 8, m->pf_ws, 4, cudaMemcpyDeviceToHost, m->stream));
+  if (m->pf_kv)
+    B200_CUDA(cudaMemcpyAsync(m->h_state_pinned + 9, m->pf_kv, 4, cudaMemcpyDeviceToHost, m->stream));
+  return B200_OK;
+}
+static int rows_status(b200_model *m) {
+  const int gemm = m->h_state_pinned[8], attn = m->h_state_pinned[9];
+  if (attn)
+    cudaMemsetAsync(m->pf_kv, 0, 4, m->stream);
+  if (gemm || attn)
+    return fail(B200_ECUDA, "prefill: a bounded wait gave up (code %d)", gemm ? gemm : attn);
+  return B200_OK;
+}
+
 int b200_model_prefill(b200_model *m, const int32_t *tokens, int n_tokens, int pos0, float *logits_host,
                        int all_rows, int *next_token) {
   if (!m || !tokens)
@@ -1814,6 +1855,9 @@ int b200_model_prefill(b200_model *m, const int32_t *tokens, int n_tokens, int p
   // w8a8: the activation scale of the last projection belongs to all rows, so all of them are computed
   const int logit_rows = ((all_rows && logits_host) || m->act_int8) ? M : 1;
   if (int rc = prefill_reserve(m, M, logit_rows)) return rc;
+  const bool tiled = prefill_attn_takes(m->pf_qkv, QKV, m->kv[0], m->kv[1], m->pf_att, QD, D, M);
+  if (tiled)
+    if (int rc = prefill_attention_reserve(m, pos0 + M, c.max_len)) return rc;
   cudaStream_t st = m->stream;
   B200_CUDA(cudaEventRecord(m->ev0, st));
   B200_CUDA(cudaMemcpyAsync(m->pf_tokens, tokens, (size_t)M * 4, cudaMemcpyHostToDevice, st));
@@ -1825,8 +1869,9 @@ int b200_model_prefill(b200_model *m, const int32_t *tokens, int n_tokens, int p
     if (int rc = rope_kv_rows_launch(m->pf_qkv, QKV, m->kv[2 * l], m->kv[2 * l + 1], m->inv_freq, L.q_norm,
                                      L.k_norm, c.eps, m->qh, m->kvh, D, c.max_len, pos0, M, st))
       return rc;
-    if (int rc = gqa_prefill_launch(m->pf_qkv, QKV, m->kv[2 * l], m->kv[2 * l + 1], m->pf_att, QD, m->qh,
-                                    m->kvh, D, c.max_len, pos0, M, st))
+    if (int rc = tiled ? prefill_attention(m, m->kv[2 * l], m->kv[2 * l + 1], c.max_len, pos0, M, nullptr, 0)
+                       : gqa_prefill_launch(m->pf_qkv, QKV, m->kv[2 * l], m->kv[2 * l + 1], m->pf_att, QD, m->qh, m->kvh, D,
+                                            c.max_len, pos0, M, st))
       return rc;
     // x1 = x + attn @ Wo ; mid = silu(gate) * up <- RMSNorm(x1) ; x2 = x1 + mid @ Wdown
     if (int rc = linear_rows(m, L.o, m->pf_att, QD, M, m->pf_x, H, m->pf_x, nullptr, false)) return rc;
@@ -1850,10 +1895,11 @@ int b200_model_prefill(b200_model *m, const int32_t *tokens, int n_tokens, int p
   else if (logits_host)
     B200_CUDA(cudaMemcpyAsync(logits_host, last_logits, (size_t)c.vocab * 4, cudaMemcpyDeviceToHost, st));
   B200_CUDA(cudaMemcpyAsync(m->h_state_pinned, m->d_state, 32, cudaMemcpyDeviceToHost, st));
+  if (int rc = rows_status_queue(m)) return rc;
   B200_CUDA(cudaStreamSynchronize(st));
   B200_CUDA(cudaEventElapsedTime(&m->last_ms, m->ev0, m->ev1));
   m->rows_fresh = false;
-  if (int rc = b200_gemm_w8_status(m->pf_ws, st)) return rc;
+  if (int rc = rows_status(m)) return rc;
   if (next_token)
     *next_token = m->h_state_pinned[2];
   return B200_OK;
@@ -1896,14 +1942,17 @@ static int batch_rows(b200_batch *b, int M, const int32_t *tokens, const int32_t
     if (int rc = dev_alloc((void **)&b->d_next, (size_t)M * 4)) return rc;
     b->rows_cap = M;
   }
+  // a prefill chunk: consecutive positions of one sequence
+  bool one_chunk = prefill_attn_takes(m->pf_qkv, QKV, b->pool[0], b->pool[1], m->pf_att, QD, D, M);
+  for (int r = 1; r < M && one_chunk; ++r)
+    one_chunk = row_seq[r] == row_seq[0] && row_pos[r] == row_pos[0] + r;
+  if (one_chunk)
+    if (int rc = prefill_attention_reserve(m, row_pos[0] + M, b->max_context)) return rc;
   B200_CUDA(cudaEventRecord(m->ev0, st));
   B200_CUDA(cudaMemcpyAsync(m->pf_tokens, tokens, (size_t)M * 4, cudaMemcpyHostToDevice, st));
   B200_CUDA(cudaMemcpyAsync(b->d_seq, row_seq, (size_t)M * 4, cudaMemcpyHostToDevice, st));
   B200_CUDA(cudaMemcpyAsync(b->d_pos, row_pos, (size_t)M * 4, cudaMemcpyHostToDevice, st));
   B200_CUDA(cudaMemcpyAsync(b->d_table, b->table.data(), b->table.size() * 4, cudaMemcpyHostToDevice, st));
-  bool one_chunk = M >= 64;
-  for (int r = 1; r < M && one_chunk; ++r)
-    one_chunk = row_seq[r] == row_seq[0] && row_pos[r] == row_pos[0] + r;
   if (int rc = embed_rows_launch(m->embed, m->pf_tokens, m->pf_x, H, M, st)) return rc;
   for (int l = 0; l < c.n_layers; ++l) {
     Layer &L = m->layers[l];
@@ -1912,17 +1961,13 @@ static int batch_rows(b200_batch *b, int M, const int32_t *tokens, const int32_t
                                       L.k_norm, c.eps, m->qh, m->kvh, D, b->page, b->d_seq, b->d_pos, b->d_table,
                                       b->table_stride, M, st))
       return rc;
-    int arc = B200_ESTATE;
-    if (one_chunk)   // a prefill chunk: consecutive positions of one sequence
-      arc = gqa_paged_prefill_launch(m->pf_qkv, QKV, b->pool[2 * l], b->pool[2 * l + 1], m->pf_att, QD, m->qh, m->kvh,
-                                     D, b->page, b->d_table + (size_t)row_seq[0] * b->table_stride, row_pos[0], M,
-                                     b->max_context, st);
-    if (arc == B200_ESTATE)
-      arc = gqa_paged_launch(m->pf_qkv, QKV, b->pool[2 * l], b->pool[2 * l + 1], m->pf_att, QD, m->qh, m->kvh, D,
-                             b->page, b->d_seq, b->d_pos, b->d_table, b->table_stride, M, b->d_part, b->part_rows,
-                             b->max_context, st);
-    if (arc)
-      return arc;
+    if (int rc = one_chunk
+                     ? prefill_attention(m, b->pool[2 * l], b->pool[2 * l + 1], b->max_context, row_pos[0], M,
+                                         b->d_table + (size_t)row_seq[0] * b->table_stride, b->page)
+                     : gqa_paged_launch(m->pf_qkv, QKV, b->pool[2 * l], b->pool[2 * l + 1], m->pf_att, QD, m->qh, m->kvh, D,
+                                        b->page, b->d_seq, b->d_pos, b->d_table, b->table_stride, M, b->d_part, b->part_rows,
+                                        b->max_context, st))
+      return rc;
     if (int rc = linear_rows(m, L.o, m->pf_att, QD, M, m->pf_x, H, m->pf_x, nullptr, false)) return rc;
     if (int rc = linear_rows(m, L.gateup, m->pf_x, H, M, m->pf_mid, m->ffn, nullptr, L.post_norm, true)) return rc;
     if (int rc = linear_rows(m, L.down, m->pf_mid, m->ffn, M, m->pf_x, H, m->pf_x, nullptr, false)) return rc;
@@ -1937,9 +1982,10 @@ static int batch_rows(b200_batch *b, int M, const int32_t *tokens, const int32_t
     B200_CUDA(cudaMemcpyAsync(logits_host, m->pf_logits, (size_t)logit_rows * c.vocab * 4, cudaMemcpyDeviceToHost, st));
   if (next_host)
     B200_CUDA(cudaMemcpyAsync(next_host, b->d_next, (size_t)logit_rows * 4, cudaMemcpyDeviceToHost, st));
+  if (int rc = rows_status_queue(m)) return rc;
   B200_CUDA(cudaStreamSynchronize(st));
   B200_CUDA(cudaEventElapsedTime(&b->last_ms, m->ev0, m->ev1));
-  return b200_gemm_w8_status(m->pf_ws, st);
+  return rows_status(m);
 }
 
 // pages for positions [len, len + n) of a sequence

@@ -33,6 +33,7 @@
 // call fails.
 #include "common.cuh"
 #include "gemv_mma.cuh"
+#include "tensor_core.cuh"
 
 #include <cuda.h>
 
@@ -51,8 +52,6 @@ constexpr int kEpiWarps = 8;
 constexpr int kMaxStages = 3;
 constexpr int kMaxPartialTiles = 320;          // split-K: shares of tiles in the workspace
 constexpr int kHeadBytes = 2048;               // workspace head: error word, scales of W8A8, arrival counters
-constexpr uint32_t kSpin = 1u << 26;
-constexpr unsigned long long kWaitNs = 2000000000ull;
 
 template <int BN> struct Ring {
   static constexpr uint32_t A_BYTES = BM * BK, W_BYTES = BN * BK, STAGE_BYTES = A_BYTES + W_BYTES;
@@ -69,55 +68,11 @@ struct Bars {
   int last;                    // split-K: this CTA completes its tile
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ unsigned long long now_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(uint64_t *bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-               : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-  return ok != 0;
-}
-// Bounded wait; false when it gave up or the CTA already failed.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *ab, int *err, int code) {
-  unsigned long long t0 = 0;
-  for (uint32_t it = 0; it < kSpin; ++it) {
-    if (mbar_try(bar, parity))
-      return !*ab;
-    if ((it & 0x3FF) == 0x3FF) {
-      if (*ab)
-        return false;
-      const unsigned long long t = now_ns();
-      if (t0 == 0)
-        t0 = t;
-      else if (t - t0 > kWaitNs)
-        break;
-    }
-  }
-  atomicCAS(err, 0, code);
-  *ab = 1;
-  return false;
-}
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y)
       : "memory");
-}
-// K-major operand tile in shared memory, rows of 128 bytes, 128-byte swizzle: start address / 16, leading byte offset
-// (unused for swizzled K-major: 1), stride byte offset = 8 rows, descriptor version 1, layout 2.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
-  return (uint64_t)((addr & 0x3FFFFu) >> 4) | (uint64_t)1 << 16 | (uint64_t)((8 * BK) >> 4) << 32 | (uint64_t)1 << 46 |
-         (uint64_t)2 << 61;
 }
 // kind::i8 instruction descriptor: D = s32, A = B = s8, both K-major, M = 128.
 template <int BN>
@@ -129,10 +84,6 @@ __device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t da, uint64_t db
       ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ void tc_commit(uint64_t *bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
 struct GemmParams {
   int M, N, K;                 // K: multiple of 64
   const float *scale, *bias;   // [N], bias may be null
@@ -233,7 +184,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // ---- epilogue ----------------------------------------------------------------------------------------------------
     // A thread reads an accumulator row (its lane of tensor memory) and half of its columns; the sums go to a padded tile in
     // shared memory (the ring is idle by then), from where the warps add up the planes and write whole rows.
-    const bool ok = mbar_wait(&bars.accum, 0, ab, p.error, 703);
+    const bool ok = mbar_wait(&bars.accum, 0, ab, p.error, 703) && !*ab;
     asm volatile("griddepcontrol.wait;" ::: "memory");   // row scales, counters (long complete: the operand was loaded)
     constexpr int LDS = 128 + 4;                      // row stride of the staging tile, in words
     float *ep = reinterpret_cast<float *>(tiles);     // [BM][LDS]: 66 KB of the ring
@@ -255,17 +206,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         for (int cb = cb0; cb < cb0 + 64; cb += 32) {
           uint32_t v[32];
           const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(h * 128 + cb);
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-              "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-              "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-              : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-                "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-                "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-              : "r"(taddr)
-              : "memory");
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          tmem_load32(taddr, v);
+          tmem_wait_load();
           float *erow = ep + row * LDS + cb;
 #pragma unroll
           for (int j = 0; j < 32; j += 4) {
@@ -612,24 +554,6 @@ int make_map(CUtensorMap *map, CUtensorMapDataType dt, int bk, void *base, uint6
                          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (rc != CUDA_SUCCESS)
     return fail(B200_ECUDA, "gemm_w8: cuTensorMapEncodeTiled failed (%d)", (int)rc);
-  return B200_OK;
-}
-
-// Launch behind the kernel before it with its start overlapping that kernel's end (it waits where it needs its results).
-template <typename... P, typename... A>
-int launch_after(void (*kern)(P...), dim3 grid, int threads, int smem, cudaStream_t st, A... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  B200_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
-  count_launch();
   return B200_OK;
 }
 

@@ -172,241 +172,6 @@ gqa_prefill_kernel(const float *qkv, int64_t ld, const float *kc, const float *v
   }
 }
 
-// Causal attention tiled over query rows (flash style, f32 on the CUDA cores).
-// A CTA takes BQ consecutive query rows of one kv head: R = BQ * G query vectors
-// (row r = query row r / G, head hk * G + r % G) against tiles of 64 keys staged in
-// shared memory, so a K/V row is read once per BQ query rows instead of once per
-// row.  512 threads as 32 x 16: thread (ty, tx) owns query vectors 4ty..4ty+3; for
-// the scores it owns keys tx, tx + 16, tx + 32, tx + 48 of the tile (rows of the K
-// tile 16 apart: no bank conflicts), for the output the float4 column
-// chunks tx + 16i.  Per key tile: S = Q K^T (register tile 4 x 4 over D), running
-// max / sum per row across the 16 threads of a row (tosa.py:14245-14252, one update
-// per tile instead of per key), P to shared memory, O += P V (register tile
-// 4 x D/16).  The next K/V tile is fetched into registers while the current one
-// is used.
-template <int G, int D>
-struct PrefillTile {
-  static constexpr int BQ = G >= 6 ? 16 : (G >= 3 ? 32 : 64);
-  static constexpr int R = BQ * G;           // <= 128
-  static constexpr int KT = 64;              // keys per tile
-  static constexpr int LDQ = D + 4, LDK = D + 4, LDP = KT + 4;
-  static constexpr size_t smem_bytes = ((size_t)R * LDQ + (size_t)KT * LDK + (size_t)KT * D + (size_t)R * LDP) * 4;
-};
-
-// PAGED: kc / vc are page pools [n_pages][kv_heads][page][D] and `table` lists the
-// pages of the one sequence all M rows belong to (positions pos0, pos0 + 1, ..).
-template <int G, int D, bool PAGED>
-__global__ void __launch_bounds__(512, 1)
-gqa_prefill_tiled_kernel(const float *qkv, int64_t ld, const float *kc, const float *vc, float *out, int64_t ldo,
-                         int max_len, int pos0, int M, const int32_t *table, int page, int kv_heads) {
-  using T = PrefillTile<G, D>;
-  constexpr int R = T::R, KT = T::KT, LDQ = T::LDQ, LDK = T::LDK, LDP = T::LDP, NCH = D / 64;
-  extern __shared__ __align__(16) float sm[];
-  float *Qs = sm, *Ks = Qs + R * LDQ, *Vs = Ks + KT * LDK, *Ps = Vs + KT * D;
-  // heavy tiles (late rows, long histories) first
-  const int qt = gridDim.x - 1 - blockIdx.x, hk = blockIdx.y;
-  const int m0 = qt * T::BQ;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const bool row_thread = 4 * ty < R;
-  const float scale = rsqrtf((float)D);
-  // keys this tile needs: up to the position of its last live row
-  const int last_m = min(m0 + T::BQ, M) - 1;
-  const int n_keys = min(pos0 + last_m, max_len - 1) + 1;
-  const float *kbase = PAGED ? kc : kc + (int64_t)hk * max_len * D;
-  const float *vbase = PAGED ? vc : vc + (int64_t)hk * max_len * D;
-
-  // ---- stage Q: row r = (query row r / G, head r % G), G heads of a row are contiguous ----
-  for (int idx = tid; idx < R * (D / 4); idx += 512) {
-    const int r = idx / (D / 4), c = idx - r * (D / 4);
-    const int m = m0 + r / G;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (m < M)
-      v = *reinterpret_cast<const float4 *>(qkv + (int64_t)m * ld + (int64_t)(hk * G + r % G) * D + 4 * c);
-    *reinterpret_cast<float4 *>(Qs + r * LDQ + 4 * c) = v;
-  }
-  // per-thread K/V fetch slots: KT * D / 4 float4 per tile over 512 threads
-  constexpr int NF = KT * (D / 4) / 512;   // 4 (D = 128) or 2 (D = 64)
-  float4 kf[NF], vf[NF];
-  auto fetch = [&](int k0) {
-#pragma unroll
-    for (int i = 0; i < NF; ++i) {
-      const int idx = tid + 512 * i;
-      const int j = idx / (D / 4), c = idx - j * (D / 4);
-      if (k0 + j < n_keys) {
-        const int key = k0 + j;
-        const int64_t roff = PAGED ? (((int64_t)table[key / page] * kv_heads + hk) * page + key % page) * D
-                                   : (int64_t)key * D;
-        kf[i] = __ldg(reinterpret_cast<const float4 *>(kbase + roff + 4 * c));
-        vf[i] = __ldg(reinterpret_cast<const float4 *>(vbase + roff + 4 * c));
-      } else {
-        kf[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        vf[i] = kf[i];
-      }
-    }
-  };
-  auto stash = [&]() {
-#pragma unroll
-    for (int i = 0; i < NF; ++i) {
-      const int idx = tid + 512 * i;
-      const int j = idx / (D / 4), c = idx - j * (D / 4);
-      *reinterpret_cast<float4 *>(Ks + j * LDK + 4 * c) = kf[i];
-      *reinterpret_cast<float4 *>(Vs + j * D + 4 * c) = vf[i];
-    }
-  };
-
-  float mrow[4], lrow[4], acc[4][NCH * 4];
-  int qpos[4];
-#pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    mrow[a] = kSeed;
-    lrow[a] = 0.f;
-    const int m = m0 + (4 * ty + a) / G;
-    qpos[a] = (row_thread && m < M) ? min(pos0 + m, max_len - 1) : -1;   // -1: every key is masked
-#pragma unroll
-    for (int c = 0; c < NCH * 4; ++c)
-      acc[a][c] = 0.f;
-  }
-
-  fetch(0);
-  for (int k0 = 0; k0 < n_keys; k0 += KT) {
-    __syncthreads();            // the previous tile is no longer read (and Q is staged)
-    stash();
-    __syncthreads();
-    if (k0 + KT < n_keys)
-      fetch(k0 + KT);
-    if (row_thread) {
-      // ---- S = Q K^T for rows 4ty.., keys tx + 16b ------------------------------------
-      float sc[4][4];
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b)
-          sc[a][b] = 0.f;
-      const float *qp = Qs + (4 * ty) * LDQ, *kp = Ks + tx * LDK;
-#pragma unroll 4
-      for (int d = 0; d < D; d += 4) {
-        float4 q4[4], k4[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-          q4[a] = *reinterpret_cast<const float4 *>(qp + a * LDQ + d);
-#pragma unroll
-        for (int b = 0; b < 4; ++b)
-          k4[b] = *reinterpret_cast<const float4 *>(kp + b * 16 * LDK + d);
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b) {
-            sc[a][b] = fmaf(q4[a].x, k4[b].x, sc[a][b]);
-            sc[a][b] = fmaf(q4[a].y, k4[b].y, sc[a][b]);
-            sc[a][b] = fmaf(q4[a].z, k4[b].z, sc[a][b]);
-            sc[a][b] = fmaf(q4[a].w, k4[b].w, sc[a][b]);
-          }
-      }
-      // ---- running softmax per row: the 16 threads tx = 0..15 of a row hold its 64 scores ----
-#pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        float tm = kSeed;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const int key = k0 + 16 * b + tx;
-          sc[a][b] = key <= qpos[a] ? sc[a][b] * scale : kSeed;
-          tm = fmaxf(tm, sc[a][b]);
-        }
-        tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 1));
-        tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 2));
-        tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 4));
-        tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 8));
-        const float nm = fmaxf(mrow[a], tm);
-        const float alpha = expf(mrow[a] - nm);
-        float ps = 0.f;
-        float pw[4];
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const int key = k0 + 16 * b + tx;
-          pw[b] = key <= qpos[a] ? expf(sc[a][b] - nm) : 0.f;
-          ps += pw[b];
-        }
-        ps += __shfl_xor_sync(0xffffffffu, ps, 1);
-        ps += __shfl_xor_sync(0xffffffffu, ps, 2);
-        ps += __shfl_xor_sync(0xffffffffu, ps, 4);
-        ps += __shfl_xor_sync(0xffffffffu, ps, 8);
-        lrow[a] = fmaf(lrow[a], alpha, ps);
-        mrow[a] = nm;
-#pragma unroll
-        for (int c = 0; c < NCH * 4; ++c)
-          acc[a][c] *= alpha;
-#pragma unroll
-        for (int b = 0; b < 4; ++b)
-          Ps[(4 * ty + a) * LDP + 16 * b + tx] = pw[b];
-      }
-    }
-    // the 16 threads of a row sit in one warp: P of a row is complete after a warp sync
-    __syncwarp();
-    if (row_thread) {
-      // ---- O += P V for rows 4ty.., column chunks tx + 16i ----------------------------
-      const float *pp = Ps + (4 * ty) * LDP;
-#pragma unroll 2
-      for (int j = 0; j < KT; j += 4) {
-        float4 p4[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-          p4[a] = *reinterpret_cast<const float4 *>(pp + a * LDP + j);
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-#pragma unroll
-          for (int i = 0; i < NCH; ++i) {
-            const float4 v4 = *reinterpret_cast<const float4 *>(Vs + (j + jj) * D + 4 * (tx + 16 * i));
-#pragma unroll
-            for (int a = 0; a < 4; ++a) {
-              const float pv = jj == 0 ? p4[a].x : jj == 1 ? p4[a].y : jj == 2 ? p4[a].z : p4[a].w;
-              acc[a][4 * i + 0] = fmaf(pv, v4.x, acc[a][4 * i + 0]);
-              acc[a][4 * i + 1] = fmaf(pv, v4.y, acc[a][4 * i + 1]);
-              acc[a][4 * i + 2] = fmaf(pv, v4.z, acc[a][4 * i + 2]);
-              acc[a][4 * i + 3] = fmaf(pv, v4.w, acc[a][4 * i + 3]);
-            }
-          }
-        }
-      }
-    }
-  }
-  if (row_thread) {
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const int r = 4 * ty + a;
-      const int m = m0 + r / G;
-      if (m < M) {
-        float *orow = out + (int64_t)m * ldo + (int64_t)(hk * G + r % G) * D;
-#pragma unroll
-        for (int i = 0; i < NCH; ++i)
-          *reinterpret_cast<float4 *>(orow + 4 * (tx + 16 * i)) =
-              make_float4(__fdiv_rn(acc[a][4 * i], lrow[a]), __fdiv_rn(acc[a][4 * i + 1], lrow[a]),
-                          __fdiv_rn(acc[a][4 * i + 2], lrow[a]), __fdiv_rn(acc[a][4 * i + 3], lrow[a]));
-      }
-    }
-  }
-}
-
-template <int G, int D, bool PAGED>
-int launch_prefill_tiled(const float *qkv, int64_t ld, const float *kc, const float *vc, float *out, int64_t ldo,
-                         int kv_heads, int max_len, int pos0, int M, const int32_t *table, int page,
-                         cudaStream_t st) {
-  using T = PrefillTile<G, D>;
-  static bool configured[64] = {};
-  int dev = 0;
-  B200_CUDA(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64 || !configured[dev]) {
-    B200_CUDA(cudaFuncSetAttribute(gqa_prefill_tiled_kernel<G, D, PAGED>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::smem_bytes));
-    if (dev >= 0 && dev < 64)
-      configured[dev] = true;
-  }
-  dim3 grid((M + T::BQ - 1) / T::BQ, kv_heads);
-  gqa_prefill_tiled_kernel<G, D, PAGED><<<grid, 512, T::smem_bytes, st>>>(qkv, ld, kc, vc, out, ldo, max_len, pos0,
-                                                                         M, table, page, kv_heads);
-  B200_LAUNCH_CHECK();
-  return B200_OK;
-}
-
 template <int G>
 int launch_prefill_attn(const float *qkv, int64_t ld, const float *kc, const float *vc, float *out, int64_t ldo,
                         int q_heads, int kv_heads, int D, int max_len, int pos0, int M, cudaStream_t st) {
@@ -872,30 +637,6 @@ int gqa_paged_launch(const float *qkv, int64_t ld, const float *k_pool, const fl
   }
 }
 
-// M rows of ONE sequence at positions pos0 .. pos0 + M - 1 (a prefill chunk) over the paged
-// pool: the attention kernel tiled over query rows.  seq_table: the sequence's row of the
-// block table (device).  Needs M >= 64 and 16-byte aligned rows; else returns B200_ESTATE
-// untouched and the caller uses gqa_paged_launch.
-int gqa_paged_prefill_launch(const float *qkv, int64_t ld, const float *k_pool, const float *v_pool, float *out,
-                             int64_t ldo, int q_heads, int kv_heads, int D, int page, const int32_t *seq_table,
-                             int pos0, int M, int max_context, cudaStream_t st) {
-  if ((D != 64 && D != 128) || M < 64 || (ld & 3) || (ldo & 3) || ((uintptr_t)qkv & 15) || ((uintptr_t)out & 15) ||
-      ((uintptr_t)k_pool & 15) || ((uintptr_t)v_pool & 15))
-    return B200_ESTATE;
-  switch (q_heads / kv_heads) {
-#define B200_G(G_)                                                                                                  \
-  case G_:                                                                                                          \
-    return D == 128 ? launch_prefill_tiled<G_, 128, true>(qkv, ld, k_pool, v_pool, out, ldo, kv_heads, max_context, \
-                                                          pos0, M, seq_table, page, st)                             \
-                    : launch_prefill_tiled<G_, 64, true>(qkv, ld, k_pool, v_pool, out, ldo, kv_heads, max_context,  \
-                                                         pos0, M, seq_table, page, st);
-    B200_G(1) B200_G(2) B200_G(3) B200_G(4) B200_G(6) B200_G(8)
-#undef B200_G
-  default:
-    return B200_ESTATE;
-  }
-}
-
 int argmax_rows_launch(const float *v, int64_t n, int rows, int32_t *out, cudaStream_t st) {
   argmax_rows_kernel<<<rows, 1024, 0, st>>>(v, n, out);
   B200_LAUNCH_CHECK();
@@ -924,17 +665,9 @@ int gqa_prefill_launch(const float *qkv, int64_t ld, const float *kc, const floa
                        int q_heads, int kv_heads, int D, int max_len, int pos0, int M, cudaStream_t st) {
   if (D != 64 && D != 128)
     return fail(B200_EINVAL, "gqa_prefill: head_dim %d (64 or 128 supported)", D);
-  // many rows: the tiled kernel (needs 16-byte aligned rows); few rows: one CTA per (row, kv head)
-  const bool tiled = M >= 64 && (ld & 3) == 0 && (ldo & 3) == 0 && ((uintptr_t)qkv & 15) == 0 &&
-                     ((uintptr_t)out & 15) == 0 && ((uintptr_t)kc & 15) == 0 && ((uintptr_t)vc & 15) == 0;
   switch (q_heads / kv_heads) {
 #define B200_G(G_)                                                                                      \
   case G_:                                                                                              \
-    if (tiled)                                                                                          \
-      return D == 128 ? launch_prefill_tiled<G_, 128, false>(qkv, ld, kc, vc, out, ldo, kv_heads, max_len, pos0, \
-                                                             M, nullptr, 0, st)                                 \
-                      : launch_prefill_tiled<G_, 64, false>(qkv, ld, kc, vc, out, ldo, kv_heads, max_len, pos0, \
-                                                            M, nullptr, 0, st);                                 \
     return launch_prefill_attn<G_>(qkv, ld, kc, vc, out, ldo, q_heads, kv_heads, D, max_len, pos0, M, st);
     B200_G(1) B200_G(2) B200_G(3) B200_G(4) B200_G(6) B200_G(8)
 #undef B200_G
