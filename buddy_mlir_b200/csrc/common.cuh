@@ -167,6 +167,28 @@ int gemm_w8a8_fused(const b200_weight *w, const float *A, int M, int64_t lda, fl
                     cudaStream_t stream);
 int argmax_rows_launch(const float *v, int64_t n, int rows, int32_t *out, cudaStream_t st);
 
+// Launch behind the kernel before it with its start overlapping that kernel's end.  Such a kernel waits (kernel_wait) before it
+// touches anything that an earlier kernel writes or reads; every kernel of a chain waits, so that "the one before is complete"
+// covers all that came before it.  kernel_go, early in a kernel, lets the next one start.
+__device__ __forceinline__ void kernel_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void kernel_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... P, typename... A>
+int launch_after(void (*kern)(P...), dim3 grid, int threads, int smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  B200_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
+  count_launch();
+  return B200_OK;
+}
+
 __device__ __forceinline__ float load_as_float(const void *p, int dtype,
                                                int64_t i) {
   if (dtype == B200_F32)

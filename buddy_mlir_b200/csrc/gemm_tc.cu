@@ -120,6 +120,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const int nkb_all = (p.K + BK - 1) / BK;
   const int kb0 = nkb_all * blockIdx.z / p.splits, nkb = nkb_all * (blockIdx.z + 1) / p.splits - kb0;
   volatile int *ab = &bars.abort_flag;
+  kernel_go();
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
@@ -154,7 +155,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const int ahead = min(S, nkb);
       for (int i = 0; i < ahead; ++i)   // the weights do not wait for the kernel before
         load_w(i);
-      asm volatile("griddepcontrol.wait;" ::: "memory");
+      kernel_wait();
       for (int i = 0; i < ahead; ++i)
         load_a(i);
       for (int i = ahead; i < nkb; ++i) {
@@ -185,7 +186,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // A thread reads an accumulator row (its lane of tensor memory) and half of its columns; the sums go to a padded tile in
     // shared memory (the ring is idle by then), from where the warps add up the planes and write whole rows.
     const bool ok = mbar_wait(&bars.accum, 0, ab, p.error, 703) && !*ab;
-    asm volatile("griddepcontrol.wait;" ::: "memory");   // row scales, counters (long complete: the operand was loaded)
+    kernel_wait();   // row scales, counters (long complete: the operand was loaded)
     constexpr int LDS = 128 + 4;                      // row stride of the staging tile, in words
     float *ep = reinterpret_cast<float *>(tiles);     // [BM][LDS]: 66 KB of the ring
     const int ew = warp - 2, quad = warp & 3;
@@ -261,16 +262,21 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             continue;
           float y[4];
           if (p.splits > 1) {
-            float4 a = __ldcg(shares + i);
-            for (int z = 1; z < p.splits; ++z) {
-              const float4 b = __ldcg(shares + (int64_t)z * kRows * 32 + i);
-              if (PLANES)
-                a = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
-              else
-                a = make_float4(__int_as_float(__float_as_int(a.x) + __float_as_int(b.x)),
-                                __int_as_float(__float_as_int(a.y) + __float_as_int(b.y)),
-                                __int_as_float(__float_as_int(a.z) + __float_as_int(b.z)),
-                                __int_as_float(__float_as_int(a.w) + __float_as_int(b.w)));
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int z0 = 0; z0 < p.splits; z0 += 8) {   // 8 loads in flight
+              float4 b[8];
+#pragma unroll
+              for (int z = 0; z < 8; ++z)
+                b[z] = z0 + z < p.splits ? __ldcg(shares + (int64_t)(z0 + z) * kRows * 32 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+              for (int z = 0; z < 8; ++z)
+                if (PLANES)
+                  a = make_float4(a.x + b[z].x, a.y + b[z].y, a.z + b[z].z, a.w + b[z].w);
+                else
+                  a = make_float4(__int_as_float(__float_as_int(a.x) + __float_as_int(b[z].x)),
+                                  __int_as_float(__float_as_int(a.y) + __float_as_int(b[z].y)),
+                                  __int_as_float(__float_as_int(a.z) + __float_as_int(b[z].z)),
+                                  __int_as_float(__float_as_int(a.w) + __float_as_int(b[z].w)));
             }
             y[0] = a.x; y[1] = a.y; y[2] = a.z; y[3] = a.w;
           } else {
@@ -349,7 +355,8 @@ constexpr int kUnits = 3;
 __global__ void __launch_bounds__(256)
 planes_kernel(const float *A, int64_t lda, int M, int K, const float *norm_w, float eps, int T, int vec, uint8_t *planes,
               float *row_scale, uint32_t *head, int head_words) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  kernel_go();
+  kernel_wait();
   __shared__ uint32_t s_mx[8];
   __shared__ float s_ss[8];
   const int t = threadIdx.x % T, m = blockIdx.x * (256 / T) + threadIdx.x / T;
@@ -451,7 +458,8 @@ constexpr int kMaxParts = 256;   // partial maxima, in the workspace head
 // word and counters.
 __global__ void __launch_bounds__(256)
 absmax_kernel(const float *A, int64_t lda, int M, int K, int vec, uint32_t *part, uint32_t *error, uint32_t *arrived) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  kernel_go();
+  kernel_wait();
   __shared__ uint32_t s_mx[8];
   if (blockIdx.x == 0) {
     if (threadIdx.x == 0)
@@ -489,8 +497,8 @@ absmax_kernel(const float *A, int64_t lda, int M, int K, int vec, uint32_t *part
 __global__ void __launch_bounds__(256)
 quantize_kernel(const float *A, int64_t lda, int M, int K, int vec, const uint32_t *part, int parts, float *scale_out,
                 uint8_t *q) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  kernel_go();
+  kernel_wait();
   __shared__ uint32_t s_mx[8];
   uint32_t mx = threadIdx.x < parts ? __ldcg(part + threadIdx.x) : 0u;
   mx = __reduce_max_sync(0xffffffffu, mx);
@@ -643,9 +651,9 @@ int b200_gemm_w8(const b200_weight *w, const float *A, int M, int64_t lda, float
   while (T < 256 && (K > T * 16 * kUnits || (int64_t)M * T < 148 * 256))
     T *= 2;
   const int vec = (lda & 3) == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)norm_weight & 15) == 0;
-  planes_kernel<<<(M + 256 / T - 1) / (256 / T), 256, 0, st>>>(A, lda, M, K, norm_weight, norm_eps, T, vec, planes, row_scale,
-                                                                reinterpret_cast<uint32_t *>(ws), 16 + kMaxPartialTiles);
-  B200_LAUNCH_CHECK();
+  if (int rc = launch_after(planes_kernel, dim3((M + 256 / T - 1) / (256 / T)), 256, 0, st, A, lda, M, K, norm_weight, norm_eps, T,
+                            vec, planes, row_scale, reinterpret_cast<uint32_t *>(ws), 16 + kMaxPartialTiles))
+    return rc;
   // 256 columns per CTA (fewer bytes per operation) when that still gives every SM its two CTAs
   if ((int64_t)((N + 255) / 256) * m_tiles >= 296) {
     p.splits = 1;
@@ -714,8 +722,9 @@ int gemm_w8a8_fused(const b200_weight *w, const float *A, int M, int64_t lda, fl
   p.arrived = reinterpret_cast<uint32_t *>(ws) + 16;
   const int vec = (lda & 3) == 0 && ((uintptr_t)A & 15) == 0;
   const int parts = (int)std::min<int64_t>(((int64_t)M * K / 4 + 1023) / 1024, kMaxParts);
-  absmax_kernel<<<parts, 256, 0, st>>>(A, lda, M, K, vec, part, reinterpret_cast<uint32_t *>(ws), p.arrived);
-  B200_LAUNCH_CHECK();
+  if (int rc = launch_after(absmax_kernel, dim3(parts), 256, 0, st, A, lda, M, K, vec, part, reinterpret_cast<uint32_t *>(ws),
+                            p.arrived))
+    return rc;
   const int64_t units = (int64_t)M * (K / 16);
   if (int rc = launch_after(quantize_kernel, dim3((unsigned)((units + 255) / 256)), 256, 0, st, A, lda, M, K, vec,
                             (const uint32_t *)part, parts, act_scale, q))

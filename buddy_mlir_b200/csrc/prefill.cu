@@ -17,6 +17,7 @@ constexpr float kSeed = -1.0e30f;
 
 // subgraph0_decode_simplify.mlir:46-49, for M tokens
 __global__ void embed_rows_kernel(const float *table, const int32_t *tokens, float *x, int64_t H) {
+  kernel_go();
   const float4 *src = reinterpret_cast<const float4 *>(table + (int64_t)tokens[blockIdx.x] * H);
   float4 *dst = reinterpret_cast<float4 *>(x + (int64_t)blockIdx.x * H);
   for (int i = threadIdx.x; i < H / 4; i += blockDim.x)
@@ -30,6 +31,8 @@ __global__ void rope_kv_rows_kernel(float *qkv, int64_t ld, float *k_cache, floa
                                     const float *inv_freq, const float *q_norm, const float *k_norm,
                                     float eps, int q_heads, int kv_heads, int D, int max_len, int pos0) {
   __shared__ float red[8];
+  kernel_go();
+  kernel_wait();
   const int half = D / 2;
   const int j = threadIdx.x;
   const int m = blockIdx.x, head = blockIdx.y;
@@ -194,6 +197,8 @@ __global__ void rope_kv_paged_kernel(float *qkv, int64_t ld, float *k_pool, floa
                                      int q_heads, int kv_heads, int D, int page, const int32_t *row_seq,
                                      const int32_t *row_pos, const int32_t *block_table, int table_stride) {
   __shared__ float red[8];
+  kernel_go();
+  kernel_wait();
   const int half = D / 2;
   const int j = threadIdx.x;
   const int m = blockIdx.x, head = blockIdx.y;
@@ -351,7 +356,9 @@ int launch_paged_attn(const float *qkv, int64_t ld, const float *kp, const float
 
 // The same scan for few rows with long histories (batched decode): the keys of a row
 // are cut into chunks of `chunk` positions (paged_chunk(): an eighth of the longest
-// context, 32..256), one CTA of 8 warps per (row, kv head, chunk); a warp owns every 8th key of the chunk and keeps four K/V rows in flight.
+// context, 32..256), one CTA per (row, kv head, chunk), a warp per 32 keys with 8 rows of V (and 8
+// 16-byte pieces of each lane's K row) in flight: the scan is a chain of memory latencies.  24 sequences of 32..700 positions,
+// 12 heads on 2, D = 128: 30 us a layer with one row in flight, 8 warps for 96 keys.
 // Partials (m, l, acc[D]) per query head go to `part`; the CTA that finishes a row's last
 // chunk folds them in chunk order.
 __host__ __device__ inline int paged_chunk(int max_context) {
@@ -359,12 +366,15 @@ __host__ __device__ inline int paged_chunk(int max_context) {
   return c < 32 ? 32 : (c > 256 ? 256 : c);
 }
 template <int G, int VEC>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 gqa_paged_split_kernel(const float *qkv, int64_t ld, const float *k_pool, const float *v_pool, float *part,
                        int kv_heads, int page, const int32_t *row_seq, const int32_t *row_pos,
                        const int32_t *block_table, int table_stride, int chunk, int *counters, float *out,
                        int64_t ldo) {
-  constexpr int D = VEC * 32, W = 8;
+  constexpr int D = VEC * 32, WMAX = 8, VB = 32 / VEC;
+  const int W = blockDim.x >> 5;
+  kernel_go();
+  kernel_wait();
   const int m = blockIdx.x, hk = blockIdx.y, sp = blockIdx.z;
   const int len = row_pos[m] + 1;
   const int j0 = sp * chunk;
@@ -403,8 +413,25 @@ gqa_paged_split_kernel(const float *qkv, int64_t ld, const float *k_pool, const 
 #pragma unroll
     for (int g = 0; g < G; ++g)
       sc[g] = 0.f;
+    const int nk = min(32, j1 - jb);
+    // values of keys t0 .. t0 + VB - 1 of the 32 (beyond nk: the last key again, with weight 0): VB rows in flight
+    float vr[VB][VEC];
+    auto fetch = [&](int t0) {
+#pragma unroll
+      for (int u = 0; u < VB; ++u) {
+        const float *vp = v_pool + (int64_t)__shfl_sync(0xffffffffu, ridx, min(t0 + u, nk - 1)) * D + lane * VEC;
+        if (VEC == 4) {
+          const float4 b = *reinterpret_cast<const float4 *>(vp);
+          vr[u][0] = b.x; vr[u][1] = b.y; vr[u][2 % VEC] = b.z; vr[u][3 % VEC] = b.w;
+        } else {
+          const float2 b = *reinterpret_cast<const float2 *>(vp);
+          vr[u][0] = b.x; vr[u][1] = b.y;
+        }
+      }
+    };
+    fetch(0);   // on their way while the scores are made
     if (live) {
-#pragma unroll 4
+#pragma unroll 8
       for (int d = 0; d < D; d += 4) {
         const float4 k4 = *reinterpret_cast<const float4 *>(kp + d);
 #pragma unroll
@@ -431,30 +458,22 @@ gqa_paged_split_kernel(const float *qkv, int64_t ld, const float *k_pool, const 
       for (int e = 0; e < VEC; ++e)
         acc[g][e] *= alpha;
     }
-    const int nk = min(32, j1 - jb);
-    for (int t = 0; t < nk; ++t) {
-      const int rt = __shfl_sync(0xffffffffu, ridx, t);
-      const float *vp = v_pool + (int64_t)rt * D + lane * VEC;
-      float vr[VEC];
-      if (VEC == 4) {
-        const float4 b = *reinterpret_cast<const float4 *>(vp);
-        vr[0] = b.x; vr[1] = b.y; vr[2 % VEC] = b.z; vr[3 % VEC] = b.w;
-      } else {
+    for (int t0 = 0; t0 < nk; t0 += VB) {
+      if (t0 > 0)
+        fetch(t0);
 #pragma unroll
-        for (int e = 0; e < VEC; ++e)
-          vr[e] = vp[e];
-      }
+      for (int u = 0; u < VB; ++u)
 #pragma unroll
-      for (int g = 0; g < G; ++g) {
-        const float pt = __shfl_sync(0xffffffffu, pw[g], t);
+        for (int g = 0; g < G; ++g) {
+          const float pt = __shfl_sync(0xffffffffu, pw[g], t0 + u);
 #pragma unroll
-        for (int e = 0; e < VEC; ++e)
-          acc[g][e] = fmaf(pt, vr[e], acc[g][e]);
-      }
+          for (int e = 0; e < VEC; ++e)
+            acc[g][e] = fmaf(pt, vr[u][e], acc[g][e]);
+        }
     }
   }
-  __shared__ float s_m[W][G], s_l[W][G];
-  __shared__ float s_acc[W][G][D];
+  __shared__ float s_m[WMAX][G], s_l[WMAX][G];
+  __shared__ float s_acc[WMAX][G][D];
 #pragma unroll
   for (int g = 0; g < G; ++g) {
     if (lane == 0) {
@@ -470,11 +489,9 @@ gqa_paged_split_kernel(const float *qkv, int64_t ld, const float *k_pool, const 
   for (int idx = threadIdx.x; idx < G * D; idx += blockDim.x) {
     const int g = idx / D, d = idx - g * D;
     float M = kSeed;
-#pragma unroll
     for (int w = 0; w < W; ++w)
       M = fmaxf(M, s_m[w][g]);
     float L = 0.f, A = 0.f;
-#pragma unroll
     for (int w = 0; w < W; ++w) {
       const float b = expf(s_m[w][g] - M);   // a warp that saw no key: l = 0, acc = 0
       L = fmaf(s_l[w][g], b, L);
@@ -526,14 +543,12 @@ int launch_paged_split(const float *qkv, int64_t ld, const float *kp, const floa
                        const int32_t *block_table, int table_stride, int M, float *part, int *counters, int chunks,
                        int chunk, cudaStream_t st) {
   dim3 grid(M, kv_heads, chunks);
+  const int threads = min(256, chunk);   // a warp per 32 keys of the chunk (32 .. 256, a multiple of 32)
   if (D == 128)
-    gqa_paged_split_kernel<G, 4><<<grid, 256, 0, st>>>(qkv, ld, kp, vp, part, kv_heads, page, row_seq, row_pos,
-                                                       block_table, table_stride, chunk, counters, out, ldo);
-  else
-    gqa_paged_split_kernel<G, 2><<<grid, 256, 0, st>>>(qkv, ld, kp, vp, part, kv_heads, page, row_seq, row_pos,
-                                                       block_table, table_stride, chunk, counters, out, ldo);
-  B200_LAUNCH_CHECK();
-  return B200_OK;
+    return launch_after(gqa_paged_split_kernel<G, 4>, grid, threads, 0, st, qkv, ld, kp, vp, part, kv_heads, page, row_seq, row_pos,
+                        block_table, table_stride, chunk, counters, out, ldo);
+  return launch_after(gqa_paged_split_kernel<G, 2>, grid, threads, 0, st, qkv, ld, kp, vp, part, kv_heads, page, row_seq, row_pos,
+                        block_table, table_stride, chunk, counters, out, ldo);
 }
 
 // one first-maximum per row of a [rows, n] matrix (Sampler.h:101-104); 1024 threads per row,
@@ -593,11 +608,9 @@ int rope_kv_paged_launch(float *qkv, int64_t ld, float *k_pool, float *v_pool, c
                          int page, const int32_t *row_seq, const int32_t *row_pos, const int32_t *block_table,
                          int table_stride, int M, cudaStream_t st) {
   dim3 grid(M, q_heads + kv_heads);
-  rope_kv_paged_kernel<<<grid, D / 2 < 32 ? 32 : D / 2, 0, st>>>(qkv, ld, k_pool, v_pool, inv_freq, q_norm, k_norm, eps,
+  return launch_after(rope_kv_paged_kernel, grid, D / 2 < 32 ? 32 : D / 2, 0, st, qkv, ld, k_pool, v_pool, inv_freq, q_norm, k_norm, eps,
                                                                q_heads, kv_heads, D, page, row_seq, row_pos,
                                                                block_table, table_stride);
-  B200_LAUNCH_CHECK();
-  return B200_OK;
 }
 
 int64_t gqa_paged_scratch_floats(int rows, int q_heads, int D, int max_context) {
@@ -655,10 +668,8 @@ int rope_kv_rows_launch(float *qkv, int64_t ld, float *k_cache, float *v_cache, 
                         const float *q_norm, const float *k_norm, float eps, int q_heads, int kv_heads, int D,
                         int max_len, int pos0, int M, cudaStream_t st) {
   dim3 grid(M, q_heads + kv_heads);
-  rope_kv_rows_kernel<<<grid, D / 2 < 32 ? 32 : D / 2, 0, st>>>(qkv, ld, k_cache, v_cache, inv_freq, q_norm, k_norm,
+  return launch_after(rope_kv_rows_kernel, grid, D / 2 < 32 ? 32 : D / 2, 0, st, qkv, ld, k_cache, v_cache, inv_freq, q_norm, k_norm,
                                                               eps, q_heads, kv_heads, D, max_len, pos0);
-  B200_LAUNCH_CHECK();
-  return B200_OK;
 }
 
 int gqa_prefill_launch(const float *qkv, int64_t ld, const float *kc, const float *vc, float *out, int64_t ldo,

@@ -83,7 +83,8 @@ template <int D>
 __global__ void __launch_bounds__(256)
 kv_image_kernel(const float *kc, const float *vc, int max_len, int n_keys, const int32_t *table, int page, uint8_t *images,
                 uint32_t *arrived, int counters) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  kernel_wait();
+  kernel_go();   // not before: the next kernel reads Q, which the kernel before this one writes, without waiting
   if (blockIdx.x + blockIdx.y + blockIdx.z == 0)
     for (int i = threadIdx.x; i < counters; i += 256)
       arrived[i] = 0u;
@@ -186,6 +187,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(const AttnPar
   const int splits = (n_all + p.chunk - 1) / p.chunk;
   if ((int)blockIdx.x >= splits)
     return;
+  kernel_go();
   const int t0 = n_all * blockIdx.x / splits, n = n_all * (blockIdx.x + 1) / splits - t0;
 
   if (threadIdx.x == 0) {
@@ -238,7 +240,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(const AttnPar
   if (warp == kSoftmaxWarps) {
     // ---- loader ----------------------------------------------------------------------------------------------------------------
     if (lane == 0) {
-      asm volatile("griddepcontrol.wait;" ::: "memory");
+      kernel_wait();
       const uint8_t *img = p.images + ((int64_t)hk * p.key_tiles + t0) * 2 * T::KV_BYTES;
       // plane j of the sequence: tile j / 3, planes 2, 1, 0
       auto load = [&](uint8_t *dst, int j, int z, uint64_t *bar) {
@@ -433,7 +435,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(const AttnPar
     bool mine = ok;
     float *part = p.part + ((int64_t)(hk * gridDim.y + qt) * gridDim.x) * T::PART;
     if (!whole) {   // leave this CTA's share; the last one of the row tile goes on
-      asm volatile("griddepcontrol.wait;" ::: "memory");   // the counters are zero
+      kernel_wait();   // the counters are zero
       float *own = part + (int64_t)blockIdx.x * T::PART;
       for (int i = half * 32 + lane; i < 32 * (D / 4); i += 64) {
         const int rr = quad * 32 + i / (D / 4), c = i % (D / 4);
@@ -531,9 +533,9 @@ int launch_attn(const AttnParams &p, const float *kc, const float *vc, int kv_he
     if (dev >= 0 && dev < 64)
       configured[dev].store(true, std::memory_order_release);
   }
-  kv_image_kernel<D><<<dim3(p.key_tiles, kv_heads, 2 * kKeys * (D / 8) / 256), 256, 0, st>>>(kc, vc, p.max_len, n_keys, table, page, images, p.arrived,
-                                                                    max_splits > 1 ? q_tiles * kv_heads : 0);
-  B200_LAUNCH_CHECK();
+  if (int rc = launch_after(kv_image_kernel<D>, dim3(p.key_tiles, kv_heads, 2 * kKeys * (D / 8) / 256), 256, 0, st, kc, vc,
+                            p.max_len, n_keys, table, page, images, p.arrived, max_splits > 1 ? q_tiles * kv_heads : 0))
+    return rc;
   return launch_after(prefill_attn_kernel<D>, dim3(max_splits, q_tiles, kv_heads), kThreads, Tile<D>::SMEM, st, p);
 }
 

@@ -1,5 +1,4 @@
-// What the tensor-core kernels (gemm_tc.cu, prefill_attn.cu) share: mbarriers with bounded waits, tcgen05 operands, the
-// launch that overlaps the kernel before.
+// What the tensor-core kernels (gemm_tc.cu, prefill_attn.cu) share: mbarriers with bounded waits, tcgen05 operands.
 #pragma once
 #include "common.cuh"
 
@@ -77,24 +76,6 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
 }
 __device__ __forceinline__ void tc_commit(uint64_t *bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-// Launch behind the kernel before it with its start overlapping that kernel's end (it waits where it needs its results).
-template <typename... P, typename... A>
-int launch_after(void (*kern)(P...), dim3 grid, int threads, int smem, cudaStream_t st, A... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  B200_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
-  count_launch();
-  return B200_OK;
 }
 
 } // namespace b200
