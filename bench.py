@@ -106,8 +106,7 @@ class ClockSampler:
 # dram__bytes_read.sum + dram__bytes_write.sum of one decode_step_kernel launch (ncu, full-size
 # 1.5B int8 model at context ~1000), and the git blob hash of the kernel source it was captured
 # from.  The figure is only reported while the source is still that one.
-TRAFFIC = {"bytes": 1717368176, "kernel_source": "buddy_mlir_b200/csrc/mega.cu",
-           "git_blob": "fbdb80c4ec6f5ae66337f7c5b248aeed4b7800a5",
+TRAFFIC = {"bytes": None, "kernel_source": "buddy_mlir_b200/csrc/decode.cu", "git_blob": "",
            "capture": "ncu --set full --clock-control none -k regex:decode_step -c 1, bench.py --resident-only"}
 
 
@@ -390,8 +389,8 @@ def gemm_microbench(lib, only=None):
         out[name]["w8a8_us"] = round(us8, 1)
         out[name]["w8a8_TOP/s"] = round(2.0 * M * N * K / us8 / 1e6, 1)
     return {"shapes": out, "peak_tflops": peak,
-            "note": "frac = algorithmic 2MNK / time / measured sustained bf16 peak; the tensor pipe does twice the "
-                    "algorithmic work (two bf16 terms per f32 activation); w8a8_* = the same shape with int8 "
+            "note": "frac = algorithmic 2MNK / time / measured sustained bf16 peak; the tensor pipe does three times the "
+                    "algorithmic work (three int8 digits per f32 activation, int8 at the bf16 rate); w8a8_* = the same shape with int8 "
                     "activations on the integer tensor-core path (no measured int8 peak on this pool: absolute only)"}
 
 

@@ -157,12 +157,12 @@ int b200_gemv(const b200_weight *w, const b200_gemv_args *a, void *stream);
  * (dequantisation fused into the B packing; known answer
  * examples/BuddyMatmul/dequant-matmul-vectorization-blis-prefill.mlir:113-115).
  * w: int8 per-channel packed rows as for b200_gemv (f32 scales, optional
- * bias), K a multiple of 64.  A: f32 [M, lda] on the device; norm_weight (or
- * NULL): RMSNorm of every row of A first.  The f32 activations are split into
- * two bf16 terms (16 significant bits), int8 -> bf16 is exact, accumulation is
- * f32 in tensor memory.  workspace: b200_gemm_w8_workspace_bytes(M, K) bytes,
- * 256-byte aligned, owned by the caller (it holds the split activations and an
- * error word).  b200_gemm_w8_status() reports a bounded wait that gave up. */
+ * bias), K a multiple of 64 up to 131008.  A: f32 [M, lda] on the device; norm_weight (or
+ * NULL): RMSNorm of every row of A first.  An activation is a 23-bit
+ * fixed-point number in units of its row, three int8 digits whose sums of
+ * products are exact (tcgen05.mma kind::i8) and added in f32.  workspace:
+ * b200_gemm_w8_workspace_bytes(M, K) bytes, 256-byte aligned, owned by the
+ * caller (it holds the digits, shares of split tiles and an error word).  b200_gemm_w8_status() reports a bounded wait that gave up. */
 int64_t b200_gemm_w8_workspace_bytes(int M, int64_t K);
 int b200_gemm_w8(const b200_weight *w, const float *A, int M, int64_t lda,
                  float *C, int64_t ldc, const float *residual, int64_t ldr,
