@@ -120,7 +120,8 @@ __global__ void __launch_bounds__(kMaxWarps<COLS> * 32, 1) gemv_mma_kernel(const
   const int nu = p.tunits;   // int4: units of the short last block
   const bool one_slab = p.slab_steps >= p.steps;
 
-  auto tile_of = [&](int r) { return ((int64_t)r * gridDim.x + blockIdx.x) * p.slots + slot; };
+  // (warps beyond the slots only help with the staging)
+  auto tile_of = [&](int r) { return slot < p.slots ? ((int64_t)r * gridDim.x + blockIdx.x) * p.slots + slot : (int64_t)p.tiles; };
   TileRows rows{};
   uint4 w[8];
   Scales sc{};
@@ -152,16 +153,15 @@ __global__ void __launch_bounds__(kMaxWarps<COLS> * 32, 1) gemv_mma_kernel(const
   };
   auto finish_rows = [&]() {
     __syncthreads();
-    if (warp == 0)
-      for (int m = 0; m < p.M; ++m) {
-        const uint32_t mx = __reduce_max_sync(0xffffffffu, lane < W ? red[m * W + lane] : 0u);
-        const float ss = p.norm_w != nullptr ? warp_sum(lane < W ? redf[m * W + lane] : 0.f) : 0.f;
-        if (lane == 0) {
-          float inv;
-          s_scale[m] = fixed_scale(mx, &inv);
-          s_inv[m] = p.norm_w != nullptr ? inv * rsqrtf(ss * (1.0f / (float)p.K) + p.eps) : inv;
-        }
+    for (int m = warp; m < p.M; m += W) {   // a warp per row
+      const uint32_t mx = __reduce_max_sync(0xffffffffu, lane < W ? red[m * W + lane] : 0u);
+      const float ss = p.norm_w != nullptr ? warp_sum(lane < W ? redf[m * W + lane] : 0.f) : 0.f;
+      if (lane == 0) {
+        float inv;
+        s_scale[m] = fixed_scale(mx, &inv);
+        s_inv[m] = p.norm_w != nullptr ? inv * rsqrtf(ss * (1.0f / (float)p.K) + p.eps) : inv;
       }
+    }
     __syncthreads();
   };
   auto add4 = [&](float4 v, float &ss) {
@@ -243,21 +243,31 @@ __global__ void __launch_bounds__(kMaxWarps<COLS> * 32, 1) gemv_mma_kernel(const
     staged = true;
     __syncthreads();
   } else {
-    for (int m = 0; m < p.M; ++m) {
-      uint32_t mx = 0;
-      float ss = 0.f;
-      for (int k = tid * 4; k < p.K; k += 4 * nthr * 4) {   // four loads in flight per thread
-        float4 v[4];
+    // four rows at a time, one or two loads of each in flight per thread: a row after the other is a chain of M latencies
+    for (int m0 = 0; m0 < p.M; m0 += 4) {
+      uint32_t mx[4] = {0, 0, 0, 0};
+      float ss[4] = {0.f, 0.f, 0.f, 0.f};
+      constexpr int kU = XF ? 2 : 1;   // (16-bit loads bring more code)
+      for (int k = tid * 4; k < p.K; k += kU * nthr * 4) {
+        float4 v[4][kU];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          v[u] = act4<XF>(p, m, k + u * nthr * 4);
+        for (int q = 0; q < 4; ++q)
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          add4(v[u], ss);
-          mx = max(mx, absbits4(normed<XF>(p, k + u * nthr * 4, v[u])));
-        }
+          for (int u = 0; u < kU; ++u)
+            v[q][u] = act4<XF>(p, min(m0 + q, p.M - 1), k + u * nthr * 4);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+          for (int u = 0; u < kU; ++u) {
+            if (p.norm_w != nullptr)
+              add4(v[q][u], ss[q]);
+            mx[q] = max(mx[q], absbits4(normed<XF>(p, k + u * nthr * 4, v[q][u])));
+          }
       }
-      reduce_row(m, mx, ss);
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (m0 + q < p.M)
+          reduce_row(m0 + q, mx[q], ss[q]);
     }
     finish_rows();
     if (U4 && nu > 0)
@@ -266,32 +276,49 @@ __global__ void __launch_bounds__(kMaxWarps<COLS> * 32, 1) gemv_mma_kernel(const
   // planes of the slab that starts at step s0; all rows' groups as one list, four loads in flight per thread
   auto stage = [&](int s0) {
     const int k0 = s0 * (U4 ? 512 : 256);
-    constexpr int kU = U4 ? 2 : 4;
+    constexpr int kU = U4 ? 1 : COLS > 16 ? 8 : 4;
     const int units = min(p.slab_k / (U4 ? 32 : 16), p.units - k0 / (U4 ? 32 : 16));
     const int groups = units * 4;   // per row (int4: a multiple of 128, so a warp never straddles two rows)
     const int total = groups * p.M;
-    for (int i0 = tid; i0 < total; i0 += kU * nthr) {
-      float4 v[kU], v2[U4 ? kU : 1];
-#pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        const int i = i0 + u * nthr;
+    const uint32_t magic = 0xffffffffu / (uint32_t)groups + 1;   // i / groups exactly for i < total <= 2^16
+    auto row_of = [&](int i) { return groups > 1 ? (int)__umulhi((uint32_t)i, magic) : i; };
+    if constexpr (U4) {   // the next group is loaded while this one is stored: one copy of the code, which is long and cold
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f), v2 = v;
+      auto load = [&](int i, float4 &x, float4 &y) {
         if (i < total) {
-          const int m = i / groups, k = k0 + k_of(i - m * groups, units);
-          v[u] = act4<XF>(p, m, k);
-          if constexpr (U4)
-            v2[u] = act4<XF>(p, m, k + 16);
+          const int m = row_of(i), k = k0 + k_of(i - m * groups, units);
+          x = act4<XF>(p, m, k);
+          y = act4<XF>(p, m, k + 16);
         }
+      };
+      load(tid, v, v2);
+#pragma unroll 1
+      for (int i = tid; i < total; i += nthr) {
+        float4 nv = v, nv2 = v2;
+        load(i + nthr, nv, nv2);
+        const int m = row_of(i), k = k0 + k_of(i - m * groups, units);
+        store_u4<COLS>(planes, start, group_u4(i - m * groups), m, normed<XF>(p, k, v), normed<XF>(p, k + 16, v2), s_scale[m]);
+        v = nv;
+        v2 = nv2;
       }
+    } else {
+      for (int i0 = tid; i0 < total; i0 += kU * nthr) {
+        float4 v[kU];
 #pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        const int i = i0 + u * nthr;
-        if (i < total) {
-          const int m = i / groups, k = k0 + k_of(i - m * groups, units);
-          if constexpr (U4)
-            store_u4<COLS>(planes, start, group_u4(i - m * groups), m, normed<XF>(p, k, v[u]), normed<XF>(p, k + 16, v2[u]),
-                     s_scale[m]);
-          else
+        for (int u = 0; u < kU; ++u) {
+          const int i = i0 + u * nthr;
+          if (i < total) {
+            const int m = row_of(i);
+            v[u] = act4<XF>(p, m, k0 + k_of(i - m * groups, units));
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+          const int i = i0 + u * nthr;
+          if (i < total) {
+            const int m = row_of(i), k = k0 + k_of(i - m * groups, units);
             store_i8<COLS>(planes, group_i8(i - m * groups, units), m, normed<XF>(p, k, v[u]), s_scale[m]);
+          }
         }
       }
     }
@@ -475,7 +502,9 @@ template <int KIND, int COLS, bool GROUPED, bool XF> static int launch_mma(MmaP 
   const int64_t ctas = ((int64_t)p.tiles + p.slots - 1) / p.slots;
   const int grid = (int)(ctas < sms ? ctas : sms);
   p.rounds = (int)((ctas + grid - 1) / grid);
-  const int threads = p.slots * p.ks * 32;
+  // Several rows: the staging takes longer than a narrow projection's products, and few warps issue it at their latency, so
+  // all warps take part (int4 14336 x 4096, 5 rows: 7 warps hold tiles).
+  const int threads = (p.M > 1 ? W : p.slots * p.ks) * 32;
   p.reg_x = p.M == 1 && nblk * blk >= span && p.units * 4 <= (U4 ? 3 : 6) * threads;
   static std::atomic<bool> configured{false};
   if (!configured.load(std::memory_order_acquire)) {
