@@ -7,7 +7,7 @@
 //
 // Bound: HBM for one row (int8 lm_head 151936 x 1536: 42 us, 5.6 TB/s; int4 152000 x 4096: 70 us; the FFMA kernel: 50 and
 // 111 us), the shared-memory reads and MMAs of four columns per activation row for many (int4 14336 x 4096, 5 rows: 130 ->
-// 28 us; 16 rows: 363 -> 61 us), and for short calls the chain launch - first load - quantise - first step - sum.
+// 27 us; 16 rows: 363 -> 61 us), and for short calls the chain launch - first load - quantise - first step - sum.
 #include "gemv_mma.cuh"
 
 #include <mutex>
