@@ -596,10 +596,13 @@ int launch_gemm(const void *a, int a_rows, const void *w, GemmParams &p, int m_t
 // CTAs along K for `tiles` output tiles of `nkb` k blocks: up to two CTAs per SM (148), within the workspace, at least 8 k
 // blocks each: a share's trip through L2 costs what 8 to 12 blocks cost.  24 x 2048 x 1536 (12 blocks): 10.1 us whole, 11.1 in
 // 6 shares; 24 x 1536 x 8960 (70 blocks): 27 us whole, 14.4 in 8, 17.2 in 24; 366 x 1536 x 8960 (108 tiles): 34.8 whole, 28.2 in 2.
-int split_k(int tiles, int nkb) {
+// A row of a tile's sums costs as much on that trip as 0.4 blocks, so tiles with many rows split only long k ranges (W8A8,
+// 1024 x 1536 x 8960: 49.8 us whole, 55.3 in 3; 200 x 4096 x 4096: 21.4 whole, 29 in 4; 64 x 1536 x 8960: 32.2 whole, 19.7 in 8).
+int split_k(int tiles, int nkb, int rows) {
   if (tiles >= 148)
     return 1;
-  return std::max(1, std::min({296 / tiles, nkb / 8, kMaxPartialTiles / tiles}));
+  const int s = std::max(1, std::min({296 / tiles, nkb / 8, kMaxPartialTiles / tiles}));
+  return (nkb - nkb / s) * 5 > rows * 2 ? s : 1;
 }
 
 } // namespace
@@ -666,7 +669,7 @@ int b200_gemm_w8(const b200_weight *w, const float *A, int M, int64_t lda, float
     p.splits = 1;
     return launch_gemm<256, true>(planes, m_tiles * BM, w->w, p, m_tiles, st);
   }
-  p.splits = split_k((N + 127) / 128 * m_tiles, (K + BK - 1) / BK);
+  p.splits = split_k((N + 127) / 128 * m_tiles, (K + BK - 1) / BK, std::min(M, kPlaneRows));
   return launch_gemm<128, true>(planes, m_tiles * BM, w->w, p, m_tiles, st);
 }
 
@@ -736,7 +739,7 @@ int gemm_w8a8_fused(const b200_weight *w, const float *A, int M, int64_t lda, fl
   if (int rc = launch_after(quantize_kernel, dim3((unsigned)((units + 255) / 256)), 256, 0, st, A, lda, M, K, vec,
                             (const uint32_t *)part, parts, act_scale, q))
     return rc;
-  p.splits = split_k((N + 127) / 128 * m_tiles, (K + BK - 1) / BK);
+  p.splits = split_k((N + 127) / 128 * m_tiles, (K + BK - 1) / BK, std::min(M, BM));
   return launch_gemm<128, false>(q, M, w->w, p, m_tiles, st);
 }
 } // namespace b200
