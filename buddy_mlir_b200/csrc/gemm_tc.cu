@@ -156,7 +156,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         tma_load_2d(tiles + s * R::STAGE_BYTES, &map_a, (kb0 + i) * BK, blockIdx.y * BM, &bars.full[s]);
       };
       // few rows: the weights' way from memory is the GEMM; all of this CTA's share starts for L2 while the kernels before run
-      if (gridDim.y <= 2)
+      // (if all CTAs are resident at once: 24 x 151936 x 1536, 594 CTAs, took 68 us with it and 60 without)
+      if (gridDim.y <= 2 && gridDim.x * gridDim.y * gridDim.z <= 296)
         for (int i = S; i < nkb; ++i)
           tma_prefetch_2d(&map_w, (kb0 + i) * BK, n0);
       const int ahead = min(S, nkb);
