@@ -123,7 +123,6 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const int nkb_all = (p.K + BK - 1) / BK;
   const int kb0 = nkb_all * blockIdx.z / p.splits, nkb = nkb_all * (blockIdx.z + 1) / p.splits - kb0;
   volatile int *ab = &bars.abort_flag;
-  kernel_go();
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
@@ -142,6 +141,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = bars.tmem_base;
+  kernel_go();   // not before the allocation: see tensor_core.cuh
 
   if (warp == 0) {
     // ---- loader --------------------------------------------------------------------------------------------------

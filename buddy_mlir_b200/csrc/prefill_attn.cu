@@ -187,7 +187,6 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(const AttnPar
   const int splits = (n_all + p.chunk - 1) / p.chunk;
   if ((int)blockIdx.x >= splits)
     return;
-  kernel_go();
   const int t0 = n_all * blockIdx.x / splits, n = n_all * (blockIdx.x + 1) / splits - t0;
 
   if (threadIdx.x == 0) {
@@ -236,6 +235,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(const AttnPar
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = __shfl_sync(0xffffffffu, bars.tmem_base, 0);
+  kernel_go();   // not before the allocation: see tensor_core.cuh
 
   if (warp == kSoftmaxWarps) {
     // ---- loader ----------------------------------------------------------------------------------------------------------------

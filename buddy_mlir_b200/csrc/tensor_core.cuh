@@ -1,4 +1,10 @@
 // What the tensor-core kernels (gemm_tc.cu, prefill_attn.cu) share: mbarriers with bounded waits, tcgen05 operands.
+//
+// Tensor memory and early starts.  tcgen05.alloc waits, without a limit, until the columns are free.  It ends because whoever
+// holds them ends: a kernel calls kernel_go() only after its own allocation, so the kernels behind it get an SM when every CTA
+// before them has its columns, and a CTA that holds columns waits (kernel_wait) only for kernels that need no more of them.
+// With kernel_go() first, a CTA of the next kernel could take the columns an earlier CTA still needs and then wait for it: at
+// head dim 64 an attention CTA (109 KB of shared memory, all 512 columns) and a GEMM CTA (98 KB) fit on one SM.
 #pragma once
 #include "common.cuh"
 
