@@ -161,10 +161,14 @@ int64_t prefill_attn_workspace_bytes(int n_keys, int kv_heads, int D);
 int prefill_attn_launch(const float *qkv, int64_t ld, const float *kc, const float *vc, float *out, int64_t ldo, int q_heads,
                         int kv_heads, int D, int max_len, int pos0, int M, const int32_t *table, int page, void *workspace,
                         int64_t workspace_bytes, int *error, cudaStream_t st);
-// gemm_tc.cu: b200_gemm_w8a8 with the residual sum or the SiLU pair folded into the store
+// gemm_tc.cu: b200_gemm_w8, and b200_gemm_w8a8 with the residual sum or the SiLU pair folded into the store.  in_pass: a call
+// of a session's pass (see there)
+int gemm_w8_run(const b200_weight *w, const float *A, int M, int64_t lda, float *C, int64_t ldc, const float *residual,
+                int64_t ldr, const float *norm_weight, float norm_eps, int silu_pairs, void *workspace,
+                int64_t workspace_bytes, bool in_pass, cudaStream_t stream);
 int gemm_w8a8_fused(const b200_weight *w, const float *A, int M, int64_t lda, float *C, int64_t ldc,
                     const float *residual, int64_t ldr, int silu_pairs, void *workspace, int64_t workspace_bytes,
-                    cudaStream_t stream);
+                    bool in_pass, cudaStream_t stream);
 int argmax_rows_launch(const float *v, int64_t n, int rows, int32_t *out, cudaStream_t st);
 
 // Launch behind the kernel before it with its start overlapping that kernel's end.  Such a kernel waits (kernel_wait) before it

@@ -1727,7 +1727,8 @@ static int linear_rows_int8(b200_model *m, const DevLinear &L, const float *X, i
     A = m->pf_norm;
     lda = K;
   }
-  return gemm_w8a8_fused(&L.w, A, M, lda, Y, ldy, residual, ldy, silu ? 1 : 0, m->pf_ws, m->pf_ws_bytes, st);
+  return gemm_w8a8_fused(&L.w, A, M, lda, Y, ldy, residual, ldy, silu ? 1 : 0, m->pf_ws, m->pf_ws_bytes, true,
+                         st);
 }
 
 // One projection over M rows: the dense tensor-core GEMM for int8 per-channel
@@ -1740,8 +1741,8 @@ static int linear_rows(b200_model *m, const DevLinear &L, const float *X, int64_
     return linear_rows_int8(m, L, X, ldx, M, Y, ldy, residual, norm_w, silu);
   }
   if (L.w.kind == B200_W_I8 && L.w.scale_dtype == B200_F32 && L.w.K % 64 == 0)
-    return b200_gemm_w8(&L.w, X, M, ldx, Y, ldy, residual, ldy, norm_w, m->cfg.eps, silu ? 1 : 0, m->pf_ws,
-                        m->pf_ws_bytes, m->stream);
+    return gemm_w8_run(&L.w, X, M, ldx, Y, ldy, residual, ldy, norm_w, m->cfg.eps, silu ? 1 : 0, m->pf_ws, m->pf_ws_bytes,
+                       true, m->stream);
   for (int m0 = 0; m0 < M; m0 += 16) {
     b200_gemv_args a{};
     a.x = X + (int64_t)m0 * ldx;

@@ -24,7 +24,8 @@
 // A CTA computes a 128 x 128 or 128 x 256 tile of sums: warp 0 issues the TMA loads (cp.async.bulk.tensor, no multicast) of
 // 128-byte k blocks into a ring of 96 KB (3 stages of 32 KB, or 2 of 48), warp 1 one thread of tcgen05.mma, warps 2..9 the
 // epilogue; two CTAs are resident per SM, so one's epilogue runs under the other's main loop.  The weight loads start
-// before the activations are there (programmatic dependent launch behind the kernel that makes the planes).  The main loop
+// before the activations are there (programmatic dependent launch behind the kernel that makes the planes; chain_start says
+// what keeps them behind the caller's earlier work).  The main loop
 // is bound by the bytes it brings from L2 (64 bytes per clock and SM), hence 256 columns where that leaves enough CTAs.
 // Few output tiles: the k range is split over gridDim.z, and the CTA that finishes a tile last adds the shares in order.
 //
@@ -342,6 +343,17 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   }
 }
 
+// The first kernel of a call.  The GEMM behind it loads weights before it waits, so nothing but this kernel's own wait keeps
+// those loads behind what the caller's stream did before: the weights may be the output of the kernel just before the call.
+// Inside a session's pass the weights were there before the pass began, and the next kernel may start at once (in_pass).
+__device__ __forceinline__ void chain_start(int in_pass) {
+  if (in_pass)
+    kernel_go();
+  kernel_wait();
+  if (!in_pass)
+    kernel_go();
+}
+
 // ---- the A operand ------------------------------------------------------------------------------------------------------
 // Four consecutive activations from k on (K is a multiple of 64; vec: 16-byte loads are possible).
 __device__ __forceinline__ float4 load4(const float *row, int k, bool vec) {
@@ -362,9 +374,8 @@ __device__ __forceinline__ int unit_k(int u, int j, int units) {
 constexpr int kUnits = 3;
 __global__ void __launch_bounds__(256)
 planes_kernel(const float *A, int64_t lda, int M, int K, const float *norm_w, float eps, int T, int vec, uint8_t *planes,
-              float *row_scale, uint32_t *head, int head_words) {
-  kernel_go();
-  kernel_wait();
+              float *row_scale, uint32_t *head, int head_words, int in_pass) {
+  chain_start(in_pass);
   __shared__ uint32_t s_mx[8];
   __shared__ float s_ss[8];
   const int t = threadIdx.x % T, m = blockIdx.x * (256 / T) + threadIdx.x / T;
@@ -465,9 +476,9 @@ constexpr int kMaxParts = 256;   // partial maxima, in the workspace head
 // max |x| of every CTA's share of the tensor (non-negative floats order like their bit patterns); clears the GEMM's error
 // word and counters.
 __global__ void __launch_bounds__(256)
-absmax_kernel(const float *A, int64_t lda, int M, int K, int vec, uint32_t *part, uint32_t *error, uint32_t *arrived) {
-  kernel_go();
-  kernel_wait();
+absmax_kernel(const float *A, int64_t lda, int M, int K, int vec, uint32_t *part, uint32_t *error, uint32_t *arrived,
+              int in_pass) {
+  chain_start(in_pass);
   __shared__ uint32_t s_mx[8];
   if (blockIdx.x == 0) {
     if (threadIdx.x == 0)
@@ -505,7 +516,7 @@ absmax_kernel(const float *A, int64_t lda, int M, int K, int vec, uint32_t *part
 __global__ void __launch_bounds__(256)
 quantize_kernel(const float *A, int64_t lda, int M, int K, int vec, const uint32_t *part, int parts, float *scale_out,
                 uint8_t *q) {
-  kernel_go();
+  kernel_go();   // absmax_kernel, before it, has waited as the call requires
   kernel_wait();
   __shared__ uint32_t s_mx[8];
   uint32_t mx = threadIdx.x < parts ? __ldcg(part + threadIdx.x) : 0u;
@@ -625,6 +636,17 @@ int64_t b200_gemm_w8_workspace_bytes(int M, int64_t K) {
 int b200_gemm_w8(const b200_weight *w, const float *A, int M, int64_t lda, float *C, int64_t ldc,
                  const float *residual, int64_t ldr, const float *norm_weight, float norm_eps,
                  int silu_pairs, void *workspace, int64_t workspace_bytes, void *stream) {
+  return b200::gemm_w8_run(w, A, M, lda, C, ldc, residual, ldr, norm_weight, norm_eps, silu_pairs, workspace, workspace_bytes,
+                           false, (cudaStream_t)stream);
+}
+
+} // extern "C"
+
+namespace b200 {
+// in_pass: a call of a session's pass, whose weights no kernel of the pass writes.
+int gemm_w8_run(const b200_weight *w, const float *A, int M, int64_t lda, float *C, int64_t ldc, const float *residual,
+                int64_t ldr, const float *norm_weight, float norm_eps, int silu_pairs, void *workspace,
+                int64_t workspace_bytes, bool in_pass, cudaStream_t st) {
   if (!w || !A || !C || !workspace)
     return fail(B200_EINVAL, "gemm_w8: null argument");
   if (w->kind != B200_W_I8 || w->scale_dtype != B200_F32 || !w->scale || !w->w)
@@ -637,7 +659,6 @@ int b200_gemm_w8(const b200_weight *w, const float *A, int M, int64_t lda, float
     return fail(B200_EINVAL, "gemm_w8: workspace too small");
   if (int rc = ensure_device())
     return rc;
-  cudaStream_t st = (cudaStream_t)stream;
   const int K = (int)w->K, N = (int)w->N, m_tiles = (M + kPlaneRows - 1) / kPlaneRows;
   char *ws = (char *)workspace;
   float *row_scale = reinterpret_cast<float *>(ws + kHeadBytes);
@@ -663,7 +684,7 @@ int b200_gemm_w8(const b200_weight *w, const float *A, int M, int64_t lda, float
     T *= 2;
   const int vec = (lda & 3) == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)norm_weight & 15) == 0;
   if (int rc = launch_after(planes_kernel, dim3((M + 256 / T - 1) / (256 / T)), 256, 0, st, A, lda, M, K, norm_weight, norm_eps, T,
-                            vec, planes, row_scale, reinterpret_cast<uint32_t *>(ws), 16 + kMaxPartialTiles))
+                            vec, planes, row_scale, reinterpret_cast<uint32_t *>(ws), 16 + kMaxPartialTiles, in_pass ? 1 : 0))
     return rc;
   // 256 columns per CTA (fewer bytes per operation) when that still gives every SM its two CTAs
   if ((int64_t)((N + 255) / 256) * m_tiles >= 296) {
@@ -673,6 +694,9 @@ int b200_gemm_w8(const b200_weight *w, const float *A, int M, int64_t lda, float
   p.splits = split_k((N + 127) / 128 * m_tiles, (K + BK - 1) / BK, std::min(M, kPlaneRows));
   return launch_gemm<128, true>(planes, m_tiles * BM, w->w, p, m_tiles, st);
 }
+} // namespace b200
+
+extern "C" {
 
 /* W8A8 (buddy-mlir's QuantizedMatmulOp): workspace = b200_gemm_w8a8_workspace_bytes(M, K). */
 int64_t b200_gemm_w8a8_workspace_bytes(int M, int64_t K) {
@@ -683,7 +707,8 @@ int64_t b200_gemm_w8a8_workspace_bytes(int M, int64_t K) {
 
 int b200_gemm_w8a8(const b200_weight *w, const float *A, int M, int64_t lda, float *C, int64_t ldc,
                    void *workspace, int64_t workspace_bytes, void *stream) {
-  return b200::gemm_w8a8_fused(w, A, M, lda, C, ldc, nullptr, 0, 0, workspace, workspace_bytes, (cudaStream_t)stream);
+  return b200::gemm_w8a8_fused(w, A, M, lda, C, ldc, nullptr, 0, 0, workspace, workspace_bytes, false,
+                               (cudaStream_t)stream);
 }
 
 } // extern "C"
@@ -695,7 +720,7 @@ namespace b200 {
 // separate operations.
 int gemm_w8a8_fused(const b200_weight *w, const float *A, int M, int64_t lda, float *C, int64_t ldc,
                     const float *residual, int64_t ldr, int silu_pairs, void *workspace, int64_t workspace_bytes,
-                    cudaStream_t stream) {
+                    bool in_pass, cudaStream_t st) {
   if (!w || !A || !C || !workspace)
     return fail(B200_EINVAL, "gemm_w8a8: null argument");
   if (silu_pairs && ((w->N & 1) || residual))
@@ -710,7 +735,6 @@ int gemm_w8a8_fused(const b200_weight *w, const float *A, int M, int64_t lda, fl
     return fail(B200_EINVAL, "gemm_w8a8: workspace too small");
   if (int rc = ensure_device())
     return rc;
-  cudaStream_t st = (cudaStream_t)stream;
   const int K = (int)w->K, N = (int)w->N, m_tiles = (M + BM - 1) / BM;
   char *ws = (char *)workspace;
   float *act_scale = reinterpret_cast<float *>(ws) + 2;
@@ -734,7 +758,7 @@ int gemm_w8a8_fused(const b200_weight *w, const float *A, int M, int64_t lda, fl
   const int vec = (lda & 3) == 0 && ((uintptr_t)A & 15) == 0;
   const int parts = (int)std::min<int64_t>(((int64_t)M * K / 4 + 1023) / 1024, kMaxParts);
   if (int rc = launch_after(absmax_kernel, dim3(parts), 256, 0, st, A, lda, M, K, vec, part, reinterpret_cast<uint32_t *>(ws),
-                            p.arrived))
+                            p.arrived, in_pass ? 1 : 0))
     return rc;
   const int64_t units = (int64_t)M * (K / 16);
   if (int rc = launch_after(quantize_kernel, dim3((unsigned)((units + 255) / 256)), 256, 0, st, A, lda, M, K, vec,

@@ -162,7 +162,9 @@ int b200_gemv(const b200_weight *w, const b200_gemv_args *a, void *stream);
  * fixed-point number in units of its row, three int8 digits whose sums of
  * products are exact (tcgen05.mma kind::i8) and added in f32.  workspace:
  * b200_gemm_w8_workspace_bytes(M, K) bytes, 256-byte aligned, owned by the
- * caller (it holds the digits, shares of split tiles and an error word).  b200_gemm_w8_status() reports a bounded wait that gave up. */
+ * caller (it holds the digits, shares of split tiles and an error word).
+ * b200_gemm_w8_status() reports a bounded wait that gave up.  All reads,
+ * weights included, come after the work that precedes the call on `stream`. */
 int64_t b200_gemm_w8_workspace_bytes(int M, int64_t K);
 int b200_gemm_w8(const b200_weight *w, const float *A, int M, int64_t lda,
                  float *C, int64_t ldc, const float *residual, int64_t ldr,
