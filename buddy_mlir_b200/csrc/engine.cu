@@ -1782,7 +1782,7 @@ static int prefill_reserve(b200_model *m, int rows, int logit_rows) {
     if (int rc = dev_alloc((void **)&m->pf_att, (size_t)rows * m->qh * D * 4)) return rc;
     if (int rc = dev_alloc((void **)&m->pf_mid, (size_t)rows * m->ffn * 4)) return rc;
     if (int rc = dev_alloc(&m->pf_ws, (size_t)m->pf_ws_bytes)) return rc;
-    B200_CUDA(cudaMemsetAsync(m->pf_ws, 0, 256, m->stream));   // the GEMM's error word (float projections never touch it)
+    B200_CUDA(cudaMemsetAsync(m->pf_ws, 0, 256, m->stream));   // the GEMMs' error word, collected over a pass
     if (int rc = dev_alloc((void **)&m->pf_tokens, (size_t)rows * 4)) return rc;
     if (m->act_int8)
       if (int rc = dev_alloc((void **)&m->pf_norm, (size_t)rows * c.hidden * 4)) return rc;
@@ -1830,6 +1830,8 @@ static int rows_status_queue(b200_model *m) {
 }
 static int rows_status(b200_model *m) {
   const int gemm = m->h_state_pinned[8], attn = m->h_state_pinned[9];
+  if (gemm)   // the words collect the first code of a pass; no kernel clears them
+    cudaMemsetAsync(m->pf_ws, 0, 4, m->stream);
   if (attn)
     cudaMemsetAsync(m->pf_kv, 0, 4, m->stream);
   if (gemm || attn)

@@ -370,7 +370,7 @@ __device__ __forceinline__ int unit_k(int u, int j, int units) {
 // A[M,K] f32 -> planes [ceil(M/42)][3][42] (+ 2 unused rows) [K] int8 in the k order of the packed weight rows, and the rows' scales; optional
 // RMSNorm of every row (the factor 1/rms goes into the scale).  T threads per row, a thread takes 16-byte units: it reads
 // four groups of four k and writes whole 16-byte pieces of the planes.  The row is read once and stays in registers up to
-// 48 T elements.  Also clears the GEMM's error word and counters.
+// 48 T elements.  Also clears the GEMM's counters and, outside a pass, its error word (head).
 constexpr int kUnits = 3;
 __global__ void __launch_bounds__(256)
 planes_kernel(const float *A, int64_t lda, int M, int K, const float *norm_w, float eps, int T, int vec, uint8_t *planes,
@@ -473,15 +473,15 @@ planes_kernel(const float *A, int64_t lda, int M, int K, const float *norm_w, fl
 // (+ bias).  Every step is reproduced operation by operation, so the result is bit-identical to the reference arithmetic.
 constexpr int kMaxParts = 256;   // partial maxima, in the workspace head
 
-// max |x| of every CTA's share of the tensor (non-negative floats order like their bit patterns); clears the GEMM's error
-// word and counters.
+// max |x| of every CTA's share of the tensor (non-negative floats order like their bit patterns); clears the GEMM's counters
+// and its error word (null in a pass: the word collects what any of its GEMMs leaves).
 __global__ void __launch_bounds__(256)
 absmax_kernel(const float *A, int64_t lda, int M, int K, int vec, uint32_t *part, uint32_t *error, uint32_t *arrived,
               int in_pass) {
   chain_start(in_pass);
   __shared__ uint32_t s_mx[8];
   if (blockIdx.x == 0) {
-    if (threadIdx.x == 0)
+    if (threadIdx.x == 0 && error != nullptr)
       *error = 0u;
     for (int i = threadIdx.x; i < kMaxPartialTiles; i += 256)
       arrived[i] = 0u;
@@ -643,7 +643,8 @@ int b200_gemm_w8(const b200_weight *w, const float *A, int M, int64_t lda, float
 } // extern "C"
 
 namespace b200 {
-// in_pass: a call of a session's pass, whose weights no kernel of the pass writes.
+// in_pass: a call of a session's pass, whose weights no kernel of the pass writes, and whose error word the session clears when
+// it reads it at the end of the pass.
 int gemm_w8_run(const b200_weight *w, const float *A, int M, int64_t lda, float *C, int64_t ldc, const float *residual,
                 int64_t ldr, const float *norm_weight, float norm_eps, int silu_pairs, void *workspace,
                 int64_t workspace_bytes, bool in_pass, cudaStream_t st) {
@@ -684,7 +685,8 @@ int gemm_w8_run(const b200_weight *w, const float *A, int M, int64_t lda, float 
     T *= 2;
   const int vec = (lda & 3) == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)norm_weight & 15) == 0;
   if (int rc = launch_after(planes_kernel, dim3((M + 256 / T - 1) / (256 / T)), 256, 0, st, A, lda, M, K, norm_weight, norm_eps, T,
-                            vec, planes, row_scale, reinterpret_cast<uint32_t *>(ws), 16 + kMaxPartialTiles, in_pass ? 1 : 0))
+                            vec, planes, row_scale, in_pass ? p.arrived : reinterpret_cast<uint32_t *>(ws),
+                            in_pass ? kMaxPartialTiles : 16 + kMaxPartialTiles, in_pass ? 1 : 0))
     return rc;
   // 256 columns per CTA (fewer bytes per operation) when that still gives every SM its two CTAs
   if ((int64_t)((N + 255) / 256) * m_tiles >= 296) {
@@ -757,8 +759,8 @@ int gemm_w8a8_fused(const b200_weight *w, const float *A, int M, int64_t lda, fl
   p.arrived = reinterpret_cast<uint32_t *>(ws) + 16;
   const int vec = (lda & 3) == 0 && ((uintptr_t)A & 15) == 0;
   const int parts = (int)std::min<int64_t>(((int64_t)M * K / 4 + 1023) / 1024, kMaxParts);
-  if (int rc = launch_after(absmax_kernel, dim3(parts), 256, 0, st, A, lda, M, K, vec, part, reinterpret_cast<uint32_t *>(ws),
-                            p.arrived, in_pass ? 1 : 0))
+  if (int rc = launch_after(absmax_kernel, dim3(parts), 256, 0, st, A, lda, M, K, vec, part,
+                            in_pass ? nullptr : reinterpret_cast<uint32_t *>(ws), p.arrived, in_pass ? 1 : 0))
     return rc;
   const int64_t units = (int64_t)M * (K / 16);
   if (int rc = launch_after(quantize_kernel, dim3((unsigned)((units + 255) / 256)), 256, 0, st, A, lda, M, K, vec,

@@ -1,0 +1,60 @@
+"""The host side of the library over the stand-in CUDA runtime (fake_cudart.c): failures that are made on the host."""
+import ctypes as C
+
+import numpy as np
+
+import fake_runtime
+
+
+def test_a_pass_keeps_the_error_of_any_of_its_gemms(tmp_path):
+    fake_runtime.run(tmp_path, "test_host_runtime", "errors_of_a_pass")
+
+
+def errors_of_a_pass(fake):
+    """Every GEMM of a pass in turn 'gives up': the n-th launch writes the code a bounded wait leaves, and what the kernels around
+    it clear is cleared.  The pass has to fail, and the pass after it to succeed."""
+    from buddy_mlir_b200 import TINY_MEGA, _lib, synthetic
+    from buddy_mlir_b200.session import BatchSession, ModelSession
+    state = {"n": 0, "fail": -1}
+
+    def launch(name, grid, args):
+        p = lambda i, kind: C.cast(args[i], C.POINTER(kind))[0]
+        if "planes_kernel" in name:
+            clear, at = p(11, C.c_int), p(10, C.c_void_p)
+            C.memset(at, 0, 4 * clear)
+        elif "absmax_kernel" in name and p(6, C.c_void_p):
+            C.memset(p(6, C.c_void_p), 0, 4)
+        elif "gemm_i8_kernel" in name:
+            if state["n"] == state["fail"]:
+                # GemmParams::error
+                C.cast(C.cast(args[2], C.POINTER(C.c_void_p))[12], C.POINTER(C.c_int))[0] = 702
+            state["n"] += 1
+    fake.on_launch(launch)
+    _, views = synthetic.make_f32_blob(TINY_MEGA, 3)
+    for int8 in (False, True):
+        s = ModelSession(TINY_MEGA)
+        s.load_tensors(views, quantize_to="w8")
+        s.set_activation_int8(int8)
+        batch = None if int8 else BatchSession(s, 2, 16, 16, 64)
+
+        def one_pass(fail):
+            state.update(n=0, fail=fail)
+            try:
+                if batch is None:
+                    s.prefill_rows(np.arange(5), 0, all_rows=False)
+                else:
+                    q = batch.add()
+                    try:
+                        batch.prefill(q, np.arange(5))
+                    finally:
+                        batch.remove(q)
+            except _lib.B200Error as e:
+                assert "code 702" in str(e)
+                return False
+            return True
+        assert one_pass(-1)
+        gemms = state["n"]
+        assert gemms == 4 * TINY_MEGA.n_layers + 1
+        for i in range(gemms):
+            assert not one_pass(i), i
+            assert one_pass(-1), i
