@@ -40,6 +40,21 @@ int ensure_device();
                           cudaGetErrorString(e_), __FILE__, __LINE__);         \
   } while (0)
 
+// A kernel's limit of dynamic shared memory belongs to a device: raised on each device a kernel is launched on, once.
+struct RaisedOn {
+  std::atomic<bool> device[64];   // (zero: static storage)
+};
+inline int raise_shared_limit(RaisedOn &done, const void *kern, int bytes) {
+  int dev = 0;
+  B200_CUDA(cudaGetDevice(&dev));
+  if (dev >= 0 && dev < 64 && done.device[dev].load(std::memory_order_acquire))
+    return B200_OK;
+  B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  if (dev >= 0 && dev < 64)
+    done.device[dev].store(true, std::memory_order_release);
+  return B200_OK;
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1)

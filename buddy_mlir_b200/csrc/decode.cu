@@ -1081,15 +1081,9 @@ int dec_launch(const DecParams &p, int grid, size_t smem, cudaStream_t st) {
 #undef B200_G
   default: return fail(B200_EINVAL, "decode kernel: group size %d not built", G);
   }
-  // the attribute belongs to the device's copy of the function: set it once per device and kernel
-  static std::atomic<bool> configured[64][9][3];
-  int dev = 0;
-  B200_CUDA(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64 || !configured[dev][G][mode].load(std::memory_order_acquire)) {
-    B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    if (dev >= 0 && dev < 64)
-      configured[dev][G][mode].store(true, std::memory_order_release);
-  }
+  static RaisedOn raised[9][3];
+  if (int rc = raise_shared_limit(raised[G][mode], kern, 227 * 1024))
+    return rc;
   void *args[] = {(void *)&p};
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);

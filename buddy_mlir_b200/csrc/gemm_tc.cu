@@ -593,14 +593,9 @@ int launch_gemm(const void *a, int a_rows, const void *w, GemmParams &p, int m_t
   if (int rc = make_map(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, BK, const_cast<void *>(w), p.K, p.N, (uint64_t)p.K,
                         CU_TENSOR_MAP_SWIZZLE_128B, BN))
     return rc;
-  static std::atomic<bool> configured[64];
-  int dev = 0;
-  B200_CUDA(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
-    B200_CUDA(cudaFuncSetAttribute(gemm_i8_kernel<BN, PLANES>, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring<BN>::SMEM));
-    if (dev >= 0 && dev < 64)
-      configured[dev].store(true, std::memory_order_release);
-  }
+  static RaisedOn raised;
+  if (int rc = raise_shared_limit(raised, (const void *)gemm_i8_kernel<BN, PLANES>, Ring<BN>::SMEM))
+    return rc;
   return launch_after(gemm_i8_kernel<BN, PLANES>, dim3((p.N + BN - 1) / BN, m_tiles, p.splits), kThreads, Ring<BN>::SMEM, st,
                       map_a, map_w, p);
 }

@@ -521,12 +521,9 @@ static int launch(const GemvP &p, int warps, cudaStream_t st) {
   auto kern = gemv_kernel<KIND, MT, R, GROUPED>;
   const size_t smem = ((size_t)MT * p.kc + (p.in_place4 ? p.kc / 4 : 0)) * sizeof(float);
   if (smem > 40 * 1024) {  // dynamic + static shared memory may exceed the 48 KB default
-    static thread_local size_t configured = 0;
-    if (smem > configured) {
-      B200_CUDA(cudaFuncSetAttribute(
-          kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-      configured = 200 * 1024;
-    }
+    static RaisedOn raised;
+    if (int rc = raise_shared_limit(raised, (const void *)kern, 200 * 1024))
+      return rc;
   }
   const int64_t rows_per_cta = (int64_t)warps * R;
   int64_t grid = (p.N + rows_per_cta - 1) / rows_per_cta;

@@ -506,11 +506,9 @@ template <int KIND, int COLS, bool GROUPED, bool XF> static int launch_mma(MmaP 
   // all warps take part (int4 14336 x 4096, 5 rows: 7 warps hold tiles).
   const int threads = (p.M > 1 ? W : p.slots * p.ks) * 32;
   p.reg_x = p.M == 1 && nblk * blk >= span && p.units * 4 <= (U4 ? 3 : 6) * threads;
-  static std::atomic<bool> configured{false};
-  if (!configured.load(std::memory_order_acquire)) {
-    B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmem));
-    configured.store(true, std::memory_order_release);
-  }
+  static RaisedOn raised;
+  if (int rc = raise_shared_limit(raised, (const void *)kern, kMmaSmem))
+    return rc;
   kern<<<grid, threads, smem, st>>>(p);
   B200_LAUNCH_CHECK();
   return B200_OK;

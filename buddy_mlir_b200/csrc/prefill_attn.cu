@@ -525,14 +525,9 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(const AttnPar
 template <int D>
 int launch_attn(const AttnParams &p, const float *kc, const float *vc, int kv_heads, int q_tiles, int max_splits, int n_keys,
                 const int32_t *table, int page, uint8_t *images, cudaStream_t st) {
-  static std::atomic<bool> configured[64];
-  int dev = 0;
-  B200_CUDA(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
-    B200_CUDA(cudaFuncSetAttribute(prefill_attn_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<D>::SMEM));
-    if (dev >= 0 && dev < 64)
-      configured[dev].store(true, std::memory_order_release);
-  }
+  static RaisedOn raised;
+  if (int rc = raise_shared_limit(raised, (const void *)prefill_attn_kernel<D>, Tile<D>::SMEM))
+    return rc;
   if (int rc = launch_after(kv_image_kernel<D>, dim3(p.key_tiles, kv_heads, 2 * kKeys * (D / 8) / 256), 256, 0, st, kc, vc,
                             p.max_len, n_keys, table, page, images, p.arrived, max_splits > 1 ? q_tiles * kv_heads : 0))
     return rc;

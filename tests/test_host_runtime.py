@@ -58,3 +58,25 @@ def errors_of_a_pass(fake):
         for i in range(gemms):
             assert not one_pass(i), i
             assert one_pass(-1), i
+
+
+def test_shared_memory_limits_are_raised_on_every_device(tmp_path):
+    fake_runtime.run(tmp_path, "test_host_runtime", "calls_on_several_devices")
+
+
+def calls_on_several_devices(fake):
+    """The calls that need more than 48 KB of shared memory, on one device after the other, and back: the limit belongs to the
+    device that is current."""
+    from buddy_mlir_b200 import _lib
+    lib, device = _lib.load(), fake.value("fake_device", C.c_int)
+    buf = np.zeros(1 << 16, dtype=np.uint8)
+    at = (buf.ctypes.data + 255) // 256 * 256
+    for d in (0, 1, 0, 5):
+        device.value = d
+        for kind, K, N, M in ((_lib.W_I8, 8960, 1536, 5), (_lib.W_I8, 8960, 1536, 1), (_lib.W_U4, 4096, 14336, 16), (_lib.W_F32, 14336, 1024, 1),
+                              (_lib.W_F32, 8960, 1536, 16), (_lib.W_I8, 70000, 1024, 4)):
+            w = _lib.Weight(kind, 128 if kind == _lib.W_U4 else 0, K, N, at, at, _lib.F16 if kind == _lib.W_U4 else _lib.F32, 0, None)
+            a = _lib.GemvArgs(at, _lib.F32, _lib.F32, K, N, at, None, None, 0.0, M, 0, 0)
+            assert lib.b200_gemv(C.byref(w), C.byref(a), None) == 0, (d, kind, K, N, M, lib.b200_last_error())
+        w = _lib.Weight(_lib.W_I8, 0, 1536, 1536, at, at, _lib.F32, 0, None)
+        assert lib.b200_gemm_w8(C.byref(w), at, 64, 1536, at, 1536, None, 0, None, 0.0, 0, at, 1 << 40, None) == 0
