@@ -306,6 +306,7 @@ struct b200_model {
   DecParams dp{};
   int dec_grid = 0;
   size_t dec_smem = 0;
+  bool persistent_tried = false;
   uint8_t *dec_stream = nullptr;     // the weights once more, as the kernel's warps consume them
   int64_t *dec_offsets = nullptr;    // [(4L+1)+1][grid * warps]: offsets of every projection, starts of the streams
   DecLayer *dec_layers = nullptr;
@@ -585,7 +586,20 @@ bool persistent_eligible(const b200_model *m, int grid, DecPhase (&ph)[5]) {
   return fits(m->lm_head, ph[4]);
 }
 
-int build_persistent(b200_model *m) {
+void release_persistent(b200_model *m) {
+  cudaStreamSynchronize(m->stream);
+  cudaFree(m->dec_stream); cudaFree(m->dec_offsets); cudaFree(m->dec_layers);
+  cudaFree(m->ll_buf); cudaFree(m->d_trace);
+  m->dec_stream = nullptr;
+  m->dec_offsets = nullptr;
+  m->dec_layers = nullptr;
+  m->ll_buf = nullptr;
+  m->d_trace = nullptr;
+  m->dp = DecParams{};
+  m->persistent = false;
+}
+
+int try_persistent(b200_model *m) {
   const b200_model_config &c = m->cfg;
   int dev = 0, sms = 0, coop = 0;
   B200_CUDA(cudaGetDevice(&dev));
@@ -695,52 +709,83 @@ int build_persistent(b200_model *m) {
   m->persistent = true;
   return B200_OK;
 }
+// The kernel's copy of the weights is there for speed only: a session whose weights fit once runs its steps as a graph.
+int build_persistent(b200_model *m) {
+  m->persistent_tried = true;
+  int rc = try_persistent(m);
+  if (rc == B200_ENOMEM) {   // once more without the projections that finalize has fused and not yet freed
+    release_persistent(m);
+    for (auto &L : m->layers) { L.gate.release(); L.up.release(); }
+    rc = try_persistent(m);
+  }
+  if (rc != B200_OK)
+    release_persistent(m);
+  return rc == B200_ENOMEM ? B200_OK : rc;
+}
+// What a session allocates once it runs: if memory is short, that copy is given back (and made again if that did not help).
+int session_alloc(b200_model *m, void **p, size_t bytes) {
+  int rc = dev_alloc(p, bytes);
+  if (rc == B200_ENOMEM && m->persistent) {
+    release_persistent(m);
+    rc = dev_alloc(p, bytes);
+    if (rc != B200_OK) {
+      (void)build_persistent(m);
+      rc = fail(B200_ENOMEM, "out of device memory (%zu bytes)", bytes);
+    }
+  }
+  return rc;
+}
 
 int set_state(b200_model *m, int token, int pos);
 
-// The decode step of the w8a8 arithmetic: the same kernels as the float step except for the int8
-// projections, captured into a graph of its own the first time it is needed.  The caller has
-// set the device state (token, position); the warm-up pass outside capture runs that very step
-// (it writes the K/V row the real step writes again), then the state is put back.
-int run_step_int8(b200_model *m) {
-  if (!m->exec_q) {
+// Records the step of the arithmetic that is set.
+int capture_step(b200_model *m, cudaGraph_t *graph, cudaGraphExec_t *exec) {
+  B200_CUDA(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
+  int rc = issue_step(m, nullptr);
+  cudaGraph_t g = nullptr;
+  cudaError_t e = cudaStreamEndCapture(m->stream, &g);
+  if (rc != B200_OK) {
+    if (g) cudaGraphDestroy(g);
+    return rc;
+  }
+  if (e != cudaSuccess)
+    return fail(B200_ECUDA, "graph capture: %s", cudaGetErrorString(e));
+  *graph = g;
+  B200_CUDA(cudaGraphInstantiate(exec, g, 0));
+  return B200_OK;
+}
+
+// A decode step as a graph of kernels.  The w8a8 arithmetic (the float step's kernels except for the int8 projections) has a
+// graph of its own; both are captured when first needed (the float one by finalize, or here if the persistent kernel has been
+// given up).  The caller has set the device state (token, position); the warm-up pass outside capture runs that very step (it
+// writes the K/V row the real step writes again), then the state is put back.
+int run_step_graph(b200_model *m) {
+  const bool q = m->act_int8;
+  cudaGraphExec_t &exec = q ? m->exec_q : m->exec;
+  int &kernels = q ? m->kernels_per_step_q : m->kernels_per_step;
+  if (!exec) {
     const b200_model_config &c = m->cfg;
     int64_t Kmax = c.hidden > m->ffn ? c.hidden : m->ffn;
     if ((int64_t)m->qh * c.head_dim > Kmax) Kmax = (int64_t)m->qh * c.head_dim;
-    if (!m->q_row) {
-      if (int rc = dev_alloc((void **)&m->q_row, (size_t)Kmax)) return rc;
-      if (int rc = dev_alloc((void **)&m->q_scale, 16)) return rc;
+    if (q && !m->q_row) {
+      if (int rc = session_alloc(m, (void **)&m->q_row, (size_t)Kmax)) return rc;
+      if (int rc = session_alloc(m, (void **)&m->q_scale, 16)) return rc;
     }
     const int token = m->h_state_pinned[0], pos = m->h_state_pinned[1];
-    if (int rc = issue_step(m, &m->kernels_per_step_q)) return rc;
+    if (int rc = issue_step(m, &kernels)) return rc;
     B200_CUDA(cudaStreamSynchronize(m->stream));
     if (int rc = set_state(m, token, pos)) return rc;
-    B200_CUDA(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
-    int rc = issue_step(m, nullptr);
-    cudaGraph_t g = nullptr;
-    cudaError_t e = cudaStreamEndCapture(m->stream, &g);
-    if (rc != B200_OK) {
-      if (g) cudaGraphDestroy(g);
-      return rc;
-    }
-    if (e != cudaSuccess)
-      return fail(B200_ECUDA, "graph capture (w8a8 step): %s", cudaGetErrorString(e));
-    m->graph_q = g;
-    B200_CUDA(cudaGraphInstantiate(&m->exec_q, m->graph_q, 0));
+    if (int rc = capture_step(m, q ? &m->graph_q : &m->graph, &exec)) return rc;
   }
-  B200_CUDA(cudaGraphLaunch(m->exec_q, m->stream));
-  count_launch(m->kernels_per_step_q);
+  B200_CUDA(cudaGraphLaunch(exec, m->stream));
+  count_launch(kernels);
   return B200_OK;
 }
 
 int run_step(b200_model *m) {
-  if (m->act_int8)
-    return run_step_int8(m);
-  if (m->persistent)
+  if (m->persistent && !m->act_int8)
     return dec_launch(m->dp, m->dec_grid, m->dec_smem, m->stream);
-  B200_CUDA(cudaGraphLaunch(m->exec, m->stream));
-  count_launch(m->kernels_per_step);
-  return B200_OK;
+  return run_step_graph(m);
 }
 
 int check_step_error(b200_model *m) {
@@ -1264,6 +1309,8 @@ int b200_model_set_activation_int8(b200_model *m, int enabled) {
   if (enabled && m->tp != 1)
     return fail(B200_ESTATE, "set_activation_int8: single-GPU sessions only");
   m->act_int8 = enabled != 0;
+  if (!enabled && m->finalized && !m->persistent_tried && m->tp == 1)
+    return build_persistent(m);
   return B200_OK;
 }
 int b200_model_activation_int8(const b200_model *m) { return m && m->act_int8 ? 1 : 0; }
@@ -1555,7 +1602,9 @@ int b200_model_finalize(b200_model *m) {
     if (int rc = fuse_linears({&L.gate, &L.up}, true, &L.gateup, m->stream)) return rc;
     L.q.release(); L.k.release(); L.v.release();
   }
-  if (int rc = build_persistent(m)) return rc;
+  if (!m->act_int8)   // the w8a8 step is a graph; set_activation_int8 builds the kernel's weights if it is switched off
+    if (int rc = build_persistent(m)) return rc;
+  // not before: with the copy in their place a step of the 1.5B int8 model at 97 keys takes 737 us instead of 729
   for (auto &L : m->layers) { L.gate.release(); L.up.release(); }
   if (m->persistent) {
     // warm the kernel once (shared-memory attribute, module load), then clear the row it wrote
@@ -1587,18 +1636,7 @@ int b200_model_finalize(b200_model *m) {
   B200_CUDA(cudaStreamSynchronize(m->stream));
   for (auto p : m->kv)  // the warm-up wrote row 0
     B200_CUDA(cudaMemsetAsync(p, 0, (size_t)m->kvh * c.max_len * c.head_dim * 4, m->stream));
-  B200_CUDA(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
-  int rc = issue_step(m, nullptr);
-  cudaGraph_t g = nullptr;
-  cudaError_t e = cudaStreamEndCapture(m->stream, &g);
-  if (rc != B200_OK) {
-    if (g) cudaGraphDestroy(g);
-    return rc;
-  }
-  if (e != cudaSuccess)
-    return fail(B200_ECUDA, "graph capture: %s", cudaGetErrorString(e));
-  m->graph = g;
-  B200_CUDA(cudaGraphInstantiate(&m->exec, m->graph, 0));
+  if (int rc = capture_step(m, &m->graph, &m->exec)) return rc;
   B200_CUDA(cudaStreamSynchronize(m->stream));
   m->finalized = true;
   return B200_OK;
@@ -1777,22 +1815,22 @@ static int prefill_reserve(b200_model *m, int rows, int logit_rows) {
     int64_t Kmax = c.hidden > m->ffn ? c.hidden : m->ffn;
     if ((int64_t)m->qh * D > Kmax) Kmax = (int64_t)m->qh * D;
     m->pf_ws_bytes = std::max(b200_gemm_w8_workspace_bytes(rows, Kmax), b200_gemm_w8a8_workspace_bytes(rows, Kmax));
-    if (int rc = dev_alloc((void **)&m->pf_x, (size_t)rows * c.hidden * 4)) return rc;
-    if (int rc = dev_alloc((void **)&m->pf_qkv, (size_t)rows * QKV * 4)) return rc;
-    if (int rc = dev_alloc((void **)&m->pf_att, (size_t)rows * m->qh * D * 4)) return rc;
-    if (int rc = dev_alloc((void **)&m->pf_mid, (size_t)rows * m->ffn * 4)) return rc;
-    if (int rc = dev_alloc(&m->pf_ws, (size_t)m->pf_ws_bytes)) return rc;
+    if (int rc = session_alloc(m, (void **)&m->pf_x, (size_t)rows * c.hidden * 4)) return rc;
+    if (int rc = session_alloc(m, (void **)&m->pf_qkv, (size_t)rows * QKV * 4)) return rc;
+    if (int rc = session_alloc(m, (void **)&m->pf_att, (size_t)rows * m->qh * D * 4)) return rc;
+    if (int rc = session_alloc(m, (void **)&m->pf_mid, (size_t)rows * m->ffn * 4)) return rc;
+    if (int rc = session_alloc(m, &m->pf_ws, (size_t)m->pf_ws_bytes)) return rc;
     B200_CUDA(cudaMemsetAsync(m->pf_ws, 0, 256, m->stream));   // the GEMMs' error word, collected over a pass
-    if (int rc = dev_alloc((void **)&m->pf_tokens, (size_t)rows * 4)) return rc;
+    if (int rc = session_alloc(m, (void **)&m->pf_tokens, (size_t)rows * 4)) return rc;
     if (m->act_int8)
-      if (int rc = dev_alloc((void **)&m->pf_norm, (size_t)rows * c.hidden * 4)) return rc;
+      if (int rc = session_alloc(m, (void **)&m->pf_norm, (size_t)rows * c.hidden * 4)) return rc;
     m->pf_rows = rows;
   }
   if (logit_rows > m->pf_logit_rows) {
     cudaFree(m->pf_logits);
     m->pf_logits = nullptr;
     m->pf_logit_rows = 0;
-    if (int rc = dev_alloc((void **)&m->pf_logits, (size_t)logit_rows * c.vocab * 4)) return rc;
+    if (int rc = session_alloc(m, (void **)&m->pf_logits, (size_t)logit_rows * c.vocab * 4)) return rc;
     m->pf_logit_rows = logit_rows;
   }
   return B200_OK;
@@ -1815,7 +1853,7 @@ static int prefill_attention_reserve(b200_model *m, int n_keys, int limit) {
   m->pf_kv = nullptr;
   m->pf_kv_bytes = 0;
   const int64_t bytes = prefill_attn_workspace_bytes((int)std::min<int64_t>(limit, 2 * (int64_t)n_keys), m->kvh, m->cfg.head_dim);
-  if (int rc = dev_alloc(&m->pf_kv, (size_t)(bytes + kPrefillKvHead))) return rc;
+  if (int rc = session_alloc(m, &m->pf_kv, (size_t)(bytes + kPrefillKvHead))) return rc;
   B200_CUDA(cudaMemsetAsync(m->pf_kv, 0, kPrefillKvHead, m->stream));
   m->pf_kv_bytes = bytes;
   return B200_OK;
@@ -1940,9 +1978,9 @@ static int batch_rows(b200_batch *b, int M, const int32_t *tokens, const int32_t
     cudaFree(b->d_seq); cudaFree(b->d_pos); cudaFree(b->d_next);
     b->d_seq = b->d_pos = b->d_next = nullptr;
     b->rows_cap = 0;
-    if (int rc = dev_alloc((void **)&b->d_seq, (size_t)M * 4)) return rc;
-    if (int rc = dev_alloc((void **)&b->d_pos, (size_t)M * 4)) return rc;
-    if (int rc = dev_alloc((void **)&b->d_next, (size_t)M * 4)) return rc;
+    if (int rc = session_alloc(m, (void **)&b->d_seq, (size_t)M * 4)) return rc;
+    if (int rc = session_alloc(m, (void **)&b->d_pos, (size_t)M * 4)) return rc;
+    if (int rc = session_alloc(m, (void **)&b->d_next, (size_t)M * 4)) return rc;
     b->rows_cap = M;
   }
   // a prefill chunk: consecutive positions of one sequence
@@ -2023,19 +2061,26 @@ int b200_batch_create(b200_model *m, int max_seqs, int page_size, int n_pages, i
     b->free_pages.push_back(i);
   const size_t pool_bytes = (size_t)n_pages * m->kvh * page_size * m->cfg.head_dim * 4;
   b->pool.assign(2 * m->cfg.n_layers, nullptr);
+  const bool persistent = m->persistent;
   int rc = B200_OK;
   for (auto &p : b->pool)
-    if (rc == B200_OK) rc = dev_alloc((void **)&p, pool_bytes);
-  if (rc == B200_OK) rc = dev_alloc((void **)&b->d_table, b->table.size() * 4);
+    if (rc == B200_OK) rc = session_alloc(m, (void **)&p, pool_bytes);
+  if (rc == B200_OK) rc = session_alloc(m, (void **)&b->d_table, b->table.size() * 4);
   b->max_context = b->table_stride * page_size;
   b->part_rows = max_seqs;
   if (rc == B200_OK)
-    rc = dev_alloc((void **)&b->d_part,
-                   (size_t)gqa_paged_scratch_floats(b->part_rows, m->qh, m->cfg.head_dim, b->max_context) * 4);
+    rc = session_alloc(m, (void **)&b->d_part,
+                       (size_t)gqa_paged_scratch_floats(b->part_rows, m->qh, m->cfg.head_dim, b->max_context) * 4);
   if (rc == B200_OK && cudaMemsetAsync(b->d_part, 0, (size_t)b->part_rows * m->qh * 4, m->stream) != cudaSuccess)   // the counters
     rc = fail(B200_ECUDA, "batch_create: cudaMemset failed");
   if (rc != B200_OK) {
     b200_batch_destroy(b);
+    if (persistent && !m->persistent) {   // given up for pools that did not fit all the same
+      char why[256];
+      snprintf(why, sizeof why, "%s", error_buffer());
+      (void)build_persistent(m);
+      fail(rc, "%s", why);
+    }
     return rc;
   }
   *out = b;

@@ -11,7 +11,7 @@ enum { OK = 0, INVALID = 1, NO_MEMORY = 2 };
 typedef struct { unsigned x, y, z; } dim3_;
 typedef struct { dim3_ grid, block; size_t smem; void *stream, *attrs; unsigned n; } config;
 
-size_t fake_memory = (size_t)1 << 40, fake_used;
+size_t fake_memory = (size_t)1 << 40, fake_used, fake_peak;
 int fake_device;
 void (*fake_on_launch)(const char *name, const unsigned *grid, void **args);
 
@@ -85,6 +85,7 @@ int cudaMalloc(void **p, size_t n) {
   memset(b + 4096, 0, (n + 8191) / 4096 * 4096 - 4096);
   *(size_t *)b = n;
   fake_used += n;
+  if (fake_used > fake_peak) fake_peak = fake_used;
   *p = b + 4096;
   return OK;
 }

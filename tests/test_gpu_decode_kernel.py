@@ -58,3 +58,26 @@ def test_mixed_float_and_int8_projections():
         s.decode(int(t))
         assert maxrel(s.logits_data(), om.decode(int(t))) < 1e-4
     s.close()
+
+
+def test_steps_without_the_kernels_copy_of_the_weights():
+    """A request that cannot be met takes the copy of the weights away and brings it back; the w8a8 arithmetic starts without it."""
+    from buddy_mlir_b200 import _lib
+    from buddy_mlir_b200.session import BatchSession
+    cfg = TINY_MEGA
+    _, views = synthetic.make_f32_blob(cfg, 5)
+    floats, ints = synthetic.split_w8a32(cfg, views, lambda w: orc.quantize_per_channel(w, 8))
+    om = orc.OracleModel(cfg, views, kinds={n: "w8" for n in synthetic.QUANTISED_BY_REFERENCE})
+    s = ModelSession(cfg)
+    s.load_blobs("w8a8", floats, ints)
+    assert not s.uses_persistent_kernel()
+    s.set_activation_int8(False)
+    assert s.uses_persistent_kernel()
+    for i, t in enumerate(synthetic.prompt_tokens(cfg, 2, 6)):
+        if i == 2:
+            with pytest.raises(_lib.B200Error):
+                BatchSession(s, 1, 16, 1 << 24, 64)     # pools of 256 GB
+            assert s.uses_persistent_kernel()
+        s.decode(int(t))
+        assert maxrel(s.logits_data(), om.decode(int(t))) < 1e-4
+    s.close()

@@ -80,3 +80,80 @@ def calls_on_several_devices(fake):
             assert lib.b200_gemv(C.byref(w), C.byref(a), None) == 0, (d, kind, K, N, M, lib.b200_last_error())
         w = _lib.Weight(_lib.W_I8, 0, 1536, 1536, at, at, _lib.F32, 0, None)
         assert lib.b200_gemm_w8(C.byref(w), at, 64, 1536, at, 1536, None, 0, None, 0.0, 0, at, 1 << 40, None) == 0
+
+
+def test_sessions_that_fit_without_the_decode_kernels_copy_of_the_weights(tmp_path):
+    fake_runtime.run(tmp_path, "test_host_runtime", "sessions_in_little_memory")
+
+
+def sessions_in_little_memory(fake):
+    """The persistent decode kernel keeps the linear weights a second time.  Where there is no room for that, a session that runs
+    without it still loads, prefills, serves batches and decodes."""
+    import os
+    from buddy_mlir_b200 import TINY_MEGA, _lib, synthetic
+    from buddy_mlir_b200.session import BatchSession, ModelSession
+    memory, used, peak = (fake.value("fake_" + n) for n in ("memory", "used", "peak"))
+    cfg = TINY_MEGA.with_(max_len=64)
+    _, views = synthetic.make_f32_blob(cfg, 3)
+
+    def session(quantize=None):
+        s = ModelSession(cfg)
+        s.load_tensors(views, quantize_to=quantize)
+        return s
+    os.environ["BUDDY_B200_DECODE"] = "graph"
+    s = session()
+    plain_peak, plain = peak.value, used.value
+    s.prefill_rows(np.arange(40), 0, all_rows=False)
+    batch = BatchSession(s, 2, 16, 8, 64)
+    busy_peak = peak.value
+    batch.close()
+    s.close()
+    del os.environ["BUDDY_B200_DECODE"]
+    s = session()
+    assert s.uses_persistent_kernel() and used.value > 1.5 * plain
+    full = used.value
+    s.close()
+    assert used.value == 0
+    # no room for the copy when the model is finalised
+    memory.value = max(plain_peak, busy_peak)
+    s = session()
+    assert not s.uses_persistent_kernel()
+    s.decode(3)
+    s.close()
+    # room for it then, but not for what a prefill or a batch needs later
+    for later in (lambda s: s.prefill_rows(np.arange(40), 0, all_rows=False), lambda s: BatchSession(s, 2, 16, 8, 64).close()):
+        memory.value = 1 << 40
+        s = session()
+        memory.value = max(full, busy_peak)
+        assert s.uses_persistent_kernel()
+        later(s)
+        assert not s.uses_persistent_kernel()
+        s.position_ = 0
+        s.decode(3)
+        s.generate(3, 2)
+        s.close()
+    # pools that never fit do not cost the session its kernel: nothing, one and several of the pools go through
+    for pages in (1 << 20, 2900, 900):
+        memory.value = 1 << 40
+        s = session()
+        memory.value = full + 1000000
+        try:
+            BatchSession(s, 2, 16, pages, 64)
+            raise SystemExit("the pools fit")
+        except _lib.B200Error as e:
+            assert "memory" in str(e)
+        assert s.uses_persistent_kernel() and used.value == full
+        s.decode(3)
+        s.close()
+    # the w8a8 arithmetic decodes without the kernel: no copy, until it is switched off
+    memory.value = 1 << 40
+    s = ModelSession(cfg)
+    floats, ints = synthetic.split_w8a32(cfg, views, lambda w: (np.ones_like(w, dtype=np.int8), np.ones((1, w.shape[1]), np.float32)))
+    s.load_blobs("w8a8", floats, ints)
+    assert not s.uses_persistent_kernel()
+    s.decode(3)
+    s.set_activation_int8(False)
+    assert s.uses_persistent_kernel()
+    s.position_ = 0
+    s.decode(3)
+    s.close()
