@@ -9,15 +9,23 @@
 // 1e-3 of the CPU restatement, as for the decode path).
 //
 // Operands.  Both are int8 and go from memory to the tensor cores as they are stored (tcgen05.mma kind::i8, s32
-// accumulators in tensor memory).  The weights are the packed decode rows.  A row of activations is a 23-bit fixed-point
+// accumulators in tensor memory).  The weights are the packed decode rows.  A row of activations is a 24-bit fixed-point
 // number per element, in units of a power of two taken from the row's largest magnitude, and its three base-256 digits are
 // three rows of the A operand: a tile of 128 rows is 42 activation rows x 3 digits (planes; two rows are left over), in the
 // k order of the packed weights.  All products and sums are exact integers; the epilogue adds the planes' sums in f32.
-// Against two bf16 terms per activation and weights converted to bf16 (the form before this one): half the bytes of the
-// weight operand, no pass that converts weights, and 2^-23 of the row's largest element instead of 2^-17 of each (measured
-// against f64: 2e-7 instead of 4e-6).  int8 runs at the bf16 rate on this part (2.4 POP/s at 2048 x 8960 x 8960), so three
-// planes are half as much again on the tensor pipe; what few rows need is bytes and latency, and what many rows save are
-// the passes around the GEMM.
+// Two bf16 terms per activation and weights converted to bf16, the form before this one, kept 2^-17 of each element; three
+// digits keep 2^-23 of the row's largest, which is less where a few channels of a row are far above the rest.  Such rows are
+// wide: six digits, in passes of their own over the tile (planes_kernel says which rows, wide_passes what they cost the others).
+// Relative error (2-norm, against f64) of the columns that do not use a channel R times the rest, 256 x 1536 x 1536:
+//   R            1        30       100      1000     10000
+//   now          1.7e-7   1.1e-6   9.4e-7   4.0e-7   8.1e-8
+//   three digits 3.2e-7   3.2e-6   1.0e-5   1.1e-4   9.9e-4    (for every row, 23 bits)
+//   two bf16     2.5e-6 for all; f32 products and sums 7.0e-7
+// Time with no wide row / one / all: 1024 x 17920 x 1536 103 / 112 / 250 us, 1000 x 1536 x 8960 50 / 77 / 139, 24 x 17920 x 1536
+// 11.5 / 21 / 29.
+// Against bf16: half the bytes of the weight operand and no pass that converts weights; three planes are three times the
+// operations of one bf16 product, at 2.4 POP/s (2048 x 8960 x 8960) against 1.6 PFLOP/s.  What few rows need is bytes and
+// latency, and what many rows save are the passes around the GEMM.
 //
 // W8A8 (b200_gemm_w8a8) is the same kernel with one plane: the tile's 128 rows are activation rows.
 //
@@ -48,6 +56,7 @@ namespace {
 constexpr int BM = 128;                        // rows of a tile of sums
 constexpr int BK = 128;                        // int8 per k block: one 128-byte swizzle row
 constexpr int kPlanes = 3, kPlaneRows = 42;    // digits per activation, activation rows per tile
+constexpr int kWidePlanes = 6, kWideRows = 21; // the same for rows that need six digits: half a tile's rows at a time
 constexpr int kThreads = 320;                  // loader, mma, 8 epilogue warps
 constexpr int kEpiWarps = 8;
 constexpr int kMaxStages = 3;
@@ -67,6 +76,7 @@ struct Bars {
   uint32_t tmem_base;
   int abort_flag;
   int last;                    // split-K: this CTA completes its tile
+  int wide;                    // halves of the tile's rows that have wide rows
 };
 
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar) {
@@ -91,7 +101,7 @@ __device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t da, uint64_t db
 struct GemmParams {
   int M, N, K;                 // K: multiple of 64
   const float *scale, *bias;   // [N], bias may be null
-  const float *row_scale;      // planes: [M]; W8A8: one value
+  const float *row_scale;      // planes: [M], negative for wide rows; W8A8: one value
   const float *residual;       // [M, ldr] or null; may alias C
   float *C;                    // [M, ldc]
   int64_t ldc, ldr;
@@ -108,9 +118,233 @@ __device__ __forceinline__ float silu_of(float g, float u) {
   return __fmul_rn(__fmul_rn(g, sg), u);
 }
 
+// The epilogue warps' part of a pass: a thread reads an accumulator row (its lane of tensor memory) and half of its columns; the
+// sums go to a padded tile in shared memory (the ring is idle by then), from where the warps add up the planes and write whole
+// rows, warp w rows w, w + 8, .. of the pass: lane j holds the scale of the j-th of them (row_scales).  SIX: the pass over the wide
+// rows of one half of the tile's rows.
+template <bool PLANES> __device__ __forceinline__ float row_scales(const GemmParams &p, int first, int rows) {
+  if (!PLANES)
+    return p.row_scale[0];
+  const int r = ((int)threadIdx.x >> 5) - 2 + (threadIdx.x & 31) * kEpiWarps;
+  return r < rows ? p.row_scale[blockIdx.y * kPlaneRows + first + r] : 0.f;
+}
+template <int BN, bool PLANES, bool SIX>
+__device__ __forceinline__ void store_tile(const GemmParams &p, Bars &bars, uint8_t *tiles, uint32_t tmem, bool ok, int half,
+                                           float scales) {
+  constexpr int kRows = PLANES ? kPlaneRows : BM;   // activation rows of the tile
+  constexpr int kStep = SIX ? kWideRows : kRows;
+  constexpr int kFold = SIX ? 1 : 8;                // shares of a split tile in flight
+  constexpr int LDS = 128 + 4;                      // row stride of the staging tile, in words
+  float *ep = reinterpret_cast<float *>(tiles);     // [BM][LDS]: 66 KB of the ring
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ew = warp - 2, quad = warp & 3;
+  const int m0 = blockIdx.y * kRows, n0 = blockIdx.x * BN, rows_all = min(kRows, p.M - m0);
+  const int first = SIX ? half * kWideRows : 0, rows = min(kStep, rows_all - first);   // the pass's rows of the tile
+#pragma unroll 1
+  for (int h = 0; h < BN / 128; ++h) {   // 128 columns of the accumulator at a time
+    const int nh = n0 + h * 128;
+    if (nh >= p.N)
+      break;
+    if (h > 0)   // the staging tile is free again once the previous half has been stored
+      asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
+    if (ok && (PLANES || quad * 32 < p.M - m0)) {   // lanes beyond M hold nothing
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      // a warp reads the 32 lanes of tensor memory that match its rank within its warpgroup; the two warps that share a
+      // lane quarter take half the columns each
+      const int row = quad * 32 + lane, cb0 = (ew >> 2) * 64;
+      const int d = row / kStep;   // PLANES: which digit; its weight is 2^16, 2^8, 1, 2^-7, 2^-15, 2^-23
+      const float f = __uint_as_float((uint32_t)(127 + 16 - 8 * d + (d >= kPlanes)) << 23);
+#pragma unroll 1
+      for (int cb = cb0; cb < cb0 + 64; cb += 32) {
+        uint32_t v[32];
+        const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(h * 128 + cb);
+        tmem_load32(taddr, v);
+        tmem_wait_load();
+        float *erow = ep + row * LDS + cb;
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+          float4 o;
+          if (PLANES)
+            o = make_float4(__int2float_rn((int)v[j]) * f, __int2float_rn((int)v[j + 1]) * f,
+                            __int2float_rn((int)v[j + 2]) * f, __int2float_rn((int)v[j + 3]) * f);
+          else
+            o = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]),
+                            __uint_as_float(v[j + 3]));
+          *reinterpret_cast<float4 *>(erow + j) = o;
+        }
+      }
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
+    const int cols = min(128, p.N - nh);
+    // sums of the pass's row r, columns c .. c + 3 of this CTA's k range
+    auto sums = [&](int r, int c) {
+      float4 a = *reinterpret_cast<const float4 *>(ep + r * LDS + c);
+      if (PLANES) {
+#pragma unroll
+        for (int q = 1; q < (SIX ? kWidePlanes : kPlanes); ++q) {
+          const float4 b = *reinterpret_cast<const float4 *>(ep + (q * kStep + r) * LDS + c);
+          a = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+        }
+      }
+      return a;
+    };
+    bool mine = ok;
+    int r0 = first, nr = rows;   // the rows to finish
+    const int tile = blockIdx.y * gridDim.x + blockIdx.x;
+    float4 *shares = reinterpret_cast<float4 *>(p.partial) + (int64_t)tile * p.splits * kRows * 32;
+    if (p.splits > 1) {   // (BN = 128) leave this CTA's share; after its last pass the last CTA of the tile goes on
+      if (ok)   // (a wide row's share is written again by the pass with six digits, which has nothing for other rows)
+#pragma unroll 1
+        for (int r = ew, j = 0; r < rows; r += kEpiWarps, ++j)
+          if (!SIX || signbit(__shfl_sync(0xffffffffu, scales, j)))
+            __stcg(shares + ((int64_t)blockIdx.z * kRows + first + r) * 32 + lane, sums(r, lane * 4));
+      mine = false;
+      if (!PLANES || bars.wide >> (SIX ? half + 1 : 0) == 0) {
+        __threadfence();
+        asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
+        if (threadIdx.x == 64)
+          bars.last = atomicAdd(p.arrived + tile, 1u) == (uint32_t)p.splits - 1;
+        asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
+        __threadfence();
+        mine = ok && bars.last;
+      }
+      r0 = 0;
+      nr = rows_all;
+      if (SIX)
+        scales = row_scales<PLANES>(p, 0, rows_all);
+    }
+    if (mine) {
+      const bool vec = (p.ldc & 3) == 0 && ((uintptr_t)p.C & 15) == 0 && (p.N & 3) == 0 &&
+                       (!p.residual || ((p.ldr & 3) == 0 && ((uintptr_t)p.residual & 15) == 0));
+#pragma unroll (SIX ? 1 : 2)
+      for (int r = ew, j = 0; r < nr; r += kEpiWarps, ++j) {
+        const float rs = PLANES ? __shfl_sync(0xffffffffu, scales, j) : scales;
+        const int i = r * 32 + lane, c = lane * 4, m = m0 + r0 + r, n = nh + c;
+        if (c >= cols || (PLANES && p.splits == 1 && signbit(rs) != SIX))   // (finished by another pass)
+          continue;
+        float y[4];
+        if (p.splits > 1) {
+          float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int z0 = 0; z0 < p.splits; z0 += kFold) {
+            float4 b[kFold];
+#pragma unroll
+            for (int z = 0; z < kFold; ++z)
+              b[z] = z0 + z < p.splits ? __ldcg(shares + (int64_t)(z0 + z) * kRows * 32 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int z = 0; z < kFold; ++z)
+              if (PLANES)
+                a = make_float4(a.x + b[z].x, a.y + b[z].y, a.z + b[z].z, a.w + b[z].w);
+              else
+                a = make_float4(__int_as_float(__float_as_int(a.x) + __float_as_int(b[z].x)),
+                                __int_as_float(__float_as_int(a.y) + __float_as_int(b[z].y)),
+                                __int_as_float(__float_as_int(a.z) + __float_as_int(b[z].z)),
+                                __int_as_float(__float_as_int(a.w) + __float_as_int(b[z].w)));
+          }
+          y[0] = a.x; y[1] = a.y; y[2] = a.z; y[3] = a.w;
+        } else {
+          const float4 a = sums(r, c);
+          y[0] = a.x; y[1] = a.y; y[2] = a.z; y[3] = a.w;
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int ne = min(n + e, p.N - 1);
+          if (PLANES)
+            y[e] = __fmul_rn(__fmul_rn(y[e], fabsf(rs)), __ldg(p.scale + ne));
+          else   // linalg.py:12836-12846: float(acc) * (act_scale * weight_scale[n])
+            y[e] = __fmul_rn(__int2float_rn(__float_as_int(y[e])), __fmul_rn(rs, __ldg(p.scale + ne)));
+          if (p.bias)
+            y[e] = __fadd_rn(y[e], __ldg(p.bias + ne));
+        }
+        if (p.silu_pairs) {
+          float *dst = p.C + (int64_t)m * p.ldc + (n >> 1);
+          dst[0] = silu_of(y[0], y[1]);
+          if (n + 3 < p.N)   // N is even
+            dst[1] = silu_of(y[2], y[3]);
+        } else {
+          float *dst = p.C + (int64_t)m * p.ldc + n;
+          const float *res = p.residual + (int64_t)m * p.ldr + n;
+          if (vec) {
+            if (p.residual) {
+              const float4 q = *reinterpret_cast<const float4 *>(res);
+              y[0] = __fadd_rn(q.x, y[0]);
+              y[1] = __fadd_rn(q.y, y[1]);
+              y[2] = __fadd_rn(q.z, y[2]);
+              y[3] = __fadd_rn(q.w, y[3]);
+            }
+            *reinterpret_cast<float4 *>(dst) = make_float4(y[0], y[1], y[2], y[3]);
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (n + e < p.N)
+                dst[e] = p.residual ? __fadd_rn(res[e], y[e]) : y[e];
+          }
+        }
+      }
+    }
+  }
+}
+
+// The tile's wide rows once more, with six digits: a half of its rows at a time (`halves`: which).  Everything a normal tile does
+// again, in a function of its own and with little code (no unrolling in SIX): the code counts even where it does not run.  Without
+// wide rows, 24 x 17920 x 1536 takes 13.5 us without this function, 13.9 with it, 16.3 with the loops unrolled as for a normal
+// tile; 1024 x 17920 x 1536 takes 106.8, 108.4, and 110.5 with these passes as a loop around the tile's code.
+template <int BN>
+__device__ __noinline__ void wide_passes(const CUtensorMap &map_x, const CUtensorMap &map_w, const GemmParams &p, uint8_t *tiles,
+                                         uint32_t tmem, int kb0, int nkb) {
+  using R = Ring<BN>;
+  constexpr int S = R::STAGES;
+  Bars &bars = *reinterpret_cast<Bars *>(tiles + S * R::STAGE_BYTES);
+  volatile int *ab = &bars.abort_flag;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, halves = bars.wide;
+  int g = nkb, phase = 1;   // k blocks that have gone through the ring, parity of the accumulator's barrier
+  for (int half = 0; half < 2; ++half) {
+    if (!(halves >> half & 1))
+      continue;
+    if (warp == 0) {
+      if (lane == 0)
+        for (int i = 0; i < nkb; ++i) {
+          const int s = (g + i) % S, u = (g + i) / S;
+          if (u > 0 && !mbar_wait(&bars.empty[s], (u - 1) & 1, ab, p.error, 701))
+            break;
+          mbar_expect_tx(&bars.full[s], R::STAGE_BYTES);
+          tma_load_2d(tiles + s * R::STAGE_BYTES + R::A_BYTES, &map_w, (kb0 + i) * BK, blockIdx.x * BN, &bars.full[s]);
+          tma_load_2d(tiles + s * R::STAGE_BYTES, &map_x, (kb0 + i) * BK, (blockIdx.y * 2 + half) * BM, &bars.full[s]);
+        }
+    } else if (warp == 1) {
+      if (lane == 0) {
+        for (int i = 0; i < nkb; ++i) {
+          const int s = (g + i) % S;
+          if (!mbar_wait(&bars.full[s], ((g + i) / S) & 1, ab, p.error, 702))
+            break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t a = smem_u32(tiles + s * R::STAGE_BYTES), w = a + R::A_BYTES;
+#pragma unroll
+          for (int k = 0; k < BK / 32; ++k)
+            mma_i8<BN>(tmem, smem_desc(a + k * 32), smem_desc(w + k * 32), (i | k) != 0);
+          tc_commit(&bars.empty[s]);
+        }
+        tc_commit(&bars.accum);
+      }
+    } else {
+      const int first = half * kWideRows;
+      const float scales = row_scales<true>(p, first, min(kWideRows, p.M - (int)blockIdx.y * kPlaneRows - first));
+      const bool ok = mbar_wait(&bars.accum, phase, ab, p.error, 703) && !*ab;
+      store_tile<BN, true, true>(p, bars, tiles, tmem, ok, half, scales);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the next pass loads over the staging tile
+    }
+    g += nkb;
+    phase ^= 1;
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (*ab)
+      break;
+  }
+}
+
 template <int BN, bool PLANES>
 __global__ void __launch_bounds__(kThreads, 2)
-gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const GemmParams p) {
+gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
+               const __grid_constant__ GemmParams p, const __grid_constant__ CUtensorMap map_x) {
   using R = Ring<BN>;
   constexpr int S = R::STAGES;
   constexpr int kRows = PLANES ? kPlaneRows : BM;   // activation rows of the tile
@@ -132,6 +366,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
     mbar_init(&bars.accum, 1);
     bars.abort_flag = 0;
+    bars.wide = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {   // tensor memory: one warp allocates, the same warp frees
@@ -192,147 +427,26 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
   } else {
     // ---- epilogue ----------------------------------------------------------------------------------------------------
-    // A thread reads an accumulator row (its lane of tensor memory) and half of its columns; the sums go to a padded tile in
-    // shared memory (the ring is idle by then), from where the warps add up the planes and write whole rows.
-    const bool ok = mbar_wait(&bars.accum, 0, ab, p.error, 703) && !*ab;
-    kernel_wait();   // row scales, counters (long complete: the operand was loaded)
-    constexpr int LDS = 128 + 4;                      // row stride of the staging tile, in words
-    float *ep = reinterpret_cast<float *>(tiles);     // [BM][LDS]: 66 KB of the ring
-    const int ew = warp - 2, quad = warp & 3;
-#pragma unroll 1
-    for (int h = 0; h < BN / 128; ++h) {   // 128 columns of the accumulator at a time
-      const int nh = n0 + h * 128;
-      if (nh >= p.N)
-        break;
-      if (h > 0)   // the staging tile is free again once the previous half has been stored
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
-      if (ok && (PLANES || quad * 32 < p.M - m0)) {   // lanes beyond M hold nothing
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        // a warp reads the 32 lanes of tensor memory that match its rank within its warpgroup; the two warps that share a
-        // lane quarter take half the columns each
-        const int row = quad * 32 + lane, cb0 = (ew >> 2) * 64;
-        const float f = row < kPlaneRows ? 65536.f : row < 2 * kPlaneRows ? 256.f : 1.f;   // PLANES: the digit's weight
-#pragma unroll 1
-        for (int cb = cb0; cb < cb0 + 64; cb += 32) {
-          uint32_t v[32];
-          const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(h * 128 + cb);
-          tmem_load32(taddr, v);
-          tmem_wait_load();
-          float *erow = ep + row * LDS + cb;
-#pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            float4 o;
-            if (PLANES)
-              o = make_float4(__int2float_rn((int)v[j]) * f, __int2float_rn((int)v[j + 1]) * f,
-                              __int2float_rn((int)v[j + 2]) * f, __int2float_rn((int)v[j + 3]) * f);
-            else
-              o = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]),
-                              __uint_as_float(v[j + 3]));
-            *reinterpret_cast<float4 *>(erow + j) = o;
-          }
-        }
-      }
-      asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
-      const int rows = min(kRows, p.M - m0), cols = min(128, p.N - nh);
-      // sums of row r, columns c .. c + 3 of this CTA's k range
-      auto sums = [&](int r, int c) {
-        float4 a = *reinterpret_cast<const float4 *>(ep + r * LDS + c);
-        if (PLANES) {
-#pragma unroll
-          for (int q = 1; q < kPlanes; ++q) {
-            const float4 b = *reinterpret_cast<const float4 *>(ep + (q * kPlaneRows + r) * LDS + c);
-            a = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
-          }
-        }
-        return a;
-      };
-      bool mine = ok;
-      const int tile = blockIdx.y * gridDim.x + blockIdx.x;
-      float4 *shares = reinterpret_cast<float4 *>(p.partial) + (int64_t)tile * p.splits * kRows * 32;
-      if (p.splits > 1) {   // (BN = 128) leave this CTA's share; the last one of the tile goes on
-        if (ok)
-          for (int i = ew * 32 + lane; i < rows * 32; i += kEpiWarps * 32)
-            __stcg(shares + (int64_t)blockIdx.z * kRows * 32 + i, sums(i >> 5, (i & 31) * 4));
-        __threadfence();
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
-        if (threadIdx.x == 64)
-          bars.last = atomicAdd(p.arrived + tile, 1u) == (uint32_t)p.splits - 1;
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
-        __threadfence();
-        mine = ok && bars.last;
-      }
-      if (mine) {
-        const bool vec = (p.ldc & 3) == 0 && ((uintptr_t)p.C & 15) == 0 && (p.N & 3) == 0 &&
-                         (!p.residual || ((p.ldr & 3) == 0 && ((uintptr_t)p.residual & 15) == 0));
-#pragma unroll 2
-        for (int i = ew * 32 + lane; i < rows * 32; i += kEpiWarps * 32) {
-          const int r = i >> 5, c = (i & 31) * 4, m = m0 + r, n = nh + c;
-          if (c >= cols)
-            continue;
-          float y[4];
-          if (p.splits > 1) {
-            float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int z0 = 0; z0 < p.splits; z0 += 8) {   // 8 loads in flight
-              float4 b[8];
-#pragma unroll
-              for (int z = 0; z < 8; ++z)
-                b[z] = z0 + z < p.splits ? __ldcg(shares + (int64_t)(z0 + z) * kRows * 32 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-              for (int z = 0; z < 8; ++z)
-                if (PLANES)
-                  a = make_float4(a.x + b[z].x, a.y + b[z].y, a.z + b[z].z, a.w + b[z].w);
-                else
-                  a = make_float4(__int_as_float(__float_as_int(a.x) + __float_as_int(b[z].x)),
-                                  __int_as_float(__float_as_int(a.y) + __float_as_int(b[z].y)),
-                                  __int_as_float(__float_as_int(a.z) + __float_as_int(b[z].z)),
-                                  __int_as_float(__float_as_int(a.w) + __float_as_int(b[z].w)));
-            }
-            y[0] = a.x; y[1] = a.y; y[2] = a.z; y[3] = a.w;
-          } else {
-            const float4 a = sums(r, c);
-            y[0] = a.x; y[1] = a.y; y[2] = a.z; y[3] = a.w;
-          }
-          const float rs = p.row_scale[PLANES ? m : 0];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int ne = min(n + e, p.N - 1);
-            if (PLANES)
-              y[e] = __fmul_rn(__fmul_rn(y[e], rs), __ldg(p.scale + ne));
-            else   // linalg.py:12836-12846: float(acc) * (act_scale * weight_scale[n])
-              y[e] = __fmul_rn(__int2float_rn(__float_as_int(y[e])), __fmul_rn(rs, __ldg(p.scale + ne)));
-            if (p.bias)
-              y[e] = __fadd_rn(y[e], __ldg(p.bias + ne));
-          }
-          if (p.silu_pairs) {
-            float *dst = p.C + (int64_t)m * p.ldc + (n >> 1);
-            dst[0] = silu_of(y[0], y[1]);
-            if (n + 3 < p.N)   // N is even
-              dst[1] = silu_of(y[2], y[3]);
-          } else {
-            float *dst = p.C + (int64_t)m * p.ldc + n;
-            const float *res = p.residual + (int64_t)m * p.ldr + n;
-            if (vec) {
-              if (p.residual) {
-                const float4 q = *reinterpret_cast<const float4 *>(res);
-                y[0] = __fadd_rn(q.x, y[0]);
-                y[1] = __fadd_rn(q.y, y[1]);
-                y[2] = __fadd_rn(q.z, y[2]);
-                y[3] = __fadd_rn(q.w, y[3]);
-              }
-              *reinterpret_cast<float4 *>(dst) = make_float4(y[0], y[1], y[2], y[3]);
-            } else {
-#pragma unroll
-              for (int e = 0; e < 4; ++e)
-                if (n + e < p.N)
-                  dst[e] = p.residual ? __fadd_rn(res[e], y[e]) : y[e];
-            }
-          }
-        }
-      }
+    kernel_wait();   // row scales, counters
+    const float scales = row_scales<PLANES>(p, 0, min(kRows, p.M - m0));
+    if (PLANES) {
+      const uint32_t wide = __ballot_sync(0xffffffffu, signbit(scales));
+      if (wide != 0 && lane == 0)   // rows warp - 2 + 8 j, the first half of the tile: below 21
+        for (int j = 0; j < (kRows + kEpiWarps - 1) / kEpiWarps; ++j)
+          if (wide >> j & 1)
+            atomicOr(&bars.wide, warp - 2 + kEpiWarps * j < kWideRows ? 1 : 2);
     }
+    const bool ok = mbar_wait(&bars.accum, 0, ab, p.error, 703) && !*ab;
+    store_tile<BN, PLANES, false>(p, bars, tiles, tmem, ok, 0, scales);
+    if (PLANES)
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // a pass over wide rows loads over the staging tile
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (PLANES && bars.wide != 0 && !*ab) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    wide_passes<BN>(map_x, map_w, p, tiles, tmem, kb0, nkb);
+  }
   if (warp == 1) {
     if (*ab) {   // copies of an abandoned tile may still be in flight: let them land before the CTA ends
       const unsigned long long t0 = now_ns();
@@ -367,17 +481,33 @@ __device__ __forceinline__ int unit_k(int u, int j, int units) {
   return b * 512 + j * (nu * 4) + 4 * (u & 31);
 }
 
-// A[M,K] f32 -> planes [ceil(M/42)][3][42] (+ 2 unused rows) [K] int8 in the k order of the packed weight rows, and the rows' scales; optional
-// RMSNorm of every row (the factor 1/rms goes into the scale).  T threads per row, a thread takes 16-byte units: it reads
-// four groups of four k and writes whole 16-byte pieces of the planes.  The row is read once and stays in registers up to
-// 48 T elements.  Also clears the GEMM's counters and, outside a pass, its error word (head).
+// A row's fixed-point scale, from the bit pattern of its largest magnitude: |X| <= 0x7F7F7F, what three signed digits hold (a
+// magnitude whose mantissa would round beyond that takes the next power of two).  *inv undoes it; NaN for a row with an infinity
+// or a NaN.  Below 2^-104 the scale stays, and six digits reach down to the smallest subnormal.
+__device__ __forceinline__ float plane_scale(uint32_t absbits, float *inv) {
+  const int e = max((int)((absbits + 0x10102u) >> 23) - 127, -104);
+  *inv = absbits >= 0x7f800000u ? __uint_as_float(0x7fffffffu) : __uint_as_float((uint32_t)(e - 22 + 127) << 23);
+  return __uint_as_float((uint32_t)(22 - e + 127) << 23);
+}
+
+// A[M,K] f32 -> planes [ceil(M/42)][3][42] (+ 2 unused rows) [K] int8 in the k order of the packed weight rows, and the rows'
+// scales (the sign says that a row is wide); optional RMSNorm of every row (the factor 1/rms goes into the scale).  T threads per row, a thread takes 16-byte
+// units: it reads four groups of four k and writes whole 16-byte pieces of the planes.  The row is read once and stays in
+// registers up to 48 T elements.  Also clears the GEMM's counters and, outside a pass, its error word (head).
+//
+// Wide rows.  Rounding to a unit leaves 0.29 units (rms) in every element, which must be no more than the 2^-19 of an element
+// that two bf16 terms leave: the row's bulk has to have an rms of at least 2^17 units.  Its bulk is what lies below a quarter of
+// the largest magnitude, and is also to have a mean of 2^16, so that a few percent of large elements do not pass for bulk.  A
+// row with channels more than about 32 times the rest misses that, and is written a second time, into `wides`
+// [ceil(M/42)][2][6][21] (+ 2 rows) [K]: three more digits, of what the first three leave over in units of 2^-23, exact down to
+// 2^-45 of the largest magnitude.  One sum decides for nearly all other rows: a mean magnitude of 2^17.5 units.
 constexpr int kUnits = 3;
 __global__ void __launch_bounds__(256)
 planes_kernel(const float *A, int64_t lda, int M, int K, const float *norm_w, float eps, int T, int vec, uint8_t *planes,
-              float *row_scale, uint32_t *head, int head_words, int in_pass) {
+              float *row_scale, uint32_t *head, int head_words, int in_pass, uint8_t *wides) {
   chain_start(in_pass);
   __shared__ uint32_t s_mx[8];
-  __shared__ float s_ss[8];
+  __shared__ float s_ss[8], s_s1[8], s_bulk[8][3];
   const int t = threadIdx.x % T, m = blockIdx.x * (256 / T) + threadIdx.x / T;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (blockIdx.x == 0)
@@ -395,7 +525,7 @@ planes_kernel(const float *A, int64_t lda, int M, int K, const float *norm_w, fl
         v[i][j] = u < units ? load4(row, unit_k(u, j, units), vec) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
   };
-  float ss = 0.f;
+  float ss = 0.f, s1 = 0.f;
   uint32_t mx = 0;
   auto weigh = [&](int u0, bool stats) {   // times the norm weight
 #pragma unroll
@@ -414,6 +544,8 @@ planes_kernel(const float *A, int64_t lda, int M, int K, const float *norm_w, fl
           const uint32_t a = 0x7fffffffu;
           mx = max(mx, max(max(__float_as_uint(x.x) & a, __float_as_uint(x.y) & a),
                            max(__float_as_uint(x.z) & a, __float_as_uint(x.w) & a)));
+          if (stats)
+            s1 += (fabsf(x.x) + fabsf(x.y)) + (fabsf(x.z) + fabsf(x.w));
         }
     }
   };
@@ -423,27 +555,79 @@ planes_kernel(const float *A, int64_t lda, int M, int K, const float *norm_w, fl
   }
   mx = __reduce_max_sync(0xffffffffu, mx);
   ss = warp_sum(ss);
+  s1 = warp_sum(s1);
+  const int w0 = (threadIdx.x / T) * (T / 32);   // the row's first warp
   if (T > 32) {
     if (lane == 0) {
       s_mx[warp] = mx;
       s_ss[warp] = ss;
+      s_s1[warp] = s1;
     }
     __syncthreads();
-    const int w0 = (threadIdx.x / T) * (T / 32);
     mx = 0;
-    ss = 0.f;
+    ss = s1 = 0.f;
     for (int w = 0; w < T / 32; ++w) {
       mx = max(mx, s_mx[w0 + w]);
       ss += s_ss[w0 + w];
+      s1 += s_s1[w0 + w];
     }
   }
   if (m >= M)
     return;
   float inv;
-  const float scale = fixed_scale<21>(mx, &inv);   // |X| < 2^22: three digits
-  if (t == 0)
-    row_scale[m] = norm_w != nullptr ? inv * rsqrtf(ss * (1.0f / (float)K) + eps) : inv;
+  const float scale = plane_scale(mx, &inv);
+  bool wide = false;
+  if (mx != 0u && mx < 0x7f800000u && !(s1 < 3e38f && s1 * scale >= 185364.f * (float)K)) {
+    float bulk2 = 0.f, bulk = 0.f, rest = 0.f;   // of |X|, and of what rounding leaves over
+    const float cut = __uint_as_float(mx) * scale * 0.25f;
+    auto add = [&](float v) {
+      const float X = fabsf(v * scale);
+      rest += fabsf(X - rintf(X));
+      if (X <= cut) {
+        bulk2 = fmaf(X, X, bulk2);
+        bulk += X;
+      }
+    };
+    for (int u0 = 0; u0 < units; u0 += step) {
+      if (units > step) {
+        load(u0);
+        weigh(u0, false);
+      }
+#pragma unroll
+      for (int i = 0; i < kUnits; ++i)   // (units beyond the row are zero)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          add(v[i][j].x);
+          add(v[i][j].y);
+          add(v[i][j].z);
+          add(v[i][j].w);
+        }
+    }
+    bulk2 = warp_sum(bulk2);
+    bulk = warp_sum(bulk);
+    rest = warp_sum(rest);
+    if (T > 32) {
+      if (lane == 0) {
+        s_bulk[warp][0] = bulk2;
+        s_bulk[warp][1] = bulk;
+        s_bulk[warp][2] = rest;
+      }
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / T), "r"(T) : "memory");   // the row's threads
+      bulk2 = bulk = rest = 0.f;
+      for (int w = 0; w < T / 32; ++w) {
+        bulk2 += s_bulk[w0 + w][0];
+        bulk += s_bulk[w0 + w][1];
+        rest += s_bulk[w0 + w][2];
+      }
+    }
+    wide = rest > 0.f && !(bulk2 >= 17179869184.f * (float)K && bulk >= 65536.f * (float)K);
+  }
+  if (t == 0) {
+    const float rs = norm_w != nullptr ? inv * rsqrtf(ss * (1.0f / (float)K) + eps) : inv;
+    row_scale[m] = __uint_as_float((__float_as_uint(rs) & 0x7fffffffu) | (wide ? 0x80000000u : 0u));
+  }
   uint8_t *dst = planes + ((int64_t)(m / kPlaneRows) * BM + m % kPlaneRows) * K;
+  uint8_t *wdst = wides + ((int64_t)(m / kWideRows) * BM + m % kWideRows) * K;   // (42 = 2 x 21)
   for (int u0 = 0; u0 < units; u0 += step) {
     if (units > step) {
       load(u0);
@@ -463,6 +647,30 @@ planes_kernel(const float *A, int64_t lda, int M, int K, const float *norm_w, fl
           *reinterpret_cast<uint4 *>(dst + (int64_t)pl * kPlaneRows * K + u * 16) =
               make_uint4(w[0][pl + 1], w[1][pl + 1], w[2][pl + 1], w[3][pl + 1]);
       }
+    }
+  }
+  if (!wide)
+    return;
+#pragma unroll 1
+  for (int u = t; u < units; u += T) {   // from memory again: few registers
+    uint32_t w[4][4], l[4][4];
+    auto rest = [&](float x) { return fixed_digits(x * scale - rintf(x * scale), 8388608.f); };   // exact, |rest| <= 2^22
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float4 x = load4(row, unit_k(u, j, units), vec);
+      if (norm_w != nullptr) {
+        const float4 n = load4(norm_w, unit_k(u, j, units), vec);
+        x = make_float4(x.x * n.x, x.y * n.y, x.z * n.z, x.w * n.w);
+      }
+      plane_words(fixed_digits(x.x, scale), fixed_digits(x.y, scale), fixed_digits(x.z, scale), fixed_digits(x.w, scale), w[j]);
+      plane_words(rest(x.x), rest(x.y), rest(x.z), rest(x.w), l[j]);
+    }
+#pragma unroll
+    for (int pl = 0; pl < kPlanes; ++pl) {
+      uint4 *at = reinterpret_cast<uint4 *>(wdst + (int64_t)pl * kWideRows * K + u * 16);
+      *at = make_uint4(w[0][pl + 1], w[1][pl + 1], w[2][pl + 1], w[3][pl + 1]);
+      *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(at) + (int64_t)kPlanes * kWideRows * K) =
+          make_uint4(l[0][pl + 1], l[1][pl + 1], l[2][pl + 1], l[3][pl + 1]);
     }
   }
 }
@@ -585,19 +793,24 @@ int make_map(CUtensorMap *map, CUtensorMapDataType dt, int bk, void *base, uint6
 }
 
 template <int BN, bool PLANES>
-int launch_gemm(const void *a, int a_rows, const void *w, GemmParams &p, int m_tiles, cudaStream_t st) {
-  CUtensorMap map_a, map_w;
+int launch_gemm(const void *a, int a_rows, const void *x, const void *w, GemmParams &p, int m_tiles, cudaStream_t st) {
+  CUtensorMap map_a, map_w, map_x;
   if (int rc = make_map(&map_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, BK, const_cast<void *>(a), p.K, a_rows, (uint64_t)p.K,
                         CU_TENSOR_MAP_SWIZZLE_128B))
     return rc;
   if (int rc = make_map(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, BK, const_cast<void *>(w), p.K, p.N, (uint64_t)p.K,
                         CU_TENSOR_MAP_SWIZZLE_128B, BN))
     return rc;
+  map_x = map_a;
+  if (PLANES)
+    if (int rc = make_map(&map_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, BK, const_cast<void *>(x), p.K, 2 * (uint64_t)a_rows,
+                          (uint64_t)p.K, CU_TENSOR_MAP_SWIZZLE_128B))
+      return rc;
   static RaisedOn raised;
   if (int rc = raise_shared_limit(raised, (const void *)gemm_i8_kernel<BN, PLANES>, Ring<BN>::SMEM))
     return rc;
   return launch_after(gemm_i8_kernel<BN, PLANES>, dim3((p.N + BN - 1) / BN, m_tiles, p.splits), kThreads, Ring<BN>::SMEM, st,
-                      map_a, map_w, p);
+                      map_a, map_w, p, map_x);
 }
 
 // CTAs along K for `tiles` output tiles of `nkb` k blocks: up to two CTAs per SM (148), within the workspace, at least 8 k
@@ -624,8 +837,8 @@ int64_t b200_gemm_w8_workspace_bytes(int M, int64_t K) {
   if (M < 1 || K < 1)
     return 0;
   const int64_t tiles = (M + kPlaneRows - 1) / kPlaneRows, Kp = packed_k(B200_W_I8, K);
-  // head, row scales, planes, the shares of split tiles
-  return kHeadBytes + tiles * kPlaneRows * 4 + 255 + tiles * BM * Kp + (int64_t)kMaxPartialTiles * kPlaneRows * 128 * 4;
+  // head, row scales, planes, the wide rows' planes, the shares of split tiles
+  return kHeadBytes + tiles * kPlaneRows * 4 + 255 + 3 * tiles * BM * Kp + (int64_t)kMaxPartialTiles * kPlaneRows * 128 * 4;
 }
 
 int b200_gemm_w8(const b200_weight *w, const float *A, int M, int64_t lda, float *C, int64_t ldc,
@@ -659,6 +872,7 @@ int gemm_w8_run(const b200_weight *w, const float *A, int M, int64_t lda, float 
   char *ws = (char *)workspace;
   float *row_scale = reinterpret_cast<float *>(ws + kHeadBytes);
   uint8_t *planes = reinterpret_cast<uint8_t *>(ws + (kHeadBytes + (int64_t)m_tiles * kPlaneRows * 4 + 255) / 256 * 256);
+  uint8_t *wides = planes + (int64_t)m_tiles * BM * K;
   GemmParams p{};
   p.M = M;
   p.N = N;
@@ -671,7 +885,7 @@ int gemm_w8_run(const b200_weight *w, const float *A, int M, int64_t lda, float 
   p.ldc = ldc;
   p.ldr = ldr;
   p.silu_pairs = silu_pairs;
-  p.partial = planes + (int64_t)m_tiles * BM * K;
+  p.partial = wides + (int64_t)m_tiles * 2 * BM * K;
   p.error = reinterpret_cast<int *>(ws);
   p.arrived = reinterpret_cast<uint32_t *>(ws) + 16;
   // threads per row: as few as keep it in registers, more when there are few rows
@@ -681,15 +895,15 @@ int gemm_w8_run(const b200_weight *w, const float *A, int M, int64_t lda, float 
   const int vec = (lda & 3) == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)norm_weight & 15) == 0;
   if (int rc = launch_after(planes_kernel, dim3((M + 256 / T - 1) / (256 / T)), 256, 0, st, A, lda, M, K, norm_weight, norm_eps, T,
                             vec, planes, row_scale, in_pass ? p.arrived : reinterpret_cast<uint32_t *>(ws),
-                            in_pass ? kMaxPartialTiles : 16 + kMaxPartialTiles, in_pass ? 1 : 0))
+                            in_pass ? kMaxPartialTiles : 16 + kMaxPartialTiles, in_pass ? 1 : 0, wides))
     return rc;
   // 256 columns per CTA (fewer bytes per operation) when that still gives every SM its two CTAs
   if ((int64_t)((N + 255) / 256) * m_tiles >= 296) {
     p.splits = 1;
-    return launch_gemm<256, true>(planes, m_tiles * BM, w->w, p, m_tiles, st);
+    return launch_gemm<256, true>(planes, m_tiles * BM, wides, w->w, p, m_tiles, st);
   }
   p.splits = split_k((N + 127) / 128 * m_tiles, (K + BK - 1) / BK, std::min(M, kPlaneRows));
-  return launch_gemm<128, true>(planes, m_tiles * BM, w->w, p, m_tiles, st);
+  return launch_gemm<128, true>(planes, m_tiles * BM, wides, w->w, p, m_tiles, st);
 }
 } // namespace b200
 
@@ -762,7 +976,7 @@ int gemm_w8a8_fused(const b200_weight *w, const float *A, int M, int64_t lda, fl
                             (const uint32_t *)part, parts, act_scale, q))
     return rc;
   p.splits = split_k((N + 127) / 128 * m_tiles, (K + BK - 1) / BK, std::min(M, BM));
-  return launch_gemm<128, false>(q, M, w->w, p, m_tiles, st);
+  return launch_gemm<128, false>(q, M, q, w->w, p, m_tiles, st);
 }
 } // namespace b200
 

@@ -158,9 +158,10 @@ int b200_gemv(const b200_weight *w, const b200_gemv_args *a, void *stream);
  * examples/BuddyMatmul/dequant-matmul-vectorization-blis-prefill.mlir:113-115).
  * w: int8 per-channel packed rows as for b200_gemv (f32 scales, optional
  * bias), K a multiple of 64 up to 131008.  A: f32 [M, lda] on the device; norm_weight (or
- * NULL): RMSNorm of every row of A first.  An activation is a 23-bit
+ * NULL): RMSNorm of every row of A first.  An activation is a 24-bit
  * fixed-point number in units of its row, three int8 digits whose sums of
- * products are exact (tcgen05.mma kind::i8) and added in f32.  workspace:
+ * products are exact (tcgen05.mma kind::i8) and added in f32; rows with
+ * channels far above the rest get six digits.  workspace:
  * b200_gemm_w8_workspace_bytes(M, K) bytes, 256-byte aligned, owned by the
  * caller (it holds the digits, shares of split tiles and an error word).
  * b200_gemm_w8_status() reports a bounded wait that gave up.  All reads,
