@@ -330,8 +330,8 @@ GEMM_SHAPES = {
 def gemm_microbench(lib, only=None):
     """Isolated b200_gemm_w8 launches (tcgen05 path): activation split + GEMM kernel, CUDA events
     on the launching stream, int8 weights that do not fit L2 rotated between launches.
-    TFLOP/s counts 2*M*N*K once (every tile is multiplied twice on the tensor cores, once per
-    bf16 term of the f32 activations, so the tensor pipe does twice that)."""
+    TFLOP/s counts 2*M*N*K once; the tensor cores do three int8 products for each, one per digit
+    of the f32 activations (int8_TOP/s)."""
     import ctypes as C
     import torch
     from buddy_mlir_b200 import _lib
@@ -368,7 +368,7 @@ def gemm_microbench(lib, only=None):
         us = e0.elapsed_time(e1) * 1000.0 / reps
         tf = 2.0 * M * N * K / us / 1e6
         out[name] = {"M": M, "N": N, "K": K, "us": round(us, 1), "TFLOP/s": round(tf, 1),
-                     "frac_of_bf16_sustained": round(tf / peak, 3), "tensor_pipe_frac": round(2 * tf / peak, 3)}
+                     "frac_of_bf16_sustained": round(tf / peak, 3), "int8_TOP/s": round(3 * tf, 1)}
         # the same shape as W8A8 (int8 activations, integer tensor cores): quantiser + GEMM
         nb8 = lib.b200_gemm_w8a8_workspace_bytes(M, K)
         ws8 = torch.zeros(nb8, dtype=torch.uint8, device="cuda")
@@ -389,9 +389,9 @@ def gemm_microbench(lib, only=None):
         out[name]["w8a8_us"] = round(us8, 1)
         out[name]["w8a8_TOP/s"] = round(2.0 * M * N * K / us8 / 1e6, 1)
     return {"shapes": out, "peak_tflops": peak,
-            "note": "frac = algorithmic 2MNK / time / measured sustained bf16 peak; the tensor pipe does three times the "
-                    "algorithmic work (three int8 digits per f32 activation, int8 at the bf16 rate); w8a8_* = the same shape with int8 "
-                    "activations on the integer tensor-core path (no measured int8 peak on this pool: absolute only)"}
+            "note": "frac = algorithmic 2MNK / time / measured sustained bf16 peak; int8_TOP/s = what the tensor cores do, three "
+                    "int8 digits per f32 activation; w8a8_* = the same shape with int8 activations (no measured int8 peak on "
+                    "this pool: int8 figures are absolute)"}
 
 
 def run_gemm_only(args):

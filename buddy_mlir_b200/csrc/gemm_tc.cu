@@ -34,7 +34,8 @@
 // epilogue; two CTAs are resident per SM, so one's epilogue runs under the other's main loop.  The weight loads start
 // before the activations are there (programmatic dependent launch behind the kernel that makes the planes; chain_start says
 // what keeps them behind the caller's earlier work).  The main loop
-// is bound by the bytes it brings from L2 (64 bytes per clock and SM), hence 256 columns where that leaves enough CTAs.
+// is bound by the bytes it brings from L2 (64 bytes per clock and SM), hence 256 columns where that leaves two CTAs
+// for every SM (with planes; W8A8 always takes 128, see there).
 // Few output tiles: the k range is split over gridDim.z, and the CTA that finishes a tile last adds the shares in order.
 //
 // Every wait is bounded (poll count and wall time); on expiry the CTA records
@@ -60,7 +61,8 @@ constexpr int kWidePlanes = 6, kWideRows = 21; // the same for rows that need si
 constexpr int kThreads = 320;                  // loader, mma, 8 epilogue warps
 constexpr int kEpiWarps = 8;
 constexpr int kMaxStages = 3;
-constexpr int kMaxPartialTiles = 320;          // split-K: shares of tiles in the workspace
+constexpr int kSms = 148, kResident = 2 * kSms;   // CTAs of the GEMM that run at once: two per SM
+constexpr int kMaxPartialTiles = 320;          // split-K: shares of tiles in the workspace (a little over one per resident CTA)
 constexpr int kHeadBytes = 2048;               // workspace head: error word, scales of W8A8, arrival counters
 
 template <int BN> struct Ring {
@@ -112,7 +114,7 @@ struct GemmParams {
   int *error;
 };
 
-// One output element: 1: sum -> y = sum * scale (+ bias); the operations and their order are the reference's.
+// The operations and their order are the reference's.
 __device__ __forceinline__ float silu_of(float g, float u) {
   const float sg = 1.0f / (1.0f + expf(-g));   // subgraph0_decode_simplify.mlir:226-231
   return __fmul_rn(__fmul_rn(g, sg), u);
@@ -393,7 +395,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       };
       // few rows: the weights' way from memory is the GEMM; all of this CTA's share starts for L2 while the kernels before run
       // (if all CTAs are resident at once: 24 x 151936 x 1536, 594 CTAs, took 68 us with it and 60 without)
-      if (gridDim.y <= 2 && gridDim.x * gridDim.y * gridDim.z <= 296)
+      if (gridDim.y <= 2 && gridDim.x * gridDim.y * gridDim.z <= kResident)
         for (int i = S; i < nkb; ++i)
           tma_prefetch_2d(&map_w, (kb0 + i) * BK, n0);
       const int ahead = min(S, nkb);
@@ -813,15 +815,15 @@ int launch_gemm(const void *a, int a_rows, const void *x, const void *w, GemmPar
                       map_a, map_w, p, map_x);
 }
 
-// CTAs along K for `tiles` output tiles of `nkb` k blocks: up to two CTAs per SM (148), within the workspace, at least 8 k
+// CTAs along K for `tiles` output tiles of `nkb` k blocks: up to two CTAs per SM, within the workspace, at least 8 k
 // blocks each: a share's trip through L2 costs what 8 to 12 blocks cost.  24 x 2048 x 1536 (12 blocks): 10.1 us whole, 11.1 in
 // 6 shares; 24 x 1536 x 8960 (70 blocks): 27 us whole, 14.4 in 8, 17.2 in 24; 366 x 1536 x 8960 (108 tiles): 34.8 whole, 28.2 in 2.
 // A row of a tile's sums costs as much on that trip as 0.4 blocks, so tiles with many rows split only long k ranges (W8A8,
 // 1024 x 1536 x 8960: 49.8 us whole, 55.3 in 3; 200 x 4096 x 4096: 21.4 whole, 29 in 4; 64 x 1536 x 8960: 32.2 whole, 19.7 in 8).
 int split_k(int tiles, int nkb, int rows) {
-  if (tiles >= 148)
+  if (tiles >= kSms)
     return 1;
-  const int s = std::max(1, std::min({296 / tiles, nkb / 8, kMaxPartialTiles / tiles}));
+  const int s = std::max(1, std::min({kResident / tiles, nkb / 8, kMaxPartialTiles / tiles}));
   return (nkb - nkb / s) * 5 > rows * 2 ? s : 1;
 }
 
@@ -890,7 +892,7 @@ int gemm_w8_run(const b200_weight *w, const float *A, int M, int64_t lda, float 
   p.arrived = reinterpret_cast<uint32_t *>(ws) + 16;
   // threads per row: as few as keep it in registers, more when there are few rows
   int T = 32;
-  while (T < 256 && (K > T * 16 * kUnits || (int64_t)M * T < 148 * 256))
+  while (T < 256 && (K > T * 16 * kUnits || (int64_t)M * T < kSms * 256))
     T *= 2;
   const int vec = (lda & 3) == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)norm_weight & 15) == 0;
   if (int rc = launch_after(planes_kernel, dim3((M + 256 / T - 1) / (256 / T)), 256, 0, st, A, lda, M, K, norm_weight, norm_eps, T,
@@ -898,7 +900,7 @@ int gemm_w8_run(const b200_weight *w, const float *A, int M, int64_t lda, float 
                             in_pass ? kMaxPartialTiles : 16 + kMaxPartialTiles, in_pass ? 1 : 0, wides))
     return rc;
   // 256 columns per CTA (fewer bytes per operation) when that still gives every SM its two CTAs
-  if ((int64_t)((N + 255) / 256) * m_tiles >= 296) {
+  if ((int64_t)((N + 255) / 256) * m_tiles >= kResident) {
     p.splits = 1;
     return launch_gemm<256, true>(planes, m_tiles * BM, wides, w->w, p, m_tiles, st);
   }
@@ -975,6 +977,8 @@ int gemm_w8a8_fused(const b200_weight *w, const float *A, int M, int64_t lda, fl
   if (int rc = launch_after(quantize_kernel, dim3((unsigned)((units + 255) / 256)), 256, 0, st, A, lda, M, K, vec,
                             (const uint32_t *)part, parts, act_scale, q))
     return rc;
+  // 128 columns for all: with 256, where that leaves two CTAs for every SM, 2048 x 20000 x 8960 takes 423 us instead of 482 and
+  // 2048 x 17920 x 1536 105 instead of 112, but 1024 x 18992 x 1536 73 instead of 69 and 600 x 17920 x 1536 51 instead of 47
   p.splits = split_k((N + 127) / 128 * m_tiles, (K + BK - 1) / BK, std::min(M, BM));
   return launch_gemm<128, false>(q, M, q, w->w, p, m_tiles, st);
 }
