@@ -217,7 +217,7 @@ __device__ __forceinline__ void store_tile(const GemmParams &p, Bars &bars, uint
     if (mine) {
       const bool vec = (p.ldc & 3) == 0 && ((uintptr_t)p.C & 15) == 0 && (p.N & 3) == 0 &&
                        (!p.residual || ((p.ldr & 3) == 0 && ((uintptr_t)p.residual & 15) == 0));
-#pragma unroll (SIX ? 1 : 2)
+#pragma unroll 1
       for (int r = ew, j = 0; r < nr; r += kEpiWarps, ++j) {
         const float rs = PLANES ? __shfl_sync(0xffffffffu, scales, j) : scales;
         const int i = r * 32 + lane, c = lane * 4, m = m0 + r0 + r, n = nh + c;
@@ -286,9 +286,10 @@ __device__ __forceinline__ void store_tile(const GemmParams &p, Bars &bars, uint
 }
 
 // The tile's wide rows once more, with six digits: a half of its rows at a time (`halves`: which).  Everything a normal tile does
-// again, in a function of its own and with little code (no unrolling in SIX): the code counts even where it does not run.  Without
-// wide rows, 24 x 17920 x 1536 takes 13.5 us without this function, 13.9 with it, 16.3 with the loops unrolled as for a normal
-// tile; 1024 x 17920 x 1536 takes 106.8, 108.4, and 110.5 with these passes as a loop around the tile's code.
+// again, in a function of its own and with little code, since code counts even where it does not run: without wide rows,
+// 24 x 17920 x 1536 takes 13.5 us without this function, 13.9 with it, 16.3 with its loops unrolled as a tile's were;
+// 1024 x 17920 x 1536 106.8, 108.4, and 110.5 with these passes as a loop around the tile's code.  For the same reason the loops
+// over the rows of a tile are not unrolled (prefill of 1000 rows: 7.59 -> 7.48 ms).
 template <int BN>
 __device__ __noinline__ void wide_passes(const CUtensorMap &map_x, const CUtensorMap &map_w, const GemmParams &p, uint8_t *tiles,
                                          uint32_t tmem, int kb0, int nkb) {
@@ -319,7 +320,7 @@ __device__ __noinline__ void wide_passes(const CUtensorMap &map_x, const CUtenso
             break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t a = smem_u32(tiles + s * R::STAGE_BYTES), w = a + R::A_BYTES;
-#pragma unroll
+#pragma unroll 1
           for (int k = 0; k < BK / 32; ++k)
             mma_i8<BN>(tmem, smem_desc(a + k * 32), smem_desc(w + k * 32), (i | k) != 0);
           tc_commit(&bars.empty[s]);
@@ -580,11 +581,10 @@ planes_kernel(const float *A, int64_t lda, int M, int K, const float *norm_w, fl
   const float scale = plane_scale(mx, &inv);
   bool wide = false;
   if (mx != 0u && mx < 0x7f800000u && !(s1 < 3e38f && s1 * scale >= 185364.f * (float)K)) {
-    float bulk2 = 0.f, bulk = 0.f, rest = 0.f;   // of |X|, and of what rounding leaves over
+    float bulk2 = 0.f, bulk = 0.f;   // of |X|
     const float cut = __uint_as_float(mx) * scale * 0.25f;
     auto add = [&](float v) {
       const float X = fabsf(v * scale);
-      rest += fabsf(X - rintf(X));
       if (X <= cut) {
         bulk2 = fmaf(X, X, bulk2);
         bulk += X;
@@ -605,24 +605,33 @@ planes_kernel(const float *A, int64_t lda, int M, int K, const float *norm_w, fl
           add(v[i][j].w);
         }
     }
-    bulk2 = warp_sum(bulk2);
-    bulk = warp_sum(bulk);
-    rest = warp_sum(rest);
-    if (T > 32) {
-      if (lane == 0) {
-        s_bulk[warp][0] = bulk2;
-        s_bulk[warp][1] = bulk;
-        s_bulk[warp][2] = rest;
+    auto over_row = [&](float a, int at) {   // a summed over the row's threads
+      a = warp_sum(a);
+      if (T > 32) {
+        if (lane == 0)
+          s_bulk[warp][at] = a;
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / T), "r"(T) : "memory");   // the row's threads
+        a = 0.f;
+        for (int w = 0; w < T / 32; ++w)
+          a += s_bulk[w0 + w][at];
       }
-      asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / T), "r"(T) : "memory");   // the row's threads
-      bulk2 = bulk = rest = 0.f;
-      for (int w = 0; w < T / 32; ++w) {
-        bulk2 += s_bulk[w0 + w][0];
-        bulk += s_bulk[w0 + w][1];
-        rest += s_bulk[w0 + w][2];
+      return a;
+    };
+    bulk2 = over_row(bulk2, 0);
+    if (!(bulk2 >= 17179869184.f * (float)K) || !(over_row(bulk, 1) >= 65536.f * (float)K)) {
+      float rest = 0.f;   // what rounding leaves over: a row without is exact as it is
+#pragma unroll 1
+      for (int k = 4 * t; k < K; k += 4 * T) {
+        float4 x = load4(row, k, vec);
+        if (norm_w != nullptr) {
+          const float4 n = load4(norm_w, k, vec);
+          x = make_float4(x.x * n.x, x.y * n.y, x.z * n.z, x.w * n.w);
+        }
+        auto left = [&](float a) { return fabsf(a * scale - rintf(a * scale)); };
+        rest += (left(x.x) + left(x.y)) + (left(x.z) + left(x.w));
       }
+      wide = over_row(rest, 2) > 0.f;
     }
-    wide = rest > 0.f && !(bulk2 >= 17179869184.f * (float)K && bulk >= 65536.f * (float)K);
   }
   if (t == 0) {
     const float rs = norm_w != nullptr ? inv * rsqrtf(ss * (1.0f / (float)K) + eps) : inv;

@@ -1,8 +1,8 @@
 """The dense weight-only GEMM (tcgen05 path) against the CPU restatement of
 buddy-mlir's prefill matmul, through the C ABI.  Tolerance 1e-3 of the
 output's magnitude (the tolerance stated for f32 logits); observed errors are
-near 1e-5 (two bf16 terms per activation, exact int8 weights, f32
-accumulation)."""
+near 1e-7 (three int8 digits per activation, exact sums per digit, f32
+additions of them)."""
 import os
 
 import numpy as np
@@ -59,8 +59,8 @@ def test_gemm_w8_matches_prefill_restatement(M, N, K):
 
 @pytest.mark.parametrize("M,K,N", [(70, 1536, 512), (600, 1600, 768)])
 def test_gemm_w8_fused_norm_bias_residual_and_silu_pairs(M, K, N):
-    """Few rows: the converting kernel (split over K); many rows: the dense kernel with the
-    warp-per-row activation split, a K that ends in a partial block of the packed rows."""
+    """Few rows: k ranges split over CTAs; many rows: whole tiles, a warp per row for the digits, a K that ends in a
+    partial block of the packed rows."""
     from gpu_util import dev, packed_weight, gemm_w8
     rng = np.random.default_rng(5)
     A = rng.standard_normal((M, K)).astype(np.float32)
