@@ -98,12 +98,97 @@ __device__ __forceinline__ uint4 block_scales(const MmaP &p, int64_t row, int b)
   return v;
 }
 
+// The whole product in f32, for calls with a row whose bulk lies too far below its largest elements for four digits (a channel
+// some thousand times the rest): the output columns that do not use those channels would lose (10000 times: 4.8e-6 of their
+// size, here 1.4e-7).  A warp takes a pair of output rows and four activation rows at a time, lanes the units.  Small and out
+// of line: the code of the products above must stay short.
+template <int KIND, bool GROUPED, bool XF>
+__device__ __noinline__ void float_rows(const MmaP &p, const float *s_scale, const float *s_inv) {
+  constexpr bool U4 = KIND == B200_W_U4;
+  const int lane = threadIdx.x & 31, W = blockDim.x >> 5, E = U4 ? 32 : 16, units = p.Kp / E;
+#pragma unroll 1
+  for (int64_t n0 = 2 * ((int64_t)blockIdx.x * W + (threadIdx.x >> 5)); n0 < p.N; n0 += 2 * (int64_t)gridDim.x * W)
+#pragma unroll 1
+    for (int m0 = 0; m0 < p.M; m0 += 4) {
+      float acc[2][4] = {};
+#pragma unroll 1
+      for (int u = lane; u < units; u += 32) {
+        const int b = u >> 5, nu = min(32, units - 32 * b);   // packed rows: blocks of 32 units, see packed_offset
+        uint4 w[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+          w[r] = ld_weights(p.w + min(n0 + r, (int64_t)p.N - 1) * p.row_bytes + (int64_t)u * 16);
+#pragma unroll 1
+        for (int j = 0; j < (U4 ? 8 : 4); ++j) {
+          const int k = b * 32 * E + j * (nu * 4) + 4 * (u & 31);
+          float q[2][4];
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const uint32_t a = U4 ? w[r].x & 0xFFFFu : w[r].x;   // this group's four weights
+            float g = 1.f;
+            if (GROUPED && k < p.K)
+              g = __half2float(__ldg(reinterpret_cast<const __half *>(p.scale) + min(n0 + r, (int64_t)p.N - 1) * p.ngroups + (k >> 7)));
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              q[r][e] = g * (float)(U4 ? (int)(a >> (4 * e) & 15u) - 8 : (int)(int8_t)(a >> (8 * e)));
+            if (U4 && !(j & 1)) {   // the next group: the upper half of the word, or the next word
+              w[r].x >>= 16;
+            } else {
+              w[r] = make_uint4(w[r].y, w[r].z, w[r].w, 0u);
+            }
+          }
+#pragma unroll
+          for (int m = 0; m < 4; ++m) {
+            const float4 x = normed<XF>(p, k, act4<XF>(p, min(m0 + m, p.M - 1), k));
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+              acc[r][m] += fmaf(x.x, q[r][0], fmaf(x.y, q[r][1], fmaf(x.z, q[r][2], x.w * q[r][3])));
+          }
+        }
+      }
+      float mine = 0.f;   // lane 2m + r: row n0 + r, activation row m0 + m
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const float v = warp_sum(acc[r][m]);
+          if (lane == 2 * m + r)
+            mine = v;
+        }
+      const int m = m0 + (lane >> 1);
+      const int64_t row = n0 + (lane & 1);
+      const bool in = lane < 8 && m < p.M && row < p.N;
+      float v = mine;
+      if (in) {
+        v *= s_inv[m] * s_scale[m];   // 1, the RMSNorm's factor, or NaN
+        if (!GROUPED)
+          v *= load_as_float(p.scale, p.scale_dtype, row);
+        if (p.bias != nullptr)
+          v = __ldg(p.bias + row) + v;
+      }
+      const float up = __shfl_down_sync(0xffffffffu, v, 1);
+      int64_t o = (int64_t)m * p.y_ld + row;
+      if (!in || (p.silu_pairs && (lane & 1)))
+        continue;
+      if (p.silu_pairs) {
+        v = silu_gate(v, up);
+        o = (int64_t)m * p.y_ld + (row >> 1);
+      } else if (p.residual != nullptr) {
+        v = p.residual[o] + v;
+      }
+      if (p.y_dtype == B200_F32)
+        ((float *)p.y)[o] = p.accumulate ? ((float *)p.y)[o] + v : v;
+      else
+        ((__half *)p.y)[o] = __float2half_rn(p.accumulate ? __half2float(((__half *)p.y)[o]) + v : v);
+    }
+}
+
 template <int COLS> constexpr int kMaxWarps = COLS <= 16 ? 16 : COLS <= 32 ? 12 : 8;   // what the accumulators leave registers for
 
 // XF: f32 activations in whole 16-byte groups.  Compiled for the two common cases so that the code a short call has to
 // fetch stays small: a GEMV of a few microseconds is bound by its chain of latencies (instruction fetch among them).
 template <int KIND, int COLS, bool GROUPED, bool XF>
-__global__ void __launch_bounds__(kMaxWarps<COLS> * 32, 1) gemv_mma_kernel(const MmaP p) {
+__global__ void __launch_bounds__(kMaxWarps<COLS> * 32, 1) gemv_mma_kernel(const __grid_constant__ MmaP p) {
   extern __shared__ __align__(16) uint8_t sm[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = blockDim.x, W = nthr >> 5;
   uint8_t *planes = sm;
@@ -113,7 +198,9 @@ __global__ void __launch_bounds__(kMaxWarps<COLS> * 32, 1) gemv_mma_kernel(const
   float *part = reinterpret_cast<float *>(sm + p.part_off);      // [2][slots][ks][M][16]
   uint32_t *red = reinterpret_cast<uint32_t *>(sm + p.red_off);  // [M][W]
   float *redf = reinterpret_cast<float *>(red + p.M * W);        // [M][W]
-  float *s_scale = redf + p.M * W, *s_inv = s_scale + p.M;       // [M] each
+  uint32_t *redb = reinterpret_cast<uint32_t *>(redf + p.M * W); // [M][W]
+  float *s_scale = reinterpret_cast<float *>(redb + p.M * W), *s_inv = s_scale + p.M;   // [M] each
+  __shared__ int s_wide;                                         // some row has too little of itself in four digits
   const int slot = warp / p.ks, kp = warp - slot * p.ks;
   const int steps = p.steps;
   constexpr bool U4 = KIND == B200_W_U4;
@@ -142,23 +229,33 @@ __global__ void __launch_bounds__(kMaxWarps<COLS> * 32, 1) gemv_mma_kernel(const
   // ---- activations: largest magnitude (and mean square, for the RMSNorm) of every row, then the planes ------------
   // Group i of a row (4 consecutive k; int4: two such 16 apart) -> its first k.
   auto k_of = [&](int i, int units) { return U4 ? group_u4(i).k : group_i8(i, units).k; };
+  // The bulk of a row, away from its few largest elements: of the warps' smallest maximum of a thread the largest.
+  const bool some = tid * 4 < p.K;   // this thread has elements of every row
   auto reduce_row = [&](int m, uint32_t mx, float ss) {
+    const uint32_t low = __reduce_min_sync(0xffffffffu, some ? mx : 0xffffffffu);
     mx = __reduce_max_sync(0xffffffffu, mx);
     if (p.norm_w != nullptr)
       ss = warp_sum(ss);
     if (lane == 0) {
       red[m * W + warp] = mx;
       redf[m * W + warp] = ss;
+      redb[m * W + warp] = low == 0xffffffffu ? 0u : low;
     }
   };
   auto finish_rows = [&]() {
+    if (tid == 0)
+      s_wide = 0;
     __syncthreads();
     for (int m = warp; m < p.M; m += W) {   // a warp per row
       const uint32_t mx = __reduce_max_sync(0xffffffffu, lane < W ? red[m * W + lane] : 0u);
+      const uint32_t bulk = __reduce_max_sync(0xffffffffu, lane < W ? redb[m * W + lane] : 0u);
       const float ss = p.norm_w != nullptr ? warp_sum(lane < W ? redf[m * W + lane] : 0.f) : 0.f;
       if (lane == 0) {
         float inv;
-        s_scale[m] = fixed_scale(mx, &inv);
+        const float scale = fixed_scale(mx, &inv);
+        s_scale[m] = scale;
+        if (mx != 0u && mx < 0x7f800000u && __uint_as_float(bulk) * scale < 2097152.f)   // 2^21 units: 2^-22 is as f32 sums round
+          s_wide = 1;
         s_inv[m] = p.norm_w != nullptr ? inv * rsqrtf(ss * (1.0f / (float)p.K) + p.eps) : inv;
       }
     }
@@ -324,6 +421,10 @@ __global__ void __launch_bounds__(kMaxWarps<COLS> * 32, 1) gemv_mma_kernel(const
     }
   };
 
+  if (s_wide) {   // (the same in all CTAs)
+    float_rows<KIND, GROUPED, XF>(p, s_scale, s_inv);
+    return;
+  }
   int s = kp, buf = 0;
   for (int r = 0; r < p.rounds; ++r) {
     const int64_t tile = tile_of(r);
@@ -463,7 +564,7 @@ template <int KIND, int COLS, bool GROUPED, bool XF> static int launch_mma(MmaP 
   const int blk = U4 ? 1024 : 512, span = U4 ? p.tail_k0 : p.units * 16;
   const int tsets = (p.tunits + 3) / 4;
   const int tail_bytes = tsets * 4 * SB, tstart_bytes = tsets * 8 * COLS * 4;
-  const int part_bytes = 2 * W * p.M * kTileRows * 4, red_bytes = p.M * (2 * W + 2) * 4;
+  const int part_bytes = 2 * W * p.M * kTileRows * 4, red_bytes = p.M * (3 * W + 2) * 4;
   const int room = kMmaSmem - tail_bytes - tstart_bytes - part_bytes - red_bytes;
   const int per_blk = blk / 64 * SB + (U4 ? 16 * COLS * 4 : 0);   // a set covers 64 k
   int nblk = (span + blk - 1) / blk;

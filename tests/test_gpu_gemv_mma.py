@@ -73,3 +73,59 @@ def test_rows_of_very_different_size_and_a_row_with_a_nan():
     ref = orc.gemv_w8_f32(x[[0, 1, 3]], Q, s)
     assert rel(y[0], ref[0]) < 1e-5 and rel(y[1], ref[1]) < 1e-5
     assert not np.isfinite(y[2]).any() and (y[3] == 0).all()
+
+
+@pytest.mark.parametrize("times", [1, 200, 3000, 1e5, 1e9])
+@pytest.mark.parametrize("kind,M,N,K", [("i8", 2, 77, 528), ("i8", 5, 1001, 1040), ("i8", 16, 250, 12304), ("i8", 1, 4100, 1552),
+                                        ("u4", 2, 130, 640), ("u4", 5, 1000, 1152), ("u4", 1, 9000, 1664), ("u4", 16, 100, 9088),
+                                        ("u4", 9, 40000, 2048)])
+def test_rows_with_one_large_channel(kind, M, N, K, times):
+    """Outputs that do not use the channel keep the precision of the rest: an element's rounding to four digits is at most 2^-22 of
+    the rest; in f32 a lane adds up to K / 128 groups of four (96 here), sqrt(96 / 3) * 2^-24 = 3.4e-7 of the sum, which is up to 127 / 73
+    of the column's size; the largest of 2000 such errors lies near 4.5 of their rms: 2.7e-6."""
+    from gpu_util import dev, gemv, packed_scales, packed_weight
+    rng = np.random.default_rng(M * 7 + N + K)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    x[0 if M < 3 else slice(1, None, 2), 17] *= np.float32(times)     # some rows only
+    if kind == "i8":
+        Q = rng.integers(-127, 128, (K, N)).astype(np.int8)
+        Q[17, ::2] = 0
+        s = rng.uniform(0.001, 0.01, N).astype(np.float32)
+        y = gemv(_lib.W_I8, packed_weight(_lib.W_I8, Q, K, N), dev(s), K, N, dev(x)).cpu().numpy()
+        want = (x.astype(np.float64) @ Q.astype(np.float64)) * s
+    else:
+        P = rng.integers(0, 256, (K, N // 2)).astype(np.uint8)
+        P[17] = P[17] & 0xF0 | 8                                      # code 8 is zero; the low nibble is the even column
+        s = rng.uniform(0.001, 0.01, (K // 128, N)).astype(np.float16)
+        y = gemv(_lib.W_U4, packed_weight(_lib.W_U4, P, K, N, 0), packed_scales(s, _lib.F16, K // 128, N), K, N, dev(x),
+                 group=128, scale_dtype=_lib.F16).cpu().numpy()
+        q = np.stack([P & 15, P >> 4], axis=2).reshape(K, N).astype(np.float64) - 8
+        want = x.astype(np.float64) @ (q * np.repeat(s.astype(np.float64), 128, axis=0))
+    off = np.abs(y - want)
+    for c in (0, 1):   # the columns without the channel, and with it, over their rms in each row
+        size = np.sqrt((want[:, c::2] ** 2).mean(1, keepdims=True))
+        assert (off[:, c::2] / size).max() < 4e-6
+
+
+def test_wide_rows_norm_silu_accumulate_and_tiny_rows():
+    from gpu_util import dev, gemv, packed_weight
+    rng = np.random.default_rng(5)
+    M, N, K = 6, 2 * 300, 1552
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    x[1, 40] = 3e5
+    nw = (1 + 0.1 * rng.standard_normal(K)).astype(np.float32)
+    Q = rng.integers(-127, 128, (K, N)).astype(np.int8)
+    s = rng.uniform(0.0005, 0.001, N).astype(np.float32)
+    w, ds = packed_weight(_lib.W_I8, Q, K, N), dev(s)
+    y = gemv(_lib.W_I8, w, ds, K, N, dev(x), norm_w=dev(nw), silu=True).cpu().numpy()
+    for m in range(M):
+        r = orc.gemv_w8_f32(orc.rmsnorm(x[m], nw, 1e-6)[None, :], Q, s)[0]
+        assert rel(y[m], orc.silu_mul(np.ascontiguousarray(r[0::2]), np.ascontiguousarray(r[1::2]))) < 1e-5
+    y0 = rng.standard_normal((M, N)).astype(np.float32)
+    y = gemv(_lib.W_I8, w, ds, K, N, dev(x), accumulate=True, y0=dev(y0.copy())).cpu().numpy()
+    assert rel(y, y0 + orc.gemv_w8_f32(x, Q, s)) < 1e-5
+    tiny = (x * np.float32(1e-36)).astype(np.float32)      # far below the smallest scale of four digits
+    y = gemv(_lib.W_I8, w, ds, K, N, dev(tiny)).cpu().numpy()
+    want = (tiny.astype(np.float64) @ Q.astype(np.float64)) * s
+    for m in range(M):
+        assert np.abs(y[m] - want[m]).max() / np.abs(want[m]).max() < 1e-5
