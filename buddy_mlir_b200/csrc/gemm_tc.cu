@@ -291,11 +291,15 @@ __device__ __forceinline__ void store_tile(const GemmParams &p, Bars &bars, uint
 // 1024 x 17920 x 1536 106.8, 108.4, and 110.5 with these passes as a loop around the tile's code.  For the same reason the loops
 // over the rows of a tile are not unrolled (prefill of 1000 rows: 7.59 -> 7.48 ms).
 template <int BN>
-__device__ __noinline__ void wide_passes(const CUtensorMap &map_x, const CUtensorMap &map_w, const GemmParams &p, uint8_t *tiles,
-                                         uint32_t tmem, int kb0, int nkb) {
+__device__ __noinline__ void wide_passes(const CUtensorMap &map_x, const CUtensorMap &map_w, const GemmParams &p) {
   using R = Ring<BN>;
   constexpr int S = R::STAGES;
+  extern __shared__ __align__(1024) uint8_t smem[];   // (all found again, so that the caller keeps nothing for it)
+  uint8_t *tiles = reinterpret_cast<uint8_t *>(((uintptr_t)smem + 1023) & ~(uintptr_t)1023);
   Bars &bars = *reinterpret_cast<Bars *>(tiles + S * R::STAGE_BYTES);
+  const uint32_t tmem = bars.tmem_base;
+  const int nkb_all = (p.K + BK - 1) / BK;
+  const int kb0 = nkb_all * blockIdx.z / p.splits, nkb = nkb_all * (blockIdx.z + 1) / p.splits - kb0;
   volatile int *ab = &bars.abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, halves = bars.wide;
   int g = nkb, phase = 1;   // k blocks that have gone through the ring, parity of the accumulator's barrier
@@ -344,8 +348,12 @@ __device__ __noinline__ void wide_passes(const CUtensorMap &map_x, const CUtenso
   }
 }
 
-template <int BN, bool PLANES>
-__global__ void __launch_bounds__(kThreads, 2)
+// SLIM: 64 registers a thread, so that a CTA of this GEMM, one of the kernel that makes the digits and one of the next GEMM,
+// which loads its weights meanwhile, are on an SM at once.  A decode step of 6 / 12 / 16 / 20 sequences takes 2.23 / 2.31 / 2.38 /
+// 2.50 ms with it and 2.39 / 2.47 / 2.49 / 2.61 without; at 24 rows it depends on the contexts, 32 and 42 rows take 2.89 / 3.00
+// with it and 2.83 / 2.93 without.
+template <int BN, bool PLANES, bool SLIM>
+__global__ void __launch_bounds__(kThreads, SLIM ? 3 : 2)
 gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                const __grid_constant__ GemmParams p, const __grid_constant__ CUtensorMap map_x) {
   using R = Ring<BN>;
@@ -448,7 +456,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   __syncthreads();
   if (PLANES && bars.wide != 0 && !*ab) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    wide_passes<BN>(map_x, map_w, p, tiles, tmem, kb0, nkb);
+    wide_passes<BN>(map_x, map_w, p);
   }
   if (warp == 1) {
     if (*ab) {   // copies of an abandoned tile may still be in flight: let them land before the CTA ends
@@ -803,7 +811,7 @@ int make_map(CUtensorMap *map, CUtensorMapDataType dt, int bk, void *base, uint6
   return B200_OK;
 }
 
-template <int BN, bool PLANES>
+template <int BN, bool PLANES, bool SLIM = false>
 int launch_gemm(const void *a, int a_rows, const void *x, const void *w, GemmParams &p, int m_tiles, cudaStream_t st) {
   CUtensorMap map_a, map_w, map_x;
   if (int rc = make_map(&map_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, BK, const_cast<void *>(a), p.K, a_rows, (uint64_t)p.K,
@@ -818,9 +826,9 @@ int launch_gemm(const void *a, int a_rows, const void *x, const void *w, GemmPar
                           (uint64_t)p.K, CU_TENSOR_MAP_SWIZZLE_128B))
       return rc;
   static RaisedOn raised;
-  if (int rc = raise_shared_limit(raised, (const void *)gemm_i8_kernel<BN, PLANES>, Ring<BN>::SMEM))
+  if (int rc = raise_shared_limit(raised, (const void *)gemm_i8_kernel<BN, PLANES, SLIM>, Ring<BN>::SMEM))
     return rc;
-  return launch_after(gemm_i8_kernel<BN, PLANES>, dim3((p.N + BN - 1) / BN, m_tiles, p.splits), kThreads, Ring<BN>::SMEM, st,
+  return launch_after(gemm_i8_kernel<BN, PLANES, SLIM>, dim3((p.N + BN - 1) / BN, m_tiles, p.splits), kThreads, Ring<BN>::SMEM, st,
                       map_a, map_w, p, map_x);
 }
 
@@ -914,6 +922,8 @@ int gemm_w8_run(const b200_weight *w, const float *A, int M, int64_t lda, float 
     return launch_gemm<256, true>(planes, m_tiles * BM, wides, w->w, p, m_tiles, st);
   }
   p.splits = split_k((N + 127) / 128 * m_tiles, (K + BK - 1) / BK, std::min(M, kPlaneRows));
+  if (M <= 20)
+    return launch_gemm<128, true, true>(planes, m_tiles * BM, wides, w->w, p, m_tiles, st);
   return launch_gemm<128, true>(planes, m_tiles * BM, wides, w->w, p, m_tiles, st);
 }
 } // namespace b200
