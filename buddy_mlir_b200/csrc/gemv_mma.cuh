@@ -2,9 +2,8 @@
 //
 // An activation row is turned into four int8 planes of one fixed-point number: with e the exponent of the row's
 // largest magnitude, X = rint(x * 2^(29-e)) (|X| < 2^30, the scale is a power of two, so every element within 2^-7 of
-// the largest is exact and the rest is within 2^-31 of it; error of the columns that do not use a channel 1, 1000, 10000 times
-// the rest of a row of 1536, against f64: 4e-8, 1.1e-6, 2.2e-6; the FFMA kernel, which adds and takes off an offset of its int8
-// weights: 1.9e-7, 1.3e-5, 2.9e-5), and
+// the largest is exact and the rest is within 2^-31 of it: tighter than f32 sums until one channel is some thousand
+// times the rest; b200_gemv multiplies such calls in f32), and
 // X = p0*2^24 + p1*2^16 + p2*2^8 + p3 with signed bytes.  The planes are columns of the B operand of
 // mma.m16n8k32.s8: sixteen weight rows are A, as stored, and the products add up exactly in s32.
 //   int8: no conversion at all: 2 loads and 2 MMAs per 1024 weights (the FFMA form: 2 instructions per weight and lane);

@@ -129,3 +129,33 @@ def test_wide_rows_norm_silu_accumulate_and_tiny_rows():
     want = (tiny.astype(np.float64) @ Q.astype(np.float64)) * s
     for m in range(M):
         assert np.abs(y[m] - want[m]).max() / np.abs(want[m]).max() < 1e-5
+
+
+@pytest.mark.parametrize("kind,M,N,K", [("u4", 3, 66, 1032), ("u4", 1, 20000, 2080), ("i8", 3, 55, 1001), ("i8", 7, 130, 8976)])
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_wide_rows_per_channel_and_odd_lengths(kind, M, N, K, dtype):
+    import torch
+    from gpu_util import dev, gemv, packed_scales, packed_weight
+    rng = np.random.default_rng(M + K)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    x[M // 2, K - 3] = 2e5
+    xt = torch.from_numpy(x).cuda() if dtype == "f32" else torch.from_numpy(x).to(torch.bfloat16).cuda()
+    x = xt.float().cpu().numpy()
+    res = rng.standard_normal((M, N)).astype(np.float32)
+    bias = rng.standard_normal(N).astype(np.float32)
+    code = _lib.F32 if dtype == "f32" else _lib.BF16
+    if kind == "i8":
+        Q = rng.integers(-128, 128, (K, N)).astype(np.int8)
+        s = rng.uniform(0.001, 0.01, N).astype(np.float32)
+        y = gemv(_lib.W_I8, packed_weight(_lib.W_I8, Q, K, N), dev(s), K, N, xt, bias=dev(bias), residual=dev(res), x_dtype=code)
+        q = Q.astype(np.float64)
+    else:
+        P = rng.integers(0, 256, (K, N // 2)).astype(np.uint8)
+        s = rng.uniform(0.001, 0.01, N).astype(np.float16)
+        y = gemv(_lib.W_U4, packed_weight(_lib.W_U4, P, K, N, 0), packed_scales(s.reshape(1, N), _lib.F16, 1, N), K, N, xt, scale_dtype=_lib.F16,
+                 bias=dev(bias), residual=dev(res), x_dtype=code)
+        q = np.stack([P & 15, P >> 4], axis=2).reshape(K, N).astype(np.float64) - 8
+    want = (x.astype(np.float64) @ q) * s.astype(np.float64) + bias + res
+    y = y.cpu().numpy()
+    for m in range(M):   # (every row on its own: only one has the large element)
+        assert np.abs(y[m] - want[m]).max() / np.abs(want[m]).max() < 1e-5
