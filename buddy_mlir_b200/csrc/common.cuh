@@ -192,20 +192,27 @@ int argmax_rows_launch(const float *v, int64_t n, int rows, int32_t *out, cudaSt
 __device__ __forceinline__ void kernel_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void kernel_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... P, typename... A>
-int launch_after(void (*kern)(P...), dim3 grid, int threads, int smem, cudaStream_t st, A... args) {
+int launch_after_clusters(int cluster, void (*kern)(P...), dim3 grid, int threads, int smem, cudaStream_t st, A... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   B200_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
   count_launch();
   return B200_OK;
+}
+template <typename... P, typename... A>
+int launch_after(void (*kern)(P...), dim3 grid, int threads, int smem, cudaStream_t st, A... args) {
+  return launch_after_clusters(1, kern, grid, threads, smem, st, args...);
 }
 
 __device__ __forceinline__ float load_as_float(const void *p, int dtype,

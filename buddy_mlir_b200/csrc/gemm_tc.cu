@@ -11,32 +11,34 @@
 // Operands.  Both are int8 and go from memory to the tensor cores as they are stored (tcgen05.mma kind::i8, s32
 // accumulators in tensor memory).  The weights are the packed decode rows.  A row of activations is a 24-bit fixed-point
 // number per element, in units of a power of two taken from the row's largest magnitude, and its three base-256 digits are
-// three rows of the A operand: a tile of 128 rows is 42 activation rows x 3 digits (planes; two rows are left over), in the
-// k order of the packed weights.  All products and sums are exact integers; the epilogue adds the planes' sums in f32.
+// three neighbouring rows of the digit operand, in the k order of the packed weights.  All products and sums are exact
+// integers; the epilogue adds the digits' sums in f32.
 // Two bf16 terms per activation and weights converted to bf16, the form before this one, kept 2^-17 of each element; three
 // digits keep 2^-23 of the row's largest, which is less where a few channels of a row are far above the rest.  Such rows are
-// wide: six digits, in passes of their own over the tile (planes_kernel says which rows, wide_passes what they cost the others).
+// wide: six digits, in passes of their own over the tile (planes_kernel says which rows).
 // Relative error (2-norm, against f64) of the columns that do not use a channel R times the rest, 256 x 1536 x 1536:
 //   R            1        30       100      1000     10000
 //   now          1.7e-7   1.1e-6   9.4e-7   4.0e-7   8.1e-8
 //   three digits 3.2e-7   3.2e-6   1.0e-5   1.1e-4   9.9e-4    (for every row, 23 bits)
 //   two bf16     2.5e-6 for all; f32 products and sums 7.0e-7
-// Time with no wide row / one / all: 1024 x 17920 x 1536 103 / 112 / 250 us, 1000 x 1536 x 8960 50 / 77 / 139, 24 x 17920 x 1536
-// 11.5 / 21 / 29.
-// Against bf16: half the bytes of the weight operand and no pass that converts weights; three planes are three times the
-// operations of one bf16 product, at 2.4 POP/s (2048 x 8960 x 8960) against 1.6 PFLOP/s.  What few rows need is bytes and
-// latency, and what many rows save are the passes around the GEMM.
 //
-// W8A8 (b200_gemm_w8a8) is the same kernel with one plane: the tile's 128 rows are activation rows.
+// W8A8 (b200_gemm_w8a8) is the same kernel with one digit per activation.
 //
-// A CTA computes a 128 x 128 or 128 x 256 tile of sums: warp 0 issues the TMA loads (cp.async.bulk.tensor, no multicast) of
-// 128-byte k blocks into a ring of 96 KB (3 stages of 32 KB, or 2 of 48), warp 1 one thread of tcgen05.mma, warps 2..9 the
-// epilogue; two CTAs are resident per SM, so one's epilogue runs under the other's main loop.  The weight loads start
-// before the activations are there (programmatic dependent launch behind the kernel that makes the planes; chain_start says
-// what keeps them behind the caller's earlier work).  The main loop
-// is bound by the bytes it brings from L2 (64 bytes per clock and SM), hence 256 columns where that leaves two CTAs
-// for every SM (with planes; W8A8 always takes 128, see there).
-// Few output tiles: the k range is split over gridDim.z, and the CTA that finishes a tile last adds the shares in order.
+// Tiles.  The weights are the operand with M rows (lanes of tensor memory), the digits the one with N columns: a thread of the
+// epilogue then holds one channel, with all digits of an activation in neighbouring registers, so it adds them, scales and
+// stores without shared memory, a warp 128 bytes of an output row at a time; gate and up are neighbouring lanes.  (Digits as M
+// rows: the sums of a row lie in three lanes and go through 66 KB of shared memory.)  The two CTAs of a pair (cta_group::2) work
+// on 256 channels x up to 84 activation rows: each brings its 128 weight rows and half of the digit rows, 32 KB per 128 k, which
+// at 64 bytes per clock takes as long as the products (512 clocks); a CTA by itself brings 48 KB for as many products.
+// The kernel stays on its SMs for all tiles: warp 0 loads (TMA, no multicast), warp 1 issues tcgen05.mma, sixteen warps are the
+// epilogue of one accumulator while the products of the next tile go to the other.  What an epilogue needs from memory it asks
+// for a tile ahead: with loads in its loop over the rows a tile took 16600 clocks, not 6100 (L2 answers late under these loads).
+// Bound by the tensor pipe and its clock: 1024 x 17920 x 1536 72 us with the digits' own pass, 108 us as CTAs of 128 x 256 for
+// a tile each; 65 % of the pipe's cycles at 1.7 GHz, 2.9 POP/s of the padded tiles.  1000 x 1536 x 8960: 41 us (49), 366 x 17920 x
+// 1536: 31 us (50), W8A8 2048 x 8960 x 8960: 143 us (213).
+// Few tiles: the k range is cut over the pairs of a cluster, whose sums meet in shared memory: make_plan().  The weight loads
+// start before the activations are there (programmatic dependent launch behind the kernel that makes the digits; chain_start says
+// what keeps them behind the caller's earlier work).
 //
 // Every wait is bounded (poll count and wall time); on expiry the CTA records
 // an error, all roles fall through, tensor memory is released and the host
@@ -54,320 +56,441 @@ namespace b200 {
 
 namespace {
 
-constexpr int BM = 128;                        // rows of a tile of sums
+constexpr int BM = 128;                        // channels of a CTA's tile
 constexpr int BK = 128;                        // int8 per k block: one 128-byte swizzle row
-constexpr int kPlanes = 3, kPlaneRows = 42;    // digits per activation, activation rows per tile
-constexpr int kWidePlanes = 6, kWideRows = 21; // the same for rows that need six digits: half a tile's rows at a time
-constexpr int kThreads = 320;                  // loader, mma, 8 epilogue warps
-constexpr int kEpiWarps = 8;
-constexpr int kMaxStages = 3;
-constexpr int kSms = 148, kResident = 2 * kSms;   // CTAs of the GEMM that run at once: two per SM
-constexpr int kMaxPartialTiles = 320;          // split-K: shares of tiles in the workspace (a little over one per resident CTA)
-constexpr int kHeadBytes = 2048;               // workspace head: error word, scales of W8A8, arrival counters
-
-template <int BN> struct Ring {
-  static constexpr uint32_t A_BYTES = BM * BK, W_BYTES = BN * BK, STAGE_BYTES = A_BYTES + W_BYTES;
-  static constexpr int STAGES = BN == 256 ? 2 : 3;
-  static constexpr int SMEM = STAGES * (int)STAGE_BYTES + 1024 + 256;
-};
+constexpr int kPlanes = 3, kWidePlanes = 6;    // digits per activation; of rows that need more
+constexpr int kMaxStages = 8;
+constexpr int kSms = 148, kPairs = kSms / 2;
+constexpr int kMaxSplits = 4;                  // along k: clusters of up to eight CTAs
+constexpr int kHeadBytes = 256;                // workspace head: error word, scales of W8A8
+constexpr int kHeadWords = 16;                 // of it, cleared at the start of a call
+constexpr uint32_t kWBytes = BM * BK;
 
 struct Bars {
-  uint64_t full[kMaxStages];   // TMA bytes of the stage have landed
+  uint64_t full[kMaxStages];   // TMA bytes of the stage have landed (in both CTAs of a pair: the first one's)
   uint64_t empty[kMaxStages];  // the tensor core is done with the stage
-  uint64_t accum;              // all MMAs have completed
+  uint64_t acc_full[2];        // an accumulator's MMAs have completed
+  uint64_t acc_empty[2];       // the epilogue warps (of both CTAs) have read it
+  uint64_t sums;               // split k: the sums of all shares for this CTA's rows are here
   uint32_t tmem_base;
   int abort_flag;
-  int last;                    // split-K: this CTA completes its tile
-  int wide;                    // halves of the tile's rows that have wide rows
 };
 
-__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar) {
+// (of a pair: the barrier may be the other CTA's)
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y)
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y)
       : "memory");
 }
 __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap *map, int x, int y) {
   asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
 }
-// kind::i8 instruction descriptor: D = s32, A = B = s8, both K-major, M = 128.
-template <int BN>
-__device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
-  constexpr uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+// kind::i8 instruction descriptor: D = s32, A = B = s8, both K-major, M = 2 x 128 channels, N = nc digits.
+__device__ __forceinline__ uint32_t mma_desc(int nc) {
+  return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nc >> 3) << 17) | ((uint32_t)(2 * BM >> 4) << 24);
+}
+// Executed by a whole warp in uniform control flow (the operands then live in uniform registers), issued by the lane whose
+// `leader` is set.
+__device__ __forceinline__ void mma_i8(uint32_t leader, uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}"
-      ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
+      "{\n .reg .pred p, l;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 l, %5, 0;\n"
+      " @l tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n}"
+      ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t in_cta(uint32_t addr, uint32_t rank) {   // the same shared-memory place in a CTA of the cluster
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void cluster_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// Arrives at `bar` in both CTAs of the pair when the MMAs issued so far have completed.
+__device__ __forceinline__ void commit(uint64_t *bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+               "h"((uint16_t)(3u << (cluster_rank() & ~1u)))
+               : "memory");
+}
+__device__ __forceinline__ void sync_cluster() {   // all its threads
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Eight columns of this warp's 32 lanes of tensor memory
+__device__ __forceinline__ void tmem_load(uint32_t addr, uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(addr)
+               : "memory");
 }
 struct GemmParams {
   int M, N, K;                 // K: multiple of 64
   const float *scale, *bias;   // [N], bias may be null
-  const float *row_scale;      // planes: [M], negative for wide rows; W8A8: one value
+  const float *row_scale;      // digits: [M], negative for wide rows; W8A8: one value
   const float *residual;       // [M, ldr] or null; may alias C
   float *C;                    // [M, ldc]
   int64_t ldc, ldr;
   int silu_pairs;              // columns (2j, 2j+1) are (gate_j, up_j): C[m, j] = silu(g) * u, ldc counts N/2 columns
-  int splits;                  // CTAs along K per tile (gridDim.z)
-  void *partial;               // [tiles][splits][rows][128]: f32 sums of the planes, or s32 (W8A8)
-  uint32_t *arrived;           // [tiles], zeroed by the kernel before
+  int splits;                  // CTAs (pairs) along K per tile: those of a cluster, which then has one tile
+  int share_rows;              // rows that each of them completes
+  int tiles, m_tiles;          // the row tiles of a column tile are neighbours
+  int stages;
   int *error;
+  int nc, rows;                // digits (columns) and activation rows of a tile
+  int cols;                    // of tensor memory: a power of two, two accumulators
 };
 
-// The operations and their order are the reference's.
+struct Tile {
+  int n0, m0, rows;
+};
+__device__ __forceinline__ Tile tile_at(const GemmParams &p, int w) {
+  const int nt = w / p.m_tiles, m0 = (w - nt * p.m_tiles) * p.rows;
+  return {nt * (2 * BM), m0, min(p.rows, p.M - m0)};
+}
+// The row scales of a tile (lane l: rows l, l + 32, l + 64; a row that is not there: 0), requested a tile ahead of their use.
+struct RowScales {
+  float v[3];
+  __device__ __forceinline__ void load(const GemmParams &p, int m0, int rows) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      v[j] = 32 * j + lane < rows ? __ldcg(p.row_scale + m0 + 32 * j + lane) : 0.f;
+  }
+  // Which halves of the rows have wide rows: those halves are passes of their own.
+  __device__ __forceinline__ uint32_t wide_halves(const GemmParams &p) const {
+    const int lane = threadIdx.x & 31, half = (p.rows + 1) >> 1;
+    uint32_t h = 0;
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      if (signbit(v[j]))
+        h |= 32 * j + lane < half ? 1u : 2u;
+    return __reduce_or_sync(0xffffffffu, h);
+  }
+  __device__ __forceinline__ float at(int r0) const { return r0 < 32 ? v[0] : r0 < 64 ? v[1] : v[2]; }   // rows r0 & ~31 ..
+};
+
+// The operations and their order are the reference's (subgraph0_decode_simplify.mlir:226-231: (g * sigmoid(g)) * u).  The
+// reciprocal is the hardware's and one Newton step, without the divide's branch for other ranges: the chains of several
+// rows run side by side.
 __device__ __forceinline__ float silu_of(float g, float u) {
-  const float sg = 1.0f / (1.0f + expf(-g));   // subgraph0_decode_simplify.mlir:226-231
-  return __fmul_rn(__fmul_rn(g, sg), u);
+  const float d = 1.0f + expf(-g);
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
+  r = d < 3.4e38f ? fmaf(r, fmaf(-d, r, 1.0f), r) : 0.f;
+  return __fmul_rn(__fmul_rn(g, r), u);
 }
 
-// The epilogue warps' part of a pass: a thread reads an accumulator row (its lane of tensor memory) and half of its columns; the
-// sums go to a padded tile in shared memory (the ring is idle by then), from where the warps add up the planes and write whole
-// rows, warp w rows w, w + 8, .. of the pass: lane j holds the scale of the j-th of them (row_scales).  SIX: the pass over the wide
-// rows of one half of the tile's rows.
-template <bool PLANES> __device__ __forceinline__ float row_scales(const GemmParams &p, int first, int rows) {
-  if (!PLANES)
-    return p.row_scale[0];
-  const int r = ((int)threadIdx.x >> 5) - 2 + (threadIdx.x & 31) * kEpiWarps;
-  return r < rows ? p.row_scale[blockIdx.y * kPlaneRows + first + r] : 0.f;
-}
-template <int BN, bool PLANES, bool SIX>
-__device__ __forceinline__ void store_tile(const GemmParams &p, Bars &bars, uint8_t *tiles, uint32_t tmem, bool ok, int half,
-                                           float scales) {
-  constexpr int kRows = PLANES ? kPlaneRows : BM;   // activation rows of the tile
-  constexpr int kStep = SIX ? kWideRows : kRows;
-  constexpr int kFold = SIX ? 1 : 8;                // shares of a split tile in flight
-  constexpr int LDS = 128 + 4;                      // row stride of the staging tile, in words
-  float *ep = reinterpret_cast<float *>(tiles);     // [BM][LDS]: 66 KB of the ring
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ew = warp - 2, quad = warp & 3;
-  const int m0 = blockIdx.y * kRows, n0 = blockIdx.x * BN, rows_all = min(kRows, p.M - m0);
-  const int first = SIX ? half * kWideRows : 0, rows = min(kStep, rows_all - first);   // the pass's rows of the tile
-#pragma unroll 1
-  for (int h = 0; h < BN / 128; ++h) {   // 128 columns of the accumulator at a time
-    const int nh = n0 + h * 128;
-    if (nh >= p.N)
-      break;
-    if (h > 0)   // the staging tile is free again once the previous half has been stored
-      asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
-    if (ok && (PLANES || quad * 32 < p.M - m0)) {   // lanes beyond M hold nothing
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      // a warp reads the 32 lanes of tensor memory that match its rank within its warpgroup; the two warps that share a
-      // lane quarter take half the columns each
-      const int row = quad * 32 + lane, cb0 = (ew >> 2) * 64;
-      const int d = row / kStep;   // PLANES: which digit; its weight is 2^16, 2^8, 1, 2^-7, 2^-15, 2^-23
-      const float f = __uint_as_float((uint32_t)(127 + 16 - 8 * d + (d >= kPlanes)) << 23);
-#pragma unroll 1
-      for (int cb = cb0; cb < cb0 + 64; cb += 32) {
-        uint32_t v[32];
-        const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(h * 128 + cb);
-        tmem_load32(taddr, v);
-        tmem_wait_load();
-        float *erow = ep + row * LDS + cb;
+// ---- epilogue ----------------------------------------------------------------------------------------------------------------
+// A warp reads the 32 lanes of tensor memory that match its rank within its warpgroup, a lane one channel; the warps that share a
+// lane quarter take CR rows of the tile in turn.
+constexpr int CR = 8;
+constexpr int kEpiWarps = 16, kGroups = kEpiWarps / 4, kThreads = 64 + 32 * kEpiWarps;
+struct Channel {
+  int n;               // this lane's
+  bool in;
+  float scale, bias;
+  __device__ __forceinline__ Channel(const GemmParams &p, int channel) : n(channel), in(channel < p.N) {
+    scale = __ldg(p.scale + min(n, p.N - 1));
+    bias = p.bias ? __ldg(p.bias + min(n, p.N - 1)) : 0.f;
+  }
+};
+// Sums of N rows from row m of C on -> results.  rs: row scales, that of row i in lane `from` + i (W8A8: the one scale).  ALL: all
+// N rows are stored, otherwise those whose bit of `live` is set.
+template <bool PLANES, bool ALL, int N>
+__device__ __forceinline__ void finish_rows(const GemmParams &p, const Channel &c, int m, float (&y)[N], float rs, int from, uint32_t live,
+                                            const float (&res)[N]) {
 #pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-          float4 o;
-          if (PLANES)
-            o = make_float4(__int2float_rn((int)v[j]) * f, __int2float_rn((int)v[j + 1]) * f,
-                            __int2float_rn((int)v[j + 2]) * f, __int2float_rn((int)v[j + 3]) * f);
-          else
-            o = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]),
-                            __uint_as_float(v[j + 3]));
-          *reinterpret_cast<float4 *>(erow + j) = o;
-        }
-      }
+  for (int i = 0; i < N; ++i) {
+    if (PLANES)
+      y[i] = __fmul_rn(__fmul_rn(y[i], fabsf(__shfl_sync(0xffffffffu, rs, from + i))), c.scale);
+    else   // linalg.py:12836-12846: float(acc) * (act_scale * weight_scale[n])
+      y[i] = __fmul_rn(__int2float_rn(__float_as_int(y[i])), __fmul_rn(rs, c.scale));
+  }
+  if (p.bias) {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      y[i] = __fadd_rn(y[i], c.bias);
+  }
+  if (p.silu_pairs) {   // (gate, up) are neighbouring lanes: of two rows the even lane takes the first, the odd one the second
+    const bool odd = c.n & 1;
+    float *dst = p.C + (int64_t)m * p.ldc + (c.n >> 1) + (odd ? p.ldc : 0);
+#pragma unroll
+    for (int i = 0; i < N; i += 2) {
+      const float other = __shfl_xor_sync(0xffffffffu, odd ? y[i] : y[i + 1], 1);
+      const float v = silu_of(odd ? other : y[i], odd ? y[i + 1] : other);
+      if (c.in && (ALL || (live >> (odd ? i + 1 : i) & 1)))
+        *dst = v;
+      dst += 2 * p.ldc;
     }
-    asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
-    const int cols = min(128, p.N - nh);
-    // sums of the pass's row r, columns c .. c + 3 of this CTA's k range
-    auto sums = [&](int r, int c) {
-      float4 a = *reinterpret_cast<const float4 *>(ep + r * LDS + c);
-      if (PLANES) {
+  } else {
+    float *dst = p.C + (int64_t)m * p.ldc + c.n;
 #pragma unroll
-        for (int q = 1; q < (SIX ? kWidePlanes : kPlanes); ++q) {
-          const float4 b = *reinterpret_cast<const float4 *>(ep + (q * kStep + r) * LDS + c);
-          a = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
-        }
-      }
-      return a;
-    };
-    bool mine = ok;
-    int r0 = first, nr = rows;   // the rows to finish
-    const int tile = blockIdx.y * gridDim.x + blockIdx.x;
-    float4 *shares = reinterpret_cast<float4 *>(p.partial) + (int64_t)tile * p.splits * kRows * 32;
-    if (p.splits > 1) {   // (BN = 128) leave this CTA's share; after its last pass the last CTA of the tile goes on
-      if (ok)   // (a wide row's share is written again by the pass with six digits, which has nothing for other rows)
-#pragma unroll 1
-        for (int r = ew, j = 0; r < rows; r += kEpiWarps, ++j)
-          if (!SIX || signbit(__shfl_sync(0xffffffffu, scales, j)))
-            __stcg(shares + ((int64_t)blockIdx.z * kRows + first + r) * 32 + lane, sums(r, lane * 4));
-      mine = false;
-      if (!PLANES || bars.wide >> (SIX ? half + 1 : 0) == 0) {
-        __threadfence();
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
-        if (threadIdx.x == 64)
-          bars.last = atomicAdd(p.arrived + tile, 1u) == (uint32_t)p.splits - 1;
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
-        __threadfence();
-        mine = ok && bars.last;
-      }
-      r0 = 0;
-      nr = rows_all;
-      if (SIX)
-        scales = row_scales<PLANES>(p, 0, rows_all);
-    }
-    if (mine) {
-      const bool vec = (p.ldc & 3) == 0 && ((uintptr_t)p.C & 15) == 0 && (p.N & 3) == 0 &&
-                       (!p.residual || ((p.ldr & 3) == 0 && ((uintptr_t)p.residual & 15) == 0));
-#pragma unroll 1
-      for (int r = ew, j = 0; r < nr; r += kEpiWarps, ++j) {
-        const float rs = PLANES ? __shfl_sync(0xffffffffu, scales, j) : scales;
-        const int i = r * 32 + lane, c = lane * 4, m = m0 + r0 + r, n = nh + c;
-        if (c >= cols || (PLANES && p.splits == 1 && signbit(rs) != SIX))   // (finished by another pass)
-          continue;
-        float y[4];
-        if (p.splits > 1) {
-          float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-          for (int z0 = 0; z0 < p.splits; z0 += kFold) {
-            float4 b[kFold];
-#pragma unroll
-            for (int z = 0; z < kFold; ++z)
-              b[z] = z0 + z < p.splits ? __ldcg(shares + (int64_t)(z0 + z) * kRows * 32 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int z = 0; z < kFold; ++z)
-              if (PLANES)
-                a = make_float4(a.x + b[z].x, a.y + b[z].y, a.z + b[z].z, a.w + b[z].w);
-              else
-                a = make_float4(__int_as_float(__float_as_int(a.x) + __float_as_int(b[z].x)),
-                                __int_as_float(__float_as_int(a.y) + __float_as_int(b[z].y)),
-                                __int_as_float(__float_as_int(a.z) + __float_as_int(b[z].z)),
-                                __int_as_float(__float_as_int(a.w) + __float_as_int(b[z].w)));
-          }
-          y[0] = a.x; y[1] = a.y; y[2] = a.z; y[3] = a.w;
-        } else {
-          const float4 a = sums(r, c);
-          y[0] = a.x; y[1] = a.y; y[2] = a.z; y[3] = a.w;
-        }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int ne = min(n + e, p.N - 1);
-          if (PLANES)
-            y[e] = __fmul_rn(__fmul_rn(y[e], fabsf(rs)), __ldg(p.scale + ne));
-          else   // linalg.py:12836-12846: float(acc) * (act_scale * weight_scale[n])
-            y[e] = __fmul_rn(__int2float_rn(__float_as_int(y[e])), __fmul_rn(rs, __ldg(p.scale + ne)));
-          if (p.bias)
-            y[e] = __fadd_rn(y[e], __ldg(p.bias + ne));
-        }
-        if (p.silu_pairs) {
-          float *dst = p.C + (int64_t)m * p.ldc + (n >> 1);
-          dst[0] = silu_of(y[0], y[1]);
-          if (n + 3 < p.N)   // N is even
-            dst[1] = silu_of(y[2], y[3]);
-        } else {
-          float *dst = p.C + (int64_t)m * p.ldc + n;
-          const float *res = p.residual + (int64_t)m * p.ldr + n;
-          if (vec) {
-            if (p.residual) {
-              const float4 q = *reinterpret_cast<const float4 *>(res);
-              y[0] = __fadd_rn(q.x, y[0]);
-              y[1] = __fadd_rn(q.y, y[1]);
-              y[2] = __fadd_rn(q.z, y[2]);
-              y[3] = __fadd_rn(q.w, y[3]);
-            }
-            *reinterpret_cast<float4 *>(dst) = make_float4(y[0], y[1], y[2], y[3]);
-          } else {
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-              if (n + e < p.N)
-                dst[e] = p.residual ? __fadd_rn(res[e], y[e]) : y[e];
-          }
-        }
-      }
+    for (int i = 0; i < N; ++i) {
+      if (c.in && (ALL || (live >> i & 1)))
+        *dst = p.residual ? __fadd_rn(res[i], y[i]) : y[i];
+      dst += p.ldc;
     }
   }
 }
-
-// The tile's wide rows once more, with six digits: a half of its rows at a time (`halves`: which).  Everything a normal tile does
-// again, in a function of its own and with little code, since code counts even where it does not run: without wide rows,
-// 24 x 17920 x 1536 takes 13.5 us without this function, 13.9 with it, 16.3 with its loops unrolled as a tile's were;
-// 1024 x 17920 x 1536 106.8, 108.4, and 110.5 with these passes as a loop around the tile's code.  For the same reason the loops
-// over the rows of a tile are not unrolled (prefill of 1000 rows: 7.59 -> 7.48 ms).
-template <int BN>
-__device__ __noinline__ void wide_passes(const CUtensorMap &map_x, const CUtensorMap &map_w, const GemmParams &p) {
-  using R = Ring<BN>;
-  constexpr int S = R::STAGES;
-  extern __shared__ __align__(1024) uint8_t smem[];   // (all found again, so that the caller keeps nothing for it)
-  uint8_t *tiles = reinterpret_cast<uint8_t *>(((uintptr_t)smem + 1023) & ~(uintptr_t)1023);
-  Bars &bars = *reinterpret_cast<Bars *>(tiles + S * R::STAGE_BYTES);
-  const uint32_t tmem = bars.tmem_base;
-  const int nkb_all = (p.K + BK - 1) / BK;
-  const int kb0 = nkb_all * blockIdx.z / p.splits, nkb = nkb_all * (blockIdx.z + 1) / p.splits - kb0;
-  volatile int *ab = &bars.abort_flag;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, halves = bars.wide;
-  int g = nkb, phase = 1;   // k blocks that have gone through the ring, parity of the accumulator's barrier
-  for (int half = 0; half < 2; ++half) {
-    if (!(halves >> half & 1))
-      continue;
-    if (warp == 0) {
-      if (lane == 0)
-        for (int i = 0; i < nkb; ++i) {
-          const int s = (g + i) % S, u = (g + i) / S;
-          if (u > 0 && !mbar_wait(&bars.empty[s], (u - 1) & 1, ab, p.error, 701))
-            break;
-          mbar_expect_tx(&bars.full[s], R::STAGE_BYTES);
-          tma_load_2d(tiles + s * R::STAGE_BYTES + R::A_BYTES, &map_w, (kb0 + i) * BK, blockIdx.x * BN, &bars.full[s]);
-          tma_load_2d(tiles + s * R::STAGE_BYTES, &map_x, (kb0 + i) * BK, (blockIdx.y * 2 + half) * BM, &bars.full[s]);
-        }
-    } else if (warp == 1) {
-      if (lane == 0) {
-        for (int i = 0; i < nkb; ++i) {
-          const int s = (g + i) % S;
-          if (!mbar_wait(&bars.full[s], ((g + i) / S) & 1, ab, p.error, 702))
-            break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a = smem_u32(tiles + s * R::STAGE_BYTES), w = a + R::A_BYTES;
-#pragma unroll 1
-          for (int k = 0; k < BK / 32; ++k)
-            mma_i8<BN>(tmem, smem_desc(a + k * 32), smem_desc(w + k * 32), (i | k) != 0);
-          tc_commit(&bars.empty[s]);
-        }
-        tc_commit(&bars.accum);
-      }
+template <int N>
+__device__ __forceinline__ void load_residual(const GemmParams &p, const Channel &c, int m, int rows, float (&res)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    res[i] = 0.f;
+  if (p.residual != nullptr) {
+    const float *src = p.residual + (int64_t)m * p.ldr + c.n;
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if (c.in && i < rows)
+        res[i] = src[(int64_t)i * p.ldr];
+  }
+}
+// The digits' sums of N rows, ND columns each, added up.
+template <int ND, int N> __device__ __forceinline__ void add_digits(const uint32_t *v, float (&y)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    if constexpr (ND == 1) {
+      y[i] = __uint_as_float(v[i]);
     } else {
-      const int first = half * kWideRows;
-      const float scales = row_scales<true>(p, first, min(kWideRows, p.M - (int)blockIdx.y * kPlaneRows - first));
-      const bool ok = mbar_wait(&bars.accum, phase, ab, p.error, 703) && !*ab;
-      store_tile<BN, true, true>(p, bars, tiles, tmem, ok, half, scales);
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the next pass loads over the staging tile
+#pragma unroll
+      for (int d = 0; d < ND; ++d) {   // the digits' weights: 2^16, 2^8, 1, 2^-7, 2^-15, 2^-23
+        const float b = __int2float_rn((int)v[i * ND + d]) * __uint_as_float((uint32_t)(127 + 16 - 8 * d + (d >= kPlanes)) << 23);
+        y[i] = d == 0 ? b : y[i] + b;
+      }
     }
-    g += nkb;
-    phase ^= 1;
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (*ab)
-      break;
   }
 }
+__device__ __forceinline__ void release_accumulator(uint32_t bar) {
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  if ((threadIdx.x & 31) == 0)
+    cluster_arrive(bar);
+}
+// Split k: a CTA's sums of row r of the tile go to the CTA of the cluster that completes the row, [split][its rows][128 channels].
+struct Shares {
+  uint32_t base;   // this lane's channel of this CTA's share
+  uint32_t rank;   // the cluster's CTA with the same channels and the first share of k
+};
+__device__ __forceinline__ void give_row(const GemmParams &p, const Shares &sh, int row, float v) {
+  const int to = row / p.share_rows;
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(in_cta(sh.base + (uint32_t)(row - to * p.share_rows) * (BM * 4), sh.rank + to * 2)), "f"(v)
+               : "memory");
+}
+// The pass over all rows of a tile.  Split k: the sums go to the CTAs that complete the rows.  wait: until the accumulator at tmem is
+// complete; what the first rows need from memory is requested before it.
+// WIDE: some of the rows are wide, and left to the passes with six digits.
+template <bool PLANES, bool SPLIT, bool WIDE, typename Wait>
+__device__ __forceinline__ void store_tile(const GemmParams &p, const Tile &t, const Channel &c, const RowScales &scales, uint32_t tmem,
+                                           uint32_t release, const Shares &sh, Wait wait) {
+  constexpr int ND = PLANES ? kPlanes : 1;
+  const int grp = (threadIdx.x - 64) >> 7;
+  int r0 = grp * CR;
+  float res[CR];
+  if (!SPLIT)
+    load_residual<CR>(p, c, t.m0 + r0, t.rows - r0, res);
+  const bool ok = wait();
+  if (r0 >= t.rows || !ok) {
+    release_accumulator(release);
+    return;
+  }
+#pragma unroll 1
+  for (; r0 < t.rows; r0 += kGroups * CR) {
+    uint32_t v[ND * CR];
+#pragma unroll
+    for (int q = 0; q < ND; ++q)
+      if (r0 * ND + q * CR < p.nc)
+        tmem_load(tmem + r0 * ND + q * CR, *reinterpret_cast<uint32_t(*)[CR]>(v + q * CR));
+    const float rs = PLANES ? scales.at(r0) : scales.v[0];
+    const int left = t.rows - r0;
+    uint32_t live = left >= CR ? (1u << CR) - 1 : (1u << left) - 1;
+    if (WIDE)
+      live &= ~(__ballot_sync(0xffffffffu, signbit(rs)) >> (r0 & 31));
+    float next[CR], y[CR];
+    if (!SPLIT)
+      load_residual<CR>(p, c, t.m0 + r0 + kGroups * CR, left - kGroups * CR, next);
+    tmem_wait_load();
+    if (left <= kGroups * CR)
+      release_accumulator(release);
+    add_digits<ND, CR>(v, y);
+    if (SPLIT) {
+#pragma unroll
+      for (int i = 0; i < CR; ++i)
+        if (live >> i & 1)
+          give_row(p, sh, r0 + i, y[i]);
+    } else {
+      if (live == (1u << CR) - 1)
+        finish_rows<PLANES, true, CR>(p, c, t.m0 + r0, y, rs, r0 & 31, live, res);
+      else
+        finish_rows<PLANES, false, CR>(p, c, t.m0 + r0, y, rs, r0 & 31, live, res);
+#pragma unroll
+      for (int i = 0; i < CR; ++i)
+        res[i] = next[i];
+    }
+  }
+}
+// The pass with six digits over `rows` rows of a tile, `first` the first: its wide rows.
+template <bool SPLIT>
+__device__ __forceinline__ void store_wide_pass(const GemmParams &p, int m0, const Channel &c, uint32_t tmem, bool ok, int first, int rows,
+                                                uint32_t release, const Shares &sh) {
+  constexpr int N = CR / 2;
+  const int lane = threadIdx.x & 31, grp = (threadIdx.x - 64) >> 7;
+  if (grp * N >= rows || !ok) {
+    release_accumulator(release);
+    return;
+  }
+#pragma unroll 1
+  for (int r0 = grp * N; r0 < rows; r0 += kGroups * N) {
+    uint32_t v[kWidePlanes * N];
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+      if (r0 * kWidePlanes + q * CR < p.nc)
+        tmem_load(tmem + r0 * kWidePlanes + q * CR, *reinterpret_cast<uint32_t(*)[CR]>(v + q * CR));
+    const int m = m0 + first + r0;
+    const float rs = lane < N && r0 + lane < rows ? __ldcg(p.row_scale + m + lane) : 0.f;
+    const uint32_t live = __ballot_sync(0xffffffffu, signbit(rs));
+    float res[N], y[N];
+    if (!SPLIT)
+      load_residual<N>(p, c, m, rows - r0, res);
+    tmem_wait_load();
+    if (r0 + kGroups * N >= rows)
+      release_accumulator(release);
+    add_digits<kWidePlanes, N>(v, y);
+    if (SPLIT) {
+#pragma unroll
+      for (int i = 0; i < N; ++i)
+        if (live >> i & 1)
+          give_row(p, sh, first + r0 + i, y[i]);
+    } else {
+      finish_rows<true, false, N>(p, c, m, y, rs, 0, live, res);
+    }
+  }
+}
+// The rows that this CTA completes, shares added in order.  sums: this lane's channel of the first share.
+template <bool PLANES>
+__device__ __forceinline__ void add_shares(const GemmParams &p, int m0, int rows, const Channel &c, const float *sums) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll 1
+  for (int r0 = ((threadIdx.x - 64) >> 7) * CR; r0 < rows; r0 += kGroups * CR) {
+    const int m = m0 + r0, live = min(CR, rows - r0);
+    float rs = 0.f, res[CR], y[CR];
+    if (!PLANES)
+      rs = p.row_scale[0];
+    else if (lane < live)
+      rs = __ldcg(p.row_scale + m + lane);
+    load_residual<CR>(p, c, m, live, res);
+#pragma unroll
+    for (int i = 0; i < CR; ++i)
+      y[i] = 0.f;
+#pragma unroll 1
+    for (int z = 0; z < p.splits; ++z)
+#pragma unroll
+      for (int i = 0; i < CR; ++i)
+        if (i < live) {
+          const float b = sums[(z * p.share_rows + r0 + i) * BM];
+          y[i] = PLANES ? y[i] + b : __int_as_float(__float_as_int(y[i]) + __float_as_int(b));
+        }
+    finish_rows<PLANES, false, CR>(p, c, m, y, rs, 0, (1u << live) - 1, res);
+  }
+}
+// mbar_wait, and what the cluster's other CTAs stored before they arrived is visible.
+__device__ __forceinline__ bool wait_shares(uint64_t *bar, volatile int *ab, int *err, int code) {
+  if (!mbar_wait(bar, 0, ab, err, code))
+    return false;
+  asm volatile("fence.acq_rel.cluster;" ::: "memory");
+  return true;
+}
 
-// SLIM: 64 registers a thread, so that a CTA of this GEMM, one of the kernel that makes the digits and one of the next GEMM,
-// which loads its weights meanwhile, are on an SM at once.  A decode step of 6 / 12 / 16 / 20 sequences takes 2.23 / 2.31 / 2.38 /
-// 2.50 ms with it and 2.39 / 2.47 / 2.49 / 2.61 without; at 24 rows it depends on the contexts, 32 and 42 rows take 2.89 / 3.00
-// with it and 2.83 / 2.93 without.
-template <int BN, bool PLANES, bool SLIM>
-__global__ void __launch_bounds__(kThreads, SLIM ? 3 : 2)
+// An epilogue warp's way through the tiles from w on; n: accumulators so far.  WIDE = false: up to a tile with wide rows.  The rest
+// is a function that is called once, so that nothing is kept across it.
+template <bool PLANES, bool SPLIT, bool WIDE>
+__device__ __forceinline__ int epilogue(const GemmParams &p, Bars &bars, float *sums, uint32_t tmem, int w, int step, int &n) {
+  const int lane = threadIdx.x & 31, quad = threadIdx.x >> 5 & 3, crank = (int)cluster_rank(), rank = crank & 1;
+  const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16);
+  const int channel = quad * 32 + lane;
+  volatile int *ab = &bars.abort_flag;
+  bool ok = true;
+  if (w >= p.tiles)
+    return w;
+  RowScales scales;
+  auto request = [&](const Tile &i) {
+    if (PLANES)
+      scales.load(p, i.m0, i.rows);
+    else
+      scales.v[0] = __ldcg(p.row_scale);
+  };
+  Tile t = tile_at(p, w);
+  Channel c(p, t.n0 + rank * BM + channel);
+  request(t);
+#pragma unroll 1
+  for (;;) {   // (a warp that gave up goes on without waiting: the barriers keep their count)
+    const uint32_t wide = PLANES ? scales.wide_halves(p) : 0u;
+    if (!WIDE && wide != 0)
+      return w;
+    const int z = crank >> 1;
+    const Shares sh{smem_u32(sums + z * p.share_rows * BM + channel), (uint32_t)rank};
+    auto wait = [&] {
+      ok = ok && __all_sync(0xffffffffu, mbar_wait(&bars.acc_full[n & 1], n >> 1 & 1, ab, p.error, 703));
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      return ok;
+    };
+    auto release = [&] { return in_cta(smem_u32(&bars.acc_empty[n & 1]), crank & ~1); };
+    store_tile<PLANES, SPLIT, WIDE>(p, t, c, scales, lanes + (n & 1) * (p.cols >> 1), release(), sh, wait);
+    ++n;
+    if constexpr (WIDE) {
+      const int half = (p.rows + 1) >> 1;
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h)
+        if (wide >> h & 1) {
+          wait();
+          store_wide_pass<SPLIT>(p, t.m0, c, lanes + (n & 1) * (p.cols >> 1), ok, h * half, min(half, t.rows - h * half), release(), sh);
+          ++n;
+        }
+    }
+    if constexpr (SPLIT) {
+      __syncwarp();
+      if (lane < p.splits)   // (release: this warp's stores come first)
+        cluster_arrive(in_cta(smem_u32(&bars.sums), lane * 2 + rank));
+      ok = __all_sync(0xffffffffu, wait_shares(&bars.sums, ab, p.error, 705)) && ok;
+      const int row = z * p.share_rows;
+      if (ok)
+        add_shares<PLANES>(p, t.m0 + row, min(p.share_rows, t.rows - row), c, sums + channel);
+    }
+    w += step;
+    if (w >= p.tiles)
+      return w;
+    t = tile_at(p, w);   // what it needs is on its way while the tile's products are made
+    c = Channel(p, t.n0 + rank * BM + channel);
+    request(t);
+  }
+}
+template <bool SPLIT>
+__device__ __noinline__ void epilogue_wide(const GemmParams &p, Bars &bars, float *sums, uint32_t tmem, int w, int step, int n) {
+  epilogue<true, SPLIT, true>(p, bars, sums, tmem, w, step, n);
+}
+
+template <bool PLANES, bool SPLIT>
+__global__ void __launch_bounds__(kThreads, 1)
 gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                const __grid_constant__ GemmParams p, const __grid_constant__ CUtensorMap map_x) {
-  using R = Ring<BN>;
-  constexpr int S = R::STAGES;
-  constexpr int kRows = PLANES ? kPlaneRows : BM;   // activation rows of the tile
+  constexpr int ND = PLANES ? kPlanes : 1;
   extern __shared__ __align__(1024) uint8_t smem[];
   // 1024-byte alignment of every swizzled tile
   uint8_t *tiles = reinterpret_cast<uint8_t *>(((uintptr_t)smem + 1023) & ~(uintptr_t)1023);
-  Bars &bars = *reinterpret_cast<Bars *>(tiles + S * R::STAGE_BYTES);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m0 = blockIdx.y * kRows, n0 = blockIdx.x * BN;
-  // this CTA's share of the k blocks
-  const int nkb_all = (p.K + BK - 1) / BK;
-  const int kb0 = nkb_all * blockIdx.z / p.splits, nkb = nkb_all * (blockIdx.z + 1) / p.splits - kb0;
+  const uint32_t stage_bytes = kWBytes + (uint32_t)(p.nc / 2) * BK;
+  const int S = p.stages;
+  float *sums = reinterpret_cast<float *>(tiles + S * stage_bytes);   // split k: [splits][share_rows][128]
+  Bars &bars = *reinterpret_cast<Bars *>(sums + (SPLIT ? p.splits * p.share_rows * BM : 0));
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  // a cluster: `splits` pairs, each with a share of the k blocks
+  const int crank = (int)cluster_rank(), rank = crank & 1, z = crank >> 1;
+  const int first = blockIdx.x / (2 * p.splits), step = gridDim.x / (2 * p.splits);
+  const int all_blocks = (p.K + BK - 1) / BK;
+  const int kb0 = all_blocks * z / p.splits, nkb = all_blocks * (z + 1) / p.splits - kb0;
   volatile int *ab = &bars.abort_flag;
 
   if (threadIdx.x == 0) {
@@ -375,96 +498,151 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       mbar_init(&bars.full[s], 1);
       mbar_init(&bars.empty[s], 1);
     }
-    mbar_init(&bars.accum, 1);
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(&bars.acc_full[a], 1);
+      mbar_init(&bars.acc_empty[a], 2 * kEpiWarps);
+    }
+    mbar_init(&bars.sums, p.splits * kEpiWarps);
     bars.abort_flag = 0;
-    bars.wide = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) {   // tensor memory: one warp allocates, the same warp frees
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars.tmem_base)), "n"(BN) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  if (warp == 1) {   // tensor memory: one warp (of each CTA) allocates, the same warp frees
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars.tmem_base)), "r"(p.cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  sync_cluster();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = bars.tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, bars.tmem_base, 0);
   kernel_go();   // not before the allocation: see tensor_core.cuh
 
   if (warp == 0) {
     // ---- loader --------------------------------------------------------------------------------------------------
+    const uint32_t base = smem_u32(tiles);
+    int s = 0, parity = 1;   // (waiting for the phase before a barrier's first ends at once)
+    auto full = [&](int st) { return in_cta(smem_u32(&bars.full[st]), crank & ~1); };
+    auto load_w = [&](const Tile &t, int i, int st) {
+      if (rank == 0)
+        mbar_expect_tx(&bars.full[st], 2 * stage_bytes);
+      tma_load_2d(base + st * stage_bytes, &map_w, (kb0 + i) * BK, t.n0 + rank * BM, full(st));
+    };
+    Tile t = tile_at(p, first);
+    const int ahead = min(S, nkb);
     if (lane == 0) {
-      auto load_w = [&](int i) {
-        const int s = i % S;
-        mbar_expect_tx(&bars.full[s], R::STAGE_BYTES);
-        tma_load_2d(tiles + s * R::STAGE_BYTES + R::A_BYTES, &map_w, (kb0 + i) * BK, n0, &bars.full[s]);
-      };
-      auto load_a = [&](int i) {
-        const int s = i % S;
-        tma_load_2d(tiles + s * R::STAGE_BYTES, &map_a, (kb0 + i) * BK, blockIdx.y * BM, &bars.full[s]);
-      };
       // few rows: the weights' way from memory is the GEMM; all of this CTA's share starts for L2 while the kernels before run
-      // (if all CTAs are resident at once: 24 x 151936 x 1536, 594 CTAs, took 68 us with it and 60 without)
-      if (gridDim.y <= 2 && gridDim.x * gridDim.y * gridDim.z <= kResident)
+      // (if it has one tile: 24 x 151936 x 1536, in several turns, took 68 us with it and 60 without)
+      if (p.m_tiles <= 2 && p.tiles <= step)
         for (int i = S; i < nkb; ++i)
-          tma_prefetch_2d(&map_w, (kb0 + i) * BK, n0);
-      const int ahead = min(S, nkb);
+          tma_prefetch_2d(&map_w, (kb0 + i) * BK, t.n0 + rank * BM);
       for (int i = 0; i < ahead; ++i)   // the weights do not wait for the kernel before
-        load_w(i);
-      kernel_wait();
-      for (int i = 0; i < ahead; ++i)
-        load_a(i);
-      for (int i = ahead; i < nkb; ++i) {
-        if (!mbar_wait(&bars.empty[i % S], (i / S - 1) & 1, ab, p.error, 701))
-          break;
-        load_w(i);
-        load_a(i);
+        load_w(t, i, i);
+    }
+    kernel_wait();
+    RowScales scales;
+    if (PLANES)
+      scales.load(p, t.m0, t.rows);
+    uint32_t wide = PLANES ? scales.wide_halves(p) : 0u;
+    int ready = ahead;   // stages whose weights are on their way
+    bool ok = true;
+    for (int w = first; w < p.tiles && ok; w += step) {
+      const Tile next = tile_at(p, min(w + step, p.tiles - 1));
+      if (PLANES)
+        scales.load(p, next.m0, next.rows);
+      for (int pass = 0; pass < 3 && ok; ++pass) {
+        if (pass > 0 && !(wide >> (pass - 1) & 1))
+          continue;
+        const CUtensorMap *map = pass ? &map_x : &map_a;
+        const int y = (pass ? kWidePlanes * (t.m0 + (pass - 1) * ((p.rows + 1) >> 1)) : ND * t.m0) + rank * (p.nc / 2);
+        if (lane == 0)
+          for (int i = 0; i < nkb; ++i) {
+            if (ready > 0) {
+              --ready;
+            } else {
+              if (!mbar_wait(&bars.empty[s], parity, ab, p.error, 701)) {
+                ok = false;
+                break;
+              }
+              load_w(t, i, s);
+            }
+            tma_load_2d(base + s * stage_bytes + kWBytes, map, (kb0 + i) * BK, y, full(s));
+            if (++s == S) {
+              s = 0;
+              parity ^= 1;
+            }
+          }
+        ok = __all_sync(0xffffffffu, ok);
       }
+      t = next;
+      wide = PLANES ? scales.wide_halves(p) : 0u;
     }
   } else if (warp == 1) {
-    // ---- tensor core issue (one thread) -----------------------------------------------------------------------------
-    if (lane == 0) {
-      for (int i = 0; i < nkb; ++i) {
-        const int s = i % S;
-        if (!mbar_wait(&bars.full[s], (i / S) & 1, ab, p.error, 702))
-          break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a = smem_u32(tiles + s * R::STAGE_BYTES), w = a + R::A_BYTES;
+    // ---- tensor core issue (of the pair's first CTA) ------------------------------------------------------------------
+    if (rank == 0) {
+      kernel_wait();
+      uint32_t leader;
+      asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(leader));
+      const uint32_t idesc = mma_desc(p.nc);
+      const uint64_t d0 = smem_desc(smem_u32(tiles));
+      int s = 0, parity = 0, n = 0;   // n: accumulators so far
+      bool ok = true;
+      Tile t = tile_at(p, first);
+      RowScales scales;
+      if (PLANES)
+        scales.load(p, t.m0, t.rows);
+      uint32_t wide = PLANES ? scales.wide_halves(p) : 0u;
+      for (int w = first; w < p.tiles && ok; w += step) {
+        const Tile next = tile_at(p, min(w + step, p.tiles - 1));
+        if (PLANES)
+          scales.load(p, next.m0, next.rows);
+        for (int pass = 0; pass < 3 && ok; ++pass) {
+          if (pass > 0 && !(wide >> (pass - 1) & 1))
+            continue;
+          ok = __all_sync(0xffffffffu, mbar_wait(&bars.acc_empty[n & 1], (n >> 1 & 1) ^ 1, ab, p.error, 704));
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t acc = tmem + (n & 1) * (p.cols >> 1);
+          for (int i = 0; i < nkb && ok; ++i) {
+            ok = __all_sync(0xffffffffu, mbar_wait(&bars.full[s], parity, ab, p.error, 702));
+            if (!ok)
+              break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t dw = d0 + ((s * stage_bytes) >> 4), dx = dw + (kWBytes >> 4);
 #pragma unroll
-        for (int k = 0; k < BK / 32; ++k)   // 32 int8 = 32 bytes along the swizzled row
-          mma_i8<BN>(tmem, smem_desc(a + k * 32), smem_desc(w + k * 32), (i | k) != 0);
-        tc_commit(&bars.empty[s]);   // arrives when the MMAs above have read the stage
+            for (int k = 0; k < BK / 32; ++k)   // 32 int8 = 32 bytes along the swizzled row
+              mma_i8(leader, acc, dw + k * 2, dx + k * 2, idesc, (i | k) != 0);
+            if (leader)
+              commit(&bars.empty[s]);   // arrives when the MMAs above have read the stage
+            if (++s == S) {
+              s = 0;
+              parity ^= 1;
+            }
+          }
+          if (ok && leader)
+            commit(&bars.acc_full[n & 1]);
+          ++n;
+        }
+        t = next;
+        wide = PLANES ? scales.wide_halves(p) : 0u;
       }
-      tc_commit(&bars.accum);
     }
   } else {
     // ---- epilogue ----------------------------------------------------------------------------------------------------
-    kernel_wait();   // row scales, counters
-    const float scales = row_scales<PLANES>(p, 0, min(kRows, p.M - m0));
-    if (PLANES) {
-      const uint32_t wide = __ballot_sync(0xffffffffu, signbit(scales));
-      if (wide != 0 && lane == 0)   // rows warp - 2 + 8 j, the first half of the tile: below 21
-        for (int j = 0; j < (kRows + kEpiWarps - 1) / kEpiWarps; ++j)
-          if (wide >> j & 1)
-            atomicOr(&bars.wide, warp - 2 + kEpiWarps * j < kWideRows ? 1 : 2);
-    }
-    const bool ok = mbar_wait(&bars.accum, 0, ab, p.error, 703) && !*ab;
-    store_tile<BN, PLANES, false>(p, bars, tiles, tmem, ok, 0, scales);
-    if (PLANES)
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // a pass over wide rows loads over the staging tile
+    kernel_wait();   // row scales
+    int n = 0, w = first;
+    w = epilogue<PLANES, SPLIT, false>(p, bars, sums, tmem, w, step, n);
+    if (PLANES && w < p.tiles)
+      epilogue_wide<SPLIT>(p, bars, sums, tmem, w, step, n);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (PLANES && bars.wide != 0 && !*ab) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    wide_passes<BN>(map_x, map_w, p);
-  }
+  sync_cluster();   // none ends while another may still signal it
   if (warp == 1) {
     if (*ab) {   // copies of an abandoned tile may still be in flight: let them land before the CTA ends
       const unsigned long long t0 = now_ns();
       while (now_ns() - t0 < 2000000ull) {
       }
     }
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(BN) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(p.cols) : "memory");
   }
 }
 
@@ -501,16 +679,16 @@ __device__ __forceinline__ float plane_scale(uint32_t absbits, float *inv) {
   return __uint_as_float((uint32_t)(22 - e + 127) << 23);
 }
 
-// A[M,K] f32 -> planes [ceil(M/42)][3][42] (+ 2 unused rows) [K] int8 in the k order of the packed weight rows, and the rows'
-// scales (the sign says that a row is wide); optional RMSNorm of every row (the factor 1/rms goes into the scale).  T threads per row, a thread takes 16-byte
+// A[M,K] f32 -> planes [M][3][K] int8 in the k order of the packed weight rows, and the rows' scales (the sign says that a row is
+// wide); optional RMSNorm of every row (the factor 1/rms goes into the scale).  T threads per row, a thread takes 16-byte
 // units: it reads four groups of four k and writes whole 16-byte pieces of the planes.  The row is read once and stays in
 // registers up to 48 T elements.  Also clears the GEMM's counters and, outside a pass, its error word (head).
 //
 // Wide rows.  Rounding to a unit leaves 0.29 units (rms) in every element, which must be no more than the 2^-19 of an element
 // that two bf16 terms leave: the row's bulk has to have an rms of at least 2^17 units.  Its bulk is what lies below a quarter of
 // the largest magnitude, and is also to have a mean of 2^16, so that a few percent of large elements do not pass for bulk.  A
-// row with channels more than about 32 times the rest misses that, and is written a second time, into `wides`
-// [ceil(M/42)][2][6][21] (+ 2 rows) [K]: three more digits, of what the first three leave over in units of 2^-23, exact down to
+// row with channels more than about 32 times the rest misses that, and is written a second time, into `wides` [M][6][K]: three
+// more digits, of what the first three leave over in units of 2^-23, exact down to
 // 2^-45 of the largest magnitude.  One sum decides for nearly all other rows: a mean magnitude of 2^17.5 units.
 constexpr int kUnits = 3;
 __global__ void __launch_bounds__(256)
@@ -645,8 +823,7 @@ planes_kernel(const float *A, int64_t lda, int M, int K, const float *norm_w, fl
     const float rs = norm_w != nullptr ? inv * rsqrtf(ss * (1.0f / (float)K) + eps) : inv;
     row_scale[m] = __uint_as_float((__float_as_uint(rs) & 0x7fffffffu) | (wide ? 0x80000000u : 0u));
   }
-  uint8_t *dst = planes + ((int64_t)(m / kPlaneRows) * BM + m % kPlaneRows) * K;
-  uint8_t *wdst = wides + ((int64_t)(m / kWideRows) * BM + m % kWideRows) * K;   // (42 = 2 x 21)
+  uint8_t *dst = planes + (int64_t)m * kPlanes * K, *wdst = wides + (int64_t)m * kWidePlanes * K;
   for (int u0 = 0; u0 < units; u0 += step) {
     if (units > step) {
       load(u0);
@@ -663,7 +840,7 @@ planes_kernel(const float *A, int64_t lda, int M, int K, const float *norm_w, fl
                       fixed_digits(v[i][j].w, scale), w[j]);
 #pragma unroll
         for (int pl = 0; pl < kPlanes; ++pl)   // (the digit of 2^24 is zero)
-          *reinterpret_cast<uint4 *>(dst + (int64_t)pl * kPlaneRows * K + u * 16) =
+          *reinterpret_cast<uint4 *>(dst + (int64_t)pl * K + u * 16) =
               make_uint4(w[0][pl + 1], w[1][pl + 1], w[2][pl + 1], w[3][pl + 1]);
       }
     }
@@ -686,9 +863,9 @@ planes_kernel(const float *A, int64_t lda, int M, int K, const float *norm_w, fl
     }
 #pragma unroll
     for (int pl = 0; pl < kPlanes; ++pl) {
-      uint4 *at = reinterpret_cast<uint4 *>(wdst + (int64_t)pl * kWideRows * K + u * 16);
+      uint4 *at = reinterpret_cast<uint4 *>(wdst + (int64_t)pl * K + u * 16);
       *at = make_uint4(w[0][pl + 1], w[1][pl + 1], w[2][pl + 1], w[3][pl + 1]);
-      *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(at) + (int64_t)kPlanes * kWideRows * K) =
+      *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(at) + (int64_t)kPlanes * K) =
           make_uint4(l[0][pl + 1], l[1][pl + 1], l[2][pl + 1], l[3][pl + 1]);
     }
   }
@@ -703,16 +880,12 @@ constexpr int kMaxParts = 256;   // partial maxima, in the workspace head
 // max |x| of every CTA's share of the tensor (non-negative floats order like their bit patterns); clears the GEMM's counters
 // and its error word (null in a pass: the word collects what any of its GEMMs leaves).
 __global__ void __launch_bounds__(256)
-absmax_kernel(const float *A, int64_t lda, int M, int K, int vec, uint32_t *part, uint32_t *error, uint32_t *arrived,
+absmax_kernel(const float *A, int64_t lda, int M, int K, int vec, uint32_t *part, uint32_t *head, int head_words,
               int in_pass) {
   chain_start(in_pass);
   __shared__ uint32_t s_mx[8];
-  if (blockIdx.x == 0) {
-    if (threadIdx.x == 0 && error != nullptr)
-      *error = 0u;
-    for (int i = threadIdx.x; i < kMaxPartialTiles; i += 256)
-      arrived[i] = 0u;
-  }
+  if (blockIdx.x == 0 && (int)threadIdx.x < head_words)
+    head[threadIdx.x] = 0u;
   float fm = 0.f;
   const int k4 = K >> 2;
   const int64_t total = (int64_t)M * k4, stride = (int64_t)gridDim.x * 256;
@@ -811,37 +984,85 @@ int make_map(CUtensorMap *map, CUtensorMapDataType dt, int bk, void *base, uint6
   return B200_OK;
 }
 
-template <int BN, bool PLANES, bool SLIM = false>
-int launch_gemm(const void *a, int a_rows, const void *x, const void *w, GemmParams &p, int m_tiles, cudaStream_t st) {
+// How a GEMM is laid over the chip's 74 pairs of SMs.
+struct Plan {
+  int nc, rows, m_tiles, tiles, splits, share_rows, stages, grid, cols, smem;
+};
+constexpr int kMostShared = 198 * 1024;
+
+// Costs in clocks.  A k block costs a pair its products (8192 of 128 x 128 x nc a clock and SM) or its bytes (64 a clock and SM),
+// whichever takes longer; a tile's epilogue runs under the next tile's products, except the last.  Sums across a cluster cost 1.5 us
+// and their rows, and clusters of four and eight CTAs leave SMs over (72 of eight took two turns): whole / in two / in four,
+//   24 x 2048 x 1536      9.2   10.2    9.9 us        24 x 1536 x 8960    25.3    -     13.5
+//   100 x 1536 x 8960    23.6   18.5   17.1           200 x 1536 x 8960   25.1   20.7   33.2 (two turns)
+//   366 x 1536 x 8960    26.4   25.5    -
+Plan make_plan(int M, int N, int K, int nd) {
+  const int nkb = (K + BK - 1) / BK, n_tiles = (N + 2 * BM - 1) / (2 * BM), most = nd == 1 ? 256 : 84, least_tiles = (M + most - 1) / most;
+  Plan best{};
+  float least = 0.f;
+  for (int mt = least_tiles; mt < least_tiles + 16 && mt <= M; ++mt) {
+    const int rows = (M + mt - 1) / mt, need = nd == 1 ? rows : kWidePlanes * ((rows + 1) / 2), nc = (need + 31) / 32 * 32;
+    const int m_tiles = (M + rows - 1) / rows, tiles = n_tiles * m_tiles;
+    const float per_kb = (float)std::max(2 * nc, 2 * BM + nc);
+    for (int splits = 1; splits <= kMaxSplits && splits <= std::max(nkb / 2, 1); splits *= 2) {
+      if (splits > 1 && tiles * splits > kPairs * 7 / 8)
+        break;
+      const float rounds = (float)((tiles + kPairs - 1) / kPairs);
+      const float cost = rounds * (float)((nkb + splits - 1) / splits) * per_kb + 1000.f + 40.f * rows + (splits > 1 ? 3000.f + 60.f * rows : 0.f);
+      if (best.nc == 0 || cost < least) {
+        least = cost;
+        best.nc = nc;
+        best.rows = rows;
+        best.m_tiles = m_tiles;
+        best.tiles = tiles;
+        best.splits = splits;
+      }
+    }
+  }
+  best.share_rows = (best.rows + best.splits - 1) / best.splits;
+  const int clusters = best.splits > 1 ? best.tiles : std::min(best.tiles, kPairs), stage = (int)kWBytes + best.nc / 2 * BK;
+  best.grid = clusters * 2 * best.splits;
+  const int blocks = (best.tiles + clusters - 1) / clusters * ((nkb + best.splits - 1) / best.splits);
+  const int extra = 1024 + (int)sizeof(Bars) + (best.splits > 1 ? best.splits * best.share_rows * BM * 4 : 0);
+  best.stages = std::min({kMaxStages, blocks, (kMostShared - extra) / stage});
+  best.smem = extra + best.stages * stage;
+  best.cols = 32;
+  while (best.cols < 2 * best.nc)
+    best.cols *= 2;
+  return best;
+}
+
+template <bool PLANES, bool SPLIT>
+int launch_gemm(const Plan &pl, const void *a, const void *x, const void *w, GemmParams &p, cudaStream_t st) {
   CUtensorMap map_a, map_w, map_x;
-  if (int rc = make_map(&map_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, BK, const_cast<void *>(a), p.K, a_rows, (uint64_t)p.K,
-                        CU_TENSOR_MAP_SWIZZLE_128B))
+  const int box = pl.nc / 2;
+  if (int rc = make_map(&map_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, BK, const_cast<void *>(a), p.K, (uint64_t)p.M * (PLANES ? kPlanes : 1),
+                        (uint64_t)p.K, CU_TENSOR_MAP_SWIZZLE_128B, box))
     return rc;
   if (int rc = make_map(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, BK, const_cast<void *>(w), p.K, p.N, (uint64_t)p.K,
-                        CU_TENSOR_MAP_SWIZZLE_128B, BN))
+                        CU_TENSOR_MAP_SWIZZLE_128B, BM))
     return rc;
   map_x = map_a;
   if (PLANES)
-    if (int rc = make_map(&map_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, BK, const_cast<void *>(x), p.K, 2 * (uint64_t)a_rows,
-                          (uint64_t)p.K, CU_TENSOR_MAP_SWIZZLE_128B))
+    if (int rc = make_map(&map_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, BK, const_cast<void *>(x), p.K, (uint64_t)p.M * kWidePlanes,
+                          (uint64_t)p.K, CU_TENSOR_MAP_SWIZZLE_128B, box))
       return rc;
+  p.nc = pl.nc;
+  p.rows = pl.rows;
+  p.m_tiles = pl.m_tiles;
+  p.tiles = pl.tiles;
+  p.splits = pl.splits;
+  p.share_rows = pl.share_rows;
+  p.stages = pl.stages;
+  p.cols = pl.cols;
   static RaisedOn raised;
-  if (int rc = raise_shared_limit(raised, (const void *)gemm_i8_kernel<BN, PLANES, SLIM>, Ring<BN>::SMEM))
+  if (int rc = raise_shared_limit(raised, (const void *)gemm_i8_kernel<PLANES, SPLIT>, kMostShared))
     return rc;
-  return launch_after(gemm_i8_kernel<BN, PLANES, SLIM>, dim3((p.N + BN - 1) / BN, m_tiles, p.splits), kThreads, Ring<BN>::SMEM, st,
-                      map_a, map_w, p, map_x);
+  return launch_after_clusters(2 * pl.splits, gemm_i8_kernel<PLANES, SPLIT>, dim3(pl.grid), kThreads, pl.smem, st, map_a, map_w, p, map_x);
 }
-
-// CTAs along K for `tiles` output tiles of `nkb` k blocks: up to two CTAs per SM, within the workspace, at least 8 k
-// blocks each: a share's trip through L2 costs what 8 to 12 blocks cost.  24 x 2048 x 1536 (12 blocks): 10.1 us whole, 11.1 in
-// 6 shares; 24 x 1536 x 8960 (70 blocks): 27 us whole, 14.4 in 8, 17.2 in 24; 366 x 1536 x 8960 (108 tiles): 34.8 whole, 28.2 in 2.
-// A row of a tile's sums costs as much on that trip as 0.4 blocks, so tiles with many rows split only long k ranges (W8A8,
-// 1024 x 1536 x 8960: 49.8 us whole, 55.3 in 3; 200 x 4096 x 4096: 21.4 whole, 29 in 4; 64 x 1536 x 8960: 32.2 whole, 19.7 in 8).
-int split_k(int tiles, int nkb, int rows) {
-  if (tiles >= kSms)
-    return 1;
-  const int s = std::max(1, std::min({kResident / tiles, nkb / 8, kMaxPartialTiles / tiles}));
-  return (nkb - nkb / s) * 5 > rows * 2 ? s : 1;
+template <bool PLANES> int launch_plan(const void *a, const void *x, const void *w, GemmParams &p, cudaStream_t st) {
+  const Plan pl = make_plan(p.M, p.N, p.K, PLANES ? kPlanes : 1);
+  return pl.splits > 1 ? launch_gemm<PLANES, true>(pl, a, x, w, p, st) : launch_gemm<PLANES, false>(pl, a, x, w, p, st);
 }
 
 } // namespace
@@ -855,9 +1076,8 @@ extern "C" {
 int64_t b200_gemm_w8_workspace_bytes(int M, int64_t K) {
   if (M < 1 || K < 1)
     return 0;
-  const int64_t tiles = (M + kPlaneRows - 1) / kPlaneRows, Kp = packed_k(B200_W_I8, K);
-  // head, row scales, planes, the wide rows' planes, the shares of split tiles
-  return kHeadBytes + tiles * kPlaneRows * 4 + 255 + 3 * tiles * BM * Kp + (int64_t)kMaxPartialTiles * kPlaneRows * 128 * 4;
+  // head, row scales, planes, the wide rows' planes
+  return kHeadBytes + (int64_t)M * 4 + 511 + (int64_t)(kPlanes + kWidePlanes) * M * packed_k(B200_W_I8, K);
 }
 
 int b200_gemm_w8(const b200_weight *w, const float *A, int M, int64_t lda, float *C, int64_t ldc,
@@ -887,11 +1107,11 @@ int gemm_w8_run(const b200_weight *w, const float *A, int M, int64_t lda, float 
     return fail(B200_EINVAL, "gemm_w8: workspace too small");
   if (int rc = ensure_device())
     return rc;
-  const int K = (int)w->K, N = (int)w->N, m_tiles = (M + kPlaneRows - 1) / kPlaneRows;
+  const int K = (int)w->K, N = (int)w->N;
   char *ws = (char *)workspace;
   float *row_scale = reinterpret_cast<float *>(ws + kHeadBytes);
-  uint8_t *planes = reinterpret_cast<uint8_t *>(ws + (kHeadBytes + (int64_t)m_tiles * kPlaneRows * 4 + 255) / 256 * 256);
-  uint8_t *wides = planes + (int64_t)m_tiles * BM * K;
+  uint8_t *planes = reinterpret_cast<uint8_t *>(ws + (kHeadBytes + (int64_t)M * 4 + 255) / 256 * 256);
+  uint8_t *wides = planes + (int64_t)M * kPlanes * K;
   GemmParams p{};
   p.M = M;
   p.N = N;
@@ -904,27 +1124,17 @@ int gemm_w8_run(const b200_weight *w, const float *A, int M, int64_t lda, float 
   p.ldc = ldc;
   p.ldr = ldr;
   p.silu_pairs = silu_pairs;
-  p.partial = wides + (int64_t)m_tiles * 2 * BM * K;
   p.error = reinterpret_cast<int *>(ws);
-  p.arrived = reinterpret_cast<uint32_t *>(ws) + 16;
   // threads per row: as few as keep it in registers, more when there are few rows
   int T = 32;
   while (T < 256 && (K > T * 16 * kUnits || (int64_t)M * T < kSms * 256))
     T *= 2;
   const int vec = (lda & 3) == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)norm_weight & 15) == 0;
   if (int rc = launch_after(planes_kernel, dim3((M + 256 / T - 1) / (256 / T)), 256, 0, st, A, lda, M, K, norm_weight, norm_eps, T,
-                            vec, planes, row_scale, in_pass ? p.arrived : reinterpret_cast<uint32_t *>(ws),
-                            in_pass ? kMaxPartialTiles : 16 + kMaxPartialTiles, in_pass ? 1 : 0, wides))
+                            vec, planes, row_scale, reinterpret_cast<uint32_t *>(ws),
+                            in_pass ? 0 : kHeadWords, in_pass ? 1 : 0, wides))
     return rc;
-  // 256 columns per CTA (fewer bytes per operation) when that still gives every SM its two CTAs
-  if ((int64_t)((N + 255) / 256) * m_tiles >= kResident) {
-    p.splits = 1;
-    return launch_gemm<256, true>(planes, m_tiles * BM, wides, w->w, p, m_tiles, st);
-  }
-  p.splits = split_k((N + 127) / 128 * m_tiles, (K + BK - 1) / BK, std::min(M, kPlaneRows));
-  if (M <= 20)
-    return launch_gemm<128, true, true>(planes, m_tiles * BM, wides, w->w, p, m_tiles, st);
-  return launch_gemm<128, true>(planes, m_tiles * BM, wides, w->w, p, m_tiles, st);
+  return launch_plan<true>(planes, wides, w->w, p, st);
 }
 } // namespace b200
 
@@ -934,7 +1144,7 @@ extern "C" {
 int64_t b200_gemm_w8a8_workspace_bytes(int M, int64_t K) {
   if (M < 1 || K < 1)
     return 0;
-  return kHeadBytes + kMaxParts * 4 + ((int64_t)M * K + 255) / 256 * 256 + (int64_t)kMaxPartialTiles * BM * 128 * 4;
+  return kHeadBytes + kMaxParts * 4 + ((int64_t)M * K + 255) / 256 * 256;
 }
 
 int b200_gemm_w8a8(const b200_weight *w, const float *A, int M, int64_t lda, float *C, int64_t ldc,
@@ -967,7 +1177,7 @@ int gemm_w8a8_fused(const b200_weight *w, const float *A, int M, int64_t lda, fl
     return fail(B200_EINVAL, "gemm_w8a8: workspace too small");
   if (int rc = ensure_device())
     return rc;
-  const int K = (int)w->K, N = (int)w->N, m_tiles = (M + BM - 1) / BM;
+  const int K = (int)w->K, N = (int)w->N;
   char *ws = (char *)workspace;
   float *act_scale = reinterpret_cast<float *>(ws) + 2;
   uint32_t *part = reinterpret_cast<uint32_t *>(ws + kHeadBytes);
@@ -984,22 +1194,17 @@ int gemm_w8a8_fused(const b200_weight *w, const float *A, int M, int64_t lda, fl
   p.residual = residual;
   p.ldr = ldr;
   p.silu_pairs = silu_pairs;
-  p.partial = q + ((int64_t)M * K + 255) / 256 * 256;
   p.error = reinterpret_cast<int *>(ws);
-  p.arrived = reinterpret_cast<uint32_t *>(ws) + 16;
   const int vec = (lda & 3) == 0 && ((uintptr_t)A & 15) == 0;
   const int parts = (int)std::min<int64_t>(((int64_t)M * K / 4 + 1023) / 1024, kMaxParts);
   if (int rc = launch_after(absmax_kernel, dim3(parts), 256, 0, st, A, lda, M, K, vec, part,
-                            in_pass ? nullptr : reinterpret_cast<uint32_t *>(ws), p.arrived, in_pass ? 1 : 0))
+                            in_pass ? nullptr : reinterpret_cast<uint32_t *>(ws), in_pass ? 0 : kHeadWords, in_pass ? 1 : 0))
     return rc;
   const int64_t units = (int64_t)M * (K / 16);
   if (int rc = launch_after(quantize_kernel, dim3((unsigned)((units + 255) / 256)), 256, 0, st, A, lda, M, K, vec,
                             (const uint32_t *)part, parts, act_scale, q))
     return rc;
-  // 128 columns for all: with 256, where that leaves two CTAs for every SM, 2048 x 20000 x 8960 takes 423 us instead of 482 and
-  // 2048 x 17920 x 1536 105 instead of 112, but 1024 x 18992 x 1536 73 instead of 69 and 600 x 17920 x 1536 51 instead of 47
-  p.splits = split_k((N + 127) / 128 * m_tiles, (K + BK - 1) / BK, std::min(M, BM));
-  return launch_gemm<128, false>(q, M, q, w->w, p, m_tiles, st);
+  return launch_plan<false>(q, q, w->w, p, st);
 }
 } // namespace b200
 
