@@ -167,6 +167,14 @@ int gqa_paged_launch(const float *qkv, int64_t ld, const float *k_pool, const fl
                      int q_heads, int kv_heads, int D, int page, const int32_t *row_seq, const int32_t *row_pos,
                      const int32_t *block_table, int table_stride, int M, float *scratch, int scratch_rows,
                      int max_context, cudaStream_t st);
+// paged_decode.cu: rope_kv_paged and gqa_paged in one, for rows that are each the newest position of a sequence of their own;
+// longest: the most positions of a row.  q and k in qkv stay as they are.
+bool paged_decode_takes(const float *qkv, int64_t ld, const float *k_pool, const float *v_pool, int q_heads, int kv_heads, int D, int M,
+                        int longest);
+int paged_decode_launch(const float *qkv, int64_t ld, float *k_pool, float *v_pool, float *out, int64_t ldo, const float *inv_freq,
+                        const float *q_norm, const float *k_norm, float eps, int q_heads, int kv_heads, int D, int page,
+                        const int32_t *row_seq, const int32_t *row_pos, const int32_t *block_table, int table_stride, int M, int longest,
+                        cudaStream_t st);
 int64_t gqa_paged_scratch_floats(int rows, int q_heads, int D, int max_context);
 // prefill_attn.cu: causal attention of M rows at positions pos0, pos0 + 1, .. of one sequence on the tensor cores.  kc / vc:
 // the contiguous cache [kv_heads][max_len][D] (table null), or page pools [pages][kv_heads][page][D] and the sequence's row

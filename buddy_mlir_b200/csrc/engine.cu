@@ -1961,8 +1961,10 @@ struct b200_batch {
   float last_ms = 0.f;
 };
 
-static int batch_rows(b200_batch *b, int M, const int32_t *tokens, const int32_t *row_seq, const int32_t *row_pos,
-                      bool all_logits, float *logits_host, int32_t *next_host) {
+// step: a decode step, every row a sequence of its own, with logits of all rows; otherwise a chunk of one sequence's prompt, with
+// those of its last row.
+static int batch_rows(b200_batch *b, int M, const int32_t *tokens, const int32_t *row_seq, const int32_t *row_pos, bool step,
+                      float *logits_host, int32_t *next_host) {
   b200_model *m = b->m;
   // A w8a8 projection scales its whole activation tensor: rows of unrelated sequences in one
   // batch would share that scale, and each sequence's result would depend on its neighbours.
@@ -1971,7 +1973,7 @@ static int batch_rows(b200_batch *b, int M, const int32_t *tokens, const int32_t
   const b200_model_config &c = m->cfg;
   const int D = c.head_dim, H = c.hidden;
   const int64_t QD = (int64_t)m->qh * D, KD = (int64_t)m->kvh * D, QKV = QD + 2 * KD;
-  const int logit_rows = all_logits ? M : 1;
+  const int logit_rows = step ? M : 1;
   if (int rc = prefill_reserve(m, M, logit_rows)) return rc;
   cudaStream_t st = m->stream;
   if (M > b->rows_cap) {
@@ -1989,6 +1991,8 @@ static int batch_rows(b200_batch *b, int M, const int32_t *tokens, const int32_t
     one_chunk = row_seq[r] == row_seq[0] && row_pos[r] == row_pos[0] + r;
   if (one_chunk)
     if (int rc = prefill_attention_reserve(m, row_pos[0] + M, b->max_context)) return rc;
+  const int longest = 1 + *std::max_element(row_pos, row_pos + M);
+  const bool one_kernel = step && paged_decode_takes(m->pf_qkv, QKV, b->pool[0], b->pool[1], m->qh, m->kvh, D, M, longest);
   B200_CUDA(cudaEventRecord(m->ev0, st));
   B200_CUDA(cudaMemcpyAsync(m->pf_tokens, tokens, (size_t)M * 4, cudaMemcpyHostToDevice, st));
   B200_CUDA(cudaMemcpyAsync(b->d_seq, row_seq, (size_t)M * 4, cudaMemcpyHostToDevice, st));
@@ -1998,22 +2002,28 @@ static int batch_rows(b200_batch *b, int M, const int32_t *tokens, const int32_t
   for (int l = 0; l < c.n_layers; ++l) {
     Layer &L = m->layers[l];
     if (int rc = linear_rows(m, L.qkv, m->pf_x, H, M, m->pf_qkv, QKV, nullptr, L.in_norm, false)) return rc;
-    if (int rc = rope_kv_paged_launch(m->pf_qkv, QKV, b->pool[2 * l], b->pool[2 * l + 1], m->inv_freq, L.q_norm,
-                                      L.k_norm, c.eps, m->qh, m->kvh, D, b->page, b->d_seq, b->d_pos, b->d_table,
-                                      b->table_stride, M, st))
-      return rc;
-    if (int rc = one_chunk
-                     ? prefill_attention(m, b->pool[2 * l], b->pool[2 * l + 1], b->max_context, row_pos[0], M,
-                                         b->d_table + (size_t)row_seq[0] * b->table_stride, b->page)
-                     : gqa_paged_launch(m->pf_qkv, QKV, b->pool[2 * l], b->pool[2 * l + 1], m->pf_att, QD, m->qh, m->kvh, D,
-                                        b->page, b->d_seq, b->d_pos, b->d_table, b->table_stride, M, b->d_part, b->part_rows,
-                                        b->max_context, st))
-      return rc;
+    if (one_kernel) {
+      if (int rc = paged_decode_launch(m->pf_qkv, QKV, b->pool[2 * l], b->pool[2 * l + 1], m->pf_att, QD, m->inv_freq, L.q_norm, L.k_norm,
+                                       c.eps, m->qh, m->kvh, D, b->page, b->d_seq, b->d_pos, b->d_table, b->table_stride, M, longest, st))
+        return rc;
+    } else {
+      if (int rc = rope_kv_paged_launch(m->pf_qkv, QKV, b->pool[2 * l], b->pool[2 * l + 1], m->inv_freq, L.q_norm,
+                                        L.k_norm, c.eps, m->qh, m->kvh, D, b->page, b->d_seq, b->d_pos, b->d_table,
+                                        b->table_stride, M, st))
+        return rc;
+      if (int rc = one_chunk
+                       ? prefill_attention(m, b->pool[2 * l], b->pool[2 * l + 1], b->max_context, row_pos[0], M,
+                                           b->d_table + (size_t)row_seq[0] * b->table_stride, b->page)
+                       : gqa_paged_launch(m->pf_qkv, QKV, b->pool[2 * l], b->pool[2 * l + 1], m->pf_att, QD, m->qh, m->kvh, D,
+                                          b->page, b->d_seq, b->d_pos, b->d_table, b->table_stride, M, b->d_part, b->part_rows,
+                                          b->max_context, st))
+        return rc;
+    }
     if (int rc = linear_rows(m, L.o, m->pf_att, QD, M, m->pf_x, H, m->pf_x, nullptr, false)) return rc;
     if (int rc = linear_rows(m, L.gateup, m->pf_x, H, M, m->pf_mid, m->ffn, nullptr, L.post_norm, true)) return rc;
     if (int rc = linear_rows(m, L.down, m->pf_mid, m->ffn, M, m->pf_x, H, m->pf_x, nullptr, false)) return rc;
   }
-  const int first = all_logits ? 0 : M - 1;
+  const int first = step ? 0 : M - 1;
   if (int rc = linear_rows(m, m->lm_head, m->pf_x + (int64_t)first * H, H, logit_rows, m->pf_logits, c.vocab, nullptr,
                            m->final_norm, false))
     return rc;

@@ -992,7 +992,8 @@ constexpr int kMostShared = 198 * 1024;
 
 // Costs in clocks.  A k block costs a pair its products (8192 of 128 x 128 x nc a clock and SM) or its bytes (64 a clock and SM),
 // whichever takes longer; a tile's epilogue runs under the next tile's products, except the last.  Sums across a cluster cost 1.5 us
-// and their rows, and clusters of four and eight CTAs leave SMs over (72 of eight took two turns): whole / in two / in four,
+// and their rows, every SM that is taken counts (the next kernel of a pass could start there: a decode step's attention after
+// q|k|v of 24 rows took 17 us behind 128 CTAs, 14 behind 16), and clusters of four and eight CTAs leave SMs over (72 of eight took two turns): whole / in two / in four,
 //   24 x 2048 x 1536      9.2   10.2    9.9 us        24 x 1536 x 8960    25.3    -     13.5
 //   100 x 1536 x 8960    23.6   18.5   17.1           200 x 1536 x 8960   25.1   20.7   33.2 (two turns)
 //   366 x 1536 x 8960    26.4   25.5    -
@@ -1008,7 +1009,8 @@ Plan make_plan(int M, int N, int K, int nd) {
       if (splits > 1 && tiles * splits > kPairs * 7 / 8)
         break;
       const float rounds = (float)((tiles + kPairs - 1) / kPairs);
-      const float cost = rounds * (float)((nkb + splits - 1) / splits) * per_kb + 1000.f + 40.f * rows + (splits > 1 ? 3000.f + 60.f * rows : 0.f);
+      const float cost = rounds * (float)((nkb + splits - 1) / splits) * per_kb + 1000.f + 40.f * rows + (splits > 1 ? 3000.f + 60.f * rows : 0.f) +
+                         20.f * (float)std::min(tiles * splits, kPairs);
       if (best.nc == 0 || cost < least) {
         least = cost;
         best.nc = nc;
