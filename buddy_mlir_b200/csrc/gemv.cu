@@ -583,12 +583,8 @@ int b200::gemv_run(const b200_weight *w, const b200_gemv_args *a, const TpPush *
     return fail(B200_EINVAL, "gemv: silu_pairs excludes accumulate/residual");
   if (int rc = ensure_device())
     return rc;
-  // int8 and int4 weights go to the integer tensor cores.  What stays here: one row over less than 6 MB of weights, f32
-  // weights, other group sizes and scale types, and the tensor-parallel push.  Device time per call in a graph, weights from
-  // memory, us there / here: int8 K = 512: 4.0 / 3.1 at 1 MB, 5.1 / 5.1 at 6; K = 1536: 4.4 / 4.6 at 1, 5.3 / 5.4 at 6,
-  // 6.3 / 5.8 at 8; K = 4096: 5.4 / 8.4 at 1, 6.0 / 8.7 at 6; K = 8960: 7.9 / 15.4 at 1; int4 K = 512: 7.3 / 5.0 at 1, 8.4 / 14
-  // at 6; K = 4096: 5.3 / 6.1 at 1, 7.0 / 7.5 at 6.  So the line is right for rows up to 1536; long rows below it would be
-  // faster there at every size.
+  // int8 and int4 weights go to the integer tensor cores.  What stays here: one short row over few weights (one_row_is_short has
+  // the times of both), f32 weights, other group sizes and scale types, and the tensor-parallel push.
   if (push == nullptr && gemv_mma_takes(w, a))
     return gemv_mma_run(w, a, stream);
 

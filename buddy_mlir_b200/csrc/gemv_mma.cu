@@ -615,16 +615,23 @@ template <int KIND, int COLS, bool GROUPED, bool XF> static int launch_mma(MmaP 
   return B200_OK;
 }
 
+// One row: short rows over few weights are faster on the CUDA cores (a chain of launch, load, product; no digits to make).  Device
+// time per call in a graph, weights from memory, us here / there: int8 K = 512: 4.0 / 3.1 at 1 MB, 4.8 / 4.9 at 5, 6.2 / 7.1 at 10;
+// K = 1536: 4.4 / 4.6 at 1, 5.3 / 5.4 at 6, 6.4 / 6.0 at 10 (weights in L2: 4.2 / 3.6 at 2); K = 2560: 5.5 / 6.1 at 1; K = 4096:
+// 5.4 / 8.4 at 1, 6.0 / 8.7 at 6; K = 8960: 7.9 / 15.4 at 1; K = 14336: 13.0 / 21.5 at 1.  int4 K = 512: 7.3 / 5.0 at 1 MB, 6.9 / 7.0
+// at 2, 8.4 / 14 at 6; K = 1536: 7.5 / 6.9 at 1, 7.2 / 8.1 at 3; K = 2560: 6.6 / 8.7 at 0.5; K = 8960: 9.6 / 23 at 1.  (f32 rows of up to four whole blocks have a
+// quicker form there: K = 4096 5.3 / 6.1 at 0.5 MB from memory, 5.2 / 4.8 at 1.2 MB from L2.)
+static bool one_row_is_short(const b200_weight *w, const b200_gemv_args *a) {
+  const bool few_blocks = w->kind == B200_W_U4 && w->K <= 4096 && w->K % 1024 == 0 && a->x_dtype == B200_F32;
+  return (w->K < 2560 || few_blocks) && packed_row_bytes(w->kind, w->K) * w->N < (w->kind == B200_W_I8 ? 6 << 20 : 3 << 20);
+}
+
 // Whether the integer-MMA kernel takes this call: per-channel int8 or int4 (any scale type), or int4 in groups of 128
 // with f16 scales (the group is then one 4-element column of a packed block), up to K = 65536 (s32 sums).
 bool gemv_mma_takes(const b200_weight *w, const b200_gemv_args *a) {
-  if (w->K > 65536 || (a->M == 1 && packed_row_bytes(w->kind, w->K) * w->N < (6 << 20)))
+  if (w->K > 65536 || (w->kind != B200_W_I8 && w->kind != B200_W_U4) || (a->M == 1 && one_row_is_short(w, a)))
     return false;
-  if (w->kind == B200_W_I8)
-    return true;
-  if (w->kind != B200_W_U4)
-    return false;
-  const bool grouped = w->group > 0 && w->group < w->K;
+  const bool grouped = w->kind == B200_W_U4 && w->group > 0 && w->group < w->K;
   return !grouped || (w->group == 128 && w->scale_dtype == B200_F16 && w->K % 128 == 0);
 }
 

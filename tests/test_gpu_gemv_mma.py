@@ -159,3 +159,31 @@ def test_wide_rows_per_channel_and_odd_lengths(kind, M, N, K, dtype):
     y = y.cpu().numpy()
     for m in range(M):   # (every row on its own: only one has the large element)
         assert np.abs(y[m] - want[m]).max() / np.abs(want[m]).max() < 1e-5
+
+
+@pytest.mark.parametrize("kind,N,K", [("i8", 1, 2560), ("i8", 3, 2561), ("i8", 70, 2559), ("i8", 129, 3056), ("i8", 17, 8960), ("i8", 9, 14336),
+                                      ("i8", 5, 40000), ("i8", 4200, 1501), ("u4", 2, 2560), ("u4", 34, 4096), ("u4", 66, 2688), ("u4", 18, 9088),
+                                      ("u4", 4, 14336), ("u4", 5000, 1280)])
+@pytest.mark.parametrize("dtype", ["f32", "f16", "bf16"])
+def test_one_row_on_both_sides_of_the_line(kind, N, K, dtype):
+    """One row over few weights, at the lengths where the kernel changes: bias, residual and accumulation against f64."""
+    import torch
+    from gpu_util import dev, gemv, packed_scales, packed_weight
+    rng = np.random.default_rng(N + K)
+    xt = torch.from_numpy(rng.standard_normal((1, K)).astype(np.float32)).to({"f32": torch.float32, "f16": torch.float16, "bf16": torch.bfloat16}[dtype]).cuda()
+    code = {"f32": _lib.F32, "f16": _lib.F16, "bf16": _lib.BF16}[dtype]
+    bias, res = rng.standard_normal(N).astype(np.float32), rng.standard_normal((1, N)).astype(np.float32)
+    if kind == "i8":
+        Q = rng.integers(-128, 128, (K, N)).astype(np.int8)
+        s = rng.uniform(0.001, 0.01, N).astype(np.float32)
+        y = gemv(_lib.W_I8, packed_weight(_lib.W_I8, Q, K, N), dev(s), K, N, xt, bias=dev(bias), residual=dev(res), x_dtype=code)
+        w = Q.astype(np.float64) * s
+    else:
+        P = rng.integers(0, 256, (K, N // 2)).astype(np.uint8)
+        s = rng.uniform(0.001, 0.01, (K // 128, N)).astype(np.float16)
+        y = gemv(_lib.W_U4, packed_weight(_lib.W_U4, P, K, N, 0), packed_scales(s, _lib.F16, K // 128, N), K, N, xt, group=128,
+                 scale_dtype=_lib.F16, bias=dev(bias), residual=dev(res), x_dtype=code)
+        w = (np.stack([P & 15, P >> 4], axis=2).reshape(K, N).astype(np.float64) - 8) * np.repeat(s.astype(np.float64), 128, axis=0)
+    want = xt.double().cpu().numpy() @ w + bias + res
+    # f32 sums of K products: sqrt(K) * 2^-24 of the largest at most, here 40000: 1.2e-5
+    assert np.abs(y.cpu().numpy() - want).max() / max(np.abs(want).max(), 1.0) < 1.2e-5
