@@ -25,59 +25,115 @@ __global__ void embed_rows_kernel(const float *table, const int32_t *tokens, flo
 }
 
 // RoPE (and QK-norm) on the q and k heads of every row, K/V rows written to the
-// cache: subgraph0_decode_simplify.mlir:52-59, 86-142 with pos = pos0 + row.
-// grid (M, q_heads + kv_heads), one thread per (j, j + D/2) pair.
-__global__ void rope_kv_rows_kernel(float *qkv, int64_t ld, float *k_cache, float *v_cache,
-                                    const float *inv_freq, const float *q_norm, const float *k_norm,
-                                    float eps, int q_heads, int kv_heads, int D, int max_len, int pos0) {
-  __shared__ float red[8];
-  kernel_go();
-  const int half = D / 2;
-  const int j = threadIdx.x;
-  const int m = blockIdx.x, head = blockIdx.y;
-  const bool is_q = head < q_heads;
-  const int h = is_q ? head : head - q_heads;
-  float *row = qkv + (int64_t)m * ld;
-  float *p = row + (is_q ? 0 : q_heads * D) + (int64_t)h * D;
-  const float *v = row + (q_heads + kv_heads) * D + (int64_t)h * D;
-  const float *nw = is_q ? q_norm : k_norm;
-  const int pos = pos0 + m;
-  // what the kernel before does not write: the angle
-  const float th = j < half ? __fmul_rn(inv_freq[j], (float)pos) : 0.f;
-  const float c = cosf(th), s = sinf(th);
-  kernel_wait();
-  float a = 0.f, b = 0.f;
-  if (j < half) {
-    a = p[j];
-    b = p[j + half];
-  }
-  if (nw != nullptr) {
-    float ssq = warp_sum(__fadd_rn(__fmul_rn(a, a), __fmul_rn(b, b)));
-    if ((threadIdx.x & 31) == 0)
-      red[threadIdx.x >> 5] = ssq;
-    __syncthreads();
-    float t = 0.f;
-    for (int i = 0; i < (int)((blockDim.x + 31) >> 5); ++i)
-      t += red[i];
-    const float r = rsqrtf(__fadd_rn(__fmul_rn(t, 1.0f / (float)D), eps));
-    if (j < half) {
-      a = __fmul_rn(nw[j], __fmul_rn(a, r));
-      b = __fmul_rn(nw[j + half], __fmul_rn(b, r));
+// cache: subgraph0_decode_simplify.mlir:52-59, 86-142.  One CTA per row: the angles' cosines and
+// sines are made once, a warp takes a head at a time (1000 rows, 14 heads of 128, a layer: 13 us
+// for a CTA and the angles per row and head, 5 here).  Where the row's K and V go: row pos0 + m of the
+// contiguous cache [kv_heads][max_len][D], or (PAGED) the page of the position, in a pool
+// [n_pages][kv_heads][page][D].
+constexpr int kRopeThreads = 512;
+struct RopeRows {
+  float *qkv;
+  int64_t ld;
+  float *k_cache, *v_cache;   // or pools
+  const float *inv_freq, *q_norm, *k_norm;
+  float eps;
+  int q_heads, kv_heads, D;
+  int max_len, pos0;
+  int page;                   // PAGED
+  const int32_t *row_seq, *row_pos, *block_table;
+  int table_stride;
+};
+// V: neighbouring elements of a lane
+template <int V> struct RopeVec {
+  float v[V];
+  __device__ __forceinline__ void load(const float *p) {
+    if constexpr (V == 2) {
+      const float2 a = *reinterpret_cast<const float2 *>(p);
+      v[0] = a.x;
+      v[1] = a.y;
+    } else {
+      v[0] = *p;
     }
   }
-  if (j >= half)
-    return;
-  const float oa = __fadd_rn(__fmul_rn(a, c), __fmul_rn(-b, s));
-  const float ob = __fadd_rn(__fmul_rn(b, c), __fmul_rn(a, s));
-  p[j] = oa;
-  p[j + half] = ob;
-  if (!is_q) {
-    const int64_t crow = ((int64_t)h * max_len + pos) * D;
-    k_cache[crow + j] = oa;
-    k_cache[crow + j + half] = ob;
-    v_cache[crow + j] = v[j];
-    v_cache[crow + j + half] = v[j + half];
+  __device__ __forceinline__ void store(float *p) const {
+    if constexpr (V == 2)
+      *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
+    else
+      *p = v[0];
   }
+};
+template <bool PAGED, int V> __global__ void __launch_bounds__(kRopeThreads) rope_rows_kernel(const RopeRows p) {
+  extern __shared__ float s_angle[];   // [D / 2] cosines, then sines
+  kernel_go();
+  const int half = p.D / 2, D = p.D, m = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // what the kernel before does not write: the angles, the page
+  const int pos = PAGED ? p.row_pos[m] : p.pos0 + m;
+  for (int j = threadIdx.x; j < half; j += kRopeThreads) {
+    const float th = __fmul_rn(p.inv_freq[j], (float)pos);
+    s_angle[j] = cosf(th);
+    s_angle[half + j] = sinf(th);
+  }
+  // of kv head h: row0 + h * step
+  const int64_t step = PAGED ? p.page : p.max_len;
+  const int64_t row0 = PAGED ? (int64_t)p.block_table[(int64_t)p.row_seq[m] * p.table_stride + pos / p.page] * p.kv_heads * p.page + pos % p.page
+                             : pos;
+  __syncthreads();
+  kernel_wait();
+  float *row = p.qkv + (int64_t)m * p.ld;
+  for (int head = warp; head < p.q_heads + 2 * p.kv_heads; head += kRopeThreads / 32) {
+    float *x = row + (int64_t)head * D;
+    const int h = head - p.q_heads;
+    RopeVec<V> a, b;
+    if (h >= p.kv_heads) {   // v
+      float *v = p.v_cache + (row0 + (h - p.kv_heads) * step) * D;
+      for (int j = lane * V; j < half; j += 32 * V) {
+        a.load(x + j);
+        b.load(x + half + j);
+        a.store(v + j);
+        b.store(v + half + j);
+      }
+      continue;
+    }
+    const float *nw = h < 0 ? p.q_norm : p.k_norm;
+    float r = 0.f;
+    if (nw != nullptr) {
+      float ss = 0.f;
+      for (int j = lane * V; j < half; j += 32 * V) {
+        a.load(x + j);
+        b.load(x + half + j);
+#pragma unroll
+        for (int e = 0; e < V; ++e)
+          ss += __fadd_rn(__fmul_rn(a.v[e], a.v[e]), __fmul_rn(b.v[e], b.v[e]));
+      }
+      r = rsqrtf(__fadd_rn(__fmul_rn(warp_sum(ss), 1.0f / (float)D), p.eps));
+    }
+    float *k = h < 0 ? nullptr : p.k_cache + (row0 + h * step) * D;
+    for (int j = lane * V; j < half; j += 32 * V) {
+      a.load(x + j);
+      b.load(x + half + j);
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        if (nw != nullptr) {
+          a.v[e] = __fmul_rn(nw[j + e], __fmul_rn(a.v[e], r));
+          b.v[e] = __fmul_rn(nw[j + half + e], __fmul_rn(b.v[e], r));
+        }
+        const float c = s_angle[j + e], s = s_angle[half + j + e], u = a.v[e], w = b.v[e];
+        a.v[e] = __fadd_rn(__fmul_rn(u, c), __fmul_rn(-w, s));
+        b.v[e] = __fadd_rn(__fmul_rn(w, c), __fmul_rn(u, s));
+      }
+      a.store(x + j);
+      b.store(x + half + j);
+      if (k != nullptr) {
+        a.store(k + j);
+        b.store(k + half + j);
+      }
+    }
+  }
+}
+template <bool PAGED> int rope_rows_launch(const RopeRows &p, int M, cudaStream_t st) {
+  const bool pairs = p.D % 128 == 0 && (p.ld & 1) == 0 && (((uintptr_t)p.qkv | (uintptr_t)p.k_cache | (uintptr_t)p.v_cache) & 7) == 0;
+  return pairs ? launch_after(rope_rows_kernel<PAGED, 2>, dim3(M), kRopeThreads, p.D * 4, st, p)
+               : launch_after(rope_rows_kernel<PAGED, 1>, dim3(M), kRopeThreads, p.D * 4, st, p);
 }
 
 // Causal attention of M query rows over the cache: grid (M, kv_heads), 4 warps.
@@ -193,60 +249,6 @@ int launch_prefill_attn(const float *qkv, int64_t ld, const float *kc, const flo
 // belongs to sequence row_seq[r] at position row_pos[r]; block_table[seq][pos / page] is
 // the page that holds the position.  (buddy-mlir has no paged cache; per sequence the
 // arithmetic is that of the contiguous cache above.)
-__global__ void rope_kv_paged_kernel(float *qkv, int64_t ld, float *k_pool, float *v_pool,
-                                     const float *inv_freq, const float *q_norm, const float *k_norm, float eps,
-                                     int q_heads, int kv_heads, int D, int page, const int32_t *row_seq,
-                                     const int32_t *row_pos, const int32_t *block_table, int table_stride) {
-  __shared__ float red[8];
-  kernel_go();
-  const int half = D / 2;
-  const int j = threadIdx.x;
-  const int m = blockIdx.x, head = blockIdx.y;
-  const bool is_q = head < q_heads;
-  const int h = is_q ? head : head - q_heads;
-  float *row = qkv + (int64_t)m * ld;
-  float *p = row + (is_q ? 0 : q_heads * D) + (int64_t)h * D;
-  const float *v = row + (q_heads + kv_heads) * D + (int64_t)h * D;
-  const float *nw = is_q ? q_norm : k_norm;
-  const int pos = row_pos[m];
-  // what the kernel before does not write: the angle, the page
-  const float th = j < half ? __fmul_rn(inv_freq[j], (float)pos) : 0.f;
-  const float c = cosf(th), s = sinf(th);
-  const int pg = block_table[(int64_t)row_seq[m] * table_stride + pos / page];
-  kernel_wait();
-  float a = 0.f, b = 0.f;
-  if (j < half) {
-    a = p[j];
-    b = p[j + half];
-  }
-  if (nw != nullptr) {
-    float ssq = warp_sum(__fadd_rn(__fmul_rn(a, a), __fmul_rn(b, b)));
-    if ((threadIdx.x & 31) == 0)
-      red[threadIdx.x >> 5] = ssq;
-    __syncthreads();
-    float t = 0.f;
-    for (int i = 0; i < (int)((blockDim.x + 31) >> 5); ++i)
-      t += red[i];
-    const float r = rsqrtf(__fadd_rn(__fmul_rn(t, 1.0f / (float)D), eps));
-    if (j < half) {
-      a = __fmul_rn(nw[j], __fmul_rn(a, r));
-      b = __fmul_rn(nw[j + half], __fmul_rn(b, r));
-    }
-  }
-  if (j >= half)
-    return;
-  const float oa = __fadd_rn(__fmul_rn(a, c), __fmul_rn(-b, s));
-  const float ob = __fadd_rn(__fmul_rn(b, c), __fmul_rn(a, s));
-  p[j] = oa;
-  p[j + half] = ob;
-  if (!is_q) {
-    const int64_t crow = (((int64_t)pg * kv_heads + h) * page + pos % page) * D;
-    k_pool[crow + j] = oa;
-    k_pool[crow + j + half] = ob;
-    v_pool[crow + j] = v[j];
-    v_pool[crow + j + half] = v[j + half];
-  }
-}
 
 template <int G, int VEC>
 __global__ void __launch_bounds__(128)
@@ -639,10 +641,8 @@ int rope_kv_paged_launch(float *qkv, int64_t ld, float *k_pool, float *v_pool, c
                          const float *q_norm, const float *k_norm, float eps, int q_heads, int kv_heads, int D,
                          int page, const int32_t *row_seq, const int32_t *row_pos, const int32_t *block_table,
                          int table_stride, int M, cudaStream_t st) {
-  dim3 grid(M, q_heads + kv_heads);
-  return launch_after(rope_kv_paged_kernel, grid, D / 2 < 32 ? 32 : D / 2, 0, st, qkv, ld, k_pool, v_pool, inv_freq, q_norm, k_norm, eps,
-                                                               q_heads, kv_heads, D, page, row_seq, row_pos,
-                                                               block_table, table_stride);
+  return rope_rows_launch<true>(RopeRows{qkv, ld, k_pool, v_pool, inv_freq, q_norm, k_norm, eps, q_heads, kv_heads, D, 0, 0, page, row_seq, row_pos,
+                               block_table, table_stride}, M, st);
 }
 
 int64_t gqa_paged_scratch_floats(int rows, int q_heads, int D, int max_context) {
@@ -701,9 +701,8 @@ int embed_rows_launch(const float *table, const int32_t *tokens_dev, float *x, i
 int rope_kv_rows_launch(float *qkv, int64_t ld, float *k_cache, float *v_cache, const float *inv_freq,
                         const float *q_norm, const float *k_norm, float eps, int q_heads, int kv_heads, int D,
                         int max_len, int pos0, int M, cudaStream_t st) {
-  dim3 grid(M, q_heads + kv_heads);
-  return launch_after(rope_kv_rows_kernel, grid, D / 2 < 32 ? 32 : D / 2, 0, st, qkv, ld, k_cache, v_cache, inv_freq, q_norm, k_norm,
-                                                              eps, q_heads, kv_heads, D, max_len, pos0);
+  return rope_rows_launch<false>(RopeRows{qkv, ld, k_cache, v_cache, inv_freq, q_norm, k_norm, eps, q_heads, kv_heads, D, max_len, pos0, 0, nullptr,
+                               nullptr, nullptr, 0}, M, st);
 }
 
 int gqa_prefill_launch(const float *qkv, int64_t ld, const float *kc, const float *vc, float *out, int64_t ldo,
