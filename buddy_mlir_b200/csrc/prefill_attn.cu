@@ -20,7 +20,7 @@
 // Bound by the tensor pipe: per key tile 48 products of 64 columns (48 clocks each, measured; half the pipe's rate, but a
 // wider tile of keys would not fit beside Q's three planes) and 24 of 128 (64 clocks), 3840 clocks at D = 128; softmax and
 // conversion run beside it.  f32 FMAs at 128 per clock would need 16384.  1000 rows, 12 heads on 2, D = 128, a layer: 219 us
-// for register-tiled FMAs, 47 here and 3.5 for the images.
+// for register-tiled FMAs, 42 here and 3.5 for the images; 366 rows 25, 64 rows 14 (with a divide per output element 45, 31 and 16).
 #include "common.cuh"
 #include "tensor_core.cuh"
 
@@ -73,6 +73,12 @@ __device__ __forceinline__ void split8(float (&v)[8], uint4 (&t)[kTerms]) {
 #pragma unroll
   for (int q = 0; q < kTerms; ++q)
     t[q] = make_uint4(take_bf16(v[0], v[1]), take_bf16(v[2], v[3]), take_bf16(v[4], v[5]), take_bf16(v[6], v[7]));
+}
+// a / b with r = 1 / b: the quotient's remainder once, as the division does it, without its branch for other ranges (b, a sum of
+// weights, is at least one; an infinite a stays infinite)
+__device__ __forceinline__ float over(float a, float b, float r) {
+  const float q = a * r, e = fmaf(-b, q, a);
+  return e == e ? fmaf(e, r, q) : q;
 }
 // byte offset of 16-byte chunk c of row r in a tile of 128-byte rows, 128-byte swizzle
 __device__ __forceinline__ uint32_t swz(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }
@@ -424,11 +430,12 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(const AttnPar
     lsum += bars.sum[half ^ 1][r];
     float *stage = reinterpret_cast<float *>(ks);
     const bool whole = splits == 1;
+    const float r_sum = __frcp_rn(lsum);
 #pragma unroll
     for (int c = 0; c < D / 2; c += 4) {
       float4 o = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
       if (whole)
-        o = make_float4(__fdiv_rn(o.x, lsum), __fdiv_rn(o.y, lsum), __fdiv_rn(o.z, lsum), __fdiv_rn(o.w, lsum));
+        o = make_float4(over(o.x, lsum, r_sum), over(o.y, lsum, r_sum), over(o.z, lsum, r_sum), over(o.w, lsum, r_sum));
       *reinterpret_cast<float4 *>(stage + r * T::LDO + half * (D / 2) + c) = o;
     }
     pair_sync();
@@ -487,6 +494,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(const AttnPar
           factor[z * kRows + r] = fz;
         }
         bars.sum[0][r] = l;
+        bars.sum[1][r] = __frcp_rn(l);
       }
       pair_sync();
       each4([&](int i0, float4 (&o)[4]) {
@@ -504,8 +512,9 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(const AttnPar
           }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const float l = bars.sum[0][quad * 32 + (i0 + 64 * u) / (D / 4)];
-          o[u] = make_float4(__fdiv_rn(o[u].x, l), __fdiv_rn(o[u].y, l), __fdiv_rn(o[u].z, l), __fdiv_rn(o[u].w, l));
+          const int rr = quad * 32 + (i0 + 64 * u) / (D / 4);
+          const float l = bars.sum[0][rr], rl = bars.sum[1][rr];
+          o[u] = make_float4(over(o[u].x, l, rl), over(o[u].y, l, rl), over(o[u].z, l, rl), over(o[u].w, l, rl));
         }
       });
     }
