@@ -578,8 +578,9 @@ int prefill_attn_launch(const float *qkv, int64_t ld, const float *kc, const flo
   p.max_len = max_len;
   p.error = error;
   // Row tiles have histories from pos0 to pos0 + M keys, and few rows make few tiles.  While there are fewer row tiles than
-  // SMs their keys are shared out: the smallest shares of which one wave (148 CTAs) holds all, at least 4 key tiles (a share
-  // costs a Q conversion and a trip through L2, as much as two).
+  // SMs their keys are shared out: the smallest shares of which one wave (148 CTAs) holds all, at least 2 key tiles, and none of
+  // up to three (a share costs a Q conversion and a trip through L2): 366 rows 3.61 ms a pass with at least 4, 3.54 with 2; 150
+  // rows 2.73 whole, 2.82 in two.
   const int q_tiles = (int)(((int64_t)M * p.G + kRows - 1) / kRows), most = p.key_tiles;
   auto shares = [&](int chunk) {
     int64_t n = 0;
@@ -592,7 +593,7 @@ int prefill_attn_launch(const float *qkv, int64_t ld, const float *kc, const flo
   p.chunk = most;
   auto slots = [&](int chunk) { return (int64_t)((most + chunk - 1) / chunk) * q_tiles * kv_heads; };
   if ((int64_t)q_tiles * kv_heads < kSms) {
-    int lo = std::min(most, std::max(4, (most + kMostSplits - 1) / kMostSplits));
+    int lo = std::min(most, std::max(most <= 3 ? 3 : 2, (most + kMostSplits - 1) / kMostSplits));
     while (lo < p.chunk) {
       const int mid = (lo + p.chunk) / 2;
       if (shares(mid) <= kSms && slots(mid) <= kMaxShares)
