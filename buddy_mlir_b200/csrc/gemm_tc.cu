@@ -990,13 +990,15 @@ struct Plan {
 };
 constexpr int kMostShared = 198 * 1024;
 
-// Costs in clocks.  A k block costs a pair its products (8192 of 128 x 128 x nc a clock and SM) or its bytes (64 a clock and SM),
-// whichever takes longer; a tile's epilogue runs under the next tile's products, except the last.  Sums across a cluster cost 1.5 us
-// and their rows, every SM that is taken counts (the next kernel of a pass could start there: a decode step's attention after
-// q|k|v of 24 rows took 17 us behind 128 CTAs, 14 behind 16), and clusters of four and eight CTAs leave SMs over (72 of eight took two turns): whole / in two / in four,
-//   24 x 2048 x 1536      9.2   10.2    9.9 us        24 x 1536 x 8960    25.3    -     13.5
-//   100 x 1536 x 8960    23.6   18.5   17.1           200 x 1536 x 8960   25.1   20.7   33.2 (two turns)
-//   366 x 1536 x 8960    26.4   25.5    -
+// Costs in clocks.  A k block costs a pair its products (8192 of 128 x 128 x nc a clock and SM) or its bytes (64 a clock and SM, 45
+// when all pairs load), whichever takes longer; a tile's epilogue runs under the next tile's products, except the last.  Every pair that
+// is taken counts: the next kernel of a pass could start there (a decode step's attention after q|k|v of 24 rows took 17 us behind
+// 128 CTAs, 14 behind 16).  Sums across a cluster cost 1.5 to 3.5 us (in a pass) and their rows, and clusters of four and eight CTAs leave SMs over (72
+// of eight took two turns).  Row tiles x shares of k, us:
+//   24 x 2048 x 1536      1 x 1  9.2    1 x 2 10.2    1 x 4  9.9        24 x 1536 x 8960      1 x 1 25.3   1 x 4 13.5
+//   100 x 1536 x 8960     4 x 1 23.6    4 x 2 18.5    2 x 4 17.1        200 x 1536 x 8960     6 x 1 25.1   5 x 2 20.7   3 x 4 33.2 (two turns)
+//   366 x 1536 x 8960    12 x 1 26.1    5 x 2 25.1    6 x 1 26.6        700 x 1536 x 8960    12 x 1 30.5   9 x 1 34.2  18 x 1 45.8
+//   W8A8 333 x 1536 x 8960  11 x 1 27.8  4 x 2 26.0   2 x 4 28.3        W8A8 333 x 1536 x 1536  11 x 1 11.6  6 x 1 10.1  2 x 1 11.0
 Plan make_plan(int M, int N, int K, int nd) {
   const int nkb = (K + BK - 1) / BK, n_tiles = (N + 2 * BM - 1) / (2 * BM), most = nd == 1 ? 256 : 84, least_tiles = (M + most - 1) / most;
   Plan best{};
@@ -1004,13 +1006,13 @@ Plan make_plan(int M, int N, int K, int nd) {
   for (int mt = least_tiles; mt < least_tiles + 16 && mt <= M; ++mt) {
     const int rows = (M + mt - 1) / mt, need = nd == 1 ? rows : kWidePlanes * ((rows + 1) / 2), nc = (need + 31) / 32 * 32;
     const int m_tiles = (M + rows - 1) / rows, tiles = n_tiles * m_tiles;
-    const float per_kb = (float)std::max(2 * nc, 2 * BM + nc);
     for (int splits = 1; splits <= kMaxSplits && splits <= std::max(nkb / 2, 1); splits *= 2) {
       if (splits > 1 && tiles * splits > kPairs * 7 / 8)
         break;
-      const float rounds = (float)((tiles + kPairs - 1) / kPairs);
-      const float cost = rounds * (float)((nkb + splits - 1) / splits) * per_kb + 1000.f + 40.f * rows + (splits > 1 ? 3000.f + 60.f * rows : 0.f) +
-                         20.f * (float)std::min(tiles * splits, kPairs);
+      const float rounds = (float)((tiles + kPairs - 1) / kPairs), busy = (float)std::min(tiles * splits, kPairs);
+      const float per_kb = std::max(2.f * nc, (2 * BM + nc) * (1.f + 0.4f * busy / kPairs));
+      const float cost = rounds * (float)((nkb + splits - 1) / splits) * per_kb + 1000.f + 20.f * rows +
+                         (splits > 1 ? 7000.f + 60.f * rows : 0.f) + 50.f * busy;
       if (best.nc == 0 || cost < least) {
         least = cost;
         best.nc = nc;

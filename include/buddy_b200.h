@@ -163,7 +163,7 @@ int b200_gemv(const b200_weight *w, const b200_gemv_args *a, void *stream);
  * products are exact (tcgen05.mma kind::i8) and added in f32; rows with
  * channels far above the rest get six digits.  workspace:
  * b200_gemm_w8_workspace_bytes(M, K) bytes, 256-byte aligned, owned by the
- * caller (it holds the digits, shares of split tiles and an error word).
+ * caller (it holds the digits, the rows' scales and an error word).
  * b200_gemm_w8_status() reports a bounded wait that gave up.  All reads,
  * weights included, come after the work that precedes the call on `stream`. */
 int64_t b200_gemm_w8_workspace_bytes(int M, int64_t K);
