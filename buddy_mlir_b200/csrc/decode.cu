@@ -526,6 +526,8 @@ __device__ __forceinline__ void gemv_phase(Ctx &c, int ph, const XSrc &xs, const
     } else if (in) {
       if (ep.kind == EP_LOGITS) {
         c.p.logits[row] = v;
+        if (c.p.logits_host != nullptr)
+          c.p.logits_host[row] = v;
         if (v > bestv) {   // rows ascend: the first maximum stays
           bestv = v;
           besti = row;
@@ -616,10 +618,15 @@ __device__ __noinline__ void attention_range(Shared &sh, const DecLayer *layers,
       dst[32 * i] = in[i] * f;
     if (h >= G && s1 == pos + 1) {   // the range that holds the new row writes it
       float *row = (h == G ? ly.k_cache : ly.v_cache) + head + (size_t)pos * D + lane;
-      float *stage = p.kv_stage + (size_t)(2 * layer + (h == G ? 0 : 1)) * KD + (size_t)hk * D + lane;
+      const size_t at = (size_t)(2 * layer + (h == G ? 0 : 1)) * KD + (size_t)hk * D + lane;
+      float *stage = p.kv_stage + at;
 #pragma unroll
       for (int i = 0; i < 4; ++i)
         row[32 * i] = stage[32 * i] = in[i];
+      if (p.rows_host != nullptr)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          p.rows_host[at + 32 * i] = in[i];
     }
   }
   if (tr != nullptr && tid == 0)

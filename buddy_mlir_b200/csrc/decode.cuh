@@ -47,6 +47,9 @@ struct DecParams {
   uint2 *ll_cand;               // [grid][2] per-CTA argmax candidates (value, index)
   float *logits;
   float *kv_stage;              // [2*L][kvh*D] rows written this step
+  // the same in page-locked host memory, or null.  Written beside the step's own work: 608 KB of logits cross the bus while the
+  // lm_head streams, where a copy behind the kernel took 15 us (and one of the rows 3)
+  float *logits_host, *rows_host;
   int32_t *state;               // token, pos, next, count, launches completed
   int32_t *history;
   int history_cap;

@@ -1696,17 +1696,22 @@ int b200_model_decode(b200_model *m, int token, int pos, float *logits_host,
   if (token < 0 || token >= m->cfg.vocab || pos < 0 || pos >= m->cfg.max_len)
     return fail(B200_EINVAL, "decode: token %d / position %d out of range", token, pos);
   if (int rc = set_state(m, token, pos)) return rc;
+  // a caller that wants the logits on the host usually mirrors the new K/V rows too: they come along, so that
+  // b200_model_read_new_kv_rows needs no second round trip.  The persistent kernel writes both there itself.
+  const bool direct = m->persistent && !m->act_int8;
+  m->dp.logits_host = direct && logits_host ? m->h_logits_pinned : nullptr;
+  m->dp.rows_host = direct && logits_host ? m->h_rows_pinned : nullptr;
   B200_CUDA(cudaEventRecord(m->ev0, m->stream));
-  if (int rc = run_step(m)) return rc;
+  const int step_rc = run_step(m);
+  m->dp.logits_host = m->dp.rows_host = nullptr;
+  if (step_rc) return step_rc;
   B200_CUDA(cudaEventRecord(m->ev1, m->stream));
   m->rows_fresh = false;
   if (logits_host && m->tp > 1 && m->tp_push.ranks > 0)   // the step itself exchanged only (value, index)
     B200_NCCL(g_nccl.AllGather(m->logits_shard, m->logits, m->vocab, kNcclFloat, g_nccl.comm, m->stream));
-  if (logits_host) {
+  if (logits_host && !direct) {
     B200_CUDA(cudaMemcpyAsync(m->h_logits_pinned, m->logits, (size_t)m->cfg.vocab * 4,
                               cudaMemcpyDeviceToHost, m->stream));
-    // a caller that wants the logits on the host usually mirrors the new K/V rows too:
-    // they ride along, so that b200_model_read_new_kv_rows needs no second round trip
     B200_CUDA(cudaMemcpyAsync(m->h_rows_pinned, m->kv_stage,
                               (size_t)2 * m->cfg.n_layers * m->kvh * m->cfg.head_dim * 4,
                               cudaMemcpyDeviceToHost, m->stream));
