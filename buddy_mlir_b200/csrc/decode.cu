@@ -158,11 +158,11 @@ __device__ __forceinline__ bool poll_expired(const DecParams &p, Shared &sh, Pol
   return false;
 }
 // The same for a whole warp, lanes with `ok` still waiting for the others: one decision for all of them.  Poll loops leave
-// together: lanes that fall out of a loop one by one stay apart, and every shuffle after it pays for it.
+// together: lanes that fall out of a loop one by one stay apart, and every shuffle after it pays for it.  (No sleep between polls:
+// with 20 ns a 1.5B int8 step at contexts 97 / 1000 takes 643 / 668 us instead of 640 / 664.)
 __device__ __forceinline__ bool poll_done(const DecParams &p, Shared &sh, Poll &w, int code, bool ok) {
   if (__all_sync(0xffffffffu, ok))
     return true;
-  __nanosleep(20);
   return __any_sync(0xffffffffu, poll_expired(p, sh, w, code));
 }
 __device__ __forceinline__ float ll_wait1(Ctx &c, const uint2 *p, uint32_t tag) {
@@ -171,7 +171,6 @@ __device__ __forceinline__ float ll_wait1(Ctx &c, const uint2 *p, uint32_t tag) 
   while (v.y != tag) {
     if (poll_expired(c.p, c.sh, w, 400 + (int)(tag & 7)))
       break;
-    __nanosleep(20);
     v = ll_load1(p);
   }
   return __uint_as_float(v.x);
