@@ -106,8 +106,8 @@ class ClockSampler:
 # dram__bytes_read.sum + dram__bytes_write.sum of one decode_step_kernel launch (ncu, full-size
 # 1.5B int8 model at context ~1000), and the git blob hash of the kernel source it was captured
 # from.  The figure is only reported while the source is still that one.
-TRAFFIC = {"bytes": 1_614_000_000, "kernel_source": "buddy_mlir_b200/csrc/decode.cu",
-           "git_blob": "61e3ac7eb1da439de78079e829ef620bf860dfda",
+TRAFFIC = {"bytes": 1_609_147_000, "kernel_source": "buddy_mlir_b200/csrc/decode.cu",
+           "git_blob": "04409092035db774d650d358d5a004d2c9e9b463",
            "capture": "ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none -k regex:decode_step -s 2 -c 1"}
 
 
