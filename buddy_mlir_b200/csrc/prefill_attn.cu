@@ -22,6 +22,7 @@
 // conversion run beside it.  f32 FMAs at 128 per clock would need 16384.  1000 rows, 12 heads on 2, D = 128, a layer: 219 us
 // for register-tiled FMAs, 42 here and 3.5 for the images; 366 rows 25, 64 rows 14 (with a divide per output element 45, 31 and 16).
 #include "common.cuh"
+#include "quotient.cuh"
 #include "tensor_core.cuh"
 
 #include <algorithm>
@@ -73,12 +74,6 @@ __device__ __forceinline__ void split8(float (&v)[8], uint4 (&t)[kTerms]) {
 #pragma unroll
   for (int q = 0; q < kTerms; ++q)
     t[q] = make_uint4(take_bf16(v[0], v[1]), take_bf16(v[2], v[3]), take_bf16(v[4], v[5]), take_bf16(v[6], v[7]));
-}
-// a / b with r = 1 / b: the quotient's remainder once, as the division does it, without its branch for other ranges (b, a sum of
-// weights, is at least one; an infinite a stays infinite)
-__device__ __forceinline__ float over(float a, float b, float r) {
-  const float q = a * r, e = fmaf(-b, q, a);
-  return e == e ? fmaf(e, r, q) : q;
 }
 // byte offset of 16-byte chunk c of row r in a tile of 128-byte rows, 128-byte swizzle
 __device__ __forceinline__ uint32_t swz(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }
@@ -435,7 +430,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(const AttnPar
     for (int c = 0; c < D / 2; c += 4) {
       float4 o = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
       if (whole)
-        o = make_float4(over(o.x, lsum, r_sum), over(o.y, lsum, r_sum), over(o.z, lsum, r_sum), over(o.w, lsum, r_sum));
+        o = make_float4(quotient(o.x, lsum, r_sum), quotient(o.y, lsum, r_sum), quotient(o.z, lsum, r_sum), quotient(o.w, lsum, r_sum));
       *reinterpret_cast<float4 *>(stage + r * T::LDO + half * (D / 2) + c) = o;
     }
     pair_sync();
@@ -514,7 +509,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(const AttnPar
         for (int u = 0; u < 4; ++u) {
           const int rr = quad * 32 + (i0 + 64 * u) / (D / 4);
           const float l = bars.sum[0][rr], rl = bars.sum[1][rr];
-          o[u] = make_float4(over(o[u].x, l, rl), over(o[u].y, l, rl), over(o[u].z, l, rl), over(o[u].w, l, rl));
+          o[u] = make_float4(quotient(o[u].x, l, rl), quotient(o[u].y, l, rl), quotient(o[u].z, l, rl), quotient(o[u].w, l, rl));
         }
       });
     }
