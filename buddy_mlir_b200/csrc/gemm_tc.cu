@@ -177,16 +177,9 @@ struct RowScales {
   __device__ __forceinline__ float at(int r0) const { return r0 < 32 ? v[0] : r0 < 64 ? v[1] : v[2]; }   // rows r0 & ~31 ..
 };
 
-// The operations and their order are the reference's (subgraph0_decode_simplify.mlir:226-231: (g * sigmoid(g)) * u).  The
-// reciprocal is the hardware's and one Newton step, without the divide's branch for other ranges: the chains of several
-// rows run side by side.
-__device__ __forceinline__ float silu_of(float g, float u) {
-  const float d = 1.0f + expf(-g);
-  float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
-  r = d < 3.4e38f ? fmaf(r, fmaf(-d, r, 1.0f), r) : 0.f;
-  return __fmul_rn(__fmul_rn(g, r), u);
-}
+// silu(g) * u.  The operations, their order and roundings are the reference's (subgraph0_decode_simplify.mlir:226-231: (g * sigmoid(g)) *
+// u) and those of b200_silu_mul.  d = 1 + e^-g; __frcp_rn is 1 / d rounded to nearest.
+__device__ __forceinline__ float silu_of(float g, float u, float d) { return __fmul_rn(__fmul_rn(g, __frcp_rn(d)), u); }
 
 // ---- epilogue ----------------------------------------------------------------------------------------------------------------
 // A warp reads the 32 lanes of tensor memory that match its rank within its warpgroup, a lane one channel; the warps that share a
@@ -222,10 +215,17 @@ __device__ __forceinline__ void finish_rows(const GemmParams &p, const Channel &
   if (p.silu_pairs) {   // (gate, up) are neighbouring lanes: of two rows the even lane takes the first, the odd one the second
     const bool odd = c.n & 1;
     float *dst = p.C + (int64_t)m * p.ldc + (c.n >> 1) + (odd ? p.ldc : 0);
+    float d[N / 2];
 #pragma unroll
     for (int i = 0; i < N; i += 2) {
       const float other = __shfl_xor_sync(0xffffffffu, odd ? y[i] : y[i + 1], 1);
-      const float v = silu_of(odd ? other : y[i], odd ? y[i + 1] : other);
+      y[i] = odd ? other : y[i];
+      y[i + 1] = odd ? y[i + 1] : other;
+      d[i / 2] = 1.0f + expf(-y[i]);   // of all rows before the first reciprocal, whose branch for other ranges parts the rows' chains
+    }
+#pragma unroll
+    for (int i = 0; i < N; i += 2) {
+      const float v = silu_of(y[i], y[i + 1], d[i / 2]);
       if (c.in && (ALL || (live >> (odd ? i + 1 : i) & 1)))
         *dst = v;
       dst += 2 * p.ldc;
