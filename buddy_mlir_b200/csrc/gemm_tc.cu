@@ -1125,7 +1125,7 @@ int gemm_w8_run(const b200_weight *w, const float *A, int M, int64_t lda, float 
   p.scale = (const float *)w->scale;
   p.bias = (const float *)w->bias;
   p.row_scale = row_scale;
-  p.residual = residual;
+  p.residual = silu_pairs ? nullptr : residual;   // SiLU pairs have none: the kernel would ask for N columns of it
   p.C = C;
   p.ldc = ldc;
   p.ldr = ldr;

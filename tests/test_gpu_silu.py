@@ -71,3 +71,24 @@ def test_int8_forms_of_one_row(N, K, size):
     torch.cuda.synchronize()
     assert same(one.cpu().numpy(), dense.cpu().numpy())
     assert same(dense.cpu().numpy(), silu_mul(plain))
+
+
+# one turn of the pairs, k in shares, wide rows: the three places that ask for residual rows
+@pytest.mark.parametrize("M,N,K,wide", [(100, 512, 512, False), (24, 256, 8960, False), (84, 514, 512, True)])
+def test_a_residual_beside_silu_pairs_is_left_alone(M, N, K, wide):
+    """b200_gemm_w8 has no residual for SiLU pairs: one that is given all the same, of the output's N / 2 columns, counts for nothing."""
+    import torch
+    from gpu_util import dev, ptr, stream
+    lib = _lib.load()
+    w, keep, rng = weight(K, N, M)
+    A = rng.standard_normal((M, K)).astype(np.float32)
+    if wide:
+        A[M // 2, 17] *= 3000
+    dA, ws = dev(A), torch.zeros(lib.b200_gemm_w8_workspace_bytes(M, K), dtype=torch.uint8, device="cuda")
+    res, out = torch.full((M, N // 2), float("nan"), device="cuda"), []
+    for r in (None, ptr(res)):
+        y = torch.empty(M, N // 2, device="cuda")
+        _lib.check(lib.b200_gemm_w8(C.byref(w), ptr(dA), M, K, ptr(y), N // 2, r, N // 2, None, 0.0, 1, ptr(ws), ws.numel(), stream()))
+        _lib.check(lib.b200_gemm_w8_status(ptr(ws), stream()))
+        out.append(y.cpu().numpy())
+    assert same(*out)
