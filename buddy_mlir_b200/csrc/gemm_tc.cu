@@ -52,6 +52,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 
 namespace b200 {
@@ -995,26 +996,29 @@ constexpr int kMostShared = 198 * 1024;
 // Costs in clocks.  A k block costs a pair its products (8192 of 128 x 128 x nc a clock and SM) or its bytes (64 a clock and SM, 45
 // when all pairs load), whichever takes longer; a tile's epilogue runs under the next tile's products, except the last.  Every pair that
 // is taken counts: the next kernel of a pass could start there (a decode step's attention after q|k|v of 24 rows took 17 us behind
-// 128 CTAs, 14 behind 16).  Sums across a cluster cost 1.5 to 3.5 us (in a pass) and their rows, and clusters of four and eight CTAs leave SMs over (72
-// of eight took two turns).  Row tiles x shares of k, us:
-//   24 x 2048 x 1536      1 x 1  9.2    1 x 2 10.2    1 x 4  9.9        24 x 1536 x 8960      1 x 1 25.3   1 x 4 13.5
-//   100 x 1536 x 8960     4 x 1 23.6    4 x 2 18.5    2 x 4 17.1        200 x 1536 x 8960     6 x 1 25.1   5 x 2 20.7   3 x 4 33.2 (two turns)
-//   366 x 1536 x 8960    12 x 1 26.1    5 x 2 25.1    6 x 1 26.6        700 x 1536 x 8960    12 x 1 30.5   9 x 1 34.2  18 x 1 45.8
-//   W8A8 333 x 1536 x 8960  11 x 1 27.8  4 x 2 26.0   2 x 4 28.3        W8A8 333 x 1536 x 1536  11 x 1 11.6  6 x 1 10.1  2 x 1 11.0
-Plan make_plan(int M, int N, int K, int nd) {
+// 128 CTAs, 14 behind 16).  Sums across a cluster cost time for themselves and for their rows, which also take memory from the ring.
+// Clusters of four, six and eight CTAs leave SMs over, which differ from part to part (SMs that are switched off): 33, 22 and 15 of
+// them fit here, and one more than fits takes a second turn: so many shares are not taken.  Row tiles x shares of k, us, weights from
+// memory, * where the clusters take two turns:
+//   24 x 2048 x 1536      1 x 1  9.4    2 x 1  9.4    1 x 4  9.7        24 x 1536 x 8960      1 x 3 14.9   1 x 4 13.8
+//   100 x 1536 x 8960     3 x 2 18.5    3 x 3 16.9    2 x 4 16.9        200 x 1536 x 8960     5 x 2 20.8   3 x 3 20.7   3 x 4 32.3 *
+//   366 x 1536 x 8960     5 x 2 25.1    5 x 1 28.6   12 x 1 26.3        700 x 1536 x 8960    11 x 1 30.5   9 x 1 34.6  18 x 1 45.7
+//   24 x 4096 x 4096      1 x 1 14.9    1 x 3 13.3    1 x 4 21.5 *      24 x 4096 x 12288     1 x 2 24.2   1 x 3 20.8   1 x 4 31.7 *
+//   W8A8 366 x 1536 x 8960  4 x 2 27.0   3 x 3 28.0   2 x 4 30.6        W8A8 366 x 1536 x 1536  6 x 1 10.3  4 x 1 10.6  2 x 2 19.1
+Plan make_plan(int M, int N, int K, int nd, const int (&held)[kMaxSplits + 1]) {
   const int nkb = (K + BK - 1) / BK, n_tiles = (N + 2 * BM - 1) / (2 * BM), most = nd == 1 ? 256 : 84, least_tiles = (M + most - 1) / most;
   Plan best{};
   float least = 0.f;
   for (int mt = least_tiles; mt < least_tiles + 16 && mt <= M; ++mt) {
     const int rows = (M + mt - 1) / mt, need = nd == 1 ? rows : kWidePlanes * ((rows + 1) / 2), nc = (need + 31) / 32 * 32;
     const int m_tiles = (M + rows - 1) / rows, tiles = n_tiles * m_tiles;
-    for (int splits = 1; splits <= kMaxSplits && splits <= std::max(nkb / 2, 1); splits *= 2) {
-      if (splits > 1 && tiles * splits > kPairs * 7 / 8)
+    for (int splits = 1; splits <= kMaxSplits && splits <= std::max(nkb / 2, 1); ++splits) {
+      if (splits > 1 && tiles > held[splits])
         break;
       const float rounds = (float)((tiles + kPairs - 1) / kPairs), busy = (float)std::min(tiles * splits, kPairs);
       const float per_kb = std::max(2.f * nc, (2 * BM + nc) * (1.f + 0.4f * busy / kPairs));
       const float cost = rounds * (float)((nkb + splits - 1) / splits) * per_kb + 1000.f + 20.f * rows +
-                         (splits > 1 ? 7000.f + 60.f * rows : 0.f) + 50.f * busy;
+                         (splits > 1 ? 2000.f + 100.f * rows : 0.f) + 50.f * busy;
       if (best.nc == 0 || cost < least) {
         least = cost;
         best.nc = nc;
@@ -1066,8 +1070,40 @@ int launch_gemm(const Plan &pl, const void *a, const void *x, const void *w, Gem
     return rc;
   return launch_after_clusters(2 * pl.splits, gemm_i8_kernel<PLANES, SPLIT>, dim3(pl.grid), kThreads, pl.smem, st, map_a, map_w, p, map_x);
 }
+// How many clusters of 2 x splits CTAs the current device holds at once.
+int clusters_held(int splits) {
+  static std::atomic<int> known[64][kMaxSplits + 1];   // per device, once it has been asked
+  int dev = 0, n = 0;
+  B200_CUDA(cudaGetDevice(&dev));
+  std::atomic<int> *seen = dev >= 0 && dev < 64 ? &known[dev][splits] : nullptr;
+  if (seen != nullptr && (n = seen->load(std::memory_order_relaxed)) > 0)
+    return n;
+  static RaisedOn raised;
+  auto kern = gemm_i8_kernel<true, true>;
+  if (int rc = raise_shared_limit(raised, (const void *)kern, kMostShared))
+    return rc;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(kSms / (2 * splits) * 2 * splits);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = kMostShared;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2 * splits;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  B200_CUDA(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));
+  n = std::max(n, 1);
+  if (seen != nullptr)
+    seen->store(n, std::memory_order_relaxed);
+  return n;
+}
 template <bool PLANES> int launch_plan(const void *a, const void *x, const void *w, GemmParams &p, cudaStream_t st) {
-  const Plan pl = make_plan(p.M, p.N, p.K, PLANES ? kPlanes : 1);
+  int held[kMaxSplits + 1] = {};
+  for (int s = 2; s <= kMaxSplits; ++s)
+    if ((held[s] = clusters_held(s)) < 0)
+      return held[s];   // an error code
+  const Plan pl = make_plan(p.M, p.N, p.K, PLANES ? kPlanes : 1, held);
   return pl.splits > 1 ? launch_gemm<PLANES, true>(pl, a, x, w, p, st) : launch_gemm<PLANES, false>(pl, a, x, w, p, st);
 }
 

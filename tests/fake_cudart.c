@@ -64,6 +64,16 @@ int cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, const void *f
   (void)fn; (void)t; (void)s; (void)f; *n = 1; return OK;
 }
 
+/* the clusters of a B200 with 148 of its SMs in use; attribute 4 is the cluster's dimension */
+int cudaOccupancyMaxActiveClusters(int *n, const void *fn, const config *c) {
+  unsigned ctas = 1;
+  for (unsigned i = 0; i < c->n; ++i)
+    if (((const unsigned *)((const char *)c->attrs + 72 * i))[0] == 4) ctas = ((const unsigned *)((const char *)c->attrs + 72 * i))[2];
+  if (at(fn) < 0 || funcs[at(fn)].smem[fake_device] < c->smem) return ret(INVALID);
+  *n = ctas == 2 ? 74 : ctas == 4 ? 33 : ctas == 6 ? 22 : ctas == 8 ? 15 : 0;
+  return *n ? OK : ret(INVALID);
+}
+
 int cudaGetDeviceCount(int *n) { *n = 8; return OK; }
 int cudaGetDevice(int *d) { *d = fake_device; return OK; }
 int cudaSetDevice(int d) { fake_device = d; return OK; }

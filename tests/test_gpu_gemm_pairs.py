@@ -73,3 +73,24 @@ def test_w8a8_pair_edges(M, N, K):
     q = np.clip(np.rint(A * (np.float32(1) / scale)), -128, 127)
     want = (q @ Q.astype(np.float64)).astype(np.float32) * (scale * s)
     assert np.array_equal(call("w8a8", A, Q, s, ldc=N + 1), want)
+
+
+# k in three shares: of one row, of rows and blocks of k that three does not divide, and of rows of which a share is empty
+@pytest.mark.parametrize("M,N,K", [(1, 4096, 4096), (2, 4090, 3200), (24, 4096, 4160), (64, 4000, 6016), (200, 1536, 8960)])
+def test_three_shares(M, N, K):
+    A, Q, s, rng = inputs(M, N, K, M + K)
+    if M > 2:
+        A[M // 2, K // 2] *= 3000
+    res = rng.standard_normal((M, N)).astype(np.float32)
+    want = (A.astype(np.float64) @ Q.astype(np.float64)) * s + res
+    got = call("w8", A, Q, s, residual=res)
+    # as above, row by row: one row is far larger than the others
+    assert (np.abs(got - want).max(1) / np.abs(want).max(1)).max() < 4e-6
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 4096, 4096), (25, 4090, 4160), (301, 1536, 8960)])
+def test_w8a8_three_shares(M, N, K):
+    A, Q, s, _ = inputs(M, N, K, M * 3 + K)
+    scale = np.maximum(np.float32(np.abs(A).max()) * (np.float32(1) / np.float32(127)), np.float32(1e-10))
+    q = np.clip(np.rint(A * (np.float32(1) / scale)), -128, 127)
+    assert np.array_equal(call("w8a8", A, Q, s), (q @ Q.astype(np.float64)).astype(np.float32) * (scale * s))
