@@ -21,8 +21,8 @@
 //   now          1.7e-7   1.1e-6   9.4e-7   4.0e-7   8.1e-8
 //   three digits 3.2e-7   3.2e-6   1.0e-5   1.1e-4   9.9e-4    (for every row, 23 bits)
 //   two bf16     2.5e-6 for all; f32 products and sums 7.0e-7
-// Time with no wide row / one / all, us: 1024 x 17920 x 1536 70 / 112 / 210, 1000 x 1536 x 8960 44 / 71 / 112, 24 x 17920 x 1536
-// 10.5 / 17 / 22.
+// Time with no wide row / one / all, us, weights from memory: 1024 x 17920 x 1536 69 / 85 / 180, 1000 x 1536 x 8960 40 / 65 / 109,
+// 24 x 17920 x 1536 12.6 / 19 / 22.
 //
 // W8A8 (b200_gemm_w8a8) is the same kernel with one digit per activation.
 //
@@ -337,11 +337,19 @@ __device__ __forceinline__ void store_tile(const GemmParams &p, const Tile &t, c
   }
 }
 // The pass with six digits over `rows` rows of a tile, `first` the first: its wide rows.
-template <bool SPLIT>
-__device__ __forceinline__ void store_wide_pass(const GemmParams &p, int m0, const Channel &c, uint32_t tmem, bool ok, int first, int rows,
-                                                uint32_t release, const Shares &sh) {
+template <bool SPLIT, typename Wait>
+__device__ __forceinline__ void store_wide_pass(const GemmParams &p, int m0, const Channel &c, uint32_t tmem, int first, int rows,
+                                                uint32_t release, const Shares &sh, Wait wait) {
   constexpr int N = CR / 2;
   const int lane = threadIdx.x & 31, grp = (threadIdx.x - 64) >> 7;
+  float rs, res[N];
+  auto request = [&](int r0, float &s, float (&r)[N]) {
+    s = lane < N && r0 + lane < rows ? __ldcg(p.row_scale + m0 + first + r0 + lane) : 0.f;
+    if (!SPLIT)
+      load_residual<N>(p, c, m0 + first + r0, rows - r0, r);
+  };
+  request(grp * N, rs, res);
+  const bool ok = wait();
   if (grp * N >= rows || !ok) {
     release_accumulator(release);
     return;
@@ -353,12 +361,9 @@ __device__ __forceinline__ void store_wide_pass(const GemmParams &p, int m0, con
     for (int q = 0; q < 3; ++q)
       if (r0 * kWidePlanes + q * CR < p.nc)
         tmem_load(tmem + r0 * kWidePlanes + q * CR, *reinterpret_cast<uint32_t(*)[CR]>(v + q * CR));
-    const int m = m0 + first + r0;
-    const float rs = lane < N && r0 + lane < rows ? __ldcg(p.row_scale + m + lane) : 0.f;
     const uint32_t live = __ballot_sync(0xffffffffu, signbit(rs));
-    float res[N], y[N];
-    if (!SPLIT)
-      load_residual<N>(p, c, m, rows - r0, res);
+    float next_rs, next[N], y[N];
+    request(r0 + kGroups * N, next_rs, next);
     tmem_wait_load();
     if (r0 + kGroups * N >= rows)
       release_accumulator(release);
@@ -369,8 +374,12 @@ __device__ __forceinline__ void store_wide_pass(const GemmParams &p, int m0, con
         if (live >> i & 1)
           give_row(p, sh, first + r0 + i, y[i]);
     } else {
-      finish_rows<true, false, N>(p, c, m, y, rs, 0, live, res);
+      finish_rows<true, false, N>(p, c, m0 + first + r0, y, rs, 0, live, res);
+#pragma unroll
+      for (int i = 0; i < N; ++i)
+        res[i] = next[i];
     }
+    rs = next_rs;
   }
 }
 // The rows that this CTA completes, shares added in order.  sums: this lane's channel of the first share.
@@ -408,8 +417,7 @@ __device__ __forceinline__ bool wait_shares(uint64_t *bar, volatile int *ab, int
   return true;
 }
 
-// An epilogue warp's way through the tiles from w on; n: accumulators so far.  WIDE = false: up to a tile with wide rows.  The rest
-// is a function that is called once, so that nothing is kept across it.
+// An epilogue warp's way through the tiles from w on; n: accumulators so far.  WIDE = false: up to a tile with wide rows.
 template <bool PLANES, bool SPLIT, bool WIDE>
 __device__ __forceinline__ int epilogue(const GemmParams &p, Bars &bars, float *sums, uint32_t tmem, int w, int step, int &n) {
   const int lane = threadIdx.x & 31, quad = threadIdx.x >> 5 & 3, crank = (int)cluster_rank(), rank = crank & 1;
@@ -449,8 +457,7 @@ __device__ __forceinline__ int epilogue(const GemmParams &p, Bars &bars, float *
 #pragma unroll 1
       for (int h = 0; h < 2; ++h)
         if (wide >> h & 1) {
-          wait();
-          store_wide_pass<SPLIT>(p, t.m0, c, lanes + (n & 1) * (p.cols >> 1), ok, h * half, min(half, t.rows - h * half), release(), sh);
+          store_wide_pass<SPLIT>(p, t.m0, c, lanes + (n & 1) * (p.cols >> 1), h * half, min(half, t.rows - h * half), release(), sh, wait);
           ++n;
         }
     }
@@ -471,12 +478,17 @@ __device__ __forceinline__ int epilogue(const GemmParams &p, Bars &bars, float *
     request(t);
   }
 }
+// The tiles from a wide one on.  Where a pair has several tiles (TURNS) this is part of the kernel: as a function, whose parameters lie
+// behind a generic pointer and are loaded again after every store, it made every later tile take twice as long (1024 x 20000 x 512 with
+// one wide row 112 us, 79 inline; without one 51 and 52).  Where it has one, it is a function all the same, with a copy of the parameters:
+// a small call is 0.35 us longer with all of it inline (24 x 1536 x 1536 8.9 / 9.3 us).
 template <bool SPLIT>
-__device__ __noinline__ void epilogue_wide(const GemmParams &p, Bars &bars, float *sums, uint32_t tmem, int w, int step, int n) {
+__device__ __noinline__ void epilogue_last(const GemmParams &p_in, Bars &bars, float *sums, uint32_t tmem, int w, int step, int n) {
+  const GemmParams p = p_in;
   epilogue<true, SPLIT, true>(p, bars, sums, tmem, w, step, n);
 }
 
-template <bool PLANES, bool SPLIT>
+template <bool PLANES, bool SPLIT, bool TURNS>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                const __grid_constant__ GemmParams p, const __grid_constant__ CUtensorMap map_x) {
@@ -633,8 +645,12 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     kernel_wait();   // row scales
     int n = 0, w = first;
     w = epilogue<PLANES, SPLIT, false>(p, bars, sums, tmem, w, step, n);
-    if (PLANES && w < p.tiles)
-      epilogue_wide<SPLIT>(p, bars, sums, tmem, w, step, n);
+    if (PLANES && w < p.tiles) {
+      if constexpr (TURNS)
+        epilogue<true, SPLIT, true>(p, bars, sums, tmem, w, step, n);
+      else
+        epilogue_last<SPLIT>(p, bars, sums, tmem, w, step, n);
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -1042,7 +1058,7 @@ Plan make_plan(int M, int N, int K, int nd, const int (&held)[kMaxSplits + 1]) {
   return best;
 }
 
-template <bool PLANES, bool SPLIT>
+template <bool PLANES, bool SPLIT, bool TURNS>
 int launch_gemm(const Plan &pl, const void *a, const void *x, const void *w, GemmParams &p, cudaStream_t st) {
   CUtensorMap map_a, map_w, map_x;
   const int box = pl.nc / 2;
@@ -1066,9 +1082,9 @@ int launch_gemm(const Plan &pl, const void *a, const void *x, const void *w, Gem
   p.stages = pl.stages;
   p.cols = pl.cols;
   static RaisedOn raised;
-  if (int rc = raise_shared_limit(raised, (const void *)gemm_i8_kernel<PLANES, SPLIT>, kMostShared))
+  if (int rc = raise_shared_limit(raised, (const void *)gemm_i8_kernel<PLANES, SPLIT, TURNS>, kMostShared))
     return rc;
-  return launch_after_clusters(2 * pl.splits, gemm_i8_kernel<PLANES, SPLIT>, dim3(pl.grid), kThreads, pl.smem, st, map_a, map_w, p, map_x);
+  return launch_after_clusters(2 * pl.splits, gemm_i8_kernel<PLANES, SPLIT, TURNS>, dim3(pl.grid), kThreads, pl.smem, st, map_a, map_w, p, map_x);
 }
 // How many clusters of 2 x splits CTAs the current device holds at once.
 int clusters_held(int splits) {
@@ -1079,7 +1095,7 @@ int clusters_held(int splits) {
   if (seen != nullptr && (n = seen->load(std::memory_order_relaxed)) > 0)
     return n;
   static RaisedOn raised;
-  auto kern = gemm_i8_kernel<true, true>;
+  auto kern = gemm_i8_kernel<true, true, false>;
   if (int rc = raise_shared_limit(raised, (const void *)kern, kMostShared))
     return rc;
   cudaLaunchConfig_t cfg{};
@@ -1104,7 +1120,13 @@ template <bool PLANES> int launch_plan(const void *a, const void *x, const void 
     if ((held[s] = clusters_held(s)) < 0)
       return held[s];   // an error code
   const Plan pl = make_plan(p.M, p.N, p.K, PLANES ? kPlanes : 1, held);
-  return pl.splits > 1 ? launch_gemm<PLANES, true>(pl, a, x, w, p, st) : launch_gemm<PLANES, false>(pl, a, x, w, p, st);
+  if (pl.splits > 1)
+    return launch_gemm<PLANES, true, false>(pl, a, x, w, p, st);
+  // several tiles per pair; with one row tile, where all are wide or none is, more than two of them: 24 x 20000 x 512 takes 9.4 us with
+  // the function and 9.8 inline, 18.3 and 16.1 when wide
+  if (PLANES && pl.tiles > (pl.m_tiles > 1 ? 1 : 2) * pl.grid / 2)
+    return launch_gemm<PLANES, false, PLANES>(pl, a, x, w, p, st);
+  return launch_gemm<PLANES, false, false>(pl, a, x, w, p, st);
 }
 
 } // namespace

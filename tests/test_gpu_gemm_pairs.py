@@ -94,3 +94,20 @@ def test_w8a8_three_shares(M, N, K):
     scale = np.maximum(np.float32(np.abs(A).max()) * (np.float32(1) / np.float32(127)), np.float32(1e-10))
     q = np.clip(np.rint(A * (np.float32(1) / scale)), -128, 127)
     assert np.array_equal(call("w8a8", A, Q, s), (q @ Q.astype(np.float64)).astype(np.float32) * (scale * s))
+
+
+# a row of six digits in one row tile of several, one turn of the pairs and several: the rows beside it are what they are without it
+@pytest.mark.parametrize("M,N,K,silu", [(90, 1000, 512, False), (170, 12000, 640, False), (333, 18000, 256, True), (700, 1536, 1088, False), (1000, 2048, 256, True)])
+def test_narrow_tiles_after_a_wide_one(M, N, K, silu):
+    A, Q, s, rng = inputs(M, N, K, M + N)
+    res = None if silu else rng.standard_normal((M, N)).astype(np.float32)
+    narrow = call("w8", A, Q, s, residual=res, silu=silu)
+    row = M // 2
+    A[row, 5] *= 3000
+    got = call("w8", A, Q, s, residual=res, silu=silu)
+    others = np.arange(M) != row
+    assert np.array_equal(got[others], narrow[others])
+    y = (A[row].astype(np.float64) @ Q.astype(np.float64)) * s
+    with np.errstate(over="ignore"):
+        want = y[0::2] / (1.0 + np.exp(-y[0::2])) * y[1::2] if silu else y + res[row]
+    assert np.abs(got[row] - want).max() / np.abs(want).max() < (1e-5 if silu else 4e-6)
