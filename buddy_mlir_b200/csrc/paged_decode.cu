@@ -129,12 +129,13 @@ template <int G, int VEC>
 __global__ void __launch_bounds__(kThreads, 2) paged_decode_kernel(const __grid_constant__ PagedParams p) {
   constexpr int D = 32 * VEC, N = kKeys * G, H = halvings(N), LEFT = N >> H;   // scores, and those a lane is left with
   __shared__ int s_row[kMaxRange];
-  __shared__ __align__(16) float s_new[2][D], s_acc[kWarps][G][D], s_sum[G][D];
+  __shared__ __align__(16) float s_new[3][D], s_acc[kWarps][G][D], s_sum[G][D];
   __shared__ float s_m[kWarps][G], s_l[kWarps][G], s_max[G], s_total[G];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int m = blockIdx.z, hk = blockIdx.y, C = gridDim.x, sp = blockIdx.x;
   kernel_go();
-  const int pos = p.row_pos[m], len = pos + 1, per = (len + C - 1) / C, j0 = min(sp * per, len), j1 = min(len, j0 + per);
+  const int pos = p.row_pos[m], len = pos + 1, per = ((len + C - 1) / C + kKeys - 1) / kKeys * kKeys;
+  const int j0 = min(sp * per, len), j1 = min(len, j0 + per);   // (only the range with the newest key may end within a warp's four)
   const int32_t *table = p.block_table + (int64_t)p.row_seq[m] * p.table_stride;
   for (int j = j0 + threadIdx.x; j < j1; j += kThreads)
     s_row[j - j0] = (table[j / p.page] * p.kv_heads + hk) * p.page + j % p.page;
@@ -199,6 +200,9 @@ __global__ void __launch_bounds__(kThreads, 2) paged_decode_kernel(const __grid_
     nv.store(p.v_pool + at);
     nk.store(&s_new[0][lane * VEC]);
     nv.store(&s_new[1][lane * VEC]);
+#pragma unroll
+    for (int e = 0; e < VEC; ++e)
+      s_new[2][lane * VEC + e] = 0.f;
   }
 #pragma unroll
   for (int g = 0; g < G; ++g) {
@@ -233,18 +237,14 @@ __global__ void __launch_bounds__(kThreads, 2) paged_decode_kernel(const __grid_
   };
 #pragma unroll 1
   for (; jb < j1; jb += kWarps * kKeys) {
-    if (jb + kKeys >= j1) {   // the range's last keys
+    // the newest key (its row in the pool may be anything yet), and in the place of keys beyond it, whose weight is zero, a value of zero
+    if (j1 == len && jb + kKeys > pos) {
 #pragma unroll
-      for (int u = 0; u < kKeys; ++u) {
-        if (jb + u == pos) {   // the newest (its row in the pool may be anything yet)
+      for (int u = 0; u < kKeys; ++u)
+        if (jb + u >= pos) {
           k[u].load(&s_new[0][lane * VEC]);
-          v[u].load(&s_new[1][lane * VEC]);
+          v[u].load(&s_new[jb + u > pos ? 2 : 1][lane * VEC]);
         }
-        if (jb + u >= j1)   // no key: its weight is zero, and so is the value, which could be infinite
-#pragma unroll
-          for (int e = 0; e < VEC; ++e)
-            v[u].v[e] = 0.f;
-      }
     }
     float sc[N];
 #pragma unroll
