@@ -375,13 +375,26 @@ int cluster_size(int M, int kv_heads, int longest) {
   return c;
 }
 
+// A CTA's range of keys is a chain of turns of 32 (0.5 to 1.2 us each, 2 at eight heads of 128, whose registers do not all fit), and no
+// more than 8 CTAs share a row: with few rows of long contexts the general kernels, which cut them in chunks of 256 keys over the whole
+// chip, are done sooner.  us a layer here / there, RoPE included, caches from memory; q heads on kv heads of 128:
+//   12 on 2   2 rows of 4000 22 / 26, of 8000 41 / 30; 4 of 8000 44 / 33; 8 of 4000 33 / 31, of 8000 61 / 58; 16 of 8000 73 / 110
+//   32 on 8   2 rows of 4000 26 / 28, of 8000 44 / 53      4 on 2   2 of 4000 17 / 21, of 8000 32 / 25; 8 of 8000 44 / 47
+//   8 on 1    2 rows of 2000 19 / 24, of 4000 34 / 24; 16 of 2000 29 / 29, of 3000 41 / 34; 24 of 3000 43 / 35, of 4000 55 / 60;
+//             37 of 1000 29 / 32, of 2000 53 / 33; 64 of 4000 109 / 116; 100 of 1000 55 / 61, of 2000 104 / 88
+bool ranges_pay(int G, int D, int ctas, int range, int longest) {
+  if (G == 8 && D == 128)
+    return range <= 320 || longest <= 1024 || ctas >= 256;
+  return range <= 512 || ctas >= 128;
+}
+
 } // namespace
 
 bool paged_decode_takes(const float *qkv, int64_t ld, const float *k_pool, const float *v_pool, int q_heads, int kv_heads, int D, int M,
                         int longest) {
   const int G = q_heads / kv_heads, C = cluster_size(M, kv_heads, longest);
   return (D == 64 || D == 128) && q_heads == G * kv_heads && (G == 1 || G == 2 || G == 3 || G == 4 || G == 6 || G == 8) && M <= 65535 &&
-         kv_heads <= 65535 && (longest + C - 1) / C <= kMaxRange && (ld & 3) == 0 &&
+         kv_heads <= 65535 && (longest + C - 1) / C <= kMaxRange && ranges_pay(G, D, M * kv_heads * C, (longest + C - 1) / C, longest) && (ld & 3) == 0 &&
          (((uintptr_t)qkv | (uintptr_t)k_pool | (uintptr_t)v_pool) & 15) == 0;
 }
 
