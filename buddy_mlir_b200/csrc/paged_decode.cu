@@ -5,8 +5,9 @@
 // What bounds it is a chain of latencies, not the 19 MB of a layer (24 sequences of 32..700 positions, 12 heads on 2, D = 128: 3 us
 // of HBM).  So the keys of a row are dealt evenly to the 8 warps of up to 8 CTAs of a cluster, four keys at a time: a lane owns
 // D / 32 dims, K and V rows are whole 512-byte loads, and 24 scores (4 keys x 6 heads) are summed across the lanes together with 27
-// shuffles.  The first rows are requested, and the others sent to L2, before the kernel waits for the one before it: nothing of this
-// pass writes them.  Warps meet in shared memory, CTAs in that of the cluster, each completing its share of the output.
+// shuffles.  The first rows are requested before the kernel waits for the one before it: nothing of this pass writes them.  (Sending the
+// others to L2 there gains nothing for 24 rows of 500 keys, and costs 16 rows of 8000 17 us a layer.)  Warps
+// meet in shared memory, CTAs in that of the cluster, each completing its share of the output.
 // That step of 24 sequences, a layer, from q|k|v on: 32 us for RoPE, a scan of 32 keys per warp with a lane per key and a fold
 // through L2; 14 us here, of which 8 for the longest rows' five turns of a warp (about 450 instructions each), 3 for the sums.
 // (Chunks of 96 keys of all rows, and the CTA that finishes a row's last one adding them up: 18 us, six of them for that; CTAs of four
@@ -159,12 +160,6 @@ __global__ void __launch_bounds__(kThreads, 2) paged_decode_kernel(const __grid_
   int jb = j0 + warp * kKeys;
   if (jb < j1)
     request(jb);
-  constexpr int kLines = D * 4 / 128;   // of a row; those after the first rows go to L2, one per thread
-  for (int i = kWarps * kKeys * kLines + threadIdx.x; i < (j1 - j0) * kLines; i += kThreads) {
-    const int64_t at = (int64_t)s_row[i / kLines] * D + i % kLines * 32;
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(p.k_pool + at));
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(p.v_pool + at));
-  }
   kernel_wait();
 
   // ---- q heads; the CTA with the newest position: k and v (first warp) --------------------------------------------------------
@@ -378,10 +373,10 @@ int cluster_size(int M, int kv_heads, int longest) {
 // A CTA's range of keys is a chain of turns of 32 (0.5 to 1.2 us each, 2 at eight heads of 128, whose registers do not all fit), and no
 // more than 8 CTAs share a row: with few rows of long contexts the general kernels, which cut them in chunks of 256 keys over the whole
 // chip, are done sooner.  us a layer here / there, RoPE included, caches from memory; q heads on kv heads of 128:
-//   12 on 2   2 rows of 4000 22 / 26, of 8000 41 / 30; 4 of 8000 44 / 33; 8 of 4000 33 / 31, of 8000 61 / 58; 16 of 8000 73 / 110
-//   32 on 8   2 rows of 4000 26 / 28, of 8000 44 / 53      4 on 2   2 of 4000 17 / 21, of 8000 32 / 25; 8 of 8000 44 / 47
-//   8 on 1    2 rows of 2000 19 / 24, of 4000 34 / 24; 16 of 2000 29 / 29, of 3000 41 / 34; 24 of 3000 43 / 35, of 4000 55 / 60;
-//             37 of 1000 29 / 32, of 2000 53 / 33; 64 of 4000 109 / 116; 100 of 1000 55 / 61, of 2000 104 / 88
+//   12 on 2   2 rows of 4000 21 / 26, of 8000 38 / 30; 4 of 8000 41 / 33; 8 of 4000 31 / 31, of 8000 54 / 58; 16 of 8000 56 / 110
+//   32 on 8   2 rows of 4000 22 / 28, of 8000 38 / 53      4 on 2   2 of 4000 16 / 21, of 8000 29 / 25; 8 of 8000 34 / 47
+//   8 on 1    2 rows of 2000 19 / 24, of 4000 34 / 24; 16 of 2000 28 / 29, of 3000 39 / 34; 24 of 3000 40 / 35, of 4000 51 / 60;
+//             37 of 1000 28 / 32, of 2000 50 / 33; 64 of 4000 93 / 116; 100 of 1000 51 / 61, of 2000 93 / 88
 bool ranges_pay(int G, int D, int ctas, int range, int longest) {
   if (G == 8 && D == 128)
     return range <= 320 || longest <= 1024 || ctas >= 256;
