@@ -621,9 +621,20 @@ template <int KIND, int COLS, bool GROUPED, bool XF> static int launch_mma(MmaP 
 // 5.4 / 8.4 at 1, 6.0 / 8.7 at 6; K = 8960: 7.9 / 15.4 at 1; K = 14336: 13.0 / 21.5 at 1.  int4 K = 512: 7.3 / 5.0 at 1 MB, 6.9 / 7.0
 // at 2, 8.4 / 14 at 6; K = 1536: 7.5 / 6.9 at 1, 7.2 / 8.1 at 3; K = 2560: 6.6 / 8.7 at 0.5; K = 8960: 9.6 / 23 at 1.  (f32 rows of up to four whole blocks have a
 // quicker form there: K = 4096 5.3 / 6.1 at 0.5 MB from memory, 5.2 / 4.8 at 1.2 MB from L2.)
+// int4 rows of 2.5 to five blocks of 1024: there, per-channel scales cost nothing and whole blocks of f32 rows have a quicker form; here, a
+// part of a block is staged by itself, and the ten steps of five blocks go to five warps, too few to keep the row in registers.  From
+// memory, us here / there (in brackets from L2), 1024 rows, f32: per channel K = 2560 6.5 / 4.9 (5.7 / 3.8), 3584 7.3 / 5.8 (6.2 / 4.4), 5120 9.1 /
+// 6.8 (8.4 / 5.0), 6144 6.5 / 7.8 (6.0 / 5.5); groups of 128 2560 7.0 / 8.8 (6.2 / 7.7), 3584 7.8 / 11.3 (6.8 / 9.6), 5120 9.6 / 7.2 (9.0 /
+// 5.7), 6144 6.6 / 8.3 (6.2 / 6.4); bf16: per channel 3584 10.6 / 8.7 (9.7 / 7.3), 4096 7.8 / 9.3 (7.5 / 7.8), 5120 11.2 / 11.1 (10.6 / 9.3), groups
+// 2560 8.9 / 10.8, 5120 11.7 / 12.6.  (int8 rows of 2560 to 3071 that lie in L2 take 0.2 to 0.8 us more here, from memory 0.5 to 1.5 less.)
 static bool one_row_is_short(const b200_weight *w, const b200_gemv_args *a) {
-  const bool few_blocks = w->kind == B200_W_U4 && w->K <= 4096 && w->K % 1024 == 0 && a->x_dtype == B200_F32;
-  return (w->K < 2560 || few_blocks) && packed_row_bytes(w->kind, w->K) * w->N < (w->kind == B200_W_I8 ? 6 << 20 : 3 << 20);
+  const int64_t bytes = packed_row_bytes(w->kind, w->K) * w->N, mb = 1 << 20;
+  if (w->kind == B200_W_I8 || w->K < 2560)
+    return w->K < 2560 && bytes < (w->kind == B200_W_I8 ? 6 * mb : 3 * mb);
+  const bool whole = w->K % 1024 == 0, grouped = w->group > 0 && w->group < w->K;
+  if (w->K > 5120 || (grouped && !whole) || (a->x_dtype != B200_F32 && (grouped || w->K == 4096)))
+    return false;
+  return bytes < (w->K == 4096 ? 3 * mb : 6 * mb);
 }
 
 // Whether the integer-MMA kernel takes this call: per-channel int8 or int4 (any scale type), or int4 in groups of 128
