@@ -66,7 +66,7 @@ constexpr int kMaxStages = 8;
 constexpr int kSms = 148, kPairs = kSms / 2;
 constexpr int kMaxSplits = 4;                  // along k: clusters of up to eight CTAs
 constexpr int kHeadBytes = 256;                // workspace head: error word, scales of W8A8
-constexpr int kHeadWords = 16;                 // of it, cleared at the start of a call
+constexpr int kHeadWords = 1;                  // of it, cleared at the start of a call: the error word
 constexpr uint32_t kWBytes = BM * BK;
 
 struct Bars {
@@ -701,7 +701,7 @@ __device__ __forceinline__ float plane_scale(uint32_t absbits, float *inv) {
 // A[M,K] f32 -> planes [M][3][K] int8 in the k order of the packed weight rows, and the rows' scales (the sign says that a row is
 // wide); optional RMSNorm of every row (the factor 1/rms goes into the scale).  T threads per row, a thread takes 16-byte
 // units: it reads four groups of four k and writes whole 16-byte pieces of the planes.  The row is read once and stays in
-// registers up to 48 T elements.  Also clears the GEMM's counters and, outside a pass, its error word (head).
+// registers up to 48 T elements.  Outside a pass it also clears the call's error word (head).
 //
 // Wide rows.  Rounding to a unit leaves 0.29 units (rms) in every element, which must be no more than the 2^-19 of an element
 // that two bf16 terms leave: the row's bulk has to have an rms of at least 2^17 units.  Its bulk is what lies below a quarter of
@@ -896,8 +896,8 @@ planes_kernel(const float *A, int64_t lda, int M, int K, const float *norm_w, fl
 // (+ bias).  Every step is reproduced operation by operation, so the result is bit-identical to the reference arithmetic.
 constexpr int kMaxParts = 256;   // partial maxima, in the workspace head
 
-// max |x| of every CTA's share of the tensor (non-negative floats order like their bit patterns); clears the GEMM's counters
-// and its error word (null in a pass: the word collects what any of its GEMMs leaves).
+// max |x| of every CTA's share of the tensor (non-negative floats order like their bit patterns); clears the call's
+// error word (null in a pass: the word collects what any of its GEMMs leaves).
 __global__ void __launch_bounds__(256)
 absmax_kernel(const float *A, int64_t lda, int M, int K, int vec, uint32_t *part, uint32_t *head, int head_words,
               int in_pass) {
