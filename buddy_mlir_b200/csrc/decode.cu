@@ -26,6 +26,7 @@
 // Int4DequantMatMulVectorizationDecode.cpp:359-430, and the attention recurrence of
 // frontend/Python/ops/tosa.py:14245-14594.
 #include "decode.cuh"
+#include "quotient.cuh"
 #include "gemv_mma.cuh"
 
 #include <algorithm>
@@ -57,12 +58,12 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// a / b for b in the normal range, one Newton step on the hardware reciprocal: within an ulp, without a slow path
+// a / b for a normal b of up to 2^125: the hardware's approximate reciprocal, improved by a step of Newton's iteration, and a product.
+// Within an ulp and a half.
 __device__ __forceinline__ float div_normal(float a, float b) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
-  r = fmaf(r, fmaf(-b, r, 1.f), r);
-  return a * r;
+  return a * newton_reciprocal(b, r);
 }
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void ll_store(uint2 *p, float v, uint32_t tag) {

@@ -41,4 +41,10 @@ void pairs(const float *a, const float *b, float *out, float *want, long n) {
   }
 }
 
+// Quotients a * newton_reciprocal(b, r) with r = 1 / b rounded and moved by `ulps`: what an approximate reciprocal may give.
+void newton(const float *a, const float *b, float *out, long n, int ulps) {
+  for (long i = 0; i < n; ++i)
+    out[i] = a[i] * b200::newton_reciprocal(b[i], bits(of(1.0f / b[i]) + ulps));
+}
+
 }

@@ -50,3 +50,18 @@ def test_zero_infinities_and_nan(check):
     for d in (1.0, 1.5, 3.0, 2.0 ** 20):
         got, want = pairs(check, a, np.full_like(a, d))
         assert np.array_equal(got, want, equal_nan=True)
+
+
+@pytest.mark.parametrize("ulps", [-2, -1, 0, 1, 2])
+def test_newton_step_from_an_approximate_reciprocal(check, ulps):
+    """The decode step's division: from a reciprocal that is off by up to two units in the last place (the hardware's by one) the
+    quotient is within an ulp and a half, the rounding of r and that of the product."""
+    rng = np.random.default_rng(3)
+    n = 1 << 22
+    a, b = (np.ldexp(rng.uniform(1, 2, n), rng.integers(-30, 31, n)).astype(np.float32) for _ in range(2))
+    b[:2 ** 12] = np.float32(1) + np.arange(2 ** 12, dtype=np.float32) * np.float32(2.0 ** -23)     # the ends of a binade
+    b[2 ** 12:2 ** 13] = np.float32(2) - np.arange(1, 2 ** 12 + 1, dtype=np.float32) * np.float32(2.0 ** -23)
+    out = np.empty_like(a)
+    check.newton(*(v.ctypes.data_as(C.c_void_p) for v in (a, b, out)), C.c_long(n), ulps)
+    want = a.astype(np.float64) / b.astype(np.float64)
+    assert (np.abs(out - want) / np.spacing(np.abs(want).astype(np.float32))).max() <= 1.5
