@@ -35,9 +35,10 @@
 // The kernel stays on its SMs for all tiles: warp 0 loads (TMA, no multicast), warp 1 issues tcgen05.mma, sixteen warps are the
 // epilogue of one accumulator while the products of the next tile go to the other.  What an epilogue needs from memory it asks
 // for a tile ahead: with loads in its loop over the rows a tile took 16600 clocks, not 6100 (L2 answers late under these loads).
-// Bound by the tensor pipe and its clock: 1024 x 17920 x 1536 72 us with the digits' own pass, 108 us as CTAs of 128 x 256 for
-// a tile each; 65 % of the pipe's cycles at 1.7 GHz, 2.9 POP/s of the padded tiles.  1000 x 1536 x 8960: 41 us (49), 366 x 17920 x
-// 1536: 31 us (50), W8A8 2048 x 8960 x 8960: 143 us (213).
+// Bound by the operands' way out of L2: a launch of 1000 x 17920 x 1536 brings 674 MB to the SMs, 46 bytes a clock and SM (10 TB/s;
+// make_plan counts 45), while the tensor pipe is active in 71 % of the cycles and L2's slices in 41 %; and by the clock, which
+// falls to 1.7 GHz.  1024 x 17920 x 1536 69 us with the digits' own pass, 108 us as CTAs of 128 x 256 for a tile each; 2.9 POP/s of the
+// padded tiles.  1000 x 1536 x 8960: 40 us (49), 366 x 17920 x 1536: 31 us (50), W8A8 2048 x 8960 x 8960: 143 us (213).
 // Few tiles: the k range is cut over the pairs of a cluster, whose sums meet in shared memory: make_plan().  The weight loads
 // start before the activations are there (programmatic dependent launch behind the kernel that makes the digits; chain_start says
 // what keeps them behind the caller's earlier work).
@@ -183,6 +184,7 @@ struct RowScales {
 __device__ __forceinline__ float silu_of(float g, float u, float d) { return __fmul_rn(__fmul_rn(g, __frcp_rn(d)), u); }
 
 // ---- epilogue ----------------------------------------------------------------------------------------------------------------
+enum { kEither, kSilu, kPlain };   // STORE: SiLU pairs, which have no residual, or not; kEither: p.silu_pairs says
 // A warp reads the 32 lanes of tensor memory that match its rank within its warpgroup, a lane one channel; the warps that share a
 // lane quarter take CR rows of the tile in turn.
 constexpr int CR = 8;
@@ -198,7 +200,7 @@ struct Channel {
 };
 // Sums of N rows from row m of C on -> results.  rs: row scales, that of row i in lane `from` + i (W8A8: the one scale).  ALL: all
 // N rows are stored, otherwise those whose bit of `live` is set.
-template <bool PLANES, bool ALL, int N>
+template <bool PLANES, int STORE, bool ALL, int N>
 __device__ __forceinline__ void finish_rows(const GemmParams &p, const Channel &c, int m, float (&y)[N], float rs, int from, uint32_t live,
                                             const float (&res)[N]) {
 #pragma unroll
@@ -213,7 +215,7 @@ __device__ __forceinline__ void finish_rows(const GemmParams &p, const Channel &
     for (int i = 0; i < N; ++i)
       y[i] = __fadd_rn(y[i], c.bias);
   }
-  if (p.silu_pairs) {   // (gate, up) are neighbouring lanes: of two rows the even lane takes the first, the odd one the second
+  if (STORE == kSilu || (STORE == kEither && p.silu_pairs)) {   // (gate, up) are neighbouring lanes: of two rows the even lane takes the first, the odd one the second
     const bool odd = c.n & 1;
     float *dst = p.C + (int64_t)m * p.ldc + (c.n >> 1) + (odd ? p.ldc : 0);
     float d[N / 2];
@@ -241,12 +243,12 @@ __device__ __forceinline__ void finish_rows(const GemmParams &p, const Channel &
     }
   }
 }
-template <int N>
+template <int STORE, int N>
 __device__ __forceinline__ void load_residual(const GemmParams &p, const Channel &c, int m, int rows, float (&res)[N]) {
 #pragma unroll
   for (int i = 0; i < N; ++i)
     res[i] = 0.f;
-  if (p.residual != nullptr) {
+  if (STORE != kSilu && p.residual != nullptr) {
     const float *src = p.residual + (int64_t)m * p.ldr + c.n;
 #pragma unroll
     for (int i = 0; i < N; ++i)
@@ -287,7 +289,7 @@ __device__ __forceinline__ void give_row(const GemmParams &p, const Shares &sh, 
 // The pass over all rows of a tile.  Split k: the sums go to the CTAs that complete the rows.  wait: until the accumulator at tmem is
 // complete; what the first rows need from memory is requested before it.
 // WIDE: some of the rows are wide, and left to the passes with six digits.
-template <bool PLANES, bool SPLIT, bool WIDE, typename Wait>
+template <bool PLANES, int STORE, bool SPLIT, bool WIDE, typename Wait>
 __device__ __forceinline__ void store_tile(const GemmParams &p, const Tile &t, const Channel &c, const RowScales &scales, uint32_t tmem,
                                            uint32_t release, const Shares &sh, Wait wait) {
   constexpr int ND = PLANES ? kPlanes : 1;
@@ -295,7 +297,7 @@ __device__ __forceinline__ void store_tile(const GemmParams &p, const Tile &t, c
   int r0 = grp * CR;
   float res[CR];
   if (!SPLIT)
-    load_residual<CR>(p, c, t.m0 + r0, t.rows - r0, res);
+    load_residual<STORE, CR>(p, c, t.m0 + r0, t.rows - r0, res);
   const bool ok = wait();
   if (r0 >= t.rows || !ok) {
     release_accumulator(release);
@@ -315,7 +317,7 @@ __device__ __forceinline__ void store_tile(const GemmParams &p, const Tile &t, c
       live &= ~(__ballot_sync(0xffffffffu, signbit(rs)) >> (r0 & 31));
     float next[CR], y[CR];
     if (!SPLIT)
-      load_residual<CR>(p, c, t.m0 + r0 + kGroups * CR, left - kGroups * CR, next);
+      load_residual<STORE, CR>(p, c, t.m0 + r0 + kGroups * CR, left - kGroups * CR, next);
     tmem_wait_load();
     if (left <= kGroups * CR)
       release_accumulator(release);
@@ -327,9 +329,9 @@ __device__ __forceinline__ void store_tile(const GemmParams &p, const Tile &t, c
           give_row(p, sh, r0 + i, y[i]);
     } else {
       if (live == (1u << CR) - 1)
-        finish_rows<PLANES, true, CR>(p, c, t.m0 + r0, y, rs, r0 & 31, live, res);
+        finish_rows<PLANES, STORE, true, CR>(p, c, t.m0 + r0, y, rs, r0 & 31, live, res);
       else
-        finish_rows<PLANES, false, CR>(p, c, t.m0 + r0, y, rs, r0 & 31, live, res);
+        finish_rows<PLANES, STORE, false, CR>(p, c, t.m0 + r0, y, rs, r0 & 31, live, res);
 #pragma unroll
       for (int i = 0; i < CR; ++i)
         res[i] = next[i];
@@ -337,7 +339,7 @@ __device__ __forceinline__ void store_tile(const GemmParams &p, const Tile &t, c
   }
 }
 // The pass with six digits over `rows` rows of a tile, `first` the first: its wide rows.
-template <bool SPLIT, typename Wait>
+template <int STORE, bool SPLIT, typename Wait>
 __device__ __forceinline__ void store_wide_pass(const GemmParams &p, int m0, const Channel &c, uint32_t tmem, int first, int rows,
                                                 uint32_t release, const Shares &sh, Wait wait) {
   constexpr int N = CR / 2;
@@ -346,7 +348,7 @@ __device__ __forceinline__ void store_wide_pass(const GemmParams &p, int m0, con
   auto request = [&](int r0, float &s, float (&r)[N]) {
     s = lane < N && r0 + lane < rows ? __ldcg(p.row_scale + m0 + first + r0 + lane) : 0.f;
     if (!SPLIT)
-      load_residual<N>(p, c, m0 + first + r0, rows - r0, r);
+      load_residual<STORE, N>(p, c, m0 + first + r0, rows - r0, r);
   };
   request(grp * N, rs, res);
   const bool ok = wait();
@@ -374,7 +376,7 @@ __device__ __forceinline__ void store_wide_pass(const GemmParams &p, int m0, con
         if (live >> i & 1)
           give_row(p, sh, first + r0 + i, y[i]);
     } else {
-      finish_rows<true, false, N>(p, c, m0 + first + r0, y, rs, 0, live, res);
+      finish_rows<true, STORE, false, N>(p, c, m0 + first + r0, y, rs, 0, live, res);
 #pragma unroll
       for (int i = 0; i < N; ++i)
         res[i] = next[i];
@@ -383,7 +385,7 @@ __device__ __forceinline__ void store_wide_pass(const GemmParams &p, int m0, con
   }
 }
 // The rows that this CTA completes, shares added in order.  sums: this lane's channel of the first share.
-template <bool PLANES>
+template <bool PLANES, int STORE>
 __device__ __forceinline__ void add_shares(const GemmParams &p, int m0, int rows, const Channel &c, const float *sums) {
   const int lane = threadIdx.x & 31;
 #pragma unroll 1
@@ -394,7 +396,7 @@ __device__ __forceinline__ void add_shares(const GemmParams &p, int m0, int rows
       rs = p.row_scale[0];
     else if (lane < live)
       rs = __ldcg(p.row_scale + m + lane);
-    load_residual<CR>(p, c, m, live, res);
+    load_residual<STORE, CR>(p, c, m, live, res);
 #pragma unroll
     for (int i = 0; i < CR; ++i)
       y[i] = 0.f;
@@ -406,7 +408,7 @@ __device__ __forceinline__ void add_shares(const GemmParams &p, int m0, int rows
           const float b = sums[(z * p.share_rows + r0 + i) * BM];
           y[i] = PLANES ? y[i] + b : __int_as_float(__float_as_int(y[i]) + __float_as_int(b));
         }
-    finish_rows<PLANES, false, CR>(p, c, m, y, rs, 0, (1u << live) - 1, res);
+    finish_rows<PLANES, STORE, false, CR>(p, c, m, y, rs, 0, (1u << live) - 1, res);
   }
 }
 // mbar_wait, and what the cluster's other CTAs stored before they arrived is visible.
@@ -418,7 +420,7 @@ __device__ __forceinline__ bool wait_shares(uint64_t *bar, volatile int *ab, int
 }
 
 // An epilogue warp's way through the tiles from w on; n: accumulators so far.  WIDE = false: up to a tile with wide rows.
-template <bool PLANES, bool SPLIT, bool WIDE>
+template <bool PLANES, int STORE, bool SPLIT, bool WIDE>
 __device__ __forceinline__ int epilogue(const GemmParams &p, Bars &bars, float *sums, uint32_t tmem, int w, int step, int &n) {
   const int lane = threadIdx.x & 31, quad = threadIdx.x >> 5 & 3, crank = (int)cluster_rank(), rank = crank & 1;
   const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16);
@@ -450,14 +452,14 @@ __device__ __forceinline__ int epilogue(const GemmParams &p, Bars &bars, float *
       return ok;
     };
     auto release = [&] { return in_cta(smem_u32(&bars.acc_empty[n & 1]), crank & ~1); };
-    store_tile<PLANES, SPLIT, WIDE>(p, t, c, scales, lanes + (n & 1) * (p.cols >> 1), release(), sh, wait);
+    store_tile<PLANES, STORE, SPLIT, WIDE>(p, t, c, scales, lanes + (n & 1) * (p.cols >> 1), release(), sh, wait);
     ++n;
     if constexpr (WIDE) {
       const int half = (p.rows + 1) >> 1;
 #pragma unroll 1
       for (int h = 0; h < 2; ++h)
         if (wide >> h & 1) {
-          store_wide_pass<SPLIT>(p, t.m0, c, lanes + (n & 1) * (p.cols >> 1), h * half, min(half, t.rows - h * half), release(), sh, wait);
+          store_wide_pass<STORE, SPLIT>(p, t.m0, c, lanes + (n & 1) * (p.cols >> 1), h * half, min(half, t.rows - h * half), release(), sh, wait);
           ++n;
         }
     }
@@ -468,7 +470,7 @@ __device__ __forceinline__ int epilogue(const GemmParams &p, Bars &bars, float *
       ok = __all_sync(0xffffffffu, wait_shares(&bars.sums, ab, p.error, 705)) && ok;
       const int row = z * p.share_rows;
       if (ok)
-        add_shares<PLANES>(p, t.m0 + row, min(p.share_rows, t.rows - row), c, sums + channel);
+        add_shares<PLANES, STORE>(p, t.m0 + row, min(p.share_rows, t.rows - row), c, sums + channel);
     }
     w += step;
     if (w >= p.tiles)
@@ -478,17 +480,17 @@ __device__ __forceinline__ int epilogue(const GemmParams &p, Bars &bars, float *
     request(t);
   }
 }
-// The tiles from a wide one on.  Where a pair has several tiles (TURNS) this is part of the kernel: as a function, whose parameters lie
-// behind a generic pointer and are loaded again after every store, it made every later tile take twice as long (1024 x 20000 x 512 with
-// one wide row 112 us, 79 inline; without one 51 and 52).  Where it has one, it is a function all the same, with a copy of the parameters:
-// a small call is 0.35 us longer with all of it inline (24 x 1536 x 1536 8.9 / 9.3 us).
-template <bool SPLIT>
+// The tiles from a wide one on, as a function with a copy of the parameters (behind a generic pointer they are loaded again after every
+// store: 1024 x 17920 x 1536 with one wide row 112 us, 94 with the copy).  Where a pair has many products to make (TURNS) this is part of
+// the kernel, so that tiles after a wide one are as quick as those before: 84 us.  Inline everywhere it would lengthen every launch without
+// a wide row: a pass of 100 rows of the 1.5B model 2.36 / 2.40 ms.
+template <int STORE, bool SPLIT>
 __device__ __noinline__ void epilogue_last(const GemmParams &p_in, Bars &bars, float *sums, uint32_t tmem, int w, int step, int n) {
   const GemmParams p = p_in;
-  epilogue<true, SPLIT, true>(p, bars, sums, tmem, w, step, n);
+  epilogue<true, STORE, SPLIT, true>(p, bars, sums, tmem, w, step, n);
 }
 
-template <bool PLANES, bool SPLIT, bool TURNS>
+template <bool PLANES, int STORE, bool SPLIT, bool TURNS>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                const __grid_constant__ GemmParams p, const __grid_constant__ CUtensorMap map_x) {
@@ -644,12 +646,12 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // ---- epilogue ----------------------------------------------------------------------------------------------------
     kernel_wait();   // row scales
     int n = 0, w = first;
-    w = epilogue<PLANES, SPLIT, false>(p, bars, sums, tmem, w, step, n);
+    w = epilogue<PLANES, STORE, SPLIT, false>(p, bars, sums, tmem, w, step, n);
     if (PLANES && w < p.tiles) {
       if constexpr (TURNS)
-        epilogue<true, SPLIT, true>(p, bars, sums, tmem, w, step, n);
+        epilogue<true, STORE, SPLIT, true>(p, bars, sums, tmem, w, step, n);
       else
-        epilogue_last<SPLIT>(p, bars, sums, tmem, w, step, n);
+        p.silu_pairs ? epilogue_last<kSilu, SPLIT>(p, bars, sums, tmem, w, step, n) : epilogue_last<kPlain, SPLIT>(p, bars, sums, tmem, w, step, n);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1058,7 +1060,7 @@ Plan make_plan(int M, int N, int K, int nd, const int (&held)[kMaxSplits + 1]) {
   return best;
 }
 
-template <bool PLANES, bool SPLIT, bool TURNS>
+template <bool PLANES, int STORE, bool SPLIT, bool TURNS>
 int launch_gemm(const Plan &pl, const void *a, const void *x, const void *w, GemmParams &p, cudaStream_t st) {
   CUtensorMap map_a, map_w, map_x;
   const int box = pl.nc / 2;
@@ -1082,9 +1084,9 @@ int launch_gemm(const Plan &pl, const void *a, const void *x, const void *w, Gem
   p.stages = pl.stages;
   p.cols = pl.cols;
   static RaisedOn raised;
-  if (int rc = raise_shared_limit(raised, (const void *)gemm_i8_kernel<PLANES, SPLIT, TURNS>, kMostShared))
+  if (int rc = raise_shared_limit(raised, (const void *)gemm_i8_kernel<PLANES, STORE, SPLIT, TURNS>, kMostShared))
     return rc;
-  return launch_after_clusters(2 * pl.splits, gemm_i8_kernel<PLANES, SPLIT, TURNS>, dim3(pl.grid), kThreads, pl.smem, st, map_a, map_w, p, map_x);
+  return launch_after_clusters(2 * pl.splits, gemm_i8_kernel<PLANES, STORE, SPLIT, TURNS>, dim3(pl.grid), kThreads, pl.smem, st, map_a, map_w, p, map_x);
 }
 // How many clusters of 2 x splits CTAs the current device holds at once.
 int clusters_held(int splits) {
@@ -1095,7 +1097,7 @@ int clusters_held(int splits) {
   if (seen != nullptr && (n = seen->load(std::memory_order_relaxed)) > 0)
     return n;
   static RaisedOn raised;
-  auto kern = gemm_i8_kernel<true, true, false>;
+  auto kern = gemm_i8_kernel<true, kEither, true, false>;
   if (int rc = raise_shared_limit(raised, (const void *)kern, kMostShared))
     return rc;
   cudaLaunchConfig_t cfg{};
@@ -1121,12 +1123,14 @@ template <bool PLANES> int launch_plan(const void *a, const void *x, const void 
       return held[s];   // an error code
   const Plan pl = make_plan(p.M, p.N, p.K, PLANES ? kPlanes : 1, held);
   if (pl.splits > 1)
-    return launch_gemm<PLANES, true, false>(pl, a, x, w, p, st);
-  // several tiles per pair; with one row tile, where all are wide or none is, more than two of them: 24 x 20000 x 512 takes 9.4 us with
-  // the function and 9.8 inline, 18.3 and 16.1 when wide
-  if (PLANES && pl.tiles > (pl.m_tiles > 1 ? 1 : 2) * pl.grid / 2)
-    return launch_gemm<PLANES, false, PLANES>(pl, a, x, w, p, st);
-  return launch_gemm<PLANES, false, false>(pl, a, x, w, p, st);
+    return launch_gemm<PLANES, kEither, true, false>(pl, a, x, w, p, st);
+  // Many products: turns of the pairs times blocks of k.  us without / with one wide row, inline / as a function: 1024 x 17920 x 1536 (13 x 12)
+  // 69.1 / 84 and 71.0 / 94, 1024 x 1536 x 8960 (2 x 70) 48.3 / 66 and 51.5 / 72, 366 x 17920 x 1536 (5 x 12) 30.2 / 41 and 30.8 / 43, 100 x
+  // 17920 x 1536 (2 x 12) 16.7 / 24 and 16.5 / 26, 1024 x 1536 x 1536 (2 x 12) 16.4 / 22 and 16.1 / 23
+  const int pairs = pl.grid / 2;
+  if (PLANES && pl.tiles > pairs && (pl.tiles + pairs - 1) / pairs * ((p.K + BK - 1) / BK) >= 56)
+    return p.silu_pairs ? launch_gemm<PLANES, kSilu, false, PLANES>(pl, a, x, w, p, st) : launch_gemm<PLANES, kPlain, false, PLANES>(pl, a, x, w, p, st);
+  return launch_gemm<PLANES, kEither, false, false>(pl, a, x, w, p, st);
 }
 
 } // namespace
