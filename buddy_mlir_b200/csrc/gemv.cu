@@ -534,8 +534,8 @@ static int launch(const GemvP &p, int warps, cudaStream_t st) {
   // one resident wave: as many CTAs as fit on the device at once, each looping
   // over its row groups.  The occupancy is asked for only where it can matter, and once per block
   // shape in a row (the last answer in one word: device, shared memory, warps, CTAs): three
-  // queries are host time of every call otherwise (1 x 1536 x 1536 int8, one call after another:
-  // 8.44 us with them, 8.30 without; 8.38 and 8.10 on another host)
+  // queries are host time of every call otherwise (issuing 1 x 1536 x 1536 int8 through ctypes 4.4
+  // to 7.8 us with them, 3.9 to 4.1 without; a call by itself, awaited, hardly shows it)
   const int sms = device_sms();
   if (grid > sms) {
     static std::atomic<uint64_t> known{0};

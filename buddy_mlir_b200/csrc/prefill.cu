@@ -358,12 +358,11 @@ int launch_paged_attn(const float *qkv, int64_t ld, const float *kp, const float
   return B200_OK;
 }
 
-// The same scan for few rows with long histories (batched decode): the keys of a row
-// are cut into chunks of `chunk` positions (paged_chunk(): an eighth of the longest
+// The same scan with the keys of a row cut into chunks of `chunk` positions (paged_chunk(): an eighth of the longest
 // context, 32..256), one CTA per (row, kv head, chunk), a warp per 32 keys with 8 rows of V (and 8
-// 16-byte pieces of each lane's K row) in flight: the scan is a chain of memory latencies.  24 sequences of 32..700 positions,
-// 12 heads on 2, D = 128, caches from HBM: 50 us a layer with one row in
-// flight, 8 warps for 96 keys and a fold that loads chunk by chunk; with the fold's loads 8 at a time the step gains 0.3 ms.
+// 16-byte pieces of each lane's K row) in flight: the scan is a chain of memory latencies.  Serves decode steps whose
+// ranges of keys would be long for a cluster per row (ranges_pay() in paged_decode.cu has the times of both: 2 rows of 8000
+// keys, 12 heads on 2, 30 us a layer behind RoPE), and chunks of a prompt that the tensor-core attention does not take.
 // Partials (m, l, acc[D]) per query head go to `part`; the CTA that finishes a row's last
 // chunk folds them in chunk order.
 __host__ __device__ inline int paged_chunk(int max_context) {

@@ -3,8 +3,9 @@
 // Tensor memory and early starts.  tcgen05.alloc waits, without a limit, until the columns are free.  It ends because whoever
 // holds them ends: a kernel calls kernel_go() only after its own allocation, so the kernels behind it get an SM when every CTA
 // before them has its columns, and a CTA that holds columns waits (kernel_wait) only for kernels that need no more of them.
-// With kernel_go() first, a CTA of the next kernel could take the columns an earlier CTA still needs and then wait for it: at
-// head dim 64 an attention CTA (109 KB of shared memory, all 512 columns) and a GEMM CTA (98 KB) fit on one SM.
+// With kernel_go() first, a CTA of the next kernel could take the columns an earlier CTA still needs and then wait for it, wherever
+// two such CTAs fit on one SM: at head dim 64 an attention CTA has 109 KB of shared memory and all 512 columns, and a
+// GEMM CTA (18 warps of up to 96 registers, up to 198 KB, 32 to 512 columns) with few columns of digits a ring that fits beside it.
 #pragma once
 #include "common.cuh"
 
