@@ -1088,14 +1088,14 @@ int launch_gemm(const Plan &pl, const void *a, const void *x, const void *w, Gem
     return rc;
   return launch_after_clusters(2 * pl.splits, gemm_i8_kernel<PLANES, STORE, SPLIT, TURNS>, dim3(pl.grid), kThreads, pl.smem, st, map_a, map_w, p, map_x);
 }
-// How many clusters of 2 x splits CTAs the current device holds at once.
+// How many clusters of 2 x splits CTAs the current device holds at once; negative: an error code.
 int clusters_held(int splits) {
-  static std::atomic<int> known[64][kMaxSplits + 1];   // per device, once it has been asked
+  static std::atomic<int> known[64][kMaxSplits + 1];   // per device, once it has been asked: one more than the number
   int dev = 0, n = 0;
   B200_CUDA(cudaGetDevice(&dev));
   std::atomic<int> *seen = dev >= 0 && dev < 64 ? &known[dev][splits] : nullptr;
   if (seen != nullptr && (n = seen->load(std::memory_order_relaxed)) > 0)
-    return n;
+    return n - 1;
   static RaisedOn raised;
   auto kern = gemm_i8_kernel<true, kEither, true, false>;
   if (int rc = raise_shared_limit(raised, (const void *)kern, kMostShared))
@@ -1111,16 +1111,15 @@ int clusters_held(int splits) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   B200_CUDA(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));
-  n = std::max(n, 1);
   if (seen != nullptr)
-    seen->store(n, std::memory_order_relaxed);
+    seen->store(n + 1, std::memory_order_relaxed);
   return n;
 }
 template <bool PLANES> int launch_plan(const void *a, const void *x, const void *w, GemmParams &p, cudaStream_t st) {
   int held[kMaxSplits + 1] = {};
   for (int s = 2; s <= kMaxSplits; ++s)
     if ((held[s] = clusters_held(s)) < 0)
-      return held[s];   // an error code
+      return held[s];
   const Plan pl = make_plan(p.M, p.N, p.K, PLANES ? kPlanes : 1, held);
   if (pl.splits > 1)
     return launch_gemm<PLANES, kEither, true, false>(pl, a, x, w, p, st);

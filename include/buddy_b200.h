@@ -151,7 +151,8 @@ int b200_gemv(const b200_weight *w, const b200_gemv_args *a, void *stream);
 
 /* Dense weight-only GEMM for prefill and batched decode, on the tcgen05 tensor
  * cores: C[M,N] = A[M,K] * dequant(W)^T (+ bias) (+ residual), or, with
- * silu_pairs, C[M,N/2] = silu(gate) * up over interleaved (gate, up) rows.
+ * silu_pairs, C[M,N/2] = silu(gate) * up over interleaved (gate, up) rows (a
+ * residual that is given with them counts for nothing).
  * Replaces the prefill matmul of
  * midend/lib/Conversion/MatMulOptimization/MatMulBlisVectorization.cpp:367-530
  * (dequantisation fused into the B packing; known answer

@@ -1,7 +1,7 @@
 """A decode step of many sequences over the page pool (attention with head norm, RoPE and the cache write in one kernel), at the
 edges of its ranges: one key, ranges that some warps or CTAs have no key of, pages of one and of odd sizes, every number of q
-heads per kv head, both head dims, one and eight CTAs per row, and contexts that only the general kernels take.  A step at
-position n has to give what a prompt of n + 1 tokens gives, which other kernels compute."""
+heads per kv head, both head dims, two to eight CTAs per row (one: test_gpu_paged_kernel.py), and contexts that the general kernels take.
+A step at position n has to give what a prompt of n + 1 tokens gives, which other kernels compute."""
 import numpy as np
 import pytest
 
