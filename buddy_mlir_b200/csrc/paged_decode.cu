@@ -15,7 +15,7 @@
 // Scores are scaled in q, in powers of two, and all exponentials are ex2.approx (2 ulp), those of the sums' factors too.  Relative error
 // against f64 (2-norm, Gaussian inputs; in brackets q six times as large) here / in the kernels that it stands in for: 24 rows of 1..700 keys,
 // 12 heads on 2, 1.5e-7 / 3.3e-7 (3.2e-7 / 1.2e-6); 300 rows, where each had one CTA and expf, 1.5e-7 / 1.6e-7 (3.3e-7 / 4.1e-7);
-// contexts of up to 30 keys 9.5e-8 / 9.2e-8.  (With expf of scores scaled after the sum 1.4e-7, 1.4e-7, 9.3e-8, but 3.7e-7 for the large
+// contexts of up to 30 keys 9.5e-8 / 9.2e-8; 300 rows of up to 97, 8 heads of 64, 1.02e-7 / 1.01e-7 (2.43e-7 / 2.31e-7).  (With expf of scores scaled after the sum 1.4e-7, 1.4e-7, 9.3e-8, but 3.7e-7 for the large
 // ones, and 3 % longer, up to 17; exp2f gives the bits of ex2.)
 #include "common.cuh"
 

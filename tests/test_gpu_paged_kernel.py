@@ -20,7 +20,7 @@ class Step:
         self.lens, self.q, self.kv, self.D, self.page, self.M = lens, q_heads, kv_heads, D, page, len(lens)
         self.stride = (max(max(lens), limit) + page - 1) // page
         pages = [(n + page - 1) // page for n in lens]
-        order = torch.randperm(sum(pages)).to(torch.int32)
+        order = torch.randperm(sum(pages), generator=torch.Generator().manual_seed(seed)).to(torch.int32)
         self.table, at = torch.zeros(self.M, self.stride, dtype=torch.int32), 0
         for m, n in enumerate(pages):
             self.table[m, :n] = order[at:at + n]
